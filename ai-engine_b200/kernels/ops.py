@@ -951,6 +951,40 @@ SSD_MIN_TOKENS = 32      # portions from this length on take the chunked state-s
 SSD_CHUNK = 64           # its chunk
 
 
+LC_CHUNK = 64            # chunk of the chunk-parallel kernels of the linear recurrence
+# Their three launches cost about 42 us whatever they do; the token-by-token kernel costs 0.42 us a token of its longest
+# portion or 0.027 us a token and head of all of them, whichever is more: at (heads, portions of n tokens each) 27 against
+# 42 us (8, 1 x 64), 51 against 43 (8, 1 x 128), 63 against 44 (16, 4 x 32), 37 against 43 (16, 4 x 16), 66 against 48
+# (8, 16 x 16), 864 against 132 (16, 1 x 2048).  In a step that takes them, portions below eight tokens (single ones above all) stay with the other kernel.
+LC_MIN_WORK = 1700       # heads x tokens, or 16 x tokens of the longest portion
+LC_MIN_TOKENS = 8
+
+
+def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, state, out, ctx, H, d, dv, lower, bias) -> bool:
+    """The portions of LC_MIN_TOKENS tokens or more by the chunk-parallel kernels; False (nothing is done) when the step is
+    small or the sizes, strides or addresses are not theirs: heads of up to 128 in steps of 4, rows that start on 16 bytes."""
+    if (ctx.max_q_len < LC_MIN_TOKENS or d > 128 or dv > 128 or d % 4 or dv % 4 or ld % 4 or ctx.R * H > 65535
+            or (decay_tok is not None and decay_tok.stride(0) % 4)
+            or any(t is not None and t.data_ptr() % 16 for t in (q, k, v, decay_tok, state, lower, bias))):
+        return False
+    lens = ctx.h_q_len[ctx.h_q_len >= LC_MIN_TOKENS]
+    if max(H * int(lens.sum()), 16 * ctx.max_q_len) < LC_MIN_WORK:
+        return False
+    chunks = int(((lens + LC_CHUNK - 1) // LC_CHUNK).sum())
+    L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
+    G = torch.empty((chunks, H, d), dtype=torch.float32, device=q.device)
+    lib = library("linear_recurrence_chunked.cu")
+    T = q.shape[0]
+    with region("linear_recurrence_chunked", _nb(out) + T * H * (2 * d + dv) * 4 + 2 * ctx.R * H * d * dv * 4, 4.0 * T * H * d * dv):
+        check(lib.aie_linear_recurrence_chunked(_p(q), _p(k), _p(v), c_int(ld), _p(decay_tok),
+                                                c_int(decay_tok.stride(0) if decay_tok is not None else 0), _p(decay_head),
+                                                c_float(q_scale), c_float(k_scale), _p(state), _p(out), _p(L), _p(G),
+                                                _p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d),
+                                                c_int(dv), c_int(state.shape[0]), c_int(LC_MIN_TOKENS), c_int(chunks), _p(lower),
+                                                _p(bias), _p(ctx.err), _stream()), "linear_recurrence_chunked")
+    return True
+
+
 def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_tok: Optional[torch.Tensor],
                       decay_head: Optional[torch.Tensor], q_scale: float, k_scale: float, state: torch.Tensor,
                       ctx, H: int, d: int, dv: int, heads_per_group: int = 1, dt_raw: Optional[torch.Tensor] = None,
@@ -998,6 +1032,12 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
         if int(ctx.h_q_len.min()) >= SSD_MIN_TOKENS:
             return out
         max_len = SSD_MIN_TOKENS - 1                # the shorter portions and single tokens of the same step
+    elif (dt_raw is None and heads_per_group == 1 and skip is None
+          and _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, state, out, ctx, H, d, dv,
+                                    forget_lower, forget_bias)):
+        if int(ctx.h_q_len.min()) >= LC_MIN_TOKENS:
+            return out
+        max_len = LC_MIN_TOKENS - 1
     lib = library("linear_recurrence.cu")
     with region("linear_recurrence", _nb(out) + T * H * (2 * d + dv) * 4 + 2 * ctx.R * H * d * dv * 4, 4.0 * T * H * d * dv):
         check(lib.aie_linear_recurrence(_p(q), _p(k), _p(v), c_int(ld), _p(decay_tok),
