@@ -110,3 +110,217 @@ extern "C" int aie_paged_attention_plain(const void* q, const void* k_pages, con
         return AIE_BAD_ARG;
     AIE_LAUNCH_CHECK();
 }
+
+// ---------------------------------------------------------------------------
+// The same for portions of prompts in float32, 64 query tokens of one request and one head a block: keys and values of a
+// chunk are read once for all of them, scores and outputs are tiles of FMAs.  A block's additions are those of the kernel
+// above, in its order (the dot product over e, the butterfly sum of a chunk's 128 weights, the values over j), so a
+// token's bits do not depend on which of the two computes it.  Bound by the FMA units and, for few heads and tokens, by
+// the longest block's chain of chunks.
+// A warp owns 16 query rows; lanes lie 4 x 8: rows lm + 4 i, keys ln + 8 j, output columns 4 (ln + 8 x) .. + 3.
+#define PT_Q 64
+#define PT_THREADS 128
+
+template <int ND>      // pieces of 32 output columns: d <= 32 ND
+__global__ void __launch_bounds__(PT_THREADS)
+paged_attention_f32_tiles_kernel(const float* __restrict__ q, const float* __restrict__ k_pages, const float* __restrict__ v_pages,
+                                 float* __restrict__ out, const int* __restrict__ tiles, int per_tile, const int* __restrict__ q_start,
+                                 const int* __restrict__ q_len, const int* __restrict__ ctx_len, const int* __restrict__ block_table,
+                                 int bt_width, int num_pages, int P, int H, int K, int d, int window, float scale, unsigned* err) {
+    extern __shared__ __align__(16) float pt_sm[];
+    const int ld = d + 4, ldp = PLAIN_CHUNK + 4;                 // padded rows: lanes' rows fall on different banks
+    float* q_s = pt_sm;                                          // [64][ld]
+    float* v_s = q_s + PT_Q * ld;                                // [128][d]
+    float* k_s = v_s + PLAIN_CHUNK * d;                          // [128][ld], then the weights [64][ldp]
+    float* p_s = k_s;
+    int* ok_s = reinterpret_cast<int*>(k_s + max(PLAIN_CHUNK * ld, PT_Q * ldp));      // [128]
+
+    const int row = tiles[2 * (blockIdx.x / per_tile)], off = tiles[2 * (blockIdx.x / per_tile) + 1] + PT_Q * (blockIdx.x % per_tile);
+    const int n = min(PT_Q, q_len[row] - off), h = blockIdx.y, kvh = h / (H / K);
+    if (n <= 0) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lm = lane >> 3, ln = lane & 7;
+    const int pos0 = ctx_len[row] + off, last = pos0 + n - 1, t0 = q_start[row] + off, d4 = d / 4;
+    const int lo0 = (window > 0 && pos0 - window + 1 > 0) ? pos0 - window + 1 : 0;
+    auto copy = [](float* dst, const float* src, bool ok) {
+        const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(src), "r"(ok ? 16 : 0) : "memory");
+    };
+    for (int i = tid; i < PT_Q * d4; i += PT_THREADS) {
+        const int r = i / d4, c = (i % d4) * 4;
+        copy(q_s + r * ld + c, r < n ? q + ((size_t)(t0 + r) * H + h) * d + c : q, r < n);
+    }
+    const bool works = warp * 16 < n;
+    float m[4], l[4];
+    float4 acc[4][ND];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int x = 0; x < ND; ++x) acc[i][x] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int c0 = (lo0 / PLAIN_CHUNK) * PLAIN_CHUNK; c0 <= last; c0 += PLAIN_CHUNK) {
+        __syncthreads();                                         // the previous chunk is done with
+        const int kp = c0 + tid;
+        int page = -1;
+        if (kp >= lo0 && kp <= last) {
+            const int pidx = kp / P;
+            page = pidx < bt_width ? block_table[(size_t)row * bt_width + pidx] : -1;
+            if (page < 0 || page >= num_pages) {
+                atomicOr(err, AIE_DEV_PAGE_OOB);
+                page = -1;
+            }
+        }
+        ok_s[tid] = page < 0 ? -1 : page * P + kp % P;           // page and place of the key
+        __syncthreads();
+        for (int i = tid; i < PLAIN_CHUNK * d4; i += PT_THREADS) {
+            const int j = i / d4, c = (i % d4) * 4, at = ok_s[j], pg = at / P;
+            copy(k_s + j * ld + c, at >= 0 ? k_pages + (((size_t)pg * K + kvh) * P + (at - pg * P)) * d + c : k_pages, at >= 0);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        for (int i = tid; i < PLAIN_CHUNK * d4; i += PT_THREADS) {
+            const int j = i / d4, c = (i % d4) * 4, at = ok_s[j], pg = at / P;
+            copy(v_s + j * d + c, at >= 0 ? v_pages + (((size_t)pg * K + kvh) * P + (at - pg * P)) * d + c : v_pages, at >= 0);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();
+        float s[4][16];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) s[i][j] = 0.f;
+        if (works) {
+            const float* qr = q_s + (warp * 16 + lm) * ld;
+            const float* kr = k_s + ln * ld;
+#pragma unroll 1
+            for (int e = 0; e < d; e += 2) {
+                float2 a[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float2*>(qr + 4 * i * ld + e);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const float2 b = *reinterpret_cast<const float2*>(kr + 8 * j * ld + e);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) s[i][j] = fmaf(a[i].y, b.y, fmaf(a[i].x, b.x, s[i][j]));
+                }
+            }
+            unsigned seen = 0;                                   // bit j: the page of key ln + 8 j is there
+#pragma unroll
+            for (int j = 0; j < 16; ++j) seen |= (ok_s[ln + 8 * j] >= 0 ? 1u : 0u) << j;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int pos = pos0 + warp * 16 + lm + 4 * i;
+                const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+                float mx = -INFINITY;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    const int key = c0 + ln + 8 * j;
+                    s[i][j] = ((seen >> j) & 1) && key >= lo && key <= pos ? s[i][j] * scale : -INFINITY;
+                    mx = fmaxf(mx, s[i][j]);
+                }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                const float m_new = fmaxf(m[i], mx);
+                float w[4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {                    // 32 keys: the butterfly 16, 8, then 4, 2, 1 over the lanes
+#pragma unroll
+                    for (int x = 0; x < 4; ++x)
+                        s[i][4 * g + x] = s[i][4 * g + x] == -INFINITY ? 0.f : expf(s[i][4 * g + x] - m_new);
+                    w[g] = (s[i][4 * g] + s[i][4 * g + 2]) + (s[i][4 * g + 1] + s[i][4 * g + 3]);
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) w[g] += __shfl_xor_sync(0xffffffffu, w[g], o);
+                }
+                const float corr = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_new);
+                l[i] = l[i] * corr + ((w[0] + w[2]) + (w[1] + w[3]));
+                m[i] = m_new;
+#pragma unroll
+                for (int x = 0; x < ND; ++x) {
+                    acc[i][x].x *= corr;
+                    acc[i][x].y *= corr;
+                    acc[i][x].z *= corr;
+                    acc[i][x].w *= corr;
+                }
+            }
+        }
+        __syncthreads();                                         // all warps have read the keys: the weights take their place
+        if (works) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 16; ++j) p_s[(warp * 16 + lm + 4 * i) * ldp + ln + 8 * j] = s[i][j];
+        }
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        if (works) {
+            const float* pr = p_s + (warp * 16 + lm) * ldp;
+            const int nk = min(PLAIN_CHUNK, last - c0 + 1);
+#pragma unroll 1
+            for (int j = 0; j < nk; j += 2) {                    // a key behind the last has weight and value 0
+                float2 a[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float2*>(pr + 4 * i * ldp + j);
+#pragma unroll
+                for (int x = 0; x < ND; ++x) {
+                    const int c = 4 * (ln + 8 * x);
+                    if (c >= d) continue;
+                    const float4 b0 = *reinterpret_cast<const float4*>(v_s + j * d + c);
+                    const float4 b1 = *reinterpret_cast<const float4*>(v_s + (j + 1) * d + c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        acc[i][x].x = fmaf(a[i].y, b1.x, fmaf(a[i].x, b0.x, acc[i][x].x));
+                        acc[i][x].y = fmaf(a[i].y, b1.y, fmaf(a[i].x, b0.y, acc[i][x].y));
+                        acc[i][x].z = fmaf(a[i].y, b1.z, fmaf(a[i].x, b0.z, acc[i][x].z));
+                        acc[i][x].w = fmaf(a[i].y, b1.w, fmaf(a[i].x, b0.w, acc[i][x].w));
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = warp * 16 + lm + 4 * i;
+        if (r >= n) continue;
+        const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+        float* o = out + ((size_t)(t0 + r) * H + h) * d;
+#pragma unroll
+        for (int x = 0; x < ND; ++x) {
+            const int c = 4 * (ln + 8 * x);
+            if (c < d) *reinterpret_cast<float4*>(o + c) = make_float4(acc[i][x].x * inv, acc[i][x].y * inv, acc[i][x].z * inv, acc[i][x].w * inv);
+        }
+    }
+}
+
+// q, out [T, H, d], pages [num_pages, K, P, d] float32, all starting on 16 bytes; tiles [n_tiles, 2] = (request row, offset
+// of `tile` tokens among those it brings), tile a multiple of 64.  d <= 128 in steps of 4 (else AIE_UNSUPPORTED: the
+// caller takes the kernel above).  Tokens that no tile names are left.
+extern "C" int aie_paged_attention_f32_tiles(const float* q, const float* k_pages, const float* v_pages, float* out, const int* tiles,
+                                             int n_tiles, int tile, const int* q_start, const int* q_len, const int* ctx_len,
+                                             const int* block_table, int bt_width, int num_pages, int P, int H, int K, int d,
+                                             int window, float scale, unsigned* err, cudaStream_t st) {
+    if (n_tiles <= 0) return 0;
+    if (d <= 0 || d > 128 || d % 4 || K <= 0 || H % K || H > 65535 || tile <= 0 || tile % PT_Q || P <= 0 ||
+        (long long)num_pages * P > 0x7fffffffLL || (((size_t)q | (size_t)k_pages | (size_t)v_pages | (size_t)out) & 15))
+        return AIE_UNSUPPORTED;
+    const int ld = d + 4, ldp = PLAIN_CHUNK + 4;
+    const size_t keys = PLAIN_CHUNK * ld > PT_Q * ldp ? (size_t)PLAIN_CHUNK * ld : (size_t)PT_Q * ldp;
+    const size_t smem = ((size_t)PT_Q * ld + (size_t)PLAIN_CHUNK * d + keys) * sizeof(float) + PLAIN_CHUNK * sizeof(int);
+    const dim3 grid((unsigned)n_tiles * (tile / PT_Q), H);
+#define GO(ND)                                                                                                              \
+    {                                                                                                                       \
+        cudaError_t e = cudaFuncSetAttribute(paged_attention_f32_tiles_kernel<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                             (int)smem);                                                                    \
+        if (e != cudaSuccess) return (int)e;                                                                                \
+        paged_attention_f32_tiles_kernel<ND><<<grid, PT_THREADS, smem, st>>>(q, k_pages, v_pages, out, tiles, tile / PT_Q,   \
+            q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, H, K, d, window, scale, err);                     \
+    }
+    switch ((d + 31) / 32) {
+        case 1: GO(1) break;
+        case 2: GO(2) break;
+        case 3: GO(3) break;
+        default: GO(4)
+    }
+#undef GO
+    AIE_LAUNCH_CHECK();
+}

@@ -614,6 +614,29 @@ def prefill_takes_pairs(n_tiles: int, n_units: int, heads: int) -> bool:
     return 0.86 * math.ceil(w2) / w2 < math.ceil(w1) / w1
 
 
+F32_TILE_MIN_TOKENS = 8      # steps whose longest portion is shorter leave all tokens to the plain kernel
+
+
+def _paged_attention_f32(q, k_pages, v_pages, ctx, work, block_table, scale, window, dec_cost, pre_cost):
+    """float32: portions of prompts by the tiled kernel, lone tokens by the plain one (the same additions in the same
+    order: a token's bits are those of the plain kernel)."""
+    T, H, d = q.shape
+    num_pages, K, P, _ = k_pages.shape
+    out = torch.empty_like(q)
+    if work.n_decode:
+        paged_attention_plain(q, k_pages, v_pages, ctx.positions, ctx.token_req, block_table, scale, window, ctx.err, out=out,
+                              token_list=work.decode_tokens, cost=dec_cost)
+    _dev(q, k_pages, v_pages, work.prefill_tiles, ctx.q_start, ctx.q_len, ctx.ctx_len, block_table, ctx.err)
+    lib = library("attention_plain.cu")
+    with region("attention_f32_tiles", *pre_cost):
+        check(lib.aie_paged_attention_f32_tiles(_p(q), _p(k_pages), _p(v_pages), _p(out), _p(work.prefill_tiles),
+                                                c_int(work.prefill_tiles.shape[0]), c_int(PREFILL_TILE), _p(ctx.q_start),
+                                                _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
+                                                c_int(num_pages), c_int(P), c_int(H), c_int(K), c_int(d), c_int(window),
+                                                c_float(scale), _p(ctx.err), _stream()), "paged_attention_f32_tiles")
+    return out
+
+
 def paged_attention(q, k_pages, v_pages, ctx, work, block_table, scale: float, window: int):
     """Attention of a step's query tokens over the cache.  `ctx` gives the step's generic arrays
     (positions, token_req, q_start, q_len, ctx_len, R), `work` the attention work lists derived from
@@ -637,6 +660,9 @@ def paged_attention(q, k_pages, v_pages, ctx, work, block_table, scale: float, w
         pairs = float((ql[~lone] * cl[~lone] + ql[~lone] * (ql[~lone] + 1) / 2).sum())
         pre_cost = (float((cl[~lone] + ql[~lone]).sum()) * K * d * 2 * es + float(ql[~lone].sum()) * H * d * 2 * es,
                     4.0 * pairs * H * d)
+    if not fast and q.dtype == torch.float32 and k_pages.dtype == torch.float32 and d <= 128 and d % 4 == 0 \
+            and getattr(ctx, "max_q_len", 0) >= F32_TILE_MIN_TOKENS and getattr(work, "prefill_tiles", None) is not None:
+        return _paged_attention_f32(q, k_pages, v_pages, ctx, work, block_table, scale, window, dec_cost, pre_cost)
     if not fast:
         return paged_attention_plain(q, k_pages, v_pages, ctx.positions, ctx.token_req, block_table,
                                      scale, window, ctx.err,

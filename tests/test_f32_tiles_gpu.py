@@ -1,6 +1,6 @@
 """The tiled kernels of the 32-bit path give the bits of the simple ones: every output is a sum in one fixed order, whatever
-the tile.  Products against the same product with its weights stored in bfloat16 (which takes the simple kernel), at the
-edges of tiles."""
+the tile.  Products against the same product with its weights stored in bfloat16 (which takes the simple kernel),
+attention against the plain kernel, at the edges of tiles, chunks, pages and windows."""
 import pytest
 import torch
 
@@ -43,3 +43,38 @@ def test_gathered_rows_batches_and_weights_per_tile():
     for out, ww in zip(outs, (w.float(), w)):
         ops.gemm_f32_ex(x, ww, out, 70, N, K, E * K, E * (N + 8), batch=E, a_bs=K, w_bs=N * K, c_bs=N + 8)
     assert torch.equal(*outs) and bool((outs[0][:, :, N:] == 0).all())
+
+
+@pytest.mark.parametrize("H,K,d,P,reqs,window", [
+    (4, 2, 64, 16, [(0, 64), (0, 65), (70, 1)], 0), (2, 1, 128, 8, [(100, 130), (5, 8)], 0), (3, 3, 20, 4, [(127, 9), (0, 200)], 0),
+    (2, 2, 96, 16, [(300, 70), (0, 1), (128, 2)], 100), (1, 1, 4, 2, [(0, 257)], 1), (8, 1, 32, 32, [(1, 127), (129, 129)], 64)])
+def test_attention_of_portions_has_the_plain_kernel_s_bits(H, K, d, P, reqs, window):
+    from ai_engine_b200.cache import PagedCache
+    from ai_engine_b200.engine.step import StepContext, StepEntry
+    from ai_engine_b200.kernels import ops
+    from ai_engine_b200.parts import ATTENTION_WORK, CacheNeed, KVRequest
+    gen = torch.Generator(device=DEV).manual_seed(H * 10 + d)
+    cache = PagedCache([CacheNeed(0, "m", KVRequest(K, d))], P, sum(-(-(c + n) // P) for c, n in reqs) + 2, len(reqs), 4096,
+                       torch.float32, DEV)
+    entries, pool = [], cache.groups[0].pool                               # unwritten places hold NaN
+    for c, n in reqs:
+        s = cache.admit()
+        cache.ensure(s, c + n)
+        entries.append(StepEntry(s, c, [0] * n, []))
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ctx = StepContext(entries, cache, torch.device(DEV), err, planners=(ATTENTION_WORK,))
+    lc = cache.layer_cache(0, ctx)["m"]
+    bt = lc.block_table.cpu().numpy()
+    for r, (c, n) in enumerate(reqs):
+        for j in range(c + n):
+            pool[0, :, int(bt[r, j // P]), :, j % P] = torch.randn(2, K, d, generator=gen, device=DEV)
+    q = torch.randn(sum(n for _, n in reqs), H, d, generator=gen, device=DEV)
+    got = ops.paged_attention(q, lc.k_pages, lc.v_pages, ctx, ctx.plan(ATTENTION_WORK), lc.block_table, 0.3, window)
+    want = ops.paged_attention_plain(q, lc.k_pages, lc.v_pages, ctx.positions, ctx.token_req, lc.block_table, 0.3, window, err)
+    assert torch.equal(got, want) and not bool(got.isnan().any()) and int(err.item()) == 0
+    bad = lc.block_table.clone()                                          # a page outside the pool is flagged and skipped
+    bad[0, 0] = pool.shape[2] + 7
+    got = ops.paged_attention(q, lc.k_pages, lc.v_pages, ctx, ctx.plan(ATTENTION_WORK), bad, 0.3, 0)
+    assert int(err.item()) == 2
+    want = ops.paged_attention_plain(q, lc.k_pages, lc.v_pages, ctx.positions, ctx.token_req, bad, 0.3, 0, err)
+    assert torch.equal(got, want)
