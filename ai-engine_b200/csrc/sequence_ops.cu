@@ -333,11 +333,74 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
     }
 }
 
+// The same 16 bytes a thread: `lanes` lanes (8, 16 or 32) of a warp share a row of 4 lanes NV floats, and a lane fetches the
+// rows of four (token, head) pairs before it uses the first.  Bound by memory: 2,048 tokens x 16 heads of 128 with a gate
+// (42 MB) 16.4 us a float at a time.
+#define HN_ROWS 4
+template <int NV, typename O>
+__global__ void head_norm_gate4_kernel(const float* __restrict__ o, const float* __restrict__ g, int ldg,
+                                       const float* __restrict__ w, O* __restrict__ out, int TH, int H, int lanes, float eps) {
+    const int dv = lanes * 4 * NV, per_warp = 32 / lanes, lane = threadIdx.x & 31, c = (lane % lanes) * 4;
+    const int first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp * HN_ROWS + lane / lanes;
+    float4 x[HN_ROWS][NV], gv[HN_ROWS][NV];
+#pragma unroll
+    for (int k = 0; k < HN_ROWS; ++k) {
+        const int wi = first + k * per_warp;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            x[k][v] = gv[k][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (wi < TH) {
+                x[k][v] = *reinterpret_cast<const float4*>(o + (size_t)wi * dv + v * lanes * 4 + c);
+                if (g) gv[k][v] = *reinterpret_cast<const float4*>(g + (size_t)(wi / H) * ldg + (size_t)(wi % H) * dv + v * lanes * 4 + c);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < HN_ROWS; ++k) {
+        const int wi = first + k * per_warp;
+        float ss = 0.f;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) ss += (x[k][v].x * x[k][v].x + x[k][v].y * x[k][v].y) + (x[k][v].z * x[k][v].z + x[k][v].w * x[k][v].w);
+        for (int off = lanes >> 1; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+        const float r = 1.0f / sqrtf(ss / (float)dv + eps);
+        if (wi >= TH) continue;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            float4 y = make_float4(x[k][v].x * r, x[k][v].y * r, x[k][v].z * r, x[k][v].w * r);
+            if (w) {
+                const float4 ww = *reinterpret_cast<const float4*>(w + v * lanes * 4 + c);
+                y = make_float4(y.x * ww.x, y.y * ww.y, y.z * ww.z, y.w * ww.w);
+            }
+            if (g) {
+                const float4 z = gv[k][v];
+                y = make_float4(y.x * (z.x / (1.0f + expf(-z.x))), y.y * (z.y / (1.0f + expf(-z.y))),
+                                y.z * (z.z / (1.0f + expf(-z.z))), y.w * (z.w / (1.0f + expf(-z.w))));
+            }
+            store4<O>(out + (size_t)wi * dv + v * lanes * 4 + c, y);
+        }
+    }
+}
+
 extern "C" int aie_head_norm_gate(const float* o, const float* g, int ldg, const float* w, void* out, int out_dtype, int T,
                                   int H, int dv, float eps, cudaStream_t st) {
     if (T <= 0) return 0;
     if (H <= 0 || dv <= 0) return AIE_BAD_ARG;
     const long long warps = (long long)T * H;
+    const size_t esz = out_dtype == AIE_F32 ? 4 : 2;
+    // rows of 32, 64, 128 or 256 floats on 16 bytes, and enough of them that four to a lane still fill the machine
+    if ((dv == 32 || dv == 64 || dv == 128 || dv == 256) && ldg % 4 == 0 && !(((size_t)o | (size_t)g | (size_t)w) & 15) &&
+        !((size_t)out & (4 * esz - 1)) && (out_dtype == AIE_F32 || out_dtype == AIE_BF16) && warps >= 4096 && warps < 0x40000000LL) {
+        const int lanes = dv >= 128 ? 32 : dv / 4, rows = 32 / lanes * HN_ROWS * 4;
+        const unsigned blocks4 = (unsigned)((warps + rows - 1) / rows);
+#define GO(NV, O) head_norm_gate4_kernel<NV, O><<<blocks4, 128, 0, st>>>(o, g, ldg, w, (O*)out, (int)warps, H, lanes, eps)
+        if (out_dtype == AIE_F32) {
+            if (dv == 256) GO(2, float); else GO(1, float);
+        } else {
+            if (dv == 256) GO(2, bf16); else GO(1, bf16);
+        }
+#undef GO
+        AIE_LAUNCH_CHECK();
+    }
     const unsigned blocks = (unsigned)((warps + 3) / 4);
     if (out_dtype == AIE_F32)
         head_norm_gate_kernel<float><<<blocks, 128, 0, st>>>(o, g, ldg, w, (float*)out, (int)warps, H, dv, eps);
@@ -364,11 +427,39 @@ __global__ void clamped_glu_kernel(const float* __restrict__ gu, int ld, O* __re
     out[i] = from_f32<O>(g / (1.0f + expf(-alpha * g)) * (u + shift));
 }
 
+// Four elements a thread, 16-byte loads; rows (optional): a row with rows[t] < 0 is padding that nobody reads and is left.
+// Bound by memory: 8,892 rows (6,844 of them live) of 1,024 took 40.7 us an element at a time.
+template <typename O>
+__global__ void clamped_glu4_kernel(const float* __restrict__ gu, int ld, O* __restrict__ out, const int* __restrict__ rows,
+                                    int F, float limit, float alpha, float shift) {
+    const int t = blockIdx.x, f = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (f >= F || (rows && rows[t] < 0)) return;
+    float4 g = *reinterpret_cast<const float4*>(gu + (size_t)t * ld + f), u = *reinterpret_cast<const float4*>(gu + (size_t)t * ld + F + f);
+    g = make_float4(fminf(g.x, limit), fminf(g.y, limit), fminf(g.z, limit), fminf(g.w, limit));
+    u = make_float4(fminf(fmaxf(u.x, -limit), limit), fminf(fmaxf(u.y, -limit), limit), fminf(fmaxf(u.z, -limit), limit),
+                    fminf(fmaxf(u.w, -limit), limit));
+    store4<O>(out + (size_t)t * F + f, make_float4(g.x / (1.0f + expf(-alpha * g.x)) * (u.x + shift), g.y / (1.0f + expf(-alpha * g.y)) * (u.y + shift),
+                                                   g.z / (1.0f + expf(-alpha * g.z)) * (u.z + shift), g.w / (1.0f + expf(-alpha * g.w)) * (u.w + shift)));
+}
+
 extern "C" int aie_clamped_glu(const float* gu, int ld, void* out, int out_dtype, long long T, int F, float limit,
-                               float alpha, float shift, cudaStream_t st) {
+                               float alpha, float shift, const int* rows, cudaStream_t st) {
     if (T <= 0) return 0;
     if (F <= 0) return AIE_BAD_ARG;
     const long long n = T * F;
+    const size_t esz = out_dtype == AIE_F32 ? 4 : 2;
+    if (F % 4 == 0 && ld % 4 == 0 && !((size_t)gu & 15) && !((size_t)out & (4 * esz - 1)) && T <= 0x7fffffffLL &&
+        (out_dtype == AIE_F32 || out_dtype == AIE_BF16)) {
+        const int threads = F >= 1024 ? 256 : (F >= 256 ? 64 : 32);
+        const dim3 grid((unsigned)T, (F / 4 + threads - 1) / threads);
+        if (grid.y <= 65535) {
+            if (out_dtype == AIE_F32)
+                clamped_glu4_kernel<float><<<grid, threads, 0, st>>>(gu, ld, (float*)out, rows, F, limit, alpha, shift);
+            else
+                clamped_glu4_kernel<bf16><<<grid, threads, 0, st>>>(gu, ld, (bf16*)out, rows, F, limit, alpha, shift);
+            AIE_LAUNCH_CHECK();
+        }
+    }
     const unsigned blocks = (unsigned)((n + 255) / 256);
     if (out_dtype == AIE_F32)
         clamped_glu_kernel<float><<<blocks, 256, 0, st>>>(gu, ld, (float*)out, n, F, limit, alpha, shift);
@@ -391,11 +482,29 @@ __global__ void gated_decay_kernel(const float* __restrict__ z, const float* __r
     out[i] = expf(ls * inv_tau);
 }
 
+// four elements a thread (N a multiple of 4): 4.2 M elements took 17 us one at a time, memory's share is 5
+__global__ void gated_decay4_kernel(const float* __restrict__ z, const float* __restrict__ bias, float* __restrict__ out,
+                                    long long n4, int N, float inv_tau) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n4) return;
+    float4 v = reinterpret_cast<const float4*>(z)[i];
+    if (bias) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + (i * 4) % N);
+        v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+    }
+    const auto decay = [&](float x) { return expf((fminf(x, 0.f) - log1pf(expf(-fabsf(x)))) * inv_tau); };
+    reinterpret_cast<float4*>(out)[i] = make_float4(decay(v.x), decay(v.y), decay(v.z), decay(v.w));
+}
+
 extern "C" int aie_gated_decay(const float* z, const float* bias, float* out, long long T, int N, float tau,
                                cudaStream_t st) {
     if (T <= 0) return 0;
     if (N <= 0 || !(tau > 0.f)) return AIE_BAD_ARG;
     const long long n = T * N;
+    if (N % 4 == 0 && !(((size_t)z | (size_t)out | (size_t)bias) & 15)) {
+        gated_decay4_kernel<<<(unsigned)((n / 4 + 255) / 256), 256, 0, st>>>(z, bias, out, n / 4, N, 1.0f / tau);
+        AIE_LAUNCH_CHECK();
+    }
     gated_decay_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(z, bias, out, n, N, 1.0f / tau);
     AIE_LAUNCH_CHECK();
 }
@@ -656,9 +765,112 @@ __global__ void causal_conv4_kernel(const float* __restrict__ u, int ld_in, cons
     }
 }
 
+// For steps of many tokens a request: a block walks CC_T tokens with the last taps - 1 inputs and all taps in registers, so
+// an input is read once (and taps - 1 of them again at a tile's start) and a weight once a tile; four inputs are on their
+// way at a time.  A request's first taps - 1 tokens, which read its tail, and the tail's renewal belong to a block of
+// their own (the first R of a row of blocks): nobody else touches the tail.  The additions and their order are those
+// above.  Bound by memory: 2,048 tokens of 6,144 channels (100 MB) took 108 us when every output read its taps anew.
+#define CC_T 16
+#define CC_THREADS 64
+template <int TAPS, typename O>
+__global__ void __launch_bounds__(CC_THREADS)
+causal_conv_tiles_kernel(const float* __restrict__ u, int ld_in, const float* __restrict__ w, const float* __restrict__ bias,
+                         float* __restrict__ state, O* __restrict__ out, int ld_out, const int* __restrict__ q_start,
+                         const int* __restrict__ q_len, const int* __restrict__ slots, const int* __restrict__ token_req, int T,
+                         int R, int C, int residual, int act, int dup_from, int dup_n, int max_slots, unsigned* err) {
+    constexpr int Hh = TAPS - 1;
+    const int c = (blockIdx.y * CC_THREADS + threadIdx.x) * 4;
+    if (c >= C) return;
+    float wc[4][TAPS];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) wc[e][j] = w[(size_t)(c + e) * TAPS + j];
+    const float4 b = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool dup = c >= dup_from && c < dup_from + dup_n;
+    const auto row = [&](int t) { return *reinterpret_cast<const float4*>(u + (size_t)t * ld_in + c); };
+    float4 win[TAPS];                                       // win[Hh]: the token's own input
+    win[0] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const auto emit = [&](int t) {
+        float4 acc = b;
+        if (residual) acc = make_float4(acc.x + win[Hh].x, acc.y + win[Hh].y, acc.z + win[Hh].z, acc.w + win[Hh].w);
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            acc.x = fmaf(wc[0][j], win[j].x, acc.x);
+            acc.y = fmaf(wc[1][j], win[j].y, acc.y);
+            acc.z = fmaf(wc[2][j], win[j].z, acc.z);
+            acc.w = fmaf(wc[3][j], win[j].w, acc.w);
+        }
+        if (act == 1) {
+            acc.x = acc.x / (1.0f + expf(-acc.x));
+            acc.y = acc.y / (1.0f + expf(-acc.y));
+            acc.z = acc.z / (1.0f + expf(-acc.z));
+            acc.w = acc.w / (1.0f + expf(-acc.w));
+        }
+        store4<O>(out + (size_t)t * ld_out + c, acc);
+        if (dup) store4<O>(out + (size_t)t * ld_out + c + dup_n, acc);
+    };
+    if ((int)blockIdx.x < R) {
+        const int r = blockIdx.x, a = q_start[r], n = q_len[r], slot = slots[r];
+        if (n <= 0) return;
+        if (slot < 0 || slot >= max_slots) {
+            if (threadIdx.x == 0) atomicOr(err, AIE_DEV_SLOT_OOB);
+            return;
+        }
+        float* st = state + (size_t)slot * Hh * C + c;      // st[k * C]: input at local index k - Hh
+        float4 old[Hh];
+#pragma unroll
+        for (int k = 0; k < Hh; ++k) win[k + 1] = old[k] = *reinterpret_cast<const float4*>(st + (size_t)k * C);
+#pragma unroll
+        for (int i = 0; i < Hh; ++i) {
+            if (i >= n) break;
+#pragma unroll
+            for (int j = 0; j < Hh; ++j) win[j] = win[j + 1];
+            win[Hh] = row(a + i);
+            emit(a + i);
+        }
+#pragma unroll
+        for (int k = 0; k < Hh; ++k) {
+            const int src = n - Hh + k;                     // the input at that index; before the portion: the old tail's
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (src >= 0) x = row(a + src);
+#pragma unroll
+            for (int m = 0; m < Hh; ++m)
+                if (src < 0 && src + Hh == m) x = old[m];
+            *reinterpret_cast<float4*>(st + (size_t)k * C) = x;
+        }
+        return;
+    }
+    int t = ((int)blockIdx.x - R) * CC_T;
+    const int end = min(T, t + CC_T);
+    while (t < end) {
+        const int r = token_req[t], a = q_start[r], stop = min(end, a + q_len[r]);
+        int s = max(t, a + Hh);
+        if (s < stop) {
+#pragma unroll
+            for (int k = 0; k < Hh; ++k) win[k + 1] = row(s - Hh + k);
+        }
+        for (; s < stop; s += 4) {
+            float4 x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (s + i < stop) x[i] = row(s + i);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (s + i < stop) {
+#pragma unroll
+                    for (int j = 0; j < Hh; ++j) win[j] = win[j + 1];
+                    win[Hh] = x[i];
+                    emit(s + i);
+                }
+        }
+        t = max(t + 1, stop);
+    }
+}
+
 extern "C" int aie_causal_conv(const float* u, int ld_in, const float* w, const float* bias, float* state, void* out,
                                int out_dtype, int ld_out, const int* q_start, const int* q_len, const int* slots,
-                               const int* token_req, int T, int C, int taps, int residual, int act, int dup_from,
+                               const int* token_req, int T, int R, int C, int taps, int residual, int act, int dup_from,
                                int dup_n, int max_slots, unsigned* err, cudaStream_t st) {
     if (T <= 0) return 0;
     if (C <= 0 || taps < 1 || act < 0 || act > 1 || dup_n < 0 || (dup_n && (dup_from < 0 || dup_from + dup_n != C)))
@@ -668,6 +880,18 @@ extern "C" int aie_causal_conv(const float* u, int ld_in, const float* w, const 
         !((size_t)state & 15) && !((size_t)out & (4 * esz - 1)) && (!bias || !((size_t)bias & 15)) &&
         (out_dtype == AIE_F32 || out_dtype == AIE_BF16)) {
         const int threads4 = 64;
+        // portions of eight tokens on average and more: below that most tokens are a request's first ones
+        if (taps >= 2 && taps <= 4 && R > 0 && T >= 8 * R) {
+            const dim3 tiles(R + (T + CC_T - 1) / CC_T, (C / 4 + CC_THREADS - 1) / CC_THREADS);
+#define GO(TAPS, O) causal_conv_tiles_kernel<TAPS, O><<<tiles, CC_THREADS, 0, st>>>(u, ld_in, w, bias, state, (O*)out, ld_out, q_start, q_len, slots, token_req, T, R, C, residual, act, dup_from, dup_n, max_slots, err)
+#define GO_O(TAPS) if (out_dtype == AIE_F32) GO(TAPS, float); else GO(TAPS, bf16)
+            if (taps == 2) { GO_O(2); }
+            else if (taps == 3) { GO_O(3); }
+            else { GO_O(4); }
+#undef GO_O
+#undef GO
+            AIE_LAUNCH_CHECK();
+        }
         dim3 grid4(T, (C / 4 + threads4 - 1) / threads4);
         if (out_dtype == AIE_F32)
             causal_conv4_kernel<float><<<grid4, threads4, 0, st>>>(u, ld_in, w, bias, state, (float*)out, ld_out, q_start, q_len, slots, token_req, C, taps, residual, act, dup_from, dup_n, max_slots, err);
@@ -712,6 +936,39 @@ __global__ void gate_group_norm_kernel(const float* __restrict__ y, const float*
     }
 }
 
+// The same with a warp a (token, part) of 128 NV floats on 16 bytes: y and z are read once, all of a lane's loads side by
+// side.  Bound by memory: 2,048 tokens of 4,096 in eight parts (84 MB) took 38 us in two passes of a block a part.
+template <int NV, typename O>
+__global__ void __launch_bounds__(256)
+gate_group_norm4_kernel(const float* __restrict__ y, const float* __restrict__ z, int ldz, const float* __restrict__ w,
+                        O* __restrict__ out, int W, int parts, int rows, float eps) {
+    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (row >= rows) return;
+    const int t = row / parts, n = 128 * NV, c0 = (row % parts) * n + lane * 4;
+    float4 yv[NV], zv[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        yv[v] = *reinterpret_cast<const float4*>(y + (size_t)t * W + c0 + v * 128);
+        zv[v] = *reinterpret_cast<const float4*>(z + (size_t)t * ldz + c0 + v * 128);
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        yv[v].x *= zv[v].x / (1.0f + expf(-zv[v].x));
+        yv[v].y *= zv[v].y / (1.0f + expf(-zv[v].y));
+        yv[v].z *= zv[v].z / (1.0f + expf(-zv[v].z));
+        yv[v].w *= zv[v].w / (1.0f + expf(-zv[v].w));
+        ss += (yv[v].x * yv[v].x + yv[v].y * yv[v].y) + (yv[v].z * yv[v].z + yv[v].w * yv[v].w);
+    }
+    ss = warp_sum(ss);
+    const float r = 1.0f / sqrtf(ss / (float)n + eps);
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const float4 wv = *reinterpret_cast<const float4*>(w + c0 + v * 128);
+        store4<O>(out + (size_t)t * W + c0 + v * 128, make_float4(yv[v].x * r * wv.x, yv[v].y * r * wv.y, yv[v].z * r * wv.z, yv[v].w * r * wv.w));
+    }
+}
+
 extern "C" int aie_gate_group_norm(const float* y, const float* z, int ldz, const float* w, void* out, int out_dtype,
                                    int T, int W, int parts, float eps, cudaStream_t st) {
     if (T <= 0) return 0;
@@ -719,6 +976,22 @@ extern "C" int aie_gate_group_norm(const float* y, const float* z, int ldz, cons
     const int n = W / parts, threads = n >= 1024 ? 256 : (n >= 256 ? 128 : 64);
     const long long blocks = (long long)T * parts;
     if (blocks > 0x7fffffffLL) return AIE_UNSUPPORTED;
+    const size_t esz = out_dtype == AIE_F32 ? 4 : 2;
+    // parts of 128, 256, 512 or 1,024 floats; fewer than 1,024 of them leave most of the machine without a warp, and a block a
+    // part is the wider reader then
+    if ((n == 128 || n == 256 || n == 512 || n == 1024) && ldz % 4 == 0 && blocks >= 1024 &&
+        !(((size_t)y | (size_t)z | (size_t)w) & 15) && !((size_t)out & (4 * esz - 1)) && (out_dtype == AIE_F32 || out_dtype == AIE_BF16)) {
+        const unsigned grid = (unsigned)((blocks + 7) / 8);
+#define GO(NV)                                                                                                              \
+    if (out_dtype == AIE_F32) gate_group_norm4_kernel<NV, float><<<grid, 256, 0, st>>>(y, z, ldz, w, (float*)out, W, parts, (int)blocks, eps); \
+    else gate_group_norm4_kernel<NV, bf16><<<grid, 256, 0, st>>>(y, z, ldz, w, (bf16*)out, W, parts, (int)blocks, eps)
+        if (n == 128) { GO(1); }
+        else if (n == 256) { GO(2); }
+        else if (n == 512) { GO(4); }
+        else { GO(8); }
+#undef GO
+        AIE_LAUNCH_CHECK();
+    }
     if (out_dtype == AIE_F32)
         gate_group_norm_kernel<float><<<(unsigned)blocks, threads, 0, st>>>(y, z, ldz, w, (float*)out, W, parts, eps);
     else if (out_dtype == AIE_BF16)
@@ -828,6 +1101,118 @@ __global__ void route_topk_kernel(float* __restrict__ z, int ld, float* __restri
         for (int k = 0; k < top; ++k) weights[(size_t)t * top + k] = weights[(size_t)t * top + k] / div * weight_scale;
 }
 
+// The same with a warp a token, for up to 64 outputs: scores and choice values in shared memory, lanes stand for outputs, or
+// for groups while the groups are weighed.  Every sum, comparison and tie is that of the kernel above.  1,711 tokens of 32
+// outputs took 24 us with a thread a token, whose rows lie apart in memory.
+#define RT_MAX 64
+#define RT_WARPS 4
+__global__ void __launch_bounds__(32 * RT_WARPS)
+route_topk_warp_kernel(float* __restrict__ z, int ld, const float* __restrict__ corr, int T, int E, int groups, int keep, int top,
+                       int* __restrict__ ids, float* __restrict__ weights, int sigmoid, int group_top, int normalise,
+                       float weight_scale) {
+    __shared__ float s_s[RT_WARPS][RT_MAX], c_s[RT_WARPS][RT_MAX], g_s[RT_WARPS][RT_MAX];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = blockIdx.x * RT_WARPS + warp;
+    if (t >= T) return;
+    float *s = s_s[warp], *c = c_s[warp], *gval = g_s[warp], *zr = z + (size_t)t * ld;
+    float m = -INFINITY;
+    for (int e = lane; e < E; e += 32) {
+        s[e] = zr[e];
+        m = fmaxf(m, s[e]);
+    }
+    if (sigmoid) {
+        for (int e = lane; e < E; e += 32) s[e] = 1.0f / (1.0f + expf(-s[e]));
+    } else {
+        m = warp_max(m);
+        for (int e = lane; e < E; e += 32) s[e] = expf(s[e] - m);
+        __syncwarp();
+        float sum = 0.f;
+        for (int e = 0; e < E; ++e) sum += s[e];            // every lane, in order
+        __syncwarp();
+        for (int e = lane; e < E; e += 32) s[e] = s[e] / sum;
+    }
+    for (int e = lane; e < E; e += 32) {
+        c[e] = s[e] + (corr ? corr[e] : 0.f);
+        zr[e] = s[e];
+    }
+    __syncwarp();
+    const int per = E / groups;
+    if (keep < groups) {
+        for (int g = lane; g < groups; g += 32) {
+            float gv = -INFINITY;
+            if (group_top <= 1) {
+                for (int e = g * per; e < (g + 1) * per; ++e) gv = fmaxf(gv, c[e]);
+            } else {
+                gv = 0.f;
+                float bound = INFINITY;
+                int bound_e = -1;
+                for (int n = 0; n < group_top && n < per; ++n) {
+                    float best = -INFINITY;
+                    int best_e = -1;
+                    for (int e = g * per; e < (g + 1) * per; ++e) {
+                        const bool below = c[e] < bound || (c[e] == bound && e > bound_e);
+                        if (below && (best_e < 0 || c[e] > best)) {
+                            best = c[e];
+                            best_e = e;
+                        }
+                    }
+                    if (best_e < 0) break;
+                    gv += best;
+                    bound = best;
+                    bound_e = best_e;
+                }
+            }
+            gval[g] = gv;
+        }
+        __syncwarp();
+        unsigned long long kept = 0ull;
+        for (int k = 0; k < keep; ++k) {                    // every lane
+            int bg = -1;
+            float bv = -INFINITY;
+            for (int g = 0; g < groups; ++g) {
+                if (kept >> g & 1ull) continue;
+                if (bg < 0 || gval[g] > bv) {
+                    bg = g;
+                    bv = gval[g];
+                }
+            }
+            if (bg >= 0) kept |= 1ull << bg;
+        }
+        for (int e = lane; e < E; e += 32)
+            if (!(kept >> (e / per) & 1ull)) c[e] = -INFINITY;
+    }
+    float div = 0.f;
+    for (int k = 0; k < top; ++k) {
+        int be = -1;                                        // the largest of the lane's outputs, the first among equals
+        float bv = -INFINITY;
+        for (int e = lane; e < E; e += 32)
+            if (c[e] > bv) {
+                be = e;
+                bv = c[e];
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+            const int oe = __shfl_xor_sync(0xffffffffu, be, o);
+            if (oe >= 0 && (be < 0 || ov > bv || (ov == bv && oe < be))) {
+                be = oe;
+                bv = ov;
+            }
+        }
+        const float wv = be >= 0 ? s[be] : 0.f;
+        div += wv;
+        if (lane == 0) {
+            ids[(size_t)t * top + k] = be;
+            weights[(size_t)t * top + k] = wv;
+        }
+        if (be >= 0 && lane == (be & 31)) c[be] = -INFINITY;
+        __syncwarp();
+    }
+    if (!normalise && weight_scale == 1.f) return;
+    div = normalise ? div + 1e-20f : 1.f;
+    if (lane == 0)
+        for (int k = 0; k < top; ++k) weights[(size_t)t * top + k] = weights[(size_t)t * top + k] / div * weight_scale;
+}
+
 extern "C" int aie_route_topk(float* z, int ld, float* scratch, const float* corr, int T, int E, int groups, int keep, int top,
                               int* ids, float* weights, int sigmoid, int group_top, int normalise, float weight_scale,
                               cudaStream_t st) {
@@ -835,6 +1220,11 @@ extern "C" int aie_route_topk(float* z, int ld, float* scratch, const float* cor
     if (E <= 0 || ld < E || groups <= 0 || E % groups || keep <= 0 || keep > groups || top <= 0 || top > E / groups * keep)
         return AIE_BAD_ARG;
     if (groups > 64) return AIE_UNSUPPORTED;
+    if (E <= RT_MAX) {
+        route_topk_warp_kernel<<<(T + RT_WARPS - 1) / RT_WARPS, 32 * RT_WARPS, 0, st>>>(z, ld, corr, T, E, groups, keep, top, ids, weights,
+                                                                                       sigmoid, group_top, normalise, weight_scale);
+        AIE_LAUNCH_CHECK();
+    }
     route_topk_kernel<<<(T + 63) / 64, 64, 0, st>>>(z, ld, scratch, corr, T, E, groups, keep, top, ids, weights, sigmoid,
                                                     group_top, normalise, weight_scale);
     AIE_LAUNCH_CHECK();
@@ -866,11 +1256,55 @@ __global__ void expert_combine_weighted_kernel(const float* __restrict__ y, cons
     }
 }
 
+// The same four columns a thread with the rows of all choices (up to eight) on their way before the first is used; the
+// additions are those of the kernel above, in its order.  Bound by memory: 1,711 tokens x 4 rows of 2,048 and a shared row
+// (84 MB) took 43 us a float at a time.
+template <typename A>
+__global__ void __launch_bounds__(256)
+expert_combine_weighted4_kernel(const float* __restrict__ y, const int* __restrict__ pair_row, const float* __restrict__ weight,
+                                int top, const A* __restrict__ h, float* __restrict__ out, int D, const float* __restrict__ shared,
+                                int shared_parts, size_t shared_stride) {
+    const int t = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+    if (c >= D) return;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), sh = acc, v[8];
+    float w[8];
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+        w[s] = 0.f;
+        v[s] = acc;
+        if (s >= top) continue;
+        const int row = pair_row[(size_t)t * top + s];
+        if (row >= 0) v[s] = *reinterpret_cast<const float4*>(y + (size_t)row * D + c);
+        else if (row == -2) v[s] = load4<A>(h + (size_t)t * D + c);
+        w[s] = row >= 0 || row == -2 ? weight[(size_t)t * top + s] : 0.f;
+    }
+    if (shared)
+        for (int p = 0; p < shared_parts; ++p) {
+            const float4 x = *reinterpret_cast<const float4*>(shared + p * shared_stride + (size_t)t * D + c);
+            sh = make_float4(sh.x + x.x, sh.y + x.y, sh.z + x.z, sh.w + x.w);
+        }
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+        if (s < top) acc = make_float4(fmaf(w[s], v[s].x, acc.x), fmaf(w[s], v[s].y, acc.y), fmaf(w[s], v[s].z, acc.z), fmaf(w[s], v[s].w, acc.w));
+    if (shared) acc = make_float4(acc.x + sh.x, acc.y + sh.y, acc.z + sh.z, acc.w + sh.w);
+    *reinterpret_cast<float4*>(out + (size_t)t * D + c) = acc;
+}
+
 extern "C" int aie_expert_combine_weighted(const float* y, const int* pair_row, const float* weight, int top,
                                            const void* h, int h_dtype, float* out, int T, int D, const float* shared,
                                            int shared_parts, long long shared_stride, cudaStream_t st) {
     if (T <= 0) return 0;
     if (D <= 0 || top <= 0) return AIE_BAD_ARG;
+    if (D % 4 == 0 && top <= 8 && shared_stride % 4 == 0 && !(((size_t)y | (size_t)out | (size_t)shared) & 15) &&
+        !((size_t)h & (h_dtype == AIE_BF16 ? 7 : 15)) && (D / 4 + 255) / 256 <= 65535) {
+        const int threads4 = D >= 1024 ? 256 : 64;
+        const dim3 grid(T, (D / 4 + threads4 - 1) / threads4);
+        if (h_dtype == AIE_BF16)
+            expert_combine_weighted4_kernel<bf16><<<grid, threads4, 0, st>>>(y, pair_row, weight, top, (const bf16*)h, out, D, shared, shared_parts, (size_t)shared_stride);
+        else
+            expert_combine_weighted4_kernel<float><<<grid, threads4, 0, st>>>(y, pair_row, weight, top, (const float*)h, out, D, shared, shared_parts, (size_t)shared_stride);
+        AIE_LAUNCH_CHECK();
+    }
     const int threads = D >= 1024 ? 256 : 128;
     if (h_dtype == AIE_BF16)
         expert_combine_weighted_kernel<bf16><<<T, threads, 0, st>>>(y, pair_row, weight, top, (const bf16*)h, out, D, shared, shared_parts, (size_t)shared_stride);

@@ -819,9 +819,10 @@ def head_norm_gate(o: torch.Tensor, gate: Optional[torch.Tensor], weight: Option
 
 
 def clamped_glu(gu: torch.Tensor, F: int, limit: float, alpha: float, shift: float,
-                out_dtype: torch.dtype) -> torch.Tensor:
+                out_dtype: torch.dtype, rows: Optional[torch.Tensor] = None) -> torch.Tensor:
     """g = min(gate, limit), u = clamp(up, +-limit): g * sigmoid(alpha g) * (u + shift).  gu [T, >= 2F] float32
-    with the gate in columns [0, F) and up in [F, 2F)."""
+    with the gate in columns [0, F) and up in [F, 2F).  rows (int32 [T]): rows with a negative entry are padding of a
+    grouping and may be left unwritten."""
     if gu.dtype != torch.float32 or gu.stride(1) != 1 or gu.shape[1] < 2 * F:
         raise KernelError("clamped_glu: float32 [T, >= 2F] input")
     T = gu.shape[0]
@@ -829,7 +830,7 @@ def clamped_glu(gu: torch.Tensor, F: int, limit: float, alpha: float, shift: flo
     lib = library("sequence_ops.cu")
     with region("clamped_glu", 2 * T * F * 4 + _nb(out)):
         check(lib.aie_clamped_glu(_p(gu), c_int(gu.stride(0)), _p(out), c_int(dtype_code(out)), c_longlong(T),
-                                  c_int(F), c_float(limit), c_float(alpha), c_float(shift), _stream()), "clamped_glu")
+                                  c_int(F), c_float(limit), c_float(alpha), c_float(shift), _p(rows), _stream()), "clamped_glu")
     return out
 
 
@@ -1137,7 +1138,7 @@ def causal_conv(u: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
     with region("causal_conv", T * C * 4 + _nb(out)):
         check(lib.aie_causal_conv(_p(u), c_int(u.stride(0)), _p(w), _p(bias), _p(state), _p(out), c_int(dtype_code(out)),
                                   c_int(out.stride(0)), _p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), _p(ctx.token_req),
-                                  c_int(T), c_int(C), c_int(taps), c_int(1 if residual else 0),
+                                  c_int(T), c_int(ctx.R), c_int(C), c_int(taps), c_int(1 if residual else 0),
                                   c_int(1 if activation == "silu" else 0), c_int(dup_from), c_int(dup_n),
                                   c_int(state.shape[0]), _p(ctx.err), _stream()), "causal_conv")
     return out

@@ -80,7 +80,7 @@ class TableMoE(FeedForward):
         T, D, F = h.shape[0], self.hidden, self.F
         row_token, pair_row, tile_expert = ops.expert_plan(ctx.token_ids, self.table, self.E, ctx.err)
         gu = ops.grouped_linear(h, self.w_gu, tile_expert, torch.float32, ctx.err, row_src=row_token, live=pair_row.numel())
-        act = ops.clamped_glu(gu, F, self.limit, self.alpha, self.shift, self.env.dtype)
+        act = ops.clamped_glu(gu, F, self.limit, self.alpha, self.shift, self.env.dtype, rows=row_token)
         y = ops.grouped_linear(act, self.w_down, tile_expert, torch.float32, ctx.err)
         shared = gate = None
         if self.Fs:
@@ -225,7 +225,7 @@ class RoutedMoE(FeedForward):
         row_token, pair_row, tile_expert = ops.expert_plan(None, ids, self.E, ctx.err, identity=self.ident)
         gu = ops.grouped_linear(h, self.w_gu, tile_expert, torch.float32, ctx.err, row_src=row_token, live=pair_row.numel())
         if self.gated:
-            act = ops.clamped_glu(gu, self.F, float("inf"), 1.0, 0.0, self.env.dtype)       # silu(gate) * up
+            act = ops.clamped_glu(gu, self.F, float("inf"), 1.0, 0.0, self.env.dtype, rows=row_token)       # silu(gate) * up
         else:
             act = ops.activate(gu, self.activation, self.env.dtype, rows=row_token, live=ids.numel())
         y = ops.grouped_linear(act, self.w_down, tile_expert, torch.float32, ctx.err)
