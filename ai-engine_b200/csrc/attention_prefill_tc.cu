@@ -28,10 +28,12 @@
 //                      rescaled on few tiles; the final division by the running sum makes the
 //                      result the same softmax.
 // The extended form (EXT) of this kernel adds, for layers that want them: a window (key tiles before it are never
-// loaded, nor are pages that the window has passed), scores kept within +-cap by a tanh, probabilities that enter the
+// loaded, nor are pages that the window has passed) that may keep the first keys, a factor a head and a distance bias on
+// the scores, a sink in the denominator, a gate a token and head, scores kept within +-cap by a tanh, probabilities that enter the
 // product with the values as two bfloat16 terms (the rounded one over the first half of the scores' columns, what
 // rounding left over the second: 16 bits of mantissa), a sigmoid gate on every output element, and cache rows
-// [k | v] or, with the values being the keys, [k] of one plane.
+// [k | v] or, with the values being the keys, [k] of one plane.  A portion of 1,900 tokens after 1,000 and a prompt of 148,
+// 16 heads of 128, window 1,024 with four kept keys, bias, sink and gates: 83 us (mma.sync kernel: 183 us).
 // The value rows of keys past the sequence's last token are zeroed in shared memory before the
 // last tile's P . V, so a probability of 0 never meets what an unwritten cache slot holds.
 // The softmax warps hand a tile's probabilities to the issuing warp at a named hardware barrier (bar.arrive /
@@ -69,6 +71,11 @@ struct AtExt {
     float cap;                    // 0: scores are not bounded
     const float* gate_logits;     // [T, >= H * HD] float32, rows ld_gate apart, or null
     int ld_gate;
+    int keep_first;               // with a window: the first keys that every query reads
+    const float* gate;            // [T, H] a factor a token and head, or null
+    const float* temp;            // [H] factor of the scores, or null
+    const float* slope;           // [H] slope * (i - j) is taken off the scores, or null
+    const float* sink;            // [H] exp(sink) joins the denominator, or null
 };
 
 // tanh(z) for |z| <= 1 as an odd polynomial of degree 15, two at a time (z2 = z^2 and z as packed pairs); the
@@ -182,7 +189,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     // first key that any row reads, and the tile it lies in; tile j of the loops below is key tile kt0 + j
     const int lo_min = EXT && ext.window > 0 ? max(p0 - ext.window + 1, 0) : 0;
     const int kt0 = lo_min / AT_N;
-    const int n_kt = p_last / AT_N + 1 - kt0;          // key tiles
+    // tiles of kept first keys that lie before the window's come first
+    const int n_kept = EXT && ext.window > 0 ? min((ext.keep_first + AT_N - 1) / AT_N, kt0) : 0;
+    const int n_kt = n_kept + p_last / AT_N + 1 - kt0;          // key tiles
+    auto tile_of = [&](int j) { return EXT && j < n_kept ? j : kt0 + j - n_kept; };
     const int ppt = AT_N / P;                          // pages per key tile
 
     if (tid == 0) {
@@ -224,30 +234,23 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // the next tile's page is read while this tile's boxes are issued
         const int* bt = block_table + (size_t)r * bt_width;
         const int lp = 31 - __clz(P);                      // P is a power of two
+        // pages that lie wholly before the window and hold no kept key may be gone: they are not loaded
+        const int first_page = lo_min >> lp;
+        auto gone = [&](int pidx) { return EXT && pidx < first_page && (pidx << lp) >= ext.keep_first; };
         auto page_of = [&](int jj) {
-            const int pidx = (kt0 + jj) * ppt + lane;
-            return (lane < ppt && (pidx << lp) <= p_last && pidx < bt_width) ? bt[pidx] : -1;
+            const int pidx = tile_of(jj) * ppt + lane;
+            return (lane < ppt && (pidx << lp) <= p_last && pidx < bt_width && !gone(pidx)) ? bt[pidx] : -1;
         };
         int page = page_of(0);
         bool ok = true;
-        // pages of the first tile that lie wholly before the window: they may be gone, so they are not loaded, and
-        // their value rows are zeroed before the tile's barrier is armed
-        const int skip = EXT ? (lo_min >> lp) - kt0 * ppt : 0;
-        if (EXT && skip > 0) {
-            for (int i = lane; i < skip * P * HV * 8; i += 32) {
-                const int row = i / (HV * 8), c = i % (HV * 8);
-                *reinterpret_cast<uint4*>(v_s + (row >> 3) * GROUP + (c >> 3) * 1024 + (row & 7) * 128 + (c & 7) * 16) =
-                    make_uint4(0, 0, 0, 0);
-            }
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            __syncwarp();
-        }
         for (int j = 0; j < n_kt && ok; ++j) {
             const int st = j % NST;
             const int page_next = j + 1 < n_kt ? page_of(j + 1) : -1;
-            const int n_pages = min(ppt, ((p_last - (kt0 + j) * AT_N) >> lp) + 1);      // pages of this tile that hold keys
-            const int from = EXT && j == 0 ? skip : 0;
-            const bool have = lane >= from && lane < n_pages;
+            const int n_pages = min(ppt, ((p_last - tile_of(j) * AT_N) >> lp) + 1);      // pages of this tile that hold keys
+            const bool lost = lane < n_pages && gone(tile_of(j) * ppt + lane);
+            const bool have = lane < n_pages && !lost;
+            unsigned missing = EXT ? __ballot_sync(0xffffffffu, lost) : 0u;
+            const int n_lost = __popc(missing);
             const bool valid = have && page >= 0 && page < num_pages;
             if (have && !valid) atomicOr(err, AIE_DEV_PAGE_OOB);
             // a missing page is flagged; page 0 stands in for it so that the byte count of the barrier holds
@@ -256,10 +259,26 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             if (lane == 0) {
                 const unsigned ph = ((j / NST) & 1) ^ 1;
                 ok = mbar_wait(&k_empty[st], ph, abort_flag, err) && mbar_wait(&v_empty[st], ph, abort_flag, err);
-                if (ok) mbar_expect_tx(&kv_full[st], 2u * (unsigned)(n_pages - from) * (unsigned)P * (unsigned)(HD * 2));
+                if (ok && !missing) mbar_expect_tx(&kv_full[st], 2u * (unsigned)n_pages * (unsigned)P * (unsigned)(HD * 2));
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
+            if (EXT && missing) {
+                // the value rows of pages that are not loaded are zeroed before the tile's barrier is armed (their
+                // scores are masked, whatever the keys' places hold)
+                for (; missing; missing &= missing - 1) {
+                    const int r0 = (__ffs(missing) - 1) * P;
+                    for (int i = lane; i < P * HV * 8; i += 32) {
+                        const int row = r0 + i / (HV * 8), c = i % (HV * 8);
+                        *reinterpret_cast<uint4*>(v_s + st * TILE + (row >> 3) * GROUP + (c >> 3) * 1024 + (row & 7) * 128 + (c & 7) * 16) =
+                            make_uint4(0, 0, 0, 0);
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_expect_tx(&kv_full[st], 2u * (unsigned)(n_pages - n_lost) * (unsigned)P * (unsigned)(HD * 2));
+                __syncwarp();
+            }
             if (have) {
                 tma_load_4d(k_s + st * TILE + lane * P * (HD * 2), &map_k, &kv_full[st], 0, 0, 0, group0);
                 tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &kv_full[st], 0, 0, 0, group0);
@@ -271,7 +290,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // the last tile: zero the value rows of keys past the sequence's end (whole warp)
         {
             const int j = n_kt - 1, st = j % NST;
-            const int first_bad = p_last + 1 - (kt0 + j) * AT_N;       // rows [first_bad, 128) are not keys
+            const int first_bad = p_last + 1 - tile_of(j) * AT_N;       // rows [first_bad, 128) are not keys
             bool ok2 = true;
             if (first_bad < AT_N) {
                 if (lane == 0) ok2 = mbar_wait(&kv_full[st], (j / NST) & 1, abort_flag, err);
@@ -368,8 +387,12 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const unsigned tmem_o = tmem_base + 256u;
         const float log2e = 1.4426950408889634f;
         const bool capped = EXT && ext.cap > 0.f;
-        const float sl2 = capped ? ext.cap * log2e : scale * log2e;      // scores in units of log2(e): exp2 below
-        const float z_of = capped ? scale / ext.cap : 0.f;
+        const float scale_h = EXT && ext.temp ? scale * ext.temp[h] : scale;
+        const float sl2 = capped ? ext.cap * log2e : scale_h * log2e;      // scores in units of log2(e): exp2 below
+        const float z_of = capped ? scale_h / ext.cap : 0.f, z_abs = fabsf(z_of);
+        // with a bias or a factor of its own, a head's scores are brought to those units before their maximum is taken
+        const bool shaped = EXT && (ext.slope || ext.temp);
+        const float slope2 = EXT && ext.slope ? ext.slope[h] * log2e : 0.f, sl2_e = shaped ? 1.f : sl2;
         const int low = EXT && ext.window > 0 ? qpos - ext.window + 1 : 0;      // first key this row reads
         const int low_last = EXT && ext.window > 0 ? p_last - ext.window + 1 : 0;
         float m_run = -INFINITY, l_run = 0.f;
@@ -387,7 +410,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 continue;
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const int kbase = (kt0 + j) * AT_N;
+            const int kbase = tile_of(j) * AT_N;
             const bool edge = kbase + AT_N - 1 > p0;     // the tile touches the diagonal or the sequence's end
             // the row of scores in registers (all four loads in flight at once), masked; its maximum
             unsigned sv[128];
@@ -402,7 +425,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
                 for (int i = 0; i < 128; i += 2)
                     big = at_max3(big, fabsf(__uint_as_float(sv[i])), fabsf(__uint_as_float(sv[i + 1])));
-                if (__all_sync(0xffffffffu, big * z_of <= 1.f)) {
+                if (__all_sync(0xffffffffu, big * z_abs <= 1.f)) {
                     constexpr float tc[8] = AT_TANH_COEFS;
                     const unsigned long long zz = at_pack2(z_of, z_of);
 #pragma unroll
@@ -427,6 +450,18 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                     }
                 }
             }
+            if (shaped) {
+                const unsigned long long off2 = at_pack2((float)(kbase - qpos), (float)(kbase - qpos));
+                const unsigned long long m2 = at_pack2(sl2, sl2), b2 = at_pack2(slope2, slope2);
+#pragma unroll
+                for (int i = 0; i < 128; i += 2) {
+                    unsigned long long dist;            // j - i, exact
+                    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(dist) : "l"(off2), "l"(at_pack2((float)i, (float)(i + 1))));
+                    const unsigned long long x = at_fma2(at_pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), m2, at_mul2(dist, b2));
+                    sv[i] = __float_as_uint(at_lo(x));
+                    sv[i + 1] = __float_as_uint(at_hi(x));
+                }
+            }
             if (edge) {
 #pragma unroll
                 for (int i = 0; i < 128; ++i)
@@ -435,7 +470,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             if (EXT && kbase < low_last) {
 #pragma unroll
                 for (int i = 0; i < 128; ++i)
-                    if (kbase + i < low) sv[i] = 0xff800000u;
+                    if (kbase + i < low && kbase + i >= ext.keep_first) sv[i] = 0xff800000u;
             }
             float tmax = -INFINITY, tmax2 = -INFINITY;
 #pragma unroll
@@ -443,7 +478,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 tmax = at_max3(tmax, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
                 tmax2 = at_max3(tmax2, __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]));
             }
-            tmax = fmaxf(tmax, tmax2) * sl2;
+            tmax = fmaxf(tmax, tmax2) * sl2_e;
             // the row's reference maximum moves only by more than AT_RESCALE_STEP
             float m_new = m_run, corr = 1.0f;
             if (tmax > m_run + AT_RESCALE_STEP) {
@@ -473,7 +508,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             }
             // probabilities exp2(s * sl2 - m), their sum, packed to bf16 and written over the scores, 32 columns
             // at a time: two keys to a column, so the P of columns [32 c, 32 c + 32) lands on [16 c, 16 c + 16)
-            const unsigned long long sl2_2 = at_pack2(sl2, sl2), negm_2 = at_pack2(-m_use, -m_use);
+            const unsigned long long sl2_2 = at_pack2(sl2_e, sl2_e), negm_2 = at_pack2(-m_use, -m_use);
             unsigned long long psum2 = 0ull, psum2b = 0ull;
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
@@ -511,7 +546,9 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         if (ok) {
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+            if (EXT && ext.sink) l_run += exp2f(ext.sink[h] * log2e - m_run);
+            float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+            if (EXT && ext.gate && row < rows_valid) inv *= ext.gate[(size_t)(t0 + row) * H + h];
             bf16* dst = out + ((size_t)(t0 + row) * H + h) * HD;
 #pragma unroll
             for (int c0 = 0; c0 < HD; c0 += 32) {
@@ -1039,19 +1076,21 @@ extern "C" int aie_paged_attention_prefill_tc(const void* q, const void* k_pages
 
 // The extended form (see the head of this file) over pages [num_pages, K, P, 2 d] of rows [k | v], or with `tied`
 // [num_pages, K, P, d] of rows that are key and value at once.  window 0: every earlier key; cap 0: unbounded scores;
-// gate_logits [T, >= H d] float32 with rows ld_gate apart, or null.  Same sizes as above.
+// gate_logits [T, >= H d] float32 with rows ld_gate apart, gate [T, H], temp, slope and sink [H] float32: see AtExt, each
+// may be null.  Same sizes as above.
 extern "C" int aie_paged_attention_prefill_tc_rows(const void* q, const void* pages, void* out, const int* tiles,
                                                    int n_tiles, const int* q_start, const int* q_len, const int* ctx_len,
                                                    const int* block_table, int bt_width, int num_pages, int P, int T,
                                                    int H, int K, int d, int window, int tied, float cap,
-                                                   const float* gate_logits, int ld_gate, float scale, unsigned* err,
-                                                   cudaStream_t stream) {
+                                                   const float* gate_logits, int ld_gate, int keep_first, const float* gate,
+                                                   const float* temp, const float* slope, const float* sink, float scale,
+                                                   unsigned* err, cudaStream_t stream) {
     if (n_tiles <= 0) return 0;
-    if (K <= 0 || H % K || window < 0 || cap < 0.f) return AIE_BAD_ARG;
+    if (K <= 0 || H % K || window < 0 || cap < 0.f || keep_first < 0) return AIE_BAD_ARG;
     if ((d != 64 && d != 128) || P < 8 || P > 128 || 128 % P || n_tiles > 65535) return AIE_UNSUPPORTED;
     if (((size_t)q & 15) || ((size_t)pages & 15) || ((size_t)out & 15)) return AIE_UNSUPPORTED;
     if (gate_logits && (((size_t)gate_logits & 15) || ld_gate % 4)) return AIE_UNSUPPORTED;
-    const AtExt ext{window, cap, gate_logits, ld_gate};
+    const AtExt ext{window, cap, gate_logits, ld_gate, keep_first, gate, temp, slope, sink};
 #define ARGS q, pages, out, tiles, n_tiles, q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, T, H, K, tied, \
              scale, ext, err, stream
     return d == 128 ? launch_prefill_tc_rows<128>(ARGS) : launch_prefill_tc_rows<64>(ARGS);
