@@ -167,14 +167,17 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     unsigned long long* p_ready = s_full + 2;
     unsigned long long* o_done = p_ready + 1;
     unsigned long long* v_fixed = o_done + 1;
-    unsigned* tmem_slot = reinterpret_cast<unsigned*>(v_fixed + 1);
+    unsigned long long* o_last = v_fixed + 1;      // the last P . V; o_done, which every tile's P . V completes, does not
+                                                   // tell it from the one before the last: a softmax warp that is a tile ahead
+                                                   // may come here while that one is still to be issued
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_last + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    constexpr int HV = HD / 64;                    // halves of 64 columns
-    constexpr int TILE = AtSmem<HD>::tile;         // bytes of a 128-row tile
-    constexpr int GROUP = HV * 1024;               // bytes of 8 rows (all halves) of a key or value tile
-    unsigned char* q_s = sm + AtSmem<HD>::q_off;
-    unsigned char* k_s = sm + AtSmem<HD>::k_off;   // stage st at + st * TILE
-    unsigned char* v_s = sm + AtSmem<HD>::v_off;
+    constexpr int HV = HD / 64, HK = HQ / 64;      // halves of 64 columns of values, of queries and keys
+    constexpr int KTILE = AtSmem<HD, HQ>::tile, TILE = AtSmem<HD, HQ>::v_tile;      // bytes of a 128-row tile of keys, of values
+    constexpr int KGROUP = HK * 1024, GROUP = HV * 1024;      // bytes of 8 rows (all halves) of a key tile, of a value tile
+    unsigned char* q_s = sm + AtSmem<HD, HQ>::q_off;
+    unsigned char* k_s = sm + AtSmem<HD, HQ>::k_off;   // stage st at + st * KTILE
+    unsigned char* v_s = sm + AtSmem<HD, HQ>::v_off;   // ... + st * TILE
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // later tiles hold more keys: start them first, for all heads (heads run fastest in the grid, so the heads
@@ -206,6 +209,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         mbar_init(&s_full[1], 1);
         mbar_init(o_done, 1);
         mbar_init(v_fixed, 1);
+        mbar_init(o_last, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -375,7 +379,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                                     dv + (unsigned long long)((ks * 2 * GROUP) >> 4), idesc_o, 1u);
                 }
                 umma_commit(&v_empty[st0]);
-                umma_commit(o_done);
+                umma_commit(j == n_kt - 1 ? o_last : o_done);
             }
         }
     } else {
@@ -541,7 +545,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         }
         // the last P . V, then this row of O divided by the row's sum
         if (ok) {
-            if (lane == 0) ok = mbar_wait(o_done, (n_kt - 1) & 1, abort_flag, err);
+            if (lane == 0) ok = mbar_wait(o_last, 0, abort_flag, err);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         }
         if (ok) {
