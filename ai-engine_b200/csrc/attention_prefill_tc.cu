@@ -172,12 +172,12 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                                                    // may come here while that one is still to be issued
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_last + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    constexpr int HV = HD / 64, HK = HQ / 64;      // halves of 64 columns of values, of queries and keys
-    constexpr int KTILE = AtSmem<HD, HQ>::tile, TILE = AtSmem<HD, HQ>::v_tile;      // bytes of a 128-row tile of keys, of values
-    constexpr int KGROUP = HK * 1024, GROUP = HV * 1024;      // bytes of 8 rows (all halves) of a key tile, of a value tile
-    unsigned char* q_s = sm + AtSmem<HD, HQ>::q_off;
-    unsigned char* k_s = sm + AtSmem<HD, HQ>::k_off;   // stage st at + st * KTILE
-    unsigned char* v_s = sm + AtSmem<HD, HQ>::v_off;   // ... + st * TILE
+    constexpr int HV = HD / 64;                    // halves of 64 columns
+    constexpr int TILE = AtSmem<HD>::tile;         // bytes of a 128-row tile
+    constexpr int GROUP = HV * 1024;               // bytes of 8 rows (all halves) of a key or value tile
+    unsigned char* q_s = sm + AtSmem<HD>::q_off;
+    unsigned char* k_s = sm + AtSmem<HD>::k_off;   // stage st at + st * TILE
+    unsigned char* v_s = sm + AtSmem<HD>::v_off;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // later tiles hold more keys: start them first, for all heads (heads run fastest in the grid, so the heads
