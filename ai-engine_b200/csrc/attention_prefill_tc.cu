@@ -54,14 +54,14 @@
 #define AT_RESCALE_STEP 8.0f     // a row's reference maximum moves in steps of more than this (log2 units)
 
 // HD: head size, HD / 64 halves of 64 columns.  A tile of 128 keys (or queries) holds 16 KB per half.
-template <int HD> struct AtSmem {
-    static constexpr int HV = HD / 64;
-    static constexpr int tile = HV * AT_HALF_BYTES;
+// HQ: elements of queries and keys (HD those of values) when they differ.
+template <int HD, int HQ = HD> struct AtSmem {
+    static constexpr int tile = HQ / 64 * AT_HALF_BYTES, v_tile = HD / 64 * AT_HALF_BYTES;
     // [alignment slack | 1 KB: barriers | Q | K x NST | V x NST]
     // rings of NST key tiles and NST value tiles: as deep as 227 KB allow (3 at head size 128), because a
     // tile is requested when its buffer is freed and a ring of two leaves the products waiting for loads
-    static constexpr int NST = HD >= 128 ? 3 : 4;
-    static constexpr int q_off = 1024, k_off = q_off + tile, v_off = k_off + NST * tile, end = v_off + NST * tile;
+    static constexpr int NST = HQ > 128 ? 2 : (HD >= 128 ? 3 : 4);
+    static constexpr int q_off = 1024, k_off = q_off + tile, v_off = k_off + NST * tile, end = v_off + NST * v_tile;
     static constexpr int bytes = 1024 + end;
 };
 
@@ -76,6 +76,10 @@ struct AtExt {
     const float* temp;            // [H] factor of the scores, or null
     const float* slope;           // [H] slope * (i - j) is taken off the scores, or null
     const float* sink;            // [H] exp(sink) joins the denominator, or null
+    // > 0: keys and values are not in pages but in rows of their own, [key (HQ) | value (HD)] of every head side by side, a
+    // request's rows from the tile of 128 keys on that its window begins in, requests that bring this many tokens or more
+    // one behind the other
+    int min_len;
 };
 
 // tanh(z) for |z| <= 1 as an odd polynomial of degree 15, two at a time (z2 = z^2 and z as packed pairs); the
@@ -148,7 +152,7 @@ __device__ __forceinline__ float at_hi(unsigned long long v) {
                    "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),   \
                    "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory")
 
-template <int HD, bool EXT>
+template <int HD, bool EXT, int HQ = HD>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out,
@@ -159,7 +163,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     extern __shared__ unsigned char at_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((size_t)at_raw + 1023) & ~(size_t)1023);
     unsigned long long* q_full = reinterpret_cast<unsigned long long*>(sm);
-    constexpr int NST = AtSmem<HD>::NST;           // stages of the key ring and of the value ring
+    constexpr int NST = AtSmem<HD, HQ>::NST;           // stages of the key ring and of the value ring
     unsigned long long* kv_full = q_full + 1;      // [NST] keys and values of a tile have landed
     unsigned long long* k_empty = kv_full + NST;   // [NST] the scores have read the keys
     unsigned long long* v_empty = k_empty + NST;   // [NST] P . V has read the values
@@ -172,12 +176,12 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                                                    // may come here while that one is still to be issued
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_last + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    constexpr int HV = HD / 64;                    // halves of 64 columns
-    constexpr int TILE = AtSmem<HD>::tile;         // bytes of a 128-row tile
-    constexpr int GROUP = HV * 1024;               // bytes of 8 rows (all halves) of a key or value tile
-    unsigned char* q_s = sm + AtSmem<HD>::q_off;
-    unsigned char* k_s = sm + AtSmem<HD>::k_off;   // stage st at + st * TILE
-    unsigned char* v_s = sm + AtSmem<HD>::v_off;
+    constexpr int HV = HD / 64, HK = HQ / 64;      // halves of 64 columns of values, of queries and keys
+    constexpr int KTILE = AtSmem<HD, HQ>::tile, TILE = AtSmem<HD, HQ>::v_tile;      // bytes of a 128-row tile of keys, of values
+    constexpr int KGROUP = HK * 1024, GROUP = HV * 1024;      // bytes of 8 rows (all halves) of a key tile, of a value tile
+    unsigned char* q_s = sm + AtSmem<HD, HQ>::q_off;
+    unsigned char* k_s = sm + AtSmem<HD, HQ>::k_off;   // stage st at + st * KTILE
+    unsigned char* v_s = sm + AtSmem<HD, HQ>::v_off;   // ... + st * TILE
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // later tiles hold more keys: start them first, for all heads (heads run fastest in the grid, so the heads
@@ -231,8 +235,8 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (warp == 0) {
             if (lane == 0) {
             // queries of this tile: rows t0 .. t0 + 127 of q [T, H * 128], columns of head h
-            mbar_expect_tx(q_full, TILE);
-            for (int hv = 0; hv < HV; ++hv) tma_load_2d(q_s + hv * AT_HALF_BYTES, &map_q, q_full, h * HD + hv * 64, t0);
+            mbar_expect_tx(q_full, KTILE);
+            for (int hv = 0; hv < HK; ++hv) tma_load_2d(q_s + hv * AT_HALF_BYTES, &map_q, q_full, h * HQ + hv * 64, t0);
         }
         // lane i owns page i of every key tile: one box per page (all 128 columns of its P keys); the id of
         // the next tile's page is read while this tile's boxes are issued
@@ -241,8 +245,21 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // pages that lie wholly before the window and hold no kept key may be gone: they are not loaded
         const int first_page = lo_min >> lp;
         auto gone = [&](int pidx) { return EXT && pidx < first_page && (pidx << lp) >= ext.keep_first; };
+        const bool in_rows = EXT && ext.min_len > 0;
+        const int blk_k = in_rows ? h * (HK + HV) : 0, blk_v = in_rows ? blk_k + HK : 0;
+        int row_page = 0;                                  // rows instead of pages: the request's first tile of 128
+        if (in_rows) {
+            for (int i = lane; i < r; i += 32)
+                if (q_len[i] >= ext.min_len) {
+                    const int lo = ext.window > 0 ? max(ctx_len[i] - ext.window + 1, 0) : 0;
+                    row_page += (ctx_len[i] + q_len[i] - 1) / AT_N - lo / AT_N + 1;
+                }
+            row_page = __reduce_add_sync(0xffffffffu, row_page);
+            row_page -= (ext.window > 0 ? max(ctx_len[r] - ext.window + 1, 0) : 0) / AT_N;
+        }
         auto page_of = [&](int jj) {
             const int pidx = tile_of(jj) * ppt + lane;
+            if (in_rows) return lane == 0 ? row_page + pidx : -1;
             return (lane < ppt && (pidx << lp) <= p_last && pidx < bt_width && !gone(pidx)) ? bt[pidx] : -1;
         };
         int page = page_of(0);
@@ -263,7 +280,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             if (lane == 0) {
                 const unsigned ph = ((j / NST) & 1) ^ 1;
                 ok = mbar_wait(&k_empty[st], ph, abort_flag, err) && mbar_wait(&v_empty[st], ph, abort_flag, err);
-                if (ok && !missing) mbar_expect_tx(&kv_full[st], 2u * (unsigned)n_pages * (unsigned)P * (unsigned)(HD * 2));
+                if (ok && !missing) mbar_expect_tx(&kv_full[st], (unsigned)n_pages * (unsigned)P * (unsigned)((HQ + HD) * 2));
             }
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
@@ -280,12 +297,12 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 }
                 asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                 __syncwarp();
-                if (lane == 0) mbar_expect_tx(&kv_full[st], 2u * (unsigned)(n_pages - n_lost) * (unsigned)P * (unsigned)(HD * 2));
+                if (lane == 0) mbar_expect_tx(&kv_full[st], (unsigned)(n_pages - n_lost) * (unsigned)P * (unsigned)((HQ + HD) * 2));
                 __syncwarp();
             }
             if (have) {
-                tma_load_4d(k_s + st * TILE + lane * P * (HD * 2), &map_k, &kv_full[st], 0, 0, 0, group0);
-                tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &kv_full[st], 0, 0, 0, group0);
+                tma_load_4d(k_s + st * KTILE + lane * P * (HQ * 2), &map_k, &kv_full[st], 0, 0, blk_k, group0);
+                tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &kv_full[st], 0, 0, blk_v, group0);
             }
             __syncwarp();
             page = page_next;
@@ -319,13 +336,13 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             const unsigned idesc_s = umma_idesc(AT_N), idesc_o = umma_idesc(HD, true);
             // descriptors of the first step of each operand, built once; a step or a stage further along is an
             // addition to the descriptor's address field (bytes / 16)
-            const unsigned long long dq0 = umma_desc(q_s), dk0 = umma_desc(k_s, GROUP), dv0 = umma_desc_mn(v_s, 1024, GROUP);
+            const unsigned long long dq0 = umma_desc(q_s), dk0 = umma_desc(k_s, KGROUP), dv0 = umma_desc_mn(v_s, 1024, GROUP);
             // S(j) = Q . K(j)^T over the head size into score buffer j & 1: steps of 16; keys from stage `st`
             auto issue_scores = [&](int j, int st) {
-                const unsigned long long dk = dk0 + (unsigned long long)((st * TILE) >> 4);
+                const unsigned long long dk = dk0 + (unsigned long long)((st * KTILE) >> 4);
                 const unsigned ts = tmem_base + (unsigned)((j & 1) * AT_N);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)
+                for (int ks = 0; ks < HQ / 16; ++ks)
                     umma(ts, dq0 + (unsigned long long)((((ks >> 2) * AT_HALF_BYTES) >> 4) + 2 * (ks & 3)),
                          dk + (unsigned long long)((((ks >> 2) * 1024) >> 4) + 2 * (ks & 3)), idesc_s, ks > 0 ? 1u : 0u);
                 umma_commit(&k_empty[st]);
@@ -1094,11 +1111,45 @@ extern "C" int aie_paged_attention_prefill_tc_rows(const void* q, const void* pa
     if ((d != 64 && d != 128) || P < 8 || P > 128 || 128 % P || n_tiles > 65535) return AIE_UNSUPPORTED;
     if (((size_t)q & 15) || ((size_t)pages & 15) || ((size_t)out & 15)) return AIE_UNSUPPORTED;
     if (gate_logits && (((size_t)gate_logits & 15) || ld_gate % 4)) return AIE_UNSUPPORTED;
-    const AtExt ext{window, cap, gate_logits, ld_gate, keep_first, gate, temp, slope, sink};
+    const AtExt ext{window, cap, gate_logits, ld_gate, keep_first, gate, temp, slope, sink, 0};
 #define ARGS q, pages, out, tiles, n_tiles, q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, T, H, K, tied, \
              scale, ext, err, stream
     return d == 128 ? launch_prefill_tc_rows<128>(ARGS) : launch_prefill_tc_rows<64>(ARGS);
 #undef ARGS
+}
+
+// Keys of 192 and values of 128 elements out of rows [rows][H][192 | 128] bf16 (see AtExt::min_len; rows a multiple of 128)
+// instead of pages; q [T, H, 192], out [T, H, 128].  tiles name requests that bring min_len tokens or more.
+extern "C" int aie_prefill_tc_expanded(const void* q, const void* rows_kv, long long rows, void* out, const int* tiles, int n_tiles,
+                                       const int* q_start, const int* q_len, const int* ctx_len, int T, int H, int window,
+                                       int min_len, const float* sink, float scale, unsigned* err, cudaStream_t stream) {
+    if (n_tiles <= 0) return 0;
+    if (H <= 0 || window < 0 || min_len < 1 || rows % AT_N || rows / AT_N > 0x7fffffffLL / AT_N) return AIE_BAD_ARG;
+    if (n_tiles > 65535 || (((size_t)q | (size_t)rows_kv | (size_t)out) & 15)) return AIE_UNSUPPORTED;
+    constexpr int HD = 128, HQ = 192, BLOCKS = (HD + HQ) / 64;
+    TcEncodeTiledFn fn = tc_encode_fn();
+    if (!fn) return AIE_UNSUPPORTED;
+    CUtensorMap mq, mk, mv;
+    int rc = tc_make_map_2d(&mq, q, (unsigned long long)T, (unsigned long long)H * HQ, (unsigned long long)H * HQ * 2, AT_M, 64);
+    if (rc) return rc;
+    // [groups of 8 rows][blocks of 64 columns of all heads][8 rows][64]: a box takes a head's key blocks, or its value blocks
+    const cuuint64_t row_bytes = (cuuint64_t)H * BLOCKS * 128;
+    const cuuint64_t dims[4] = {64, 8, (cuuint64_t)H * BLOCKS, (cuuint64_t)(rows / 8)}, strides[3] = {row_bytes, 128, row_bytes * 8};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    for (int v = 0; v < 2; ++v) {
+        const cuuint32_t box[4] = {64, 8, (cuuint32_t)((v ? HD : HQ) / 64), AT_N / 8};
+        if (fn(v ? &mv : &mk, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(rows_kv), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return AIE_UNSUPPORTED;
+    }
+    const AtExt ext{window, 0.f, nullptr, 0, 0, nullptr, nullptr, nullptr, sink, min_len};
+    auto kern = paged_prefill_tc_kernel<HD, true, HQ>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AtSmem<HD, HQ>::bytes);
+    if (e != cudaSuccess) return (int)e;
+    launch_pdl(kern, dim3(H, n_tiles), dim3(AT_THREADS), AtSmem<HD, HQ>::bytes, stream, mq, mk, mv, (bf16*)out, tiles, n_tiles,
+               q_start, q_len, ctx_len, (const int*)nullptr, 0, (int)(rows / AT_N), AT_N, H, 1, scale, err, ext);
+    AIE_LAUNCH_CHECK();
 }
 
 // The same with two query tiles per CTA.  units: [n_units][2] = (request row, offset of the 256-token unit

@@ -5,8 +5,9 @@
 // kernel reads the cache rows as they are: score_j = (qa . c_j + q_rot . kr_j) * scale, one "kv head" for all
 // query heads.
 //
-// latent_prepare: from the fused projection [q heads | c | kr] of the step's tokens it writes the plain
-//   query parts (compute dtype, for the folding product), the rotated query parts (float32), and the
+// latent_prepare (q_plain with q_full, and q_all, may be left out: null): from the fused projection [q heads | c | kr] of the step's tokens it writes the plain
+//   query parts (compute dtype, for the folding product), the rotated query parts (float32), in q_all both parts side by
+//   side (compute dtype, for queries that meet expanded keys), and the
 //   normalised c and rotated kr into the token's cache row.  The rotation pairs element 2i with 2i+1 over the
 //   first `rot_dims` elements of the rot-wide part (or, with `halves`, element i with i + rot_dims / 2); the
 //   angle is float(position) * inv_freq[i] in float32, and cosine and sine are multiplied by `mag`.  The latent and the key part may come from a projection
@@ -19,22 +20,22 @@
 #define LAT_CHUNK 128
 #define LAT_PREP 128       // threads that share the sum over a latent
 
-// element i of a rot-wide vector x after the rotation by `pos`
-__device__ __forceinline__ float latent_rotated(const float* x, int i, int half, int halves, int pos,
-                                                const float* __restrict__ inv_freq, float mag) {
-    if (i >= 2 * half) return x[i];
+#define LAT_ANGLES 128     // angles a token that fit the table below (a rotation over up to 256 elements)
+
+__device__ __forceinline__ float2 latent_angle(int pos, float freq, float mag) {
     float sn, cs;
-    if (halves) {
-        const int j = i < half ? i : i - half;
-        sincosf((float)pos * inv_freq[j], &sn, &cs);
-        sn *= mag;
-        cs *= mag;
-        return i < half ? x[i] * cs - x[i + half] * sn : x[i] * cs + x[j] * sn;
-    }
-    sincosf((float)pos * inv_freq[i >> 1], &sn, &cs);
-    sn *= mag;
-    cs *= mag;
-    return (i & 1) ? x[i] * cs + x[i - 1] * sn : x[i] * cs - x[i + 1] * sn;
+    sincosf((float)pos * freq, &sn, &cs);
+    return make_float2(cs * mag, sn * mag);
+}
+
+// element i of a rot-wide vector x after the rotation by `pos`; tab: the token's cosines and sines, or null
+__device__ __forceinline__ float latent_rotated(const float* x, int i, int half, int halves, int pos,
+                                                const float* __restrict__ inv_freq, float mag, const float2* tab) {
+    if (i >= 2 * half) return x[i];
+    const int j = halves ? (i < half ? i : i - half) : i >> 1;
+    const float2 a = tab ? tab[j] : latent_angle(pos, inv_freq[j], mag);
+    if (halves) return i < half ? x[i] * a.x - x[i + half] * a.y : x[i] * a.x + x[j] * a.y;
+    return (i & 1) ? x[i] * a.x + x[i - 1] * a.y : x[i] * a.x - x[i + 1] * a.y;
 }
 
 template <typename A, typename C>
@@ -44,23 +45,44 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int ld, in
                                       float* __restrict__ q_full, C* __restrict__ pages,
                                       const int* __restrict__ positions, const int* __restrict__ token_req,
                                       const int* __restrict__ block_table, int bt_width, int num_pages, int P,
-                                      unsigned* err, const float* __restrict__ kv, int ld_kv, int halves, float mag) {
+                                      unsigned* err, const float* __restrict__ kv, int ld_kv, int halves, float mag,
+                                      A* __restrict__ q_all) {
     __shared__ float red[32];
+    __shared__ float2 angles[LAT_ANGLES];              // made once a token, for all heads
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x, tid = threadIdx.x;
     const float* row = proj + (size_t)t * ld;
     const int pos = positions[t];
     const int dq = d + rot, dk = rank + rot, half = rot_dims / 2;
+    const float2* tab = half <= LAT_ANGLES ? angles : nullptr;
+    if (tab) {
+        for (int j = tid; j < half; j += blockDim.x) angles[j] = latent_angle(pos, inv_freq[j], mag);
+        __syncthreads();
+    }
     // queries: the plain part as it is, the rotated part turned by the position
-    for (int e = tid; e < H * d; e += blockDim.x) {
-        const int hh = e / d, i = e % d;
-        q_plain[((size_t)t * H + hh) * d + i] = from_f32<A>(row[hh * dq + i]);
+    const bool vec = ((d | rot | ld) & 3) == 0 && (((size_t)proj | (size_t)q_plain | (size_t)q_all) & 15) == 0;      // (rows of A: 4 elements)
+    if (vec) {
+        for (int e = tid * 4; e < H * d; e += blockDim.x * 4) {
+            const int hh = e / d, i = e % d;
+            const float4 v = *reinterpret_cast<const float4*>(row + hh * dq + i);
+            if (q_plain) store4<A>(q_plain + ((size_t)t * H + hh) * d + i, v);
+            if (q_all) store4<A>(q_all + ((size_t)t * H + hh) * dq + i, v);
+        }
+    } else {
+        for (int e = tid; e < H * d; e += blockDim.x) {
+            const int hh = e / d, i = e % d;
+            const A v = from_f32<A>(row[hh * dq + i]);
+            if (q_plain) q_plain[((size_t)t * H + hh) * d + i] = v;
+            if (q_all) q_all[((size_t)t * H + hh) * dq + i] = v;
+        }
     }
     for (int e = tid; e < H * rot; e += blockDim.x) {
         const int hh = e / rot, i = e % rot;
         const float* qr = row + hh * dq + d;
-        q_full[((size_t)t * H + hh) * dk + rank + i] = latent_rotated(qr, i, half, halves, pos, inv_freq, mag);
+        const float v = latent_rotated(qr, i, half, halves, pos, inv_freq, mag, tab);
+        if (q_full) q_full[((size_t)t * H + hh) * dk + rank + i] = v;
+        if (q_all) q_all[((size_t)t * H + hh) * dq + d + i] = from_f32<A>(v);
     }
     if (!has_kv) return;
     const float* z = kv ? kv + (size_t)t * ld_kv : row + H * dq;
@@ -78,21 +100,21 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int ld, in
     C* dst = pages + ((size_t)page * P + (pos - pidx * P)) * dk;
     for (int i = tid; i < rank; i += blockDim.x) dst[i] = from_f32<C>((z[i] * rinv) * c_weight[i]);
     const float* kr = z + rank;
-    for (int i = tid; i < rot; i += blockDim.x) dst[rank + i] = from_f32<C>(latent_rotated(kr, i, half, halves, pos, inv_freq, mag));
+    for (int i = tid; i < rot; i += blockDim.x) dst[rank + i] = from_f32<C>(latent_rotated(kr, i, half, halves, pos, inv_freq, mag, tab));
 }
 
 extern "C" int aie_latent_prepare(const float* proj, int ld, int T, int H, int d, int rot, int rank, int rot_dims,
                                   int has_kv, const float* c_weight, float eps, const float* inv_freq, void* q_plain,
                                   int q_dtype, float* q_full, void* pages, int cache_dtype, const int* positions,
                                   const int* token_req, const int* block_table, int bt_width, int num_pages, int P,
-                                  unsigned* err, const float* kv, int ld_kv, int halves, float mag, cudaStream_t st) {
+                                  unsigned* err, const float* kv, int ld_kv, int halves, float mag, void* q_all, cudaStream_t st) {
     if (T <= 0) return 0;
     if (rot_dims % 2 || rot_dims > rot || H <= 0 || d < 0 || rank <= 0) return AIE_BAD_ARG;
     const int threads = T <= 2 * aie_sm_count() ? 1024 : LAT_PREP;      // few tokens: a block has an SM to itself
 #define GO(A, C)                                                                                                      \
     launch_pdl(latent_prepare_kernel<A, C>, dim3(T), dim3(threads), 0, st, proj, ld, H, d, rot, rank, rot_dims, has_kv, c_weight, eps, inv_freq, \
                                                    (A*)q_plain, q_full, (C*)pages, positions, token_req, block_table,  \
-                                                   bt_width, num_pages, P, err, kv, ld_kv, halves, mag)
+                                                   bt_width, num_pages, P, err, kv, ld_kv, halves, mag, (A*)q_all)
     if (q_dtype == AIE_F32 && cache_dtype == AIE_F32) GO(float, float);
     else if (q_dtype == AIE_BF16 && cache_dtype == AIE_BF16) GO(bf16, bf16);
     else if (q_dtype == AIE_BF16 && cache_dtype == AIE_F32) GO(bf16, float);

@@ -28,7 +28,7 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
                            const int* __restrict__ q_start, const int* __restrict__ q_len,
                            const int* __restrict__ ctx_len, const int* __restrict__ block_table, int bt_width,
                            int num_pages, int P, int H, int dk, int window, float scale, int splits,
-                           const float* __restrict__ sink, unsigned* err) {
+                           const float* __restrict__ sink, int max_len, unsigned* err) {
     constexpr int RANK = 4 * CW, NT = CW / 8, THREADS = LT_THREADS * TQ;
     extern __shared__ __align__(16) unsigned char lt_raw[];
     const int SK = dk + 8;                                        // padded row: ldmatrix rows fall on different banks
@@ -44,6 +44,7 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
     pdl_launch_dependents();
     pdl_wait();
     const int row = tiles[2 * blockIdx.x], off = tiles[2 * blockIdx.x + 1];
+    if (max_len > 0 && q_len[row] > max_len) return;              // a longer portion meets expanded keys in another kernel
     const int h0 = blockIdx.y * LT_ROWS, part = blockIdx.z;
     const int tid = threadIdx.x, tq = tid / LT_THREADS, ltid = tid % LT_THREADS, warp = (tid >> 5) & 3, lane = tid & 31;
     const int n_act = min(TQ, q_len[row] - off);                  // tokens of this CTA that exist
@@ -290,7 +291,7 @@ extern "C" int aie_latent_attention_tc(const float* q_full, const void* pages, v
                                        const int* tiles, int n_tiles, int tq, const int* q_start, const int* q_len,
                                        const int* ctx_len, const int* block_table, int bt_width,
                                        int num_pages, int P, int T, int H, int rank, int dk, int window, float scale,
-                                       int splits, const float* sink, int pair, unsigned* err, cudaStream_t st) {
+                                       int splits, const float* sink, int pair, int max_len, unsigned* err, cudaStream_t st) {
     if (T <= 0 || n_tiles <= 0) return 0;
     if (rank < 64 || rank > 512 || rank % 64 || dk % 16 || dk < rank || dk > 1024 || H <= 0) return AIE_UNSUPPORTED;
     if (splits < 1 || splits > 64 || (splits > 1 && (!part_o || !part_ml)) || (tq != 1 && tq != 4)) return AIE_BAD_ARG;
@@ -306,7 +307,7 @@ extern "C" int aie_latent_attention_tc(const float* q_full, const void* pages, v
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
         launch_pdl(kern, grid, dim3(LT_THREADS * TQV), smem, st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, tiles,    \
                                                    q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, H,   \
-                                                   dk, window, scale, splits, sink, err);                                   \
+                                                   dk, window, scale, splits, sink, max_len, err);                                   \
     }
 #define GO1(CWV, TQV)                                                                                                 \
     if (pair) GO2(CWV, TQV, true) else GO2(CWV, TQV, false)
@@ -399,5 +400,73 @@ extern "C" int aie_head_linear_small(const void* x, long long xt, long long xh, 
     }
 #undef GO_O
 #undef GO
+    AIE_LAUNCH_CHECK();
+}
+
+// ---------------------------------------------------------------------------
+// The cached rows that prompts read, one behind the other: for every request that brings min_len tokens or more, its rows
+// from the tile of 128 keys on that its first token's window begins in, to the last tile; rows outside the window or behind
+// the last token are zeros.  A block copies 32 rows of a tile, 16 bytes a thread.
+#define LG_ROWS 32
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const bf16* __restrict__ pages, bf16* __restrict__ rows, const int* __restrict__ q_len,
+                     const int* __restrict__ ctx_len, const int* __restrict__ block_table, int bt_width, int num_pages, int P,
+                     int dk, int window, int min_len, int R, unsigned* err) {
+    __shared__ int found[2];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tile_i = blockIdx.x / (128 / LG_ROWS), sub = blockIdx.x % (128 / LG_ROWS), tid = threadIdx.x;
+    const auto low = [&](int r) { return window > 0 ? max(ctx_len[r] - window + 1, 0) : 0; };
+    if (tid < 32) {                                     // whose tile this is: requests in order, 32 at a time
+        int rr = -1, tile = 0, before = 0;
+        for (int base = 0; base < R && rr < 0; base += 32) {
+            const int r = base + tid;
+            const int m = r < R && q_len[r] >= min_len ? (ctx_len[r] + q_len[r] - 1) / 128 - low(r) / 128 + 1 : 0;
+            int run = m;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, run, o);
+                if (tid >= o) run += up;
+            }
+            const unsigned hit = __ballot_sync(0xffffffffu, tile_i < before + run);
+            if (hit) {
+                const int l = __ffs(hit) - 1;
+                rr = base + l;
+                tile = low(rr) / 128 + tile_i - before - __shfl_sync(0xffffffffu, run - m, l);
+            }
+            before += __shfl_sync(0xffffffffu, run, 31);
+        }
+        if (tid == 0) {
+            found[0] = rr;
+            found[1] = tile;
+        }
+    }
+    __syncthreads();
+    const int r = found[0];
+    if (r < 0) return;
+    const int key0 = found[1] * 128 + sub * LG_ROWS, lo = low(r), last = ctx_len[r] + q_len[r] - 1, pieces = dk / 8;
+    uint4* dst = reinterpret_cast<uint4*>(rows + ((size_t)tile_i * 128 + sub * LG_ROWS) * dk);
+    for (int i = tid; i < LG_ROWS * pieces; i += 256) {
+        const int key = key0 + i / pieces, c = i % pieces;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (key >= lo && key <= last) {
+            const int pidx = key / P, page = pidx < bt_width ? block_table[(size_t)r * bt_width + pidx] : -1;
+            if (page < 0 || page >= num_pages) {
+                if (c == 0) atomicOr(err, AIE_DEV_PAGE_OOB);
+            } else {
+                v = reinterpret_cast<const uint4*>(pages + ((size_t)page * P + (key - pidx * P)) * dk)[c];
+            }
+        }
+        dst[i] = v;
+    }
+}
+
+// pages [num_pages, P, dk] bf16, dk a multiple of 8; rows [n_tiles * 128, dk].
+extern "C" int aie_latent_gather(const void* pages, void* rows, int n_tiles, const int* q_len, const int* ctx_len,
+                                 const int* block_table, int bt_width, int num_pages, int P, int dk, int window, int min_len,
+                                 int R, unsigned* err, cudaStream_t st) {
+    if (n_tiles <= 0) return 0;
+    if (dk % 8 || P <= 0 || min_len < 1 || n_tiles > 0x1fffffff || (((size_t)pages | (size_t)rows) & 15)) return AIE_BAD_ARG;
+    launch_pdl(latent_gather_kernel, dim3((unsigned)n_tiles * (128 / LG_ROWS)), dim3(256), 0, st, (const bf16*)pages, (bf16*)rows, q_len,
+               ctx_len, block_table, bt_width, num_pages, P, dk, window, min_len, R, err);
     AIE_LAUNCH_CHECK();
 }

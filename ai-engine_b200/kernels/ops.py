@@ -894,13 +894,15 @@ def expert_combine(y: torch.Tensor, pair_row: torch.Tensor, top: int, weight: fl
 def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_weight: Optional[torch.Tensor],
                    eps: float, inv_freq: torch.Tensor, pages: torch.Tensor, ctx, block_table: torch.Tensor,
                    q_dtype: torch.dtype, write: bool, kv: Optional[torch.Tensor] = None, halves: bool = False,
-                   magnitude: float = 1.0):
+                   magnitude: float = 1.0, folded: bool = True, whole: bool = False):
     """From the fused projection [q heads (d plain | rot rotated) | latent (rank) | shared key part (rot)] of a
     step: (q_plain [T, H, d] in q_dtype, q_full [T, H, rank + rot] float32 whose last rot columns hold the
     rotated query parts); with `write`, the normalised latent and the rotated key part go into the tokens'
     cache rows.  pages [num_pages, 1, P, rank + rot].  kv: the latent and the key part come from this float32 view
     [T, >= rank + rot] (rows any stride) instead of the columns behind the queries.  halves: the rotation pairs
-    element i with i + rot_dims / 2 instead of 2i with 2i + 1.  magnitude: factor of all cosines and sines."""
+    element i with i + rot_dims / 2 instead of 2i with 2i + 1.  magnitude: factor of all cosines and sines.
+    folded False: (None, None) for the two; whole: a third result [T, H, d + rot] in q_dtype, a head's plain and rotated
+    parts side by side."""
     _dev(proj, c_weight, inv_freq, pages, block_table)
     T, ld = proj.shape
     need = H * (d + rot) + ((rank + rot) if write and kv is None else 0)
@@ -908,29 +910,77 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
         raise KernelError("latent_prepare: the latent projection is a float32 view [T, >= rank + rot]")
     if proj.dtype != torch.float32 or ld < need or pages.shape[1] != 1 or pages.shape[3] != rank + rot:
         raise KernelError("latent_prepare: shapes or dtypes do not fit")
-    q_plain = torch.empty((T, H, d), dtype=q_dtype, device=proj.device)
-    q_full = torch.empty((T, H, rank + rot), dtype=torch.float32, device=proj.device)
+    q_plain = torch.empty((T, H, d), dtype=q_dtype, device=proj.device) if folded else None
+    q_full = torch.empty((T, H, rank + rot), dtype=torch.float32, device=proj.device) if folded else None
+    q_all = torch.empty((T, H, d + rot), dtype=q_dtype, device=proj.device) if whole else None
     lib = library("latent_attention.cu")
-    with region("latent_prepare", _nb(proj, q_plain) + T * H * rot * 4):
+    with region("latent_prepare", _nb(proj, q_plain, q_all) + (T * H * rot * 4 if folded else 0)):
         check(lib.aie_latent_prepare(_p(proj), c_int(ld), c_int(T), c_int(H), c_int(d), c_int(rot), c_int(rank),
                                      c_int(2 * inv_freq.shape[0]), c_int(1 if write else 0), _p(c_weight),
-                                     c_float(eps), _p(inv_freq), _p(q_plain), c_int(dtype_code(q_plain)), _p(q_full),
+                                     c_float(eps), _p(inv_freq), _p(q_plain), c_int(dtype_code(q_dtype)), _p(q_full),
                                      _p(pages), c_int(dtype_code(pages)), _p(ctx.positions), _p(ctx.token_req),
                                      _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]),
                                      c_int(pages.shape[2]), _p(ctx.err), _p(kv), c_int(kv.stride(0) if kv is not None else 0),
-                                     c_int(1 if halves else 0), c_float(magnitude), _stream()), "latent_prepare")
-    return q_plain, q_full
+                                     c_int(1 if halves else 0), c_float(magnitude), _p(q_all), _stream()), "latent_prepare")
+    return (q_plain, q_full, q_all) if whole else (q_plain, q_full)
+
+
+# Portions from this length on meet their keys and values expanded: 10 tokens' worth of products a key make heads of 192 and
+# 128 out of a row of 576, and a (query, key) pair then costs 640 operations instead of 2,176.
+LATENT_EXPAND_TOKENS = 64
+LATENT_EXPAND_BYTES = 1 << 30      # the most that a step's expanded rows may take; beyond, rows are read as they are
+
+
+def latent_expanded_tiles(ctx, window: int) -> int:
+    """Tiles of 128 cache rows that the step's portions of LATENT_EXPAND_TOKENS tokens or more read under a window."""
+    n = ctx.h_q_len >= LATENT_EXPAND_TOKENS
+    c, q = ctx.h_ctx_len[n].astype(np.int64), ctx.h_q_len[n].astype(np.int64)
+    low = np.maximum(c - window + 1, 0) if window > 0 else np.zeros_like(c)
+    return int(((c + q - 1) // 128 - low // 128 + 1).sum())
+
+
+def latent_prompt(q: torch.Tensor, pages: torch.Tensor, w_expand: torch.Tensor, ctx, block_table: torch.Tensor, tiles: torch.Tensor,
+                  n_rows: int, scale: float, window: int, sink: Optional[torch.Tensor], out: torch.Tensor) -> None:
+    """Attention of the step's portions of LATENT_EXPAND_TOKENS tokens or more over cache rows that are first expanded:
+    rows gathered one behind the other, one product with w_expand [H * (192 + 128), dk] (a head's key, its shared rotated part
+    copied by ones, and its value), then the tcgen05 prompt kernel on heads of 192 and 128.  q [T, H, 192] bfloat16, tiles
+    [n, 2] of those portions, n_rows = 128 * latent_expanded_tiles; their rows of out [T, H, 128] are written."""
+    _dev(q, pages, w_expand, block_table, tiles, sink, out)
+    T, H, _ = q.shape
+    dk = pages.shape[3]
+    if (q.shape[2] != 192 or out.shape != (T, H, 128) or w_expand.shape != (H * 320, dk) or pages.shape[1] != 1
+            or any(t.dtype != torch.bfloat16 for t in (q, pages, w_expand, out))
+            or (sink is not None and (sink.dtype != torch.float32 or sink.shape != (H,)))):
+        raise KernelError("latent_prompt: shapes or dtypes do not fit")
+    rows = torch.empty((n_rows, dk), dtype=torch.bfloat16, device=q.device)
+    with region("latent_gather", 2 * _nb(rows)):
+        check(library("latent_attention_tc.cu").aie_latent_gather(
+            _p(pages), _p(rows), c_int(n_rows // 128), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
+            c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(dk), c_int(window), c_int(LATENT_EXPAND_TOKENS), c_int(ctx.R),
+            _p(ctx.err), _stream()), "latent_gather")
+    kv = linear(rows, w_expand, torch.bfloat16)
+    pairs = 0.0
+    if _profiling() and hasattr(ctx, "h_q_len"):
+        for n, c in zip(ctx.h_q_len.tolist(), ctx.h_ctx_len.tolist()):
+            if n >= LATENT_EXPAND_TOKENS:
+                pairs += float(sum(min(c + i + 1, window) if window > 0 else c + i + 1 for i in range(n)))
+    with region("latent_prompt_tcgen05", _nb(q, kv, out), 2.0 * pairs * H * 320):
+        check(library("attention_prefill_tc.cu").aie_prefill_tc_expanded(
+            _p(q), _p(kv), c_longlong(n_rows), _p(out), _p(tiles), c_int(tiles.shape[0]), _p(ctx.q_start), _p(ctx.q_len),
+            _p(ctx.ctx_len), c_int(T), c_int(H), c_int(window), c_int(LATENT_EXPAND_TOKENS), _p(sink), c_float(scale), _p(ctx.err),
+            _stream()), "prefill_tc_expanded")
 
 
 def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table: torch.Tensor, rank: int,
                      scale: float, window: int, out_dtype: torch.dtype, work=None,
-                     sink: Optional[torch.Tensor] = None, exact_weights: bool = False) -> torch.Tensor:
+                     sink: Optional[torch.Tensor] = None, exact_weights: bool = False, max_len: int = 0) -> torch.Tensor:
     """softmax over the visible cache rows of (q_full . row) * scale, times the rows' first `rank` elements:
     [T, H, rank].  q_full [T, H, dk] float32; pages [num_pages, 1, P, dk].  `work`: the step's units of tokens
     (`tiles` [n, 2], `tq`) for the tensor-core kernel, which bfloat16 takes when the sizes fit (a latent of
     64 .. 512 in steps of 64, rows a multiple of 16); everything else takes the plain kernel.  sink [H] float32: the
     denominator also holds exp(sink[h]).  exact_weights: the tensor-core kernel multiplies weights of 16 bits of mantissa
-    (two terms) instead of 8."""
+    (two terms) instead of 8.  max_len > 0: the tensor-core kernel leaves requests that bring more tokens alone (their rows
+    of the result stay unwritten)."""
     _dev(q_full, pages, block_table, sink)
     T, H, dk = q_full.shape
     if (q_full.dtype != torch.float32 or pages.shape[3] != dk or pages.shape[1] != 1
@@ -965,7 +1015,8 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
                                               _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
                                               c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(T), c_int(H),
                                               c_int(rank), c_int(dk), c_int(window), c_float(scale), c_int(splits),
-                                              _p(sink), c_int(1 if exact_weights else 0), _p(ctx.err), _stream()), "latent_attention_tc")
+                                              _p(sink), c_int(1 if exact_weights else 0), c_int(max_len), _p(ctx.err),
+                                              _stream()), "latent_attention_tc")
         return out
     lib = library("latent_attention.cu")
     with region("latent_attention", *cost):

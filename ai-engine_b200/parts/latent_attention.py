@@ -8,7 +8,9 @@ over the keys the mask shows (all earlier ones, or the last `window`), output W_
 The up-projections never touch the cache: W_uk is folded into the query (qa_h = W_uk,h^T q_plain,h, so
 qa_h . c = q_plain,h . W_uk,h c) and W_uv is applied to the attention-weighted sum of latents
 (sum_j p_j W_uv c_j = W_uv sum_j p_j c_j).  The attention kernel then reads the cache rows as they are, as
-one key/value head for all query heads, for prompts and decoded tokens alike.
+one key/value head for all query heads.  Portions of prompts in bfloat16 with heads of 128 + 64 over values of 128 turn
+this around: the rows they read are expanded to every head's key and value once a step, by one product, and a (query,
+key) pair then costs 320 multiply-adds instead of 2 kv_rank + rot.
 
 The queries may go through a latent of their own (`q_rank`): c_q = RMSnorm(W_dq h) with a weight, q = W_uq c_q.  A
 gate per head (`head_gate`) multiplies head h's output by sigmoid(W_g h)_h; it is applied to the head's values before
@@ -32,14 +34,18 @@ from .base import KVRequest, Mixer, StepPlanner
 class LatentWork(StepPlanner):
     """The work list of the tensor-core kernel: `tiles` [n, 2] = (request row, offset among the tokens it brings)
     of units of `tq` consecutive tokens of one request, which share the cache rows they gather.  A step in which
-    every request brings one token has units of one token, all others units of four."""
+    every request brings one token has units of one token, all others units of four.  `prompt_tiles` [n, 2]: tiles of
+    `ops.PREFILL_TILE` tokens of the requests that bring `ops.LATENT_EXPAND_TOKENS` or more."""
 
     key = "latent"
 
     def plan(self, ctx):
         tq = 1 if ctx.max_q_len <= 1 else 4
-        tiles = [(r, off) for r, n in enumerate(ctx.h_q_len.tolist()) for off in range(0, n, tq)]
-        return dict(tiles=np.asarray(tiles, dtype=np.int32).reshape(-1, 2)), dict(tq=tq)
+        lens = ctx.h_q_len.tolist()
+        tiles = [(r, off) for r, n in enumerate(lens) for off in range(0, n, tq)]
+        prompts = [(r, off) for r, n in enumerate(lens) if n >= ops.LATENT_EXPAND_TOKENS for off in range(0, n, ops.PREFILL_TILE)]
+        return (dict(tiles=np.asarray(tiles, dtype=np.int32).reshape(-1, 2),
+                     prompt_tiles=np.asarray(prompts, dtype=np.int32).reshape(-1, 2)), dict(tq=tq))
 
 
 LATENT_WORK = LatentWork()
@@ -78,7 +84,7 @@ class LatentAttention(Mixer):
         if (self.q_rank or self.head_gate) and self.shares_cache:
             raise ValueError("latent attention: a layer that reads another's cache has neither a query latent nor a gate")
         self.w_uq = self.cq_weight = self.sink = None
-        self.w_in = self.w_ukT = self.w_uv = self.w_o = self.c_weight = self._no_rope = None
+        self.w_in = self.w_ukT = self.w_uv = self.w_o = self.c_weight = self._no_rope = self.w_expand = None
 
     def tensor_specs(self):
         t, dq = self.spec.tensors, self.d + self.rot
@@ -116,8 +122,17 @@ class LatentAttention(Mixer):
             self.w_in = torch.cat([w.to(dt) for w in ws], dim=0).contiguous()
             self.c_weight = source.get(t["dkv_norm"]).float().contiguous()
         # [H, kv_rank, d]: the folding product reads W_uk,h transposed
-        self.w_ukT = source.get(t["uk"]).view(self.H, self.d, self.rank).transpose(1, 2).contiguous()
+        uk = source.get(t["uk"]).view(self.H, self.d, self.rank)
+        self.w_ukT = uk.transpose(1, 2).contiguous()
         self.w_uv = source.get(t["uv"]).view(self.H, self.dv, self.rank).contiguous()
+        if (self.d, self.rot, self.dv) == (128, 64, 128) and self.env.dtype == uk.dtype == self.w_uv.dtype == torch.bfloat16 \
+                and self.rank % 8 == 0:
+            # what makes a head's key [W_uk c | kr] and value W_uv c out of a cached row [c | kr] in one product
+            w = torch.zeros((self.H, self.d + self.rot + self.dv, self.rank + self.rot), dtype=torch.bfloat16, device=uk.device)
+            w[:, :self.d, :self.rank] = uk
+            w[:, self.d:self.d + self.rot, self.rank:] = torch.eye(self.rot, dtype=torch.bfloat16, device=uk.device)
+            w[:, self.d + self.rot:, :self.rank] = self.w_uv
+            self.w_expand = w.view(-1, self.rank + self.rot)
         self.w_o = source.get(t["o"])
         if self.has_sink:
             self.sink = source.get(t["sink"]).float().contiguous()
@@ -154,16 +169,28 @@ class LatentAttention(Mixer):
             q_src = ops.linear(cq, self.w_uq, torch.float32, ctx.err)
         else:
             q_src = proj
-        q_plain, q_full = ops.latent_prepare(q_src, self.H, self.d, self.rot, self.rank, self.c_weight, self.eps,
-                                             inv_freq, cache.k_pages, ctx, cache.block_table, self.env.dtype,
-                                             write=cache.writes and not self.shares_cache, kv=kv, halves=self.halves,
-                                             magnitude=self.magnitude)
-        ops.head_linear(q_plain, self.w_ukT, q_full)
-        mixed = ops.latent_attention(q_full, cache.k_pages, ctx, cache.block_table, self.rank, self.scale,
-                                     self.window, self.env.dtype, ctx.plan(LATENT_WORK), sink=self.sink,
-                                     exact_weights=self.exact_weights)
+        work = ctx.plan(LATENT_WORK)
+        # portions of prompts meet their keys and values expanded; the others read the rows as they are
+        rows = 0
+        if self.w_expand is not None and work.prompt_tiles.shape[0]:
+            rows = 128 * ops.latent_expanded_tiles(ctx, self.window)
+            if rows * self.w_expand.shape[0] * 2 > ops.LATENT_EXPAND_BYTES:
+                rows = 0
+        folded = not rows or int(ctx.h_q_len.min()) < ops.LATENT_EXPAND_TOKENS
+        made = ops.latent_prepare(q_src, self.H, self.d, self.rot, self.rank, self.c_weight, self.eps, inv_freq, cache.k_pages,
+                                  ctx, cache.block_table, self.env.dtype, write=cache.writes and not self.shares_cache, kv=kv,
+                                  halves=self.halves, magnitude=self.magnitude, folded=folded, whole=rows > 0)
         a = torch.empty((T, self.H, self.dv), dtype=self.env.dtype, device=h.device)
-        ops.head_linear(mixed, self.w_uv, a)
+        if folded:
+            q_plain, q_full = made[:2]
+            ops.head_linear(q_plain, self.w_ukT, q_full)
+            mixed = ops.latent_attention(q_full, cache.k_pages, ctx, cache.block_table, self.rank, self.scale,
+                                         self.window, self.env.dtype, work, sink=self.sink, exact_weights=self.exact_weights,
+                                         max_len=ops.LATENT_EXPAND_TOKENS - 1 if rows else 0)
+            ops.head_linear(mixed, self.w_uv, a)
+        if rows:
+            ops.latent_prompt(made[2], cache.k_pages, self.w_expand, ctx, cache.block_table, work.prompt_tiles, rows, self.scale,
+                              self.window, self.sink, a)
         a = a.view(T, self.H * self.dv)
         if self.head_gate:
             g0 = first + self.rank + self.rot

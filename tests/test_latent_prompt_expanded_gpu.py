@@ -1,0 +1,56 @@
+"""Latent attention of prompt portions over expanded rows: against the plain implementation in 64 bits and beside the path
+that reads rows as they are (whose error it must not exceed), with windows at the edges of key tiles and pages, portions at
+the edges of its query tiles and of the shortest it takes, and requests beside them that are too short for it."""
+import pytest
+import torch
+
+import plain_vatazen as pv
+from test_vatazen_parts_gpu import DT, Rig, f64, latent_part, lm, rnd, yarn
+from zupitar_helpers import load
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,rank,page,window,scaling", [(2, 64, 16, None, None), (3, 128, 8, 200, yarn(4.0, 100, 8.0, 0.5)),
+                                                            (1, 512, 32, 129, None), (2, 256, 16, 64, yarn(16.0, 64))])
+def test_portions_over_expanded_rows(heads, rank, page, window, scaling, monkeypatch):
+    from ai_engine_b200.kernels import ops
+    hidden, lens = 128, (420, 64, 200, 90)
+    cuts = [[129, 64, 1, 128, 63, 35], [64], [1, 130, 2, 67], [63, 27]]
+    # queries of deviation 0.3 sqrt(128) on keys of 0.3 sqrt(rank): scores of about 1.5.  A score's relative error (a rounded
+    # query on a rounded key, or its latent form: 2^-9 each) is then an error of 1.5 x 2^-8.5 in the exponent; scores ten
+    # times as large, with which this was first written, bring either path to 2.6 % at a latent of 512
+    m = lm(heads, 128, 64, 128, rank, 1.5 / (0.3 * 128 ** 0.5 * 0.3 * rank ** 0.5 * 128 ** 0.5), window, 20000.0, scaling)
+    gen = torch.Generator().manual_seed(rank + (window or 0))
+    part, t = latent_part(m, hidden, 1e-5, "bfloat16", gen)
+    load(part, {k: v.to(torch.bfloat16) for k, v in t.items()}, torch.bfloat16)
+    assert part.w_expand is not None
+    seqs = [rnd(gen, n, hidden) for n in lens]
+    refs = [pv.latent_attention(s.double(), f64(t), "", m, 1e-5) for s in seqs]
+    calls, real = [], ops.latent_prompt
+    monkeypatch.setattr(ops, "latent_prompt", lambda *a, **k: calls.append(a[6]) or real(*a, **k))
+    run = lambda: Rig(part, DT["bfloat16"], page=page, pages=-(-sum(lens) // page) + 8).run([s.to(torch.bfloat16) for s in seqs], cuts)
+    got = run()
+    assert len(calls) == 3                                   # steps with a portion of 64 or more
+    monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", 0)      # no room: every row is read as it is
+    folded = run()
+    assert len(calls) == 3
+    errors = [[float(((o - r).norm() / r.norm())) for o, r in zip(os, refs)] for os in (got, folded)]
+    # 1.5 x 2^-8.5 from the scores, and latents, values, outputs and their projection of 2^-9 / sqrt(3) each
+    assert max(errors[0]) <= 6 * 2.0 ** -9, errors
+    assert sum(errors[0]) <= 1.05 * sum(errors[1]), errors     # 5 %: what the errors of two draws of roundings differ by
+
+
+def test_a_page_outside_the_pool_is_flagged():
+    from ai_engine_b200.kernels import ops
+    gen = torch.Generator().manual_seed(1)
+    m = lm(1, 128, 64, 128, 64, 0.1, None)
+    part, t = latent_part(m, 128, 1e-5, "bfloat16", gen)
+    load(part, {k: v.to(torch.bfloat16) for k, v in t.items()}, torch.bfloat16)
+    rig = Rig(part, DT["bfloat16"], page=16, pages=16)
+    slot = rig.admit()
+    ctx, lc = rig.step([(slot, 70)])
+    lc.block_table = lc.block_table.clone()
+    lc.block_table[0, 2] = 99
+    part.forward(rnd(gen, 70, 128).to(torch.bfloat16).cuda(), ctx, lc)
+    assert int(rig.err.item()) == 2
