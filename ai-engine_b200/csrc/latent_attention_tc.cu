@@ -5,7 +5,7 @@
 // of 64 that start at multiples of 64 of the absolute key position (a row's additions depend on its position
 // only, not on how the prompt was cut or on the batch).  A CTA of a prompt's portion takes TQ = 4 consecutive tokens
 // of one request (four warps each): they share the gathered cache rows, whose traffic from L2 bounds the kernel,
-// and differ only in their masks.
+// and differ only in their masks.  (Lone tokens take latent_decode_kernel below.)
 //
 // Per chunk: the 64 cache rows are gathered page by page into shared memory by 16-byte cp.async copies (rows
 // outside the mask or the block table are zero-filled, so a probability of 0 never meets an unwritten row);
@@ -20,6 +20,7 @@
 #define LT_KEYS 64
 #define LT_ROWS 16
 #define LT_THREADS 128
+#define LT_TOKENS 4
 
 template <int CW, int TQ, bool PAIR>      // latent columns per warp (rank = 4 CW); tokens per CTA; weights as two terms
 __global__ void __launch_bounds__(LT_THREADS * TQ)
@@ -28,7 +29,7 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
                            const int* __restrict__ q_start, const int* __restrict__ q_len,
                            const int* __restrict__ ctx_len, const int* __restrict__ block_table, int bt_width,
                            int num_pages, int P, int H, int dk, int window, float scale, int splits,
-                           const float* __restrict__ sink, int max_len, unsigned* err) {
+                           const float* __restrict__ sink, int min_len, int max_len, unsigned* err) {
     constexpr int RANK = 4 * CW, NT = CW / 8, THREADS = LT_THREADS * TQ;
     extern __shared__ __align__(16) unsigned char lt_raw[];
     const int SK = dk + 8;                                        // padded row: ldmatrix rows fall on different banks
@@ -44,7 +45,8 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
     pdl_launch_dependents();
     pdl_wait();
     const int row = tiles[2 * blockIdx.x], off = tiles[2 * blockIdx.x + 1];
-    if (max_len > 0 && q_len[row] > max_len) return;              // a longer portion meets expanded keys in another kernel
+    const int brings = q_len[row];                                // lone tokens and longer portions are other kernels'
+    if (brings < min_len || (max_len > 0 && brings > max_len)) return;
     const int h0 = blockIdx.y * LT_ROWS, part = blockIdx.z;
     const int tid = threadIdx.x, tq = tid / LT_THREADS, ltid = tid % LT_THREADS, warp = (tid >> 5) & 3, lane = tid & 31;
     const int n_act = min(TQ, q_len[row] - off);                  // tokens of this CTA that exist
@@ -245,6 +247,345 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
     }
 }
 
+// ---------------------------------------------------------------------------
+// Requests that bring one token.  What bounds them is the stream of their cache rows, so the rows are cut evenly over the
+// machine whatever the requests' lengths: the visible chunks of 32 keys of all such requests stand in one line, CTA i takes
+// the i-th of gridDim.x equal stretches of it, and the rows of the chunks ahead are on their way (a ring of NST stages)
+// across the requests' ends while a chunk is multiplied.  Eight warps: the scores' products are split over four groups of
+// eight keys and two halves of a row, the values' over eight ranges of the latent's columns.  A stretch that holds a whole
+// request writes its result; others leave (maximum, sum, unnormalised output) in slot CTA + request for the join.
+// 64 requests of 512 .. 4,096 keys, 16 heads, a latent of 512 (170 MB of rows, 26 us at the copy bandwidth): 162 us with a
+// CTA a (request, quarter of its keys) that loaded and multiplied in turn.
+#define LD_KEYS 32
+#define LD_THREADS 256
+#define LD_MIN_CHUNKS 2       // a stretch is at least this long: a CTA's start costs about as much as two chunks
+
+__device__ __forceinline__ int ld_chunks(const int* q_len, const int* ctx_len, int R, int window, int r, int& first) {
+    first = 0;
+    if (r >= R || q_len[r] != 1) return 0;
+    const int pos = ctx_len[r];
+    first = (window > 0 && pos - window + 1 > 0 ? pos - window + 1 : 0) / LD_KEYS;
+    return pos / LD_KEYS - first + 1;
+}
+// Chunks of all requests and the length of a stretch, by any whole warp.
+__device__ __forceinline__ int ld_stretch(const int* q_len, const int* ctx_len, int R, int window, int G, int& total) {
+    total = 0;
+    int first;
+    for (int base = 0; base < R; base += 32) total += ld_chunks(q_len, ctx_len, R, window, base + (threadIdx.x & 31), first);
+    total = __reduce_add_sync(0xffffffffu, total);
+    return max((total + G - 1) / G, LD_MIN_CHUNKS);
+}
+
+template <int NT, bool PAIR, int NST>      // NT: tiles of 8 latent columns a warp (rank = 64 NT)
+__global__ void __launch_bounds__(LD_THREADS, 1)
+latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ pages, bf16* __restrict__ out,
+                     float* __restrict__ part_o, float* __restrict__ part_ml, const int* __restrict__ q_start,
+                     const int* __restrict__ q_len, const int* __restrict__ ctx_len, const int* __restrict__ block_table,
+                     int bt_width, int num_pages, int P, int R, int H, int dk, int window, float scale,
+                     const float* __restrict__ sink, unsigned* err) {
+    constexpr int RANK = 64 * NT, SP = LD_KEYS + 8, SS = LD_KEYS + 2;
+    extern __shared__ __align__(16) unsigned char lt_raw[];
+    const int SK = dk + 8;
+    bf16* q_s = reinterpret_cast<bf16*>(lt_raw);                  // [16][SK]
+    bf16* k_s = q_s + LT_ROWS * SK;                               // [NST][32][SK]
+    bf16* p_s = k_s + NST * LD_KEYS * SK + 32;                    // [1 or 2][16][SP] (32: what a last odd step reads past a row)
+    float* s_s = reinterpret_cast<float*>(p_s + (PAIR ? 2 : 1) * LT_ROWS * SP);      // [2][16][SS]
+    float* m_s = s_s + 2 * LT_ROWS * SS;                          // [16] running maximum, sum, correction
+    float* l_s = m_s + LT_ROWS;
+    float* c_s = l_s + LT_ROWS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h0 = blockIdx.y * LT_ROWS, pieces = dk / 8;
+    pdl_launch_dependents();
+    pdl_wait();
+    int total, first;
+    const int per = ld_stretch(q_len, ctx_len, R, window, gridDim.x, total);
+    const int begin = blockIdx.x * per, cnt = min(total - begin, per);
+    if (cnt <= 0) return;
+    int r = 0, c = 0;                                             // request and chunk that the stretch starts in
+    for (int base = 0, before = 0; base < R; base += 32) {
+        const int m = ld_chunks(q_len, ctx_len, R, window, base + lane, first);
+        int run = m;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, run, o);
+            if (lane >= o) run += up;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, begin < before + run);
+        if (hit) {
+            const int l = __ffs(hit) - 1;
+            r = base + l;
+            c = begin - before - __shfl_sync(0xffffffffu, run - m, l);
+            break;
+        }
+        before += __shfl_sync(0xffffffffu, run, 31);
+    }
+    int lr = r, lc = c, lfirst, ln = ld_chunks(q_len, ctx_len, R, window, r, lfirst);      // the chunk that is asked for next
+    auto fetch = [&](int i) {
+        if (i < cnt) {
+            bf16* dst = k_s + (i % NST) * LD_KEYS * SK;
+            const int pos = ctx_len[lr], lo = window > 0 ? max(pos - window + 1, 0) : 0;
+#pragma unroll
+            for (int jj = 0; jj < LD_KEYS / 8; ++jj) {
+                const int j = warp * (LD_KEYS / 8) + jj, kp = (lfirst + lc) * LD_KEYS + j;
+                bool ok = kp >= lo && kp <= pos;
+                const bf16* src = pages;
+                if (ok) {
+                    const int pidx = kp / P, page = pidx < bt_width ? block_table[(size_t)lr * bt_width + pidx] : -1;
+                    if (page < 0 || page >= num_pages) {
+                        if (lane == 0) atomicOr(err, AIE_DEV_PAGE_OOB);
+                        ok = false;
+                    } else {
+                        src = pages + ((size_t)page * P + (kp - pidx * P)) * dk;
+                    }
+                }
+                for (int x = lane; x < pieces; x += 32) cp_async16(dst + j * SK + x * 8, ok ? src + x * 8 : pages, ok);
+            }
+            if (++lc == ln && i + 1 < cnt) {
+                lc = 0;
+                do ln = ld_chunks(q_len, ctx_len, R, window, ++lr, lfirst);
+                while (ln == 0 && lr < R);
+            }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int i = 0; i < NST - 1; ++i) fetch(i);
+    const int steps = dk / 16, kg = warp & 3, kh = warp >> 2;
+    const int step0 = kh ? (steps + 1) / 2 : 0, step1 = kh ? steps : (steps + 1) / 2;
+    float acc[NT][4];
+    int n = 0, c_begin = 0;
+    bool fresh = true;
+    for (int i = 0; i < cnt; ++i) {
+        if (fresh) {                                              // a request begins: its queries, an empty softmax
+            fresh = false;
+            n = ld_chunks(q_len, ctx_len, R, window, r, first);
+            c_begin = c;
+            if (i > 0) __syncthreads();                           // the last one's sums have been read
+            const int t = q_start[r];
+            for (int rr = warp; rr < LT_ROWS; rr += LD_THREADS / 32) {
+                const bool on = h0 + rr < H;
+                const float* src = q_full + ((size_t)t * H + h0 + rr) * dk;
+                for (int x = lane * 4; x < dk; x += 128) {
+                    const float4 v = on ? *reinterpret_cast<const float4*>(src + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    *reinterpret_cast<uint2*>(q_s + rr * SK + x) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+                }
+            }
+            if (tid < LT_ROWS) {
+                const bool leaks = sink && c == 0 && h0 + tid < H;
+                m_s[tid] = leaks ? sink[h0 + tid] : -INFINITY;
+                l_s[tid] = leaks ? 1.f : 0.f;
+            }
+#pragma unroll
+            for (int x = 0; x < NT; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
+        }
+        cp_async_wait<NST - 2>();
+        __syncthreads();                                          // chunk i is here for all; chunk i - 1 is done with
+        fetch(i + NST - 1);
+        const bf16* ks = k_s + (i % NST) * LD_KEYS * SK;
+        {
+            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+            const bf16* qa = q_s + (lane & 15) * SK + (lane >> 4) * 8;
+            const bf16* kb = ks + (kg * 8 + (lane & 7)) * SK + (lane >> 3) * 8;
+#pragma unroll 3
+            for (int st = step0; st < step1; st += 2) {           // two steps of 16: one load of keys
+                unsigned a[4], b0, b1, b2, b3;
+                ldsm_x4(b0, b1, b2, b3, kb + st * 16);
+                ldsm_x4(a[0], a[1], a[2], a[3], qa + st * 16);
+                mma16816(s0, a, b0, b1);
+                if (st + 1 < step1) {
+                    ldsm_x4(a[0], a[1], a[2], a[3], qa + st * 16 + 16);
+                    mma16816(s1, a, b2, b3);
+                }
+            }
+            float* d = s_s + kh * LT_ROWS * SS + (lane >> 2) * SS + kg * 8 + (lane & 3) * 2;
+            *reinterpret_cast<float2*>(d) = make_float2(s0[0] + s1[0], s0[1] + s1[1]);
+            *reinterpret_cast<float2*>(d + 8 * SS) = make_float2(s0[2] + s1[2], s0[3] + s1[3]);
+        }
+        __syncthreads();
+        {                                                         // running softmax: sixteen threads a row, two keys a thread
+            const int row = tid >> 4, g = tid & 15, key = (first + c) * LD_KEYS + 2 * g, pos = ctx_len[r];
+            const int lo = window > 0 ? max(pos - window + 1, 0) : 0;
+            const float2 x = *reinterpret_cast<const float2*>(s_s + row * SS + 2 * g);
+            const float2 y = *reinterpret_cast<const float2*>(s_s + (LT_ROWS + row) * SS + 2 * g);
+            const float v0 = key >= lo && key <= pos ? (x.x + y.x) * scale : -INFINITY;
+            const float v1 = key + 1 >= lo && key + 1 <= pos ? (x.y + y.y) * scale : -INFINITY;
+            float mx = fmaxf(v0, v1);
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float m_old = m_s[row], m_new = fmaxf(m_old, mx);
+            const float p0 = v0 == -INFINITY ? 0.f : expf(v0 - m_new), p1 = v1 == -INFINITY ? 0.f : expf(v1 - m_new);
+            const unsigned pb = pack_bf16(p0, p1);
+            const float2 pf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pb));
+            *reinterpret_cast<unsigned*>(p_s + row * SP + 2 * g) = pb;
+            if (PAIR) *reinterpret_cast<unsigned*>(p_s + (LT_ROWS + row) * SP + 2 * g) = pack_bf16(p0 - pf.x, p1 - pf.y);
+            float sum = PAIR ? p0 + p1 : pf.x + pf.y;             // the sum of what the product will multiply
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            __syncwarp();
+            if (g == 0) {
+                const float corr = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
+                c_s[row] = corr;
+                l_s[row] = l_s[row] * corr + sum;
+                m_s[row] = m_new;
+            }
+        }
+        __syncthreads();
+        {                                                         // O = O * corr + P V over this warp's columns
+            const float ca = c_s[lane >> 2], cb = c_s[(lane >> 2) + 8];
+#pragma unroll
+            for (int x = 0; x < NT; ++x) {
+                acc[x][0] *= ca;
+                acc[x][1] *= ca;
+                acc[x][2] *= cb;
+                acc[x][3] *= cb;
+            }
+#pragma unroll
+            for (int kk = 0; kk < LD_KEYS; kk += 16) {
+                unsigned a[4], a2[4];
+                ldsm_x4(a[0], a[1], a[2], a[3], p_s + (lane & 15) * SP + kk + (lane >> 4) * 8);
+                if (PAIR) ldsm_x4(a2[0], a2[1], a2[2], a2[3], p_s + LT_ROWS * SP + (lane & 15) * SP + kk + (lane >> 4) * 8);
+                const bf16* vb = ks + (kk + (lane & 7) + ((lane >> 3) & 1) * 8) * SK + warp * 8 * NT + (lane >> 4) * 8;
+#pragma unroll
+                for (int np = 0; np < (NT + 1) / 2; ++np) {
+                    unsigned b0, b1, b2, b3;
+                    ldsm_x4_t(b0, b1, b2, b3, vb + np * 16);
+                    mma16816(acc[2 * np], a, b0, b1);
+                    if (2 * np + 1 < NT) mma16816(acc[2 * np + 1 < NT ? 2 * np + 1 : 0], a, b2, b3);
+                    if (PAIR) {
+                        mma16816(acc[2 * np], a2, b0, b1);
+                        if (2 * np + 1 < NT) mma16816(acc[2 * np + 1 < NT ? 2 * np + 1 : 0], a2, b2, b3);
+                    }
+                }
+            }
+        }
+        ++c;
+        if (c < n && i + 1 < cnt) continue;
+        // the request, or the stretch, ends here
+        const int ra = lane >> 2, rb = ra + 8, t = q_start[r];
+        const bool whole = c_begin == 0 && c == n;
+        const size_t slot = (size_t)(blockIdx.x + r) * H;
+        const float ia = whole ? (l_s[ra] > 0.f ? 1.0f / l_s[ra] : 0.f) : 1.f, ib = whole ? (l_s[rb] > 0.f ? 1.0f / l_s[rb] : 0.f) : 1.f;
+#pragma unroll
+        for (int x = 0; x < NT; ++x) {
+            const int col = warp * 8 * NT + x * 8 + (lane & 3) * 2;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int hh = h0 + (e ? rb : ra);
+                if (hh >= H) continue;
+                const float u = acc[x][2 * e] * (e ? ib : ia), v = acc[x][2 * e + 1] * (e ? ib : ia);
+                if (whole) *reinterpret_cast<unsigned*>(out + ((size_t)t * H + hh) * RANK + col) = pack_bf16(u, v);
+                else *reinterpret_cast<float2*>(part_o + (slot + hh) * RANK + col) = make_float2(u, v);
+            }
+        }
+        if (!whole && tid < LT_ROWS && h0 + tid < H) {
+            part_ml[(slot + h0 + tid) * 2] = m_s[tid];
+            part_ml[(slot + h0 + tid) * 2 + 1] = l_s[tid];
+        }
+        c = 0;
+        fresh = true;
+        if (i + 1 < cnt)
+            do n = ld_chunks(q_len, ctx_len, R, window, ++r, first);
+            while (n == 0 && r < R);
+    }
+}
+
+// One block a (request, head): the parts that the stretches of latent_decode_kernel left of it, in their order.
+__global__ void __launch_bounds__(128)
+latent_decode_join_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, bf16* __restrict__ out,
+                          const int* __restrict__ q_start, const int* __restrict__ q_len, const int* __restrict__ ctx_len, int R,
+                          int H, int rank, int window, int G) {
+    extern __shared__ float ld_w[];                               // [G] weights
+    __shared__ int range_s[2];
+    __shared__ float inv_s;
+    pdl_launch_dependents();
+    pdl_wait();
+    const int r = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
+    if (q_len[r] != 1) return;
+    if (tid < 32) {
+        int total, first, start = 0;
+        const int per = ld_stretch(q_len, ctx_len, R, window, G, total);
+        for (int base = 0; base < r; base += 32) {
+            const int i = base + tid;
+            start += i < r ? ld_chunks(q_len, ctx_len, R, window, i, first) : 0;
+        }
+        start = __reduce_add_sync(0xffffffffu, start);
+        const int p0 = start / per, p1 = (start + ld_chunks(q_len, ctx_len, R, window, r, first) - 1) / per;
+        float mx = -INFINITY;
+        for (int p = p0 + tid; p <= p1 && p1 > p0; p += 32) {
+            const float* ml = part_ml + ((size_t)(p + r) * H + h) * 2;
+            if (ml[1] > 0.f) mx = fmaxf(mx, ml[0]);
+        }
+        mx = warp_max(mx);
+        float den = 0.f;
+        for (int p = p0 + tid; p <= p1 && p1 > p0; p += 32) {
+            const float* ml = part_ml + ((size_t)(p + r) * H + h) * 2;
+            const float w = ml[1] > 0.f ? expf(ml[0] - mx) : 0.f;
+            ld_w[p - p0] = w;
+            den += w * ml[1];
+        }
+        den = warp_sum(den);
+        if (tid == 0) {
+            range_s[0] = p0;
+            range_s[1] = p1;
+            inv_s = den > 0.f ? 1.0f / den : 0.f;
+        }
+    }
+    __syncthreads();
+    const int p0 = range_s[0], parts = range_s[1] - p0 + 1;
+    if (parts <= 1) return;                                       // one stretch held it whole
+    for (int c = tid * 4; c < rank; c += blockDim.x * 4) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+        for (int p = 0; p < parts; ++p) {
+            const float4 v = *reinterpret_cast<const float4*>(part_o + ((size_t)(p0 + p + r) * H + h) * rank + c);
+            const float w = ld_w[p];
+            acc = make_float4(fmaf(w, v.x, acc.x), fmaf(w, v.y, acc.y), fmaf(w, v.z, acc.z), fmaf(w, v.w, acc.w));
+        }
+        store4<bf16>(out + ((size_t)q_start[r] * H + h) * rank + c, make_float4(acc.x * inv_s, acc.y * inv_s, acc.z * inv_s, acc.w * inv_s));
+    }
+}
+
+// The requests of the step that bring one token (the others are left alone).  q_full [T, H, dk] float32, pages [num_pages, P,
+// dk] bfloat16, out [T, H, rank] bfloat16; part_o [G + R, H, rank] and part_ml [G + R, H, 2] float32 scratch.  rank = 64 ..
+// 512 in steps of 64, dk a multiple of 16 up to 1,024 (else AIE_UNSUPPORTED).
+extern "C" int aie_latent_decode(const float* q_full, const void* pages, void* out, float* part_o, float* part_ml,
+                                 const int* q_start, const int* q_len, const int* ctx_len, const int* block_table, int bt_width,
+                                 int num_pages, int P, int R, int H, int rank, int dk, int window, float scale, int G,
+                                 const float* sink, int pair, unsigned* err, cudaStream_t st) {
+    if (R <= 0) return 0;
+    if (rank < 64 || rank > 512 || rank % 64 || dk % 16 || dk < rank || dk > 1024 || H <= 0) return AIE_UNSUPPORTED;
+    if (G < 1 || G > 4096 || !part_o || !part_ml || P <= 0) return AIE_BAD_ARG;
+    const dim3 grid(G, (H + LT_ROWS - 1) / LT_ROWS);
+    if (grid.y > 65535 || H > 65535) return AIE_UNSUPPORTED;
+    const auto smem = [&](int nst) {
+        return (size_t)(LT_ROWS + nst * LD_KEYS) * (dk + 8) * 2 + 64 + (size_t)(pair ? 2 : 1) * LT_ROWS * (LD_KEYS + 8) * 2 +
+               (size_t)(2 * LT_ROWS * (LD_KEYS + 2) + 3 * LT_ROWS) * 4;
+    };
+    const bool deep = smem(4) <= 225 * 1024;             // four stages, or two for the longest rows
+    cudaError_t e = cudaSuccess;
+#define GO2(NT, PV, NS)                                                                                                 \
+    {                                                                                                                   \
+        auto kern = latent_decode_kernel<NT, PV, NS>;                                                                   \
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(NS));                     \
+        if (e == cudaSuccess)                                                                                           \
+            e = launch_pdl(kern, grid, dim3(LD_THREADS), smem(NS), st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, \
+                           q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, R, H, dk, window, scale, sink, err); \
+    }
+#define GO(NT)                                                                                                          \
+    case NT:                                                                                                            \
+        if (pair) { if (deep) GO2(NT, true, 4) else GO2(NT, true, 2) }                                                  \
+        else { if (deep) GO2(NT, false, 4) else GO2(NT, false, 2) }                                                     \
+        break;
+    switch (rank / 64) {
+        GO(1) GO(2) GO(3) GO(4) GO(5) GO(6) GO(7) GO(8)
+        default: return AIE_UNSUPPORTED;
+    }
+#undef GO
+#undef GO2
+    if (e != cudaSuccess) return (int)e;
+    launch_pdl(latent_decode_join_kernel, dim3(R, H), dim3(128), G * sizeof(float), st, part_o, part_ml, (bf16*)out, q_start, q_len,
+               ctx_len, R, H, rank, window, G);
+    AIE_LAUNCH_CHECK();
+}
+
 // out[t, h] = sum_p w_p O_p / sum_p w_p l_p with w_p = exp(m_p - max m), parts in order.  The first warp makes the
 // weights of all parts (at most 64), then every thread adds its column with several parts' loads in flight.
 __global__ void latent_join_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
@@ -284,17 +625,18 @@ __global__ void latent_join_kernel(const float* __restrict__ part_o, const float
 }
 
 // q_full [T, H, dk] float32; pages [num_pages, P, dk] bfloat16; out [T, H, rank] bfloat16.  tiles [n_tiles, 2] =
-// (request row, offset among the tokens it brings) of units of `tq` tokens (1 or 4).  Takes rank = 64 .. 512 in
+// (request row, offset among the tokens it brings) of units of `tq` = 4 tokens.  Requests that bring fewer than min_len or
+// (max_len > 0) more than max_len tokens are left alone.  Takes rank = 64 .. 512 in
 // steps of 64 and dk a multiple of 16 (else AIE_UNSUPPORTED: the caller takes the plain kernel).  splits > 1 needs
 // part_o [T, H, splits, rank] and part_ml [T, H, splits, 2] float32.
 extern "C" int aie_latent_attention_tc(const float* q_full, const void* pages, void* out, float* part_o, float* part_ml,
                                        const int* tiles, int n_tiles, int tq, const int* q_start, const int* q_len,
                                        const int* ctx_len, const int* block_table, int bt_width,
                                        int num_pages, int P, int T, int H, int rank, int dk, int window, float scale,
-                                       int splits, const float* sink, int pair, int max_len, unsigned* err, cudaStream_t st) {
+                                       int splits, const float* sink, int pair, int min_len, int max_len, unsigned* err, cudaStream_t st) {
     if (T <= 0 || n_tiles <= 0) return 0;
     if (rank < 64 || rank > 512 || rank % 64 || dk % 16 || dk < rank || dk > 1024 || H <= 0) return AIE_UNSUPPORTED;
-    if (splits < 1 || splits > 64 || (splits > 1 && (!part_o || !part_ml)) || (tq != 1 && tq != 4)) return AIE_BAD_ARG;
+    if (splits < 1 || splits > 64 || (splits > 1 && (!part_o || !part_ml)) || tq != LT_TOKENS) return AIE_BAD_ARG;
     const int SK = dk + 8;
     const size_t smem = (size_t)(tq * LT_ROWS + LT_KEYS) * SK * 2 + (size_t)tq * LT_ROWS * (LT_KEYS + 8) * 2 * (pair ? 2 : 1) +
                         (size_t)tq * (LT_ROWS * (LT_KEYS + 1) + 3 * LT_ROWS) * 4;
@@ -307,13 +649,13 @@ extern "C" int aie_latent_attention_tc(const float* q_full, const void* pages, v
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
         launch_pdl(kern, grid, dim3(LT_THREADS * TQV), smem, st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, tiles,    \
                                                    q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, H,   \
-                                                   dk, window, scale, splits, sink, max_len, err);                                   \
+                                                   dk, window, scale, splits, sink, min_len, max_len, err);                                   \
     }
 #define GO1(CWV, TQV)                                                                                                 \
     if (pair) GO2(CWV, TQV, true) else GO2(CWV, TQV, false)
 #define GO(CWV)                                                                                                       \
     case CWV:                                                                                                         \
-        if (tq == 1) { GO1(CWV, 1) } else { GO1(CWV, 4) }                                                             \
+        GO1(CWV, LT_TOKENS)                                                                                           \
         break;
     switch (rank / 4) {
         GO(16) GO(32) GO(48) GO(64) GO(80) GO(96) GO(112) GO(128)

@@ -979,7 +979,7 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
     (`tiles` [n, 2], `tq`) for the tensor-core kernel, which bfloat16 takes when the sizes fit (a latent of
     64 .. 512 in steps of 64, rows a multiple of 16); everything else takes the plain kernel.  sink [H] float32: the
     denominator also holds exp(sink[h]).  exact_weights: the tensor-core kernel multiplies weights of 16 bits of mantissa
-    (two terms) instead of 8.  max_len > 0: the tensor-core kernel leaves requests that bring more tokens alone (their rows
+    (two terms) instead of 8.  Lone tokens take a kernel of their own there.  max_len > 0: the tensor-core kernel leaves requests that bring more tokens alone (their rows
     of the result stay unwritten)."""
     _dev(q_full, pages, block_table, sink)
     T, H, dk = q_full.shape
@@ -998,25 +998,39 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
     if (work is not None and pages.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and rank % 64 == 0
             and 64 <= rank <= 512 and dk % 16 == 0 and dk <= 1024
             and (work.tq * 16 + 64) * (dk + 8) * 2 + work.tq * (9400 if exact_weights else 7000) <= 220 * 1024):
-        # tensor cores; a step of few tokens cuts each token's keys into parts so that the grid fills the machine
-        keys = ctx.bt_width * ctx.page_size if ctx.bucketed else ctx.max_total_len
-        if window > 0:
-            keys = min(keys, window + 63)
-        ctas = work.tiles.shape[0] * ((H + 15) // 16)
-        splits = max(1, min(64, (keys + 63) // 64, (2 * sm_count()) // ctas))
-        part_o = part_ml = None
-        if splits > 1:
-            part_o = torch.empty((T, H, splits, rank), dtype=torch.float32, device=q_full.device)
-            part_ml = torch.empty((T, H, splits, 2), dtype=torch.float32, device=q_full.device)
         lib = library("latent_attention_tc.cu")
-        with region("latent_attention_tc", *cost):
-            check(lib.aie_latent_attention_tc(_p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(work.tiles),
-                                              c_int(work.tiles.shape[0]), c_int(work.tq), _p(ctx.q_start),
-                                              _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
-                                              c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(T), c_int(H),
-                                              c_int(rank), c_int(dk), c_int(window), c_float(scale), c_int(splits),
-                                              _p(sink), c_int(1 if exact_weights else 0), c_int(max_len), _p(ctx.err),
-                                              _stream()), "latent_attention_tc")
+        lone = ctx.max_q_len <= 1 or bool((ctx.h_q_len == 1).any())
+        if ctx.max_q_len > 1 and (not max_len or bool(((ctx.h_q_len > 1) & (ctx.h_q_len <= max_len)).any())):
+            # short portions; a step of few tokens cuts each token's keys into parts so that the grid fills the machine
+            keys = ctx.bt_width * ctx.page_size if ctx.bucketed else ctx.max_total_len
+            if window > 0:
+                keys = min(keys, window + 63)
+            ctas = work.tiles.shape[0] * ((H + 15) // 16)
+            splits = max(1, min(64, (keys + 63) // 64, (2 * sm_count()) // ctas))
+            part_o = part_ml = None
+            if splits > 1:
+                part_o = torch.empty((T, H, splits, rank), dtype=torch.float32, device=q_full.device)
+                part_ml = torch.empty((T, H, splits, 2), dtype=torch.float32, device=q_full.device)
+            with region("latent_attention_tc", *cost):
+                check(lib.aie_latent_attention_tc(_p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(work.tiles),
+                                                  c_int(work.tiles.shape[0]), c_int(work.tq), _p(ctx.q_start),
+                                                  _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
+                                                  c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(T), c_int(H),
+                                                  c_int(rank), c_int(dk), c_int(window), c_float(scale), c_int(splits),
+                                                  _p(sink), c_int(1 if exact_weights else 0), c_int(2 if lone else 1), c_int(max_len),
+                                                  _p(ctx.err), _stream()), "latent_attention_tc")
+        if lone:
+            # one token a request: the visible rows of all of them in equal stretches, one a CTA.  (Behind the other kernel, whose
+            # join of parts runs over every token's row.)
+            G = max(1, sm_count() // ((H + 15) // 16))
+            part_o = torch.empty((G + ctx.R, H, rank), dtype=torch.float32, device=q_full.device)
+            part_ml = torch.empty((G + ctx.R, H, 2), dtype=torch.float32, device=q_full.device)
+            with region("latent_attention_tc", *cost):
+                check(lib.aie_latent_decode(_p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(ctx.q_start), _p(ctx.q_len),
+                                            _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]),
+                                            c_int(pages.shape[2]), c_int(ctx.R), c_int(H), c_int(rank), c_int(dk), c_int(window),
+                                            c_float(scale), c_int(G), _p(sink), c_int(1 if exact_weights else 0), _p(ctx.err),
+                                            _stream()), "latent_decode")
         return out
     lib = library("latent_attention.cu")
     with region("latent_attention", *cost):
