@@ -250,12 +250,13 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
 // ---------------------------------------------------------------------------
 // Requests that bring one token.  What bounds them is the stream of their cache rows, so the rows are cut evenly over the
 // machine whatever the requests' lengths: the visible chunks of 32 keys of all such requests stand in one line, CTA i takes
-// the i-th of gridDim.x equal stretches of it, and the rows of the chunks ahead are on their way (a ring of NST stages)
-// across the requests' ends while a chunk is multiplied.  Eight warps: the scores' products are split over four groups of
+// the i-th of gridDim.x equal stretches of it, and the rows of the next chunk are on their way, across the requests' ends,
+// while a chunk is multiplied; two CTAs share an SM, so that one's chain of products and softmax fills the other's waits.  Eight warps: the scores' products are split over four groups of
 // eight keys and two halves of a row, the values' over eight ranges of the latent's columns.  A stretch that holds a whole
 // request writes its result; others leave (maximum, sum, unnormalised output) in slot CTA + request for the join.
-// 64 requests of 512 .. 4,096 keys, 16 heads, a latent of 512 (170 MB of rows, 26 us at the copy bandwidth): 162 us with a
-// CTA a (request, quarter of its keys) that loaded and multiplied in turn.
+// 64 requests of 512 .. 4,096 keys, 16 heads, a latent of 512 (170 MB of rows, 26 us at the copy bandwidth): 63 us; 162 us with
+// a CTA a (request, quarter of its keys) that loaded and multiplied in turn, 109 us with one CTA an SM and four chunks in
+// flight, whose eight warps waited on one another.
 #define LD_KEYS 32
 #define LD_THREADS 256
 #define LD_MIN_CHUNKS 2       // a stretch is at least this long: a CTA's start costs about as much as two chunks
@@ -276,14 +277,14 @@ __device__ __forceinline__ int ld_stretch(const int* q_len, const int* ctx_len, 
     return max((total + G - 1) / G, LD_MIN_CHUNKS);
 }
 
-template <int NT, bool PAIR, int NST>      // NT: tiles of 8 latent columns a warp (rank = 64 NT)
-__global__ void __launch_bounds__(LD_THREADS, 1)
+template <int NT, bool PAIR, int CTAS>     // NT: tiles of 8 latent columns a warp (rank = 64 NT); CTAS: blocks an SM
+__global__ void __launch_bounds__(LD_THREADS, CTAS)
 latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ pages, bf16* __restrict__ out,
                      float* __restrict__ part_o, float* __restrict__ part_ml, const int* __restrict__ q_start,
                      const int* __restrict__ q_len, const int* __restrict__ ctx_len, const int* __restrict__ block_table,
                      int bt_width, int num_pages, int P, int R, int H, int dk, int window, float scale,
                      const float* __restrict__ sink, unsigned* err) {
-    constexpr int RANK = 64 * NT, SP = LD_KEYS + 8, SS = LD_KEYS + 2;
+    constexpr int RANK = 64 * NT, SP = LD_KEYS + 8, SS = LD_KEYS + 2, NST = 2;
     extern __shared__ __align__(16) unsigned char lt_raw[];
     const int SK = dk + 8;
     bf16* q_s = reinterpret_cast<bf16*>(lt_raw);                  // [16][SK]
@@ -318,25 +319,16 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
         before += __shfl_sync(0xffffffffu, run, 31);
     }
     int lr = r, lc = c, lfirst, ln = ld_chunks(q_len, ctx_len, R, window, r, lfirst);      // the chunk that is asked for next
-    auto fetch = [&](int i) {
+    // lane l: place (page * P + offset) of key l of the chunk that is asked for next, -1: none or not to be seen.  Looked up a
+    // chunk ahead, so that no copy waits for a block table.
+    auto places = [&](int i) {
+        int at = -1;
         if (i < cnt) {
-            bf16* dst = k_s + (i % NST) * LD_KEYS * SK;
-            const int pos = ctx_len[lr], lo = window > 0 ? max(pos - window + 1, 0) : 0;
-#pragma unroll
-            for (int jj = 0; jj < LD_KEYS / 8; ++jj) {
-                const int j = warp * (LD_KEYS / 8) + jj, kp = (lfirst + lc) * LD_KEYS + j;
-                bool ok = kp >= lo && kp <= pos;
-                const bf16* src = pages;
-                if (ok) {
-                    const int pidx = kp / P, page = pidx < bt_width ? block_table[(size_t)lr * bt_width + pidx] : -1;
-                    if (page < 0 || page >= num_pages) {
-                        if (lane == 0) atomicOr(err, AIE_DEV_PAGE_OOB);
-                        ok = false;
-                    } else {
-                        src = pages + ((size_t)page * P + (kp - pidx * P)) * dk;
-                    }
-                }
-                for (int x = lane; x < pieces; x += 32) cp_async16(dst + j * SK + x * 8, ok ? src + x * 8 : pages, ok);
+            const int pos = ctx_len[lr], kp = (lfirst + lc) * LD_KEYS + lane;
+            if (kp <= pos && (window <= 0 || kp > pos - window)) {
+                const int pidx = kp / P, page = pidx < bt_width ? block_table[(size_t)lr * bt_width + pidx] : -1;
+                if (page < 0 || page >= num_pages) atomicOr(err, AIE_DEV_PAGE_OOB);
+                else at = page * P + (kp - pidx * P);
             }
             if (++lc == ln && i + 1 < cnt) {
                 lc = 0;
@@ -344,20 +336,35 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
                 while (ln == 0 && lr < R);
             }
         }
-        cp_async_commit();
+        return at;
     };
+    int next_at = places(0);
+    auto fetch = [&](int i) {
+        if (i < cnt) {
+            bf16* dst = k_s + ((i % NST) * LD_KEYS + warp * (LD_KEYS / 8)) * SK + lane * 8;
 #pragma unroll
-    for (int i = 0; i < NST - 1; ++i) fetch(i);
+            for (int jj = 0; jj < LD_KEYS / 8; ++jj) {
+                const int at = __shfl_sync(0xffffffffu, next_at, warp * (LD_KEYS / 8) + jj);
+                const bf16* src = pages + (size_t)max(at, 0) * dk + lane * 8;
+                for (int x = lane; x < pieces; x += 32, src += 256) cp_async16(dst + jj * SK + (x - lane) * 8, src, at >= 0);
+            }
+        }
+        cp_async_commit();
+        next_at = places(i + 1);
+    };
+    fetch(0);
     const int steps = dk / 16, kg = warp & 3, kh = warp >> 2;
     const int step0 = kh ? (steps + 1) / 2 : 0, step1 = kh ? steps : (steps + 1) / 2;
     float acc[NT][4];
-    int n = 0, c_begin = 0;
+    int n = 0, c_begin = 0, pos = 0, lo = 0;
     bool fresh = true;
     for (int i = 0; i < cnt; ++i) {
         if (fresh) {                                              // a request begins: its queries, an empty softmax
             fresh = false;
             n = ld_chunks(q_len, ctx_len, R, window, r, first);
             c_begin = c;
+            pos = ctx_len[r];
+            lo = window > 0 ? max(pos - window + 1, 0) : 0;
             if (i > 0) __syncthreads();                           // the last one's sums have been read
             const int t = q_start[r];
             for (int rr = warp; rr < LT_ROWS; rr += LD_THREADS / 32) {
@@ -401,8 +408,7 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
         }
         __syncthreads();
         {                                                         // running softmax: sixteen threads a row, two keys a thread
-            const int row = tid >> 4, g = tid & 15, key = (first + c) * LD_KEYS + 2 * g, pos = ctx_len[r];
-            const int lo = window > 0 ? max(pos - window + 1, 0) : 0;
+            const int row = tid >> 4, g = tid & 15, key = (first + c) * LD_KEYS + 2 * g;
             const float2 x = *reinterpret_cast<const float2*>(s_s + row * SS + 2 * g);
             const float2 y = *reinterpret_cast<const float2*>(s_s + (LT_ROWS + row) * SS + 2 * g);
             const float v0 = key >= lo && key <= pos ? (x.x + y.x) * scale : -INFINITY;
@@ -552,27 +558,25 @@ extern "C" int aie_latent_decode(const float* q_full, const void* pages, void* o
                                  const float* sink, int pair, unsigned* err, cudaStream_t st) {
     if (R <= 0) return 0;
     if (rank < 64 || rank > 512 || rank % 64 || dk % 16 || dk < rank || dk > 1024 || H <= 0) return AIE_UNSUPPORTED;
-    if (G < 1 || G > 4096 || !part_o || !part_ml || P <= 0) return AIE_BAD_ARG;
+    if (G < 1 || G > 4096 || !part_o || !part_ml || P <= 0 || (long long)num_pages * P > 0x7fffffffLL) return AIE_BAD_ARG;
     const dim3 grid(G, (H + LT_ROWS - 1) / LT_ROWS);
     if (grid.y > 65535 || H > 65535) return AIE_UNSUPPORTED;
-    const auto smem = [&](int nst) {
-        return (size_t)(LT_ROWS + nst * LD_KEYS) * (dk + 8) * 2 + 64 + (size_t)(pair ? 2 : 1) * LT_ROWS * (LD_KEYS + 8) * 2 +
-               (size_t)(2 * LT_ROWS * (LD_KEYS + 2) + 3 * LT_ROWS) * 4;
-    };
-    const bool deep = smem(4) <= 225 * 1024;             // four stages, or two for the longest rows
+    const size_t smem = (size_t)(LT_ROWS + 2 * LD_KEYS) * (dk + 8) * 2 + 64 + (size_t)(pair ? 2 : 1) * LT_ROWS * (LD_KEYS + 8) * 2 +
+                        (size_t)(2 * LT_ROWS * (LD_KEYS + 2) + 3 * LT_ROWS) * 4;
+    const bool two = 2 * (smem + 1024) <= (size_t)aie_smem_per_sm();      // rows of up to about 640 elements
     cudaError_t e = cudaSuccess;
-#define GO2(NT, PV, NS)                                                                                                 \
+#define GO2(NT, PV, CTAS)                                                                                               \
     {                                                                                                                   \
-        auto kern = latent_decode_kernel<NT, PV, NS>;                                                                   \
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(NS));                     \
+        auto kern = latent_decode_kernel<NT, PV, CTAS>;                                                                 \
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                         \
         if (e == cudaSuccess)                                                                                           \
-            e = launch_pdl(kern, grid, dim3(LD_THREADS), smem(NS), st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, \
+            e = launch_pdl(kern, grid, dim3(LD_THREADS), smem, st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, \
                            q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, R, H, dk, window, scale, sink, err); \
     }
 #define GO(NT)                                                                                                          \
     case NT:                                                                                                            \
-        if (pair) { if (deep) GO2(NT, true, 4) else GO2(NT, true, 2) }                                                  \
-        else { if (deep) GO2(NT, false, 4) else GO2(NT, false, 2) }                                                     \
+        if (pair) { if (two) GO2(NT, true, 2) else GO2(NT, true, 1) }                                                   \
+        else { if (two) GO2(NT, false, 2) else GO2(NT, false, 1) }                                                      \
         break;
     switch (rank / 64) {
         GO(1) GO(2) GO(3) GO(4) GO(5) GO(6) GO(7) GO(8)

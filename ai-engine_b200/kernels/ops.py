@@ -1022,7 +1022,7 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
         if lone:
             # one token a request: the visible rows of all of them in equal stretches, one a CTA.  (Behind the other kernel, whose
             # join of parts runs over every token's row.)
-            G = max(1, sm_count() // ((H + 15) // 16))
+            G = max(1, 2 * sm_count() // ((H + 15) // 16))
             part_o = torch.empty((G + ctx.R, H, rank), dtype=torch.float32, device=q_full.device)
             part_ml = torch.empty((G + ctx.R, H, 2), dtype=torch.float32, device=q_full.device)
             with region("latent_attention_tc", *cost):
