@@ -11,7 +11,7 @@
 // product underflows to the zero it stands for.  All sums and products are float32 on the FMA units, as they were: one
 // bfloat16 or TF32 term would lose bits of keys, queries and the state, and three terms cost what this does.
 // What bounds it: the products' multiply-adds (2.7 M per chunk and head of 128 x 128).
-#include "common.cuh"
+#include "chunk_find.cuh"
 
 #define LC_T 64             // tokens of a chunk
 #define LC_THREADS 256
@@ -24,42 +24,6 @@ struct LcArgs {
     int ld, ld_decay, H, R, d, dv, max_slots, min_len;
     float q_scale, k_scale;
 };
-
-__device__ __forceinline__ int lc_chunks(const LcArgs& p, int r) {
-    const int n = r < p.R ? p.q_len[r] : 0;
-    return n >= p.min_len ? (n + LC_T - 1) / LC_T : 0;
-}
-
-// Request and chunk of the idx-th chunk of the step (requests in order, those below min_len left out); r < 0: none.
-// All threads of the block call it.
-__device__ __forceinline__ void lc_find(const LcArgs& p, int idx, int* found, int& r, int& c) {
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        int rr = -1, cc = 0, before = 0;
-        for (int base = 0; base < p.R && rr < 0; base += 32) {
-            const int m = lc_chunks(p, base + lane);
-            int run = m;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, run, o);
-                if (lane >= o) run += up;
-            }
-            const unsigned hit = __ballot_sync(0xffffffffu, idx < before + run);
-            if (hit) {
-                const int l = __ffs(hit) - 1;
-                rr = base + l;
-                cc = idx - before - __shfl_sync(0xffffffffu, run - m, l);
-            }
-            before += __shfl_sync(0xffffffffu, run, 31);
-        }
-        if (lane == 0) {
-            found[0] = rr;
-            found[1] = cc;
-        }
-    }
-    __syncthreads();
-    r = found[0];
-    c = found[1];
-}
 
 __device__ __forceinline__ float4 f4(float x) { return make_float4(x, x, x, x); }
 __device__ __forceinline__ float4 mul4(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
@@ -144,7 +108,7 @@ __global__ void __launch_bounds__(LC_THREADS, 2) lc_chunk_kernel(LcArgs p) {
     float* vs = as + LC_T * D;         // [64][DV]
     const int tid = threadIdx.x, h = blockIdx.y;
     int r, c;
-    lc_find(p, blockIdx.x, found, r, c);
+    chunk_find<LC_T>(p.q_len, p.R, p.min_len, blockIdx.x, found, r, c);
     if (r < 0) return;
     const int nt = min(LC_T, p.q_len[r] - c * LC_T);
     const size_t a0 = (size_t)p.q_start[r] + c * LC_T;
@@ -202,7 +166,7 @@ __global__ void __launch_bounds__(LC_THREADS, 2) lc_chunk_kernel(LcArgs p) {
 // four elements; eight chunks' loads are in flight while the chain of multiply-adds runs.
 __global__ void __launch_bounds__(LC_THREADS) lc_scan_kernel(LcArgs p) {
     const int r = blockIdx.y / p.H, h = blockIdx.y % p.H;
-    const int n = lc_chunks(p, r);
+    const int n = chunk_count<LC_T>(p.q_len, p.R, p.min_len, r);
     if (n == 0) return;
     const int slot = p.slots[r];
     if (slot < 0 || slot >= p.max_slots) {
@@ -212,7 +176,7 @@ __global__ void __launch_bounds__(LC_THREADS) lc_scan_kernel(LcArgs p) {
     const int e = (blockIdx.x * LC_THREADS + threadIdx.x) * 4, size = p.d * p.dv;
     if (e >= size) return;
     int first = 0;
-    for (int i = 0; i < r; ++i) first += lc_chunks(p, i);
+    for (int i = 0; i < r; ++i) first += chunk_count<LC_T>(p.q_len, p.R, p.min_len, i);
     const int row = e / p.dv;
     float* sp = p.state + ((size_t)slot * p.H + h) * size + e;
     float* L = p.L + ((size_t)first * p.H + h) * size + e;
@@ -297,7 +261,7 @@ __global__ void __launch_bounds__(LC_THREADS, 2) lc_out_kernel(LcArgs p) {
     float* A = as + LC_T * D;          // [64][64]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
     int r, c;
-    lc_find(p, blockIdx.x, found, r, c);
+    chunk_find<LC_T>(p.q_len, p.R, p.min_len, blockIdx.x, found, r, c);
     if (r < 0) return;
     const int nt = min(LC_T, p.q_len[r] - c * LC_T);
     const size_t a0 = (size_t)p.q_start[r] + c * LC_T;

@@ -1044,6 +1044,10 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
 
 SSD_MIN_TOKENS = 32      # portions from this length on take the chunked state-space kernel (bfloat16 mode)
 SSD_CHUNK = 64           # its chunk
+# Steps whose portions hold this many tokens together take the kernels that are parallel over chunks: (heads, portions of n
+# tokens each) 12 us walking the chunks against 18 in parallel (64, 1 x 64), 19 against 18 (32, 1 x 128), 33 against 24 (64, 1 x
+# 256), 36 against 27 (64, 4 x 64), 242 against 137 (64, 1 x 2048)
+SSD_PARALLEL_TOKENS = 160
 
 
 LC_CHUNK = 64            # chunk of the chunk-parallel kernels of the linear recurrence
@@ -1116,14 +1120,20 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
     max_len = 0
     if (chunked and dt_raw is not None and decay_tok is None and d <= 128 and ctx.max_q_len >= SSD_MIN_TOKENS
             and not os.environ.get("AI_ENGINE_B200_NO_CHUNKED_SCAN")):      # the switch is for measurement
-        lib = library("state_space_chunked.cu")
+        args = (_p(q), _p(k), _p(v), c_int(ld), _p(dt_raw), c_int(dt_raw.stride(0)), _p(dt_bias), _p(a_log), _p(skip), _p(state), _p(out))
+        lists = (_p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d), c_int(dv), c_int(heads_per_group),
+                 c_int(state.shape[0]), c_int(SSD_MIN_TOKENS))
         with region("state_space_chunked", _nb(out) + T * H * (2 * d // heads_per_group + dv) * 4,
                     2.0 * T * H * (SSD_CHUNK * (d + dv) / 2 + 2 * d * dv)):
-            check(lib.aie_state_space_chunked(_p(q), _p(k), _p(v), c_int(ld), _p(dt_raw), c_int(dt_raw.stride(0)), _p(dt_bias),
-                                              _p(a_log), _p(skip), _p(state), _p(out), _p(ctx.q_start), _p(ctx.q_len),
-                                              _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d), c_int(dv),
-                                              c_int(heads_per_group), c_int(state.shape[0]), c_int(SSD_MIN_TOKENS),
-                                              _p(ctx.err), _stream()), "state_space_chunked")
+            lens = ctx.h_q_len[ctx.h_q_len >= SSD_MIN_TOKENS]
+            if int(lens.sum()) >= SSD_PARALLEL_TOKENS and ctx.R * H <= 65535:
+                chunks = int(((lens + SSD_CHUNK - 1) // SSD_CHUNK).sum())
+                L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
+                G = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
+                check(library("state_space_parallel.cu").aie_state_space_parallel(
+                    *args, _p(L), _p(G), *lists, c_int(chunks), _p(ctx.err), _stream()), "state_space_parallel")
+            else:
+                check(library("state_space_chunked.cu").aie_state_space_chunked(*args, *lists, _p(ctx.err), _stream()), "state_space_chunked")
         if int(ctx.h_q_len.min()) >= SSD_MIN_TOKENS:
             return out
         max_len = SSD_MIN_TOKENS - 1                # the shorter portions and single tokens of the same step
