@@ -61,6 +61,13 @@ template <int BN> struct TcSmem {
 };
 
 #define TC_EPI_STORE 0
+// Grouped rows: from so many tiles of 64 rows an expert on (its share of the empty ones too), two of an expert's tiles share a
+// weight tile.  Single tiles are bound by what 128 x 64 of weights and 64 x 64 of tokens a stage cost between L2 and shared memory;
+// a pair moves a third less for each.  us, single -> pairs, at 128 / 192 / 256 / 512 / 1,024 rows an expert: 32 experts of 2,048 x
+// 2,048 72 / 86 / 117 / 183 / 382 -> 69 / 82 / 102 / 157 / 301; 8 of 4,096 x 2,048 40 / 44 / 58 / 99 / 203 -> 36 / 51 / 56 / 87 / 162;
+// 64 of 1,024 x 2,048 73 / 89 / 119 / 195 / 383 -> 71 / 89 / 105 / 168 / 318; at 64 rows 56, 30, 56 -> 65, 35, 68.  Two
+// blocks an SM with three stages instead of three with two: 106 and 327 at 256 and 1,024 rows of the first.
+#define TC_PAIR_TILES 4
 #define TC_EPI_SWIGLU 1
 #define TC_EPI_ROPE 2       // the fused q/k/v projection: rotate q and k by position, write k and v into their pages
 
@@ -118,16 +125,30 @@ template <int BN, int EPI, typename OT>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                OT* __restrict__ C, int T, int N, int K, int ldc, int kb_per_split, int STAGES, int raw_parts,
-               unsigned* err, const TcRope rope, const int* __restrict__ tile_w, const TcGlu glu) {
+               unsigned* err, const TcRope rope, const int* __restrict__ tile_w, int tile_rows, const TcGlu glu) {
     constexpr int TMEM_COLS = BN < 32 ? 32 : BN;
     // grouped rows: token tile y multiplies the weight tile_w[y] of a stack of [N, K] weights (-1: an empty tile).
     // The list is the previous kernel's output, so it is read behind the dependency wait.
-    int w_row0 = 0;
+    // Tiles of half of BN tokens: the first, third, ... of an expert's tiles take the next one with them where it is there (a
+    // weight tile is then read once for both), the others have nothing to do.
+    constexpr bool PAIRS = BN == 128 && EPI == TC_EPI_STORE;
+    int w_row0 = 0, t0 = blockIdx.y * BN, tokens = BN;
     if (tile_w) {
         pdl_wait();
-        const int e = tile_w[blockIdx.y];
+        const int y = blockIdx.y, e = tile_w[y];
         if (e < 0) return;
         w_row0 = e * N;
+        if (PAIRS && tile_rows == BN / 2) {
+            int first = y;
+            for (unsigned same = ~0u; same == ~0u;) {     // a warp looks at the 32 tiles before
+                const int i = first - 1 - (int)(threadIdx.x & 31);
+                same = __ballot_sync(0xffffffffu, i >= 0 && tile_w[max(i, 0)] == e);
+                first -= same == ~0u ? 32 : __ffs(~same) - 1;
+            }
+            if ((y - first) & 1) return;
+            t0 = y * tile_rows;
+            tokens = y + 1 < (int)gridDim.y && tile_w[y + 1] == e ? BN : BN / 2;
+        }
     }
     extern __shared__ unsigned char tc_raw[];
     unsigned char* bars = reinterpret_cast<unsigned char*>(((size_t)tc_raw + 1023) & ~(size_t)1023);
@@ -140,7 +161,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     float* tile_s = reinterpret_cast<float*>(base);      // [BN][128] partial tile, after the ring is idle
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n0 = blockIdx.x * TC_BM, t0 = blockIdx.y * BN;
+    const int n0 = blockIdx.x * TC_BM;
     // parts of K: joined inside a cluster (parts == cluster size), or left to the consumer
     // (raw_parts: part z is stored as it is at C + z * T * ldc and the next kernel adds them)
     const int parts = raw_parts ? 1 : gridDim.z;
@@ -172,30 +193,35 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
     if (warp == 0) {
         if (lane == 0) {
+            const int bytes = TcSmem<BN>::stage_bytes - (BN - tokens) * TC_BK * 2;
+            auto load_x = [&](unsigned char* st, unsigned long long* bar, int k) {     // in the map's boxes
+                tma_load_2d(st + TC_BM * TC_BK * 2, &map_x, bar, k, t0);
+                if (PAIRS && tile_rows == BN / 2 && tokens == BN)
+                    tma_load_2d(st + (TC_BM + BN / 2) * TC_BK * 2, &map_x, bar, k, t0 + BN / 2);
+            };
             // weights do not depend on the previous kernel: request the first ring of W tiles now
             const int pre = min(nkb, STAGES);
             for (int i = 0; i < pre; ++i) {
-                mbar_expect_tx(&full[i], TcSmem<BN>::stage_bytes);
+                mbar_expect_tx(&full[i], bytes);
                 tma_load_2d(base + i * TcSmem<BN>::stage_bytes, &map_w, &full[i], (kb_begin + i) * TC_BK, w_row0 + n0);
             }
             pdl_wait();        // the tokens are the previous kernel's output
             for (int i = 0; i < pre; ++i)
-                tma_load_2d(base + i * TcSmem<BN>::stage_bytes + TC_BM * TC_BK * 2, &map_x, &full[i],
-                            (kb_begin + i) * TC_BK, t0);
+                load_x(base + i * TcSmem<BN>::stage_bytes, &full[i], (kb_begin + i) * TC_BK);
             for (int i = pre; i < nkb; ++i) {
                 const int s = i % STAGES;
                 const unsigned ph = (i / STAGES) & 1;
                 if (!mbar_wait(&empty[s], ph ^ 1, abort_flag, err)) break;
                 unsigned char* st = base + s * TcSmem<BN>::stage_bytes;
-                mbar_expect_tx(&full[s], TcSmem<BN>::stage_bytes);
+                mbar_expect_tx(&full[s], bytes);
                 const int k = (kb_begin + i) * TC_BK;
                 tma_load_2d(st, &map_w, &full[s], k, w_row0 + n0);
-                tma_load_2d(st + TC_BM * TC_BK * 2, &map_x, &full[s], k, t0);
+                load_x(st, &full[s], k);
             }
         }
     } else if (warp == 1) {
         if (lane == 0 && nkb > 0) {
-            const unsigned idesc = umma_idesc(BN);
+            const unsigned idesc = umma_idesc(tokens);
             bool ok = true;
             for (int i = 0; i < nkb; ++i) {
                 const int s = i % STAGES;
@@ -224,6 +250,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         const bool direct = parts == 1 && EPI == TC_EPI_STORE;
 #pragma unroll
         for (int c0 = 0; c0 < BN; c0 += 16) {
+            if (PAIRS && c0 >= tokens) break;
             unsigned v[16];
             if (ok) {
                 const unsigned taddr = tmem_d + ((unsigned)(quarter * 32) << 16) + (unsigned)c0;
@@ -262,9 +289,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             const int e = tid - 64;                        // 0 .. 127
             const unsigned tile_addr = tc_smem(tile_s);
             const int rank = (int)cluster_rank();
-            const int tokens = min(BN, T - t0);
+            const int rows = min(BN, T - t0);
             constexpr int COLS = EPI == TC_EPI_STORE ? TC_BM : TC_BM / 2;      // outputs per token
-            const int total = tokens * COLS;
+            const int total = rows * COLS;
             const int share = (total + parts - 1) / parts;
             const int f0 = blockIdx.x * COLS, width = EPI == TC_EPI_STORE ? N : N / 2;
             for (int idx = rank * share + e; idx < min((rank + 1) * share, total); idx += 128) {
@@ -355,12 +382,12 @@ static int make_map(CUtensorMap* map, const void* ptr, int rows, int K, int box_
 template <int BN, int EPI, typename OT>
 static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int T, int N, int K, int ldc,
                      int splits, int raw_parts, unsigned* err, cudaStream_t st, const TcRope& rope = TcRope(),
-                     const int* tile_w = nullptr, const TcGlu glu = TcGlu{INFINITY, 1.f, 0.f}) {
+                     const int* tile_w = nullptr, const TcGlu glu = TcGlu{INFINITY, 1.f, 0.f}, int tile_rows = BN) {
     const int kb_total = (K + TC_BK - 1) / TC_BK;
     const int kbps = (kb_total + splits - 1) / splits;
     auto kern = gemm_tc_kernel<BN, EPI, OT>;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((N + TC_BM - 1) / TC_BM, (T + BN - 1) / BN, splits);
+    cfg.gridDim = dim3((N + TC_BM - 1) / TC_BM, (T + tile_rows - 1) / tile_rows, splits);
     const long long ctas = (long long)cfg.gridDim.x * cfg.gridDim.y * cfg.gridDim.z;
     // the deepest ring that still lets the grid's CTAs sit beside each other: one, two or three to an SM
     // (228 KB of shared memory an SM, 1 KB of it reserved per CTA); a grid of more than three waves
@@ -390,7 +417,7 @@ static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, void* C, int 
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mw, mx, (OT*)C, T, N, K, ldc, kbps, stages, raw_parts, err, rope, tile_w, glu);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mw, mx, (OT*)C, T, N, K, ldc, kbps, stages, raw_parts, err, rope, tile_w, tile_rows, glu);
     return (int)e;
 }
 
@@ -447,12 +474,15 @@ extern "C" int aie_gemm_tc_grouped(const void* X, const void* W, void* C, int ou
     rc = make_map(&mx, X, rows, K, bn);
     if (rc) return rc;
     if (N % TC_BM) return AIE_UNSUPPORTED;       // a weight tile must not reach into the next expert's rows
+    const TcGlu none = {INFINITY, 1.f, 0.f};
 #define GG(BNV)                                                                                                   \
-    rc = out_dtype == AIE_BF16 ? launch_tc<BNV, TC_EPI_STORE, bf16>(mw, mx, C, rows, N, K, ldc, 1, 0, err, stream, TcRope(), tile_w) \
-       : out_dtype == AIE_F32 ? launch_tc<BNV, TC_EPI_STORE, float>(mw, mx, C, rows, N, K, ldc, 1, 0, err, stream, TcRope(), tile_w) \
+    rc = out_dtype == AIE_BF16 ? launch_tc<BNV, TC_EPI_STORE, bf16>(mw, mx, C, rows, N, K, ldc, 1, 0, err, stream, TcRope(), tile_w, none, bn) \
+       : out_dtype == AIE_F32 ? launch_tc<BNV, TC_EPI_STORE, float>(mw, mx, C, rows, N, K, ldc, 1, 0, err, stream, TcRope(), tile_w, none, bn) \
        : AIE_BAD_ARG
     switch (bn) {
-        case 64: GG(64); break;
+        case 64:
+            if (rows / bn >= TC_PAIR_TILES * E) { GG(128); } else { GG(64); }
+            break;
         case 128: GG(128); break;
         default: return AIE_BAD_ARG;
     }
