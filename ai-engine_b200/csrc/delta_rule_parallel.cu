@@ -8,10 +8,10 @@
 //   walk     every (request, head, 16 or 32 columns): U = U0 - W S,  S <- exp(l_Q) S + (w K)^T U  from chunk to chunk; U takes
 //            U0's place, the states that chunks start from are kept
 //   out      every (chunk, head): O = exp(l_t) Q S_0 + P U
-// The walk is the chain that bounds it, 2.7 us a chunk with 16 columns a block and 3.5 with 32: half of it is the rate of mma.sync
-// (128 instructions a scheduler), the rest two products, two barriers and the exchange of the state one after the other.  W and
-// the keys straight from L2 to the registers of their products instead of through shared memory: 2.4 us at d = 128, but 5 %
-// slower at d = 64.
+// The walk is the chain that bounds it, 2.7 us a chunk with 16 columns a block and 3.5 with 32: two products, two barriers and the
+// exchange of the state one after the other on eight warps an SM, no unit near its limit (shared memory 50 %, L2 26 %).  A third
+// stage of W and the keys in shared memory changed nothing; both straight from L2 to the registers of their products: 2.4 us at
+// d = 128, but 5 % slower at d = 64.
 // T is made in float32: diagonal blocks of 16 by forward substitution, what is below from them.  T, beta V and beta exp(l)
 // enter the products of U0 and W as three bfloat16 values, all 24 bits; on the FMA units prepare took 39 us.  Everything else
 // enters mma.sync as pairs of bfloat16 values, as before, with float32 sums; the products that the state or the output is summed
