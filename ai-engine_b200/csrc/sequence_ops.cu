@@ -334,17 +334,17 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const float* 
 }
 
 // The same 16 bytes a thread: `lanes` lanes (8, 16 or 32) of a warp share a row of 4 lanes NV floats, and a lane fetches the
-// rows of four (token, head) pairs before it uses the first.  Bound by memory: 2,048 tokens x 16 heads of 128 with a gate
-// (42 MB) 16.4 us a float at a time.
-#define HN_ROWS 4
-template <int NV, typename O>
+// rows of ROWS (token, head) pairs before it uses the first.  Every sum that could become a fused multiply-add is written out as
+// one or kept from it: a row's bits are the same for any ROWS, so they do not depend on how many rows there are.  Bound by memory: 2,048 tokens x 16 heads of 128 with a gate (42 MB) 16.4 us a float at a time.
+template <int NV, int ROWS, typename O>
 __global__ void head_norm_gate4_kernel(const float* __restrict__ o, const float* __restrict__ g, int ldg,
                                        const float* __restrict__ w, O* __restrict__ out, int TH, int H, int lanes, float eps) {
     const int dv = lanes * 4 * NV, per_warp = 32 / lanes, lane = threadIdx.x & 31, c = (lane % lanes) * 4;
-    const int first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp * HN_ROWS + lane / lanes;
-    float4 x[HN_ROWS][NV], gv[HN_ROWS][NV];
+    const auto one_plus = [](float e) { return __fadd_rn(1.0f, e); };
+    const int first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp * ROWS + lane / lanes;
+    float4 x[ROWS][NV], gv[ROWS][NV];
 #pragma unroll
-    for (int k = 0; k < HN_ROWS; ++k) {
+    for (int k = 0; k < ROWS; ++k) {
         const int wi = first + k * per_warp;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -356,11 +356,12 @@ __global__ void head_norm_gate4_kernel(const float* __restrict__ o, const float*
         }
     }
 #pragma unroll
-    for (int k = 0; k < HN_ROWS; ++k) {
+    for (int k = 0; k < ROWS; ++k) {
         const int wi = first + k * per_warp;
         float ss = 0.f;
 #pragma unroll
-        for (int v = 0; v < NV; ++v) ss += (x[k][v].x * x[k][v].x + x[k][v].y * x[k][v].y) + (x[k][v].z * x[k][v].z + x[k][v].w * x[k][v].w);
+        for (int v = 0; v < NV; ++v)
+            ss = fmaf(x[k][v].w, x[k][v].w, fmaf(x[k][v].z, x[k][v].z, fmaf(x[k][v].y, x[k][v].y, fmaf(x[k][v].x, x[k][v].x, ss))));
         for (int off = lanes >> 1; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
         const float r = 1.0f / sqrtf(ss / (float)dv + eps);
         if (wi >= TH) continue;
@@ -373,8 +374,8 @@ __global__ void head_norm_gate4_kernel(const float* __restrict__ o, const float*
             }
             if (g) {
                 const float4 z = gv[k][v];
-                y = make_float4(y.x * (z.x / (1.0f + expf(-z.x))), y.y * (z.y / (1.0f + expf(-z.y))),
-                                y.z * (z.z / (1.0f + expf(-z.z))), y.w * (z.w / (1.0f + expf(-z.w))));
+                y = make_float4(y.x * (z.x / one_plus(expf(-z.x))), y.y * (z.y / one_plus(expf(-z.y))),
+                                y.z * (z.z / one_plus(expf(-z.z))), y.w * (z.w / one_plus(expf(-z.w))));
             }
             store4<O>(out + (size_t)wi * dv + v * lanes * 4 + c, y);
         }
@@ -387,18 +388,20 @@ extern "C" int aie_head_norm_gate(const float* o, const float* g, int ldg, const
     if (H <= 0 || dv <= 0) return AIE_BAD_ARG;
     const long long warps = (long long)T * H;
     const size_t esz = out_dtype == AIE_F32 ? 4 : 2;
-    // rows of 32, 64, 128 or 256 floats on 16 bytes, and enough of them that four to a lane still fill the machine
+    // rows of 32, 64, 128 or 256 floats on 16 bytes; four of them a lane where that still fills the machine
     if ((dv == 32 || dv == 64 || dv == 128 || dv == 256) && ldg % 4 == 0 && !(((size_t)o | (size_t)g | (size_t)w) & 15) &&
-        !((size_t)out & (4 * esz - 1)) && (out_dtype == AIE_F32 || out_dtype == AIE_BF16) && warps >= 4096 && warps < 0x40000000LL) {
-        const int lanes = dv >= 128 ? 32 : dv / 4, rows = 32 / lanes * HN_ROWS * 4;
+        !((size_t)out & (4 * esz - 1)) && (out_dtype == AIE_F32 || out_dtype == AIE_BF16) && warps < 0x40000000LL) {
+        const int lanes = dv >= 128 ? 32 : dv / 4, each = warps >= 4096 ? 4 : 1, rows = 32 / lanes * each * 4;
         const unsigned blocks4 = (unsigned)((warps + rows - 1) / rows);
-#define GO(NV, O) head_norm_gate4_kernel<NV, O><<<blocks4, 128, 0, st>>>(o, g, ldg, w, (O*)out, (int)warps, H, lanes, eps)
+#define GO2(NV, ROWS, O) head_norm_gate4_kernel<NV, ROWS, O><<<blocks4, 128, 0, st>>>(o, g, ldg, w, (O*)out, (int)warps, H, lanes, eps)
+#define GO(NV, O) if (each == 4) GO2(NV, 4, O); else GO2(NV, 1, O)
         if (out_dtype == AIE_F32) {
-            if (dv == 256) GO(2, float); else GO(1, float);
+            if (dv == 256) { GO(2, float); } else { GO(1, float); }
         } else {
-            if (dv == 256) GO(2, bf16); else GO(1, bf16);
+            if (dv == 256) { GO(2, bf16); } else { GO(1, bf16); }
         }
 #undef GO
+#undef GO2
         AIE_LAUNCH_CHECK();
     }
     const unsigned blocks = (unsigned)((warps + 3) / 4);
@@ -936,20 +939,23 @@ __global__ void gate_group_norm_kernel(const float* __restrict__ y, const float*
     }
 }
 
-// The same with a warp a (token, part) of 128 NV floats on 16 bytes: y and z are read once, all of a lane's loads side by
-// side.  Bound by memory: 2,048 tokens of 4,096 in eight parts (84 MB) took 38 us in two passes of a block a part.
-template <int NV, typename O>
+// The same with WARPS warps a (token, part) of 128 NV WARPS floats on 16 bytes: y and z are read once, all of a lane's loads side
+// by side.  Bound by memory: 2,048 tokens of 4,096 in eight parts (84 MB) took 38 us in two passes of a block a part.  Parts of
+// 1,024 are shared by four warps: one warp's sixteen loads and exponentials took 2 us longer where parts are few.
+template <int NV, int WARPS, typename O>
 __global__ void __launch_bounds__(256)
 gate_group_norm4_kernel(const float* __restrict__ y, const float* __restrict__ z, int ldz, const float* __restrict__ w,
                         O* __restrict__ out, int W, int parts, int rows, float eps) {
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= rows) return;
-    const int t = row / parts, n = 128 * NV, c0 = (row % parts) * n + lane * 4;
+    __shared__ float red[8];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = blockIdx.x * (8 / WARPS) + warp / WARPS;
+    const int t = row / parts, n = 128 * NV * WARPS, c0 = (row % parts) * n + (warp % WARPS) * 128 * NV + lane * 4;
+    const bool on = row < rows;
+    if (WARPS == 1 && !on) return;
     float4 yv[NV], zv[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        yv[v] = *reinterpret_cast<const float4*>(y + (size_t)t * W + c0 + v * 128);
-        zv[v] = *reinterpret_cast<const float4*>(z + (size_t)t * ldz + c0 + v * 128);
+        yv[v] = on ? *reinterpret_cast<const float4*>(y + (size_t)t * W + c0 + v * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
+        zv[v] = on ? *reinterpret_cast<const float4*>(z + (size_t)t * ldz + c0 + v * 128) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     float ss = 0.f;
 #pragma unroll
@@ -961,6 +967,14 @@ gate_group_norm4_kernel(const float* __restrict__ y, const float* __restrict__ z
         ss += (yv[v].x * yv[v].x + yv[v].y * yv[v].y) + (yv[v].z * yv[v].z + yv[v].w * yv[v].w);
     }
     ss = warp_sum(ss);
+    if (WARPS > 1) {
+        if (lane == 0) red[warp] = ss;
+        __syncthreads();
+        ss = 0.f;
+#pragma unroll
+        for (int i = 0; i < WARPS; ++i) ss += red[warp / WARPS * WARPS + i];
+        if (!on) return;
+    }
     const float r = 1.0f / sqrtf(ss / (float)n + eps);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
@@ -977,18 +991,17 @@ extern "C" int aie_gate_group_norm(const float* y, const float* z, int ldz, cons
     const long long blocks = (long long)T * parts;
     if (blocks > 0x7fffffffLL) return AIE_UNSUPPORTED;
     const size_t esz = out_dtype == AIE_F32 ? 4 : 2;
-    // parts of 128, 256, 512 or 1,024 floats; fewer than 1,024 of them leave most of the machine without a warp, and a block a
-    // part is the wider reader then
-    if ((n == 128 || n == 256 || n == 512 || n == 1024) && ldz % 4 == 0 && blocks >= 1024 &&
+    // parts of 128, 256, 512 or 1,024 floats, however many there are: a part's bits do not depend on the others
+    if ((n == 128 || n == 256 || n == 512 || n == 1024) && ldz % 4 == 0 &&
         !(((size_t)y | (size_t)z | (size_t)w) & 15) && !((size_t)out & (4 * esz - 1)) && (out_dtype == AIE_F32 || out_dtype == AIE_BF16)) {
-        const unsigned grid = (unsigned)((blocks + 7) / 8);
-#define GO(NV)                                                                                                              \
-    if (out_dtype == AIE_F32) gate_group_norm4_kernel<NV, float><<<grid, 256, 0, st>>>(y, z, ldz, w, (float*)out, W, parts, (int)blocks, eps); \
-    else gate_group_norm4_kernel<NV, bf16><<<grid, 256, 0, st>>>(y, z, ldz, w, (bf16*)out, W, parts, (int)blocks, eps)
-        if (n == 128) { GO(1); }
-        else if (n == 256) { GO(2); }
-        else if (n == 512) { GO(4); }
-        else { GO(8); }
+#define GO(NV, WARPS)                                                                                                       \
+    const unsigned grid = (unsigned)((blocks * WARPS + 7) / 8);                                                             \
+    if (out_dtype == AIE_F32) gate_group_norm4_kernel<NV, WARPS, float><<<grid, 256, 0, st>>>(y, z, ldz, w, (float*)out, W, parts, (int)blocks, eps); \
+    else gate_group_norm4_kernel<NV, WARPS, bf16><<<grid, 256, 0, st>>>(y, z, ldz, w, (bf16*)out, W, parts, (int)blocks, eps)
+        if (n == 128) { GO(1, 1); }
+        else if (n == 256) { GO(2, 1); }
+        else if (n == 512) { GO(4, 1); }
+        else { GO(2, 4); }
 #undef GO
         AIE_LAUNCH_CHECK();
     }
