@@ -1053,27 +1053,34 @@ CHUNK_STATES_BYTES = 1 << 30       # the most that the states of a step's chunks
 
 
 LC_CHUNK = 64            # chunk of the chunk-parallel kernels of the linear recurrence
-# Their three launches cost about 42 us whatever they do; the token-by-token kernel costs 0.42 us a token of its longest
-# portion or 0.027 us a token and head of all of them, whichever is more: at (heads, portions of n tokens each) 27 against
-# 42 us (8, 1 x 64), 51 against 43 (8, 1 x 128), 63 against 44 (16, 4 x 32), 37 against 43 (16, 4 x 16), 66 against 48
-# (8, 16 x 16), 864 against 132 (16, 1 x 2048).  In a step that takes them, portions below eight tokens (single ones above all) stay with the other kernel.
-LC_MIN_WORK = 1700       # heads x tokens, or 16 x tokens of the longest portion
+# Their three launches take about 50 us however short the portions; the token-by-token kernel takes 7 us and 0.39 us a token of
+# the longest portion, and 0.025 us a token and head of all of them once these fill the machine.  us, token by token against in
+# chunks, heads of 128 x 128: 16 heads, one portion of 64 / 96 / 128 / 192 tokens 36 / 49 / 62 / 87 against 52 / 50 / 50 / 52, four
+# of 64 120 against 54, sixteen of 48 313 against 83, 618 + 350 + 55 tokens 398 against 77; 64 heads, one of 32 / 64: 68 / 119 against
+# 50 / 54.  A portion by itself breaks even at about 1,700 (heads x tokens), one beside others, which costs next to
+# nothing more in chunks, far earlier; the line lies at half of that, where one portion loses at most about 25 us either way.
+LC_MIN_WORK = 850        # heads x tokens, or 16 x tokens where heads are fewer, of a portion that takes them
 LC_MIN_TOKENS = 8
 
 
-def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, state, out, ctx, H, d, dv, lower, bias) -> bool:
-    """The portions of LC_MIN_TOKENS tokens or more by the chunk-parallel kernels; False (nothing is done) when the step is
-    small or the sizes, strides or addresses are not theirs: heads of up to 128 in steps of 4, rows that start on 16 bytes."""
-    if (ctx.max_q_len < LC_MIN_TOKENS or d > 128 or dv > 128 or d % 4 or dv % 4 or ld % 4 or ctx.R * H > 65535
+def lc_min_len(H: int) -> int:
+    """Portions from this length on take the chunk-parallel kernels.  A portion's own size decides, never what else is in
+    the step: its bits must not depend on its neighbours."""
+    return max(LC_MIN_TOKENS, -(-LC_MIN_WORK // max(H, 16)))
+
+
+def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, state, out, ctx, H, d, dv, lower, bias) -> int:
+    """The portions of lc_min_len(H) tokens or more by the chunk-parallel kernels: that length; 0 (nothing is done) when there
+    is none or the sizes, strides or addresses are not theirs: heads of up to 128 in steps of 4, rows that start on 16 bytes."""
+    min_len = lc_min_len(H)
+    if (ctx.max_q_len < min_len or d > 128 or dv > 128 or d % 4 or dv % 4 or ld % 4 or ctx.R * H > 65535
             or (decay_tok is not None and decay_tok.stride(0) % 4)
             or any(t is not None and t.data_ptr() % 16 for t in (q, k, v, decay_tok, state, lower, bias))):
-        return False
-    lens = ctx.h_q_len[ctx.h_q_len >= LC_MIN_TOKENS]
-    if max(H * int(lens.sum()), 16 * ctx.max_q_len) < LC_MIN_WORK:
-        return False
+        return 0
+    lens = ctx.h_q_len[ctx.h_q_len >= min_len]
     chunks = int(((lens + LC_CHUNK - 1) // LC_CHUNK).sum())
     if 4 * chunks * H * d * dv > CHUNK_STATES_BYTES:
-        return False
+        return 0
     L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
     G = torch.empty((chunks, H, d), dtype=torch.float32, device=q.device)
     lib = library("linear_recurrence_chunked.cu")
@@ -1083,9 +1090,9 @@ def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, 
                                                 c_int(decay_tok.stride(0) if decay_tok is not None else 0), _p(decay_head),
                                                 c_float(q_scale), c_float(k_scale), _p(state), _p(out), _p(L), _p(G),
                                                 _p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d),
-                                                c_int(dv), c_int(state.shape[0]), c_int(LC_MIN_TOKENS), c_int(chunks), _p(lower),
+                                                c_int(dv), c_int(state.shape[0]), c_int(min_len), c_int(chunks), _p(lower),
                                                 _p(bias), _p(ctx.err), _stream()), "linear_recurrence_chunked")
-    return True
+    return min_len
 
 
 def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_tok: Optional[torch.Tensor],
@@ -1093,7 +1100,8 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
                       ctx, H: int, d: int, dv: int, heads_per_group: int = 1, dt_raw: Optional[torch.Tensor] = None,
                       dt_bias: Optional[torch.Tensor] = None, a_log: Optional[torch.Tensor] = None,
                       skip: Optional[torch.Tensor] = None, chunked: bool = False, wide_state: bool = False,
-                      forget_lower: Optional[torch.Tensor] = None, forget_bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      forget_lower: Optional[torch.Tensor] = None, forget_bias: Optional[torch.Tensor] = None,
+                      in_order: bool = False) -> torch.Tensor:
     """S <- diag(a_t) S + k_t v_t^T, o_t = S^T q_t per request and head over the step's tokens, the state
     [max_seqs, H, d, dv] float32 read and left in each request's slot.  q, k [T, H * d] and v [T, H * dv] are
     float32 views with one row stride; decay_tok [T, H * d] float32 (rows any stride) or decay_head [H].
@@ -1106,6 +1114,8 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
     once, when it returns to its float32 slot.
     forget_lower [H * d] float32 (with forget_bias [H * d] or None): the keyless form.  k is None, decay_tok holds the
     forget gate's logits z, and the kernel makes a = l + (1 - l) sigmoid(z + bias), k = 1 - a and q = silu(q) itself.
+    in_order: tokens are walked one behind the other whatever the portion (the float32 engine: a request's bits depend
+    neither on its neighbours nor on how its prompt was cut); else portions of lc_min_len(H) tokens or more go in chunks.
     Returns o [T, H, dv] float32."""
     _dev(state, decay_head, dt_bias, a_log, skip, forget_lower, forget_bias)
     if forget_lower is not None:
@@ -1141,12 +1151,13 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
         if int(ctx.h_q_len.min()) >= SSD_MIN_TOKENS:
             return out
         max_len = SSD_MIN_TOKENS - 1                # the shorter portions and single tokens of the same step
-    elif (dt_raw is None and heads_per_group == 1 and skip is None
-          and _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, state, out, ctx, H, d, dv,
-                                    forget_lower, forget_bias)):
-        if int(ctx.h_q_len.min()) >= LC_MIN_TOKENS:
-            return out
-        max_len = LC_MIN_TOKENS - 1
+    elif dt_raw is None and heads_per_group == 1 and skip is None and not in_order:
+        taken = _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, state, out, ctx, H, d, dv,
+                                      forget_lower, forget_bias)
+        if taken:
+            if int(ctx.h_q_len.min()) >= taken:
+                return out
+            max_len = taken - 1
     lib = library("linear_recurrence.cu")
     with region("linear_recurrence", _nb(out) + T * H * (2 * d + dv) * 4 + 2 * ctx.R * H * d * dv * 4, 4.0 * T * H * d * dv):
         check(lib.aie_linear_recurrence(_p(q), _p(k), _p(v), c_int(ld), _p(decay_tok),

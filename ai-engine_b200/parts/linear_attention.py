@@ -100,7 +100,7 @@ class DecayLinearAttention(Mixer):
             ops.gemm_f32_ex(proj[:, 2 * Hd + 2 * Hv:], self.w_a2, z, T, Hd, self.r, proj.stride(0), Hd)
             decay_tok = ops.gated_decay(z, self.a2_bias, self.tau)
         o = ops.linear_recurrence(q, k, v, decay_tok, self.decay_head, self.q_scale, self.k_scale, cache.state, ctx,
-                                  self.H, self.d, self.dv)
+                                  self.H, self.d, self.dv, in_order=self.env.dtype == torch.float32)
         y = ops.head_norm_gate(o, g, self.out_weight, self.eps, self.env.dtype)
         if add_to is not None and ops.linear_add(add_to, y, self.w_o):
             return None
@@ -158,6 +158,7 @@ class ForgetGateLinearAttention(Mixer):
         proj = ops.linear(h, self.w_in, torch.float32, ctx.err)
         q, z, v = proj[:, :Hd], proj[:, Hd:2 * Hd], proj[:, 2 * Hd:]
         o = ops.linear_recurrence(q, None, v, z, None, 1.0, 1.0, cache.state, ctx, self.H, self.d, self.dv,
-                                  forget_lower=self.lower, forget_bias=self.f_bias)
+                                  forget_lower=self.lower, forget_bias=self.f_bias,
+                                  in_order=self.env.dtype == torch.float32)
         y = ops.head_norm_gate(o, None, self.out_weight, self.eps, self.env.dtype)
         return ops.linear_parts(y, self.w_o, ctx.err)

@@ -1,0 +1,66 @@
+"""Which kernel takes a portion is decided by the portion, never by what else is in the step: the state that a request leaves has
+the same bits alone and beside others, its outputs up to the order of the token-by-token kernel's sum over a state's rows, which
+follows the step's shape.  The float32 engine walks a recurrence token by token, so there the state's bits do not depend on how
+a prompt was cut either."""
+import pytest
+import torch
+
+from test_linear_recurrence_chunked_gpu import DEV, Ctx
+from test_pifutar_parts_gpu import linear_part
+from zupitar_helpers import Rig, load
+
+pytestmark = pytest.mark.gpu
+
+
+def alone_and_beside(run, lens, exact):
+    """run([(request, tokens)]): (outputs, state) of every request of one step.  exact(n): the outputs' bits are the same too."""
+    together = run(list(enumerate(lens)))
+    for i, n in enumerate(lens):
+        (out, state), (out2, state2) = run([(i, n)])[0], together[i]
+        assert torch.equal(state, state2), (i, n)
+        assert torch.equal(out, out2) if exact(n) else float((out - out2).abs().max()) <= 1e-5 * float(out.abs().max()), (i, n)
+
+
+@pytest.mark.parametrize("keyless", [False, True])
+@pytest.mark.parametrize("H,lens", [(16, [40, 300, 1, 53, 54, 9]), (40, [41, 12, 43, 42])])
+def test_linear_recurrence(H, lens, keyless):
+    from ai_engine_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    d = 32
+    rows = [rnd(n, 4 * H * d) for n in lens]
+    states, lower = rnd(len(lens), H, d, d), torch.rand(H * d, generator=gen, device=DEV)
+
+    def run(reqs):
+        x, state = torch.cat([rows[i] for i, _ in reqs]), states.clone()
+        q, k, v, a = (x[:, j * H * d:(j + 1) * H * d] for j in range(4))
+        ctx = Ctx([n for _, n in reqs], [i for i, _ in reqs])
+        out = ops.linear_recurrence(q, None if keyless else k, v, a if keyless else torch.sigmoid(a), None, 0.3, 1.0, state, ctx, H, d, d,
+                                    forget_lower=lower if keyless else None)
+        assert int(ctx.err.item()) == 0
+        return [(o, state[i]) for o, (i, _) in zip(out.split([n for _, n in reqs]), reqs)]
+
+    alone_and_beside(run, lens, lambda n: n >= ops.lc_min_len(H))
+
+
+@pytest.mark.parametrize("kind,extra", [("retention", [0.5, 0.9, 0.99]), ("gla", 8.0)])
+def test_float32_linear_attention_whole_and_in_portions(kind, extra):
+    D, H, d, dv, n = 48, 3, 16, 32, 190
+    g = torch.Generator().manual_seed(5)
+    r = lambda *s: torch.randn(*s, generator=g) / s[-1] ** 0.5
+    ts = {"q": r(H * d, D), "k": r(H * d, D), "v": r(H * dv, D), "g": r(H * dv, D), "o": r(D, H * dv)}
+    ts.update({"norm": 1.0 + r(dv), "a1": r(6, D), "a2": r(H * d, 6), "a2.b": 2.0 + r(H * d)} if kind == "gla" else {})
+    part = load(linear_part(torch.float32, D, kind, H, d, dv, extra), ts, torch.float32)
+    h, outs, states = torch.randn(n, D, generator=g), [], []
+    for cuts in ([n], [120, 7, 1, 62]):
+        rig, at, got = Rig(part, torch.float32), 0, []
+        slot = rig.admit()
+        for c in cuts:
+            ctx, lc = rig.step([(slot, c)])
+            got.append(part.forward(h[at:at + c].to(DEV), ctx, lc))
+            rig.done([(slot, c)])
+            at += c
+        outs.append(torch.cat([o.sum(0) if o.dim() == 3 else o for o in got]))
+        states.append(lc.state[slot].clone())
+    assert torch.equal(*states)
+    assert float((outs[0] - outs[1]).abs().max()) <= 1e-5 * float(outs[0].abs().max())
