@@ -43,12 +43,12 @@ state_space_chunked_kernel(const float* __restrict__ Cg, const float* __restrict
                            const float* __restrict__ a_log, const float* __restrict__ skip, float* __restrict__ state,
                            float* __restrict__ out, const int* __restrict__ q_start, const int* __restrict__ q_len,
                            const int* __restrict__ slots, int H, int N, int dv, int hpg, int col_blocks, int max_slots,
-                           int min_len, unsigned* err) {
+                           int min_len, int max_len, unsigned* err) {
     extern __shared__ __align__(128) unsigned char sc_sm[];
     const int tid = threadIdx.x, warp = tid >> 5;
     const int cb = blockIdx.x % col_blocks, h = (blockIdx.x / col_blocks) % H, r = blockIdx.x / (col_blocks * H);
     const int n_tok = q_len[r];
-    if (n_tok < min_len) return;                       // short portions and single tokens take the token-by-token kernel
+    if (n_tok < min_len || (max_len > 0 && n_tok > max_len)) return;       // shorter and longer portions are other kernels'
     const int slot = slots[r];
     if (slot < 0 || slot >= max_slots) {
         if (tid == 0) atomicOr(err, AIE_DEV_SLOT_OOB);
@@ -249,11 +249,11 @@ template <int NP, int DV> static size_t sc_smem() {
 
 // C, B [T, .] with head h's N channels at column (h / hpg) N of rows `ld` floats apart; X likewise with dv columns a
 // head at column h dv; dt_raw [T, .] rows ld_dt apart; state [max_slots, H, N, dv]; out [T, H, dv].  Requests that
-// bring fewer than min_len tokens are left alone.  N <= 128.
+// bring fewer than min_len or (max_len > 0) more than max_len tokens are left alone.  N <= 128.
 extern "C" int aie_state_space_chunked(const float* C, const float* B, const float* X, int ld, const float* dt_raw, int ld_dt,
                                        const float* dt_bias, const float* a_log, const float* skip, float* state, float* out,
                                        const int* q_start, const int* q_len, const int* slots, int R, int H, int N, int dv,
-                                       int hpg, int max_slots, int min_len, unsigned* err, cudaStream_t st) {
+                                       int hpg, int max_slots, int min_len, int max_len, unsigned* err, cudaStream_t st) {
     if (R <= 0) return 0;
     if (H <= 0 || N <= 0 || dv <= 0 || hpg < 1 || H % hpg || !dt_raw || !dt_bias || !a_log) return AIE_BAD_ARG;
     if (N > 128) return AIE_UNSUPPORTED;
@@ -273,7 +273,7 @@ extern "C" int aie_state_space_chunked(const float* C, const float* B, const flo
         }                                                                                                               \
         state_space_chunked_kernel<NP, DV><<<(unsigned)blocks, SC_THREADS, sc_smem<NP, DV>(), st>>>(                    \
             C, B, X, ld, dt_raw, ld_dt, dt_bias, a_log, skip, state, out, q_start, q_len, slots, H, N, dv, hpg, col_blocks, \
-            max_slots, min_len, err);                                                                                   \
+            max_slots, min_len, max_len, err);                                                                                   \
     } while (0)
 #define GO2(NP)            \
     do {                   \

@@ -1044,8 +1044,8 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
 
 SSD_MIN_TOKENS = 32      # portions from this length on take the chunked state-space kernel (bfloat16 mode)
 SSD_CHUNK = 64           # its chunk
-# Steps whose portions hold this many tokens together take the kernels that are parallel over chunks: (heads, portions of n
-# tokens each) 12 us walking the chunks against 18 in parallel (64, 1 x 64), 19 against 18 (32, 1 x 128), 33 against 24 (64, 1 x
+# Portions from this length on, whatever stands beside them, take the kernels that are parallel over chunks: (heads, portions of
+# n tokens each) 12 us walking the chunks against 18 in parallel (64, 1 x 64), 19 against 18 (32, 1 x 128), 33 against 24 (64, 1 x
 # 256), 36 against 27 (64, 4 x 64), 242 against 137 (64, 1 x 2048)
 SSD_PARALLEL_TOKENS = 160
 CHUNK_STATES_BYTES = 1 << 30       # the most that the states of a step's chunks may take (65,536 tokens x 16 heads of 128 x 128);
@@ -1136,18 +1136,22 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
             and not os.environ.get("AI_ENGINE_B200_NO_CHUNKED_SCAN")):      # the switch is for measurement
         args = (_p(q), _p(k), _p(v), c_int(ld), _p(dt_raw), c_int(dt_raw.stride(0)), _p(dt_bias), _p(a_log), _p(skip), _p(state), _p(out))
         lists = (_p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d), c_int(dv), c_int(heads_per_group),
-                 c_int(state.shape[0]), c_int(SSD_MIN_TOKENS))
+                 c_int(state.shape[0]))
         with region("state_space_chunked", _nb(out) + T * H * (2 * d // heads_per_group + dv) * 4,
                     2.0 * T * H * (SSD_CHUNK * (d + dv) / 2 + 2 * d * dv)):
-            lens = ctx.h_q_len[ctx.h_q_len >= SSD_MIN_TOKENS]
+            from_len = max(SSD_MIN_TOKENS, SSD_PARALLEL_TOKENS)
+            lens = ctx.h_q_len[ctx.h_q_len >= from_len]
             chunks = int(((lens + SSD_CHUNK - 1) // SSD_CHUNK).sum())
-            if int(lens.sum()) >= SSD_PARALLEL_TOKENS and ctx.R * H <= 65535 and 4 * chunks * H * d * dv <= CHUNK_STATES_BYTES:
+            if not chunks or ctx.R * H > 65535 or 4 * chunks * H * d * dv > CHUNK_STATES_BYTES:
+                from_len = 0
+            else:
                 L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
                 G = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
                 check(library("state_space_parallel.cu").aie_state_space_parallel(
-                    *args, _p(L), _p(G), *lists, c_int(chunks), _p(ctx.err), _stream()), "state_space_parallel")
-            else:
-                check(library("state_space_chunked.cu").aie_state_space_chunked(*args, *lists, _p(ctx.err), _stream()), "state_space_chunked")
+                    *args, _p(L), _p(G), *lists, c_int(from_len), c_int(chunks), _p(ctx.err), _stream()), "state_space_parallel")
+            if not from_len or bool(((ctx.h_q_len >= SSD_MIN_TOKENS) & (ctx.h_q_len < from_len)).any()):
+                check(library("state_space_chunked.cu").aie_state_space_chunked(
+                    *args, *lists, c_int(SSD_MIN_TOKENS), c_int(max(from_len - 1, 0)), _p(ctx.err), _stream()), "state_space_chunked")
         if int(ctx.h_q_len.min()) >= SSD_MIN_TOKENS:
             return out
         max_len = SSD_MIN_TOKENS - 1                # the shorter portions and single tokens of the same step
