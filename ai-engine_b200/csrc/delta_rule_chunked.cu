@@ -74,12 +74,13 @@ delta_rule_chunked_kernel(const float* __restrict__ qg, const float* __restrict_
                           const float* __restrict__ a_log, const float* __restrict__ dt_bias, float q_scale, float unit_eps,
                           float* __restrict__ state, float* __restrict__ out, const int* __restrict__ q_start,
                           const int* __restrict__ q_len, const int* __restrict__ slots, const int* __restrict__ live, int H,
-                          int G, int d, int e, int col_blocks, int max_slots, int min_len, int vec4, unsigned* err) {
+                          int G, int d, int e, int col_blocks, int max_slots, int min_len, int max_len, int vec4,
+                          unsigned* err) {
     extern __shared__ __align__(128) unsigned char dc_sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int cb = blockIdx.x % col_blocks, h = (blockIdx.x / col_blocks) % H, r = blockIdx.x / (col_blocks * H);
     const int n_tok = q_len[r];
-    if (n_tok < min_len) return;                       // short portions and single tokens take the token-by-token kernel
+    if (n_tok < min_len || (max_len > 0 && n_tok > max_len)) return;       // shorter and longer portions are other kernels'
     const int slot = slots[r];
     if (slot < 0 || slot >= max_slots) {
         if (tid == 0) atomicOr(err, AIE_DEV_SLOT_OOB);
@@ -358,12 +359,12 @@ template <int NP, int DV> static size_t dc_smem() {
 
 // q, k [T, .] with head h's d channels at column (h / (H / G)) d of rows `ld` floats apart; v likewise with e columns a
 // head at column h e; b_raw, a_raw [T, .] rows ldb, lda apart; state [max_slots, H, d, e]; out [T, H, e].  Requests that
-// bring fewer than min_len tokens are left alone.  d <= 128.
+// bring fewer than min_len or (max_len > 0) more than max_len tokens are left alone.  d <= 128.
 extern "C" int aie_delta_rule_chunked(const float* q, const float* k, const float* v, int ld, const float* b_raw, int ldb,
                                       const float* a_raw, int lda, const float* a_log, const float* dt_bias, float q_scale,
                                       float unit_eps, float* state, float* out, const int* q_start, const int* q_len,
                                       const int* slots, const int* live, int R, int H, int G, int d, int e, int max_slots,
-                                      int min_len, unsigned* err, cudaStream_t st) {
+                                      int min_len, int max_len, unsigned* err, cudaStream_t st) {
     if (R <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || e <= 0) return AIE_BAD_ARG;
     if (d > 128) return AIE_UNSUPPORTED;
@@ -387,7 +388,7 @@ extern "C" int aie_delta_rule_chunked(const float* q, const float* k, const floa
         }                                                                                                               \
         delta_rule_chunked_kernel<NP, DV><<<(unsigned)blocks, DC_THREADS, dc_smem<NP, DV>(), st>>>(                     \
             q, k, v, ld, b_raw, ldb, a_raw, lda, a_log, dt_bias, q_scale, unit_eps, state, out, q_start, q_len, slots,  \
-            live, H, G, d, e, col_blocks, max_slots, min_len, vec4, err);                                                \
+            live, H, G, d, e, col_blocks, max_slots, min_len, max_len, vec4, err);                                                \
     } while (0)
 #define GO3(NP)                                  \
     do {                                         \

@@ -1529,19 +1529,28 @@ def sink_attention(q: torch.Tensor, pages: torch.Tensor, gate: Optional[torch.Te
 
 DELTA_MIN_TOKENS = 32    # portions from this length on take the chunked delta-rule kernel (bfloat16 mode)
 DELTA_CHUNK = 64         # its chunk
-# Steps do in parallel what does not need the state, within this much scratch, from so many chunks of the longest portion on (us,
-# 16 heads of 128 x 128, a portion of 128 / 256 / 1024 tokens: 26 / 48 / 181 chunk after chunk, 40 / 45 / 87 in parallel; 8 heads of
-# 64 x 64: 19 / 35 / 130 and 28 / 30 / 47), or from so many (chunk, head, d e) of all portions on (16 portions of 64 tokens, 16 heads
-# of 128 x 128: 129 and 86; 4 of them: 37 and 44; 16 portions of 64, 8 heads of 64 x 64: 26 and 31).
+# A portion does in parallel what does not need the state, within this much scratch, from so many chunks of its own on (us, 16
+# heads of 128 x 128, a portion of 128 / 256 / 1024 tokens: 26 / 48 / 181 chunk after chunk, 40 / 45 / 87 in parallel; 8 heads of
+# 64 x 64: 19 / 35 / 130 and 28 / 30 / 47), or from so many (chunk, head, d e) of its own on (16 portions of 64 tokens, 16 heads
+# of 128 x 128, fill the machine alike: 129 and 86; 4 of them: 37 and 44; 16 portions of 64, 8 heads of 64 x 64: 26 and 31).
 DELTA_PARALLEL_CHUNKS = 4
 DELTA_PARALLEL_WORK = 96 * 128 * 128
 DELTA_PARALLEL_BYTES = 1 << 30
 
 
-def _delta_in_parallel(args, lists, ctx, q, k, v, state, out, chunks: int, H: int, d: int, e: int) -> bool:
-    """The chunks of a step's portions side by side; False: the shapes, the rows' alignment or the scratch do not fit."""
+def delta_parallel_len(H: int, d: int, e: int) -> int:
+    """Portions from this length on go in parallel over chunks, whatever stands beside them."""
+    chunks = min(DELTA_PARALLEL_CHUNKS, -(-DELTA_PARALLEL_WORK // (H * d * e)))
+    return max(DELTA_MIN_TOKENS, DELTA_CHUNK * (chunks - 1) + 1)
+
+
+def _delta_in_parallel(args, lists, ctx, q, k, v, state, out, from_len: int, H: int, d: int, e: int) -> bool:
+    """The chunks of portions of from_len tokens or more side by side; False: there are none, or the shapes, the rows'
+    alignment or the scratch do not fit."""
+    lens = ctx.h_q_len[ctx.h_q_len >= from_len]
+    chunks = int(((lens + DELTA_CHUNK - 1) // DELTA_CHUNK).sum())
     scratch = chunks * H * (DELTA_CHUNK * (8 * d + 4 * e) + 4 * d * e + 4)
-    if (d not in (64, 128) or e % 16 or q.stride(0) % 4 or scratch > DELTA_PARALLEL_BYTES or max(H, ctx.R) > 65535
+    if (not chunks or d not in (64, 128) or e % 16 or q.stride(0) % 4 or scratch > DELTA_PARALLEL_BYTES or max(H, ctx.R) > 65535
             or any(t.data_ptr() % 16 for t in (q, k, v, state, out))):
         return False
     pairs = torch.empty((2, chunks, H, 2, DELTA_CHUNK, d), dtype=torch.bfloat16, device=q.device)
@@ -1549,7 +1558,8 @@ def _delta_in_parallel(args, lists, ctx, q, k, v, state, out, chunks: int, H: in
     S0 = torch.empty((chunks, H, d, e), dtype=torch.float32, device=q.device)
     decay = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
     check(library("delta_rule_parallel.cu").aie_delta_rule_parallel(
-        *args, _p(pairs[0]), _p(pairs[1]), _p(U), _p(S0), _p(decay), *lists, c_int(chunks), _p(ctx.err), _stream()), "delta_rule_parallel")
+        *args, _p(pairs[0]), _p(pairs[1]), _p(U), _p(S0), _p(decay), *lists, c_int(from_len), c_int(chunks), _p(ctx.err), _stream()),
+        "delta_rule_parallel")
     return True
 
 
@@ -1576,17 +1586,18 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
     if (chunked and d <= 128 and ctx.max_q_len >= DELTA_MIN_TOKENS
             and not os.environ.get("AI_ENGINE_B200_NO_CHUNKED_SCAN")):      # the switch is for measurement
         Q = DELTA_CHUNK
-        lens = ctx.h_q_len[ctx.h_q_len >= DELTA_MIN_TOKENS]
-        chunks = int(((lens + Q - 1) // Q).sum())
+        from_len = delta_parallel_len(H, d, e)
         args = (_p(q), _p(k), _p(v), c_int(ld), _p(b_raw), c_int(b_raw.stride(0)), _p(a_raw), c_int(a_raw.stride(0)), _p(a_log),
                 _p(dt_bias), c_float(q_scale), c_float(unit_eps), _p(state), _p(out))
         lists = (_p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), _p(ctx.live), c_int(ctx.R), c_int(H), c_int(G), c_int(d), c_int(e),
-                 c_int(state.shape[0]), c_int(DELTA_MIN_TOKENS))
+                 c_int(state.shape[0]))
         with region("delta_rule_chunked", _nb(out) + T * (2 * G * d + H * e) * 4 + 2 * ctx.R * H * d * e * 4,
                     2.0 * T * H * (Q * d + Q * e + 3 * d * e)):
-            if not ((ctx.max_q_len > Q * (DELTA_PARALLEL_CHUNKS - 1) or chunks * H * d * e >= DELTA_PARALLEL_WORK)
-                    and _delta_in_parallel(args, lists, ctx, q, k, v, state, out, chunks, H, d, e)):
-                check(library("delta_rule_chunked.cu").aie_delta_rule_chunked(*args, *lists, _p(ctx.err), _stream()), "delta_rule_chunked")
+            if not _delta_in_parallel(args, lists, ctx, q, k, v, state, out, from_len, H, d, e):
+                from_len = 0
+            if not from_len or bool(((ctx.h_q_len >= DELTA_MIN_TOKENS) & (ctx.h_q_len < from_len)).any()):
+                check(library("delta_rule_chunked.cu").aie_delta_rule_chunked(
+                    *args, *lists, c_int(DELTA_MIN_TOKENS), c_int(max(from_len - 1, 0)), _p(ctx.err), _stream()), "delta_rule_chunked")
         if int(ctx.h_q_len.min()) >= DELTA_MIN_TOKENS:
             return out
         max_len = DELTA_MIN_TOKENS - 1              # the shorter portions and single tokens of the same step

@@ -86,3 +86,24 @@ def test_state_space(H, hpg, lens):
         return [(o, state[i]) for o, (i, _) in zip(out.split([n for _, n in reqs]), reqs)]
 
     alone_and_beside(run, lens, lambda n: n >= ops.SSD_MIN_TOKENS)
+
+
+@pytest.mark.parametrize("H,G,lens", [(4, 2, [192, 40, 193, 5, 300, 1, 64]), (24, 24, [31, 32, 130, 100, 280])])
+def test_delta_rule(H, G, lens):
+    from ai_engine_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(H)
+    rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    d, e = 64, 32
+    rows, gates = [rnd(n, 2 * G * d + H * e) for n in lens], [rnd(n, 2 * H) for n in lens]
+    states, a_log, bias = rnd(len(lens), H, d, e), rnd(H) - 1.0, rnd(H)
+
+    def run(reqs):
+        x, g, state = torch.cat([rows[i] for i, _ in reqs]), torch.cat([gates[i] for i, _ in reqs]), states.clone()
+        ctx = Ctx([n for _, n in reqs], [i for i, _ in reqs])
+        ctx.live = None
+        out = ops.delta_rule(x[:, :G * d], x[:, G * d:2 * G * d], x[:, 2 * G * d:], g[:, :H], g[:, H:], a_log, bias, d ** -0.5, 1e-6,
+                             state, ctx, H, G, d, e, chunked=True)
+        assert int(ctx.err.item()) == 0
+        return [(o, state[i]) for o, (i, _) in zip(out.split([n for _, n in reqs]), reqs)]
+
+    alone_and_beside(run, lens, lambda n: n > 1)
