@@ -39,3 +39,33 @@ __device__ __forceinline__ void chunk_find(const int* q_len, int R, int min_len,
     r = found[0];
     c = found[1];
 }
+
+// Request r of the idx-th of those portions and the number of its first chunk; r < 0: there is none.  All threads of the block
+// call it; found: two ints of shared memory.
+template <int CT>
+__device__ __forceinline__ void portion_find(const int* q_len, int R, int min_len, int idx, int* found, int& r, int& first) {
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int rr = -1, portions = 0, chunks = 0;
+        for (int base = 0; base < R && rr < 0; base += 32) {
+            int m = chunk_count<CT>(q_len, R, min_len, base + lane);
+            unsigned takes = __ballot_sync(0xffffffffu, m > 0);
+            const int n = __popc(takes);
+            if (idx < portions + n) {
+                for (int i = portions; i < idx; ++i) takes &= takes - 1;
+                const int l = __ffs(takes) - 1;
+                rr = base + l;
+                if (lane >= l) m = 0;
+            }
+            portions += n;
+            chunks += __reduce_add_sync(0xffffffffu, m);
+        }
+        if (lane == 0) {
+            found[0] = rr;
+            found[1] = chunks;
+        }
+    }
+    __syncthreads();
+    r = found[0];
+    first = found[1];
+}

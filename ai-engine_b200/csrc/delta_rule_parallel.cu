@@ -333,16 +333,16 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
     bf16* SL = SH + D * LD;
     bf16* UH = SL + D * LD;                            // [64][LD]
     bf16* UL = UH + DP_T * LD;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * DV, h = blockIdx.y, r = blockIdx.z;
-    const int n = chunk_count<DP_T>(p.q_len, p.R, p.min_len, r);
-    if (n == 0) return;
-    const int slot = p.slots[r];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * DV, h = blockIdx.y;
+    __shared__ int found[2];
+    int r, first;
+    portion_find<DP_T>(p.q_len, p.R, p.min_len, blockIdx.z, found, r, first);
+    if (r < 0) return;
+    const int n = chunk_count<DP_T>(p.q_len, p.R, p.min_len, r), slot = p.slots[r];
     if (slot < 0 || slot >= p.max_slots) {
         if (tid == 0) atomicOr(p.err, AIE_DEV_SLOT_OOB);
         return;
     }
-    int first = 0;
-    for (int i = 0; i < r; ++i) first += chunk_count<DP_T>(p.q_len, p.R, p.min_len, i);
     auto fetch = [&](int c) {
         if (c < n) {
             const size_t at = (size_t)(first + c) * p.H + h;
@@ -596,7 +596,7 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_out_kernel(DpArgs p) {
 }
 
 template <int D>
-static int dp_go(const DpArgs& p, int n_chunks, cudaStream_t st) {
+static int dp_go(const DpArgs& p, int n_portions, int n_chunks, cudaStream_t st) {
     constexpr int LN = D + 8, LA = DP_T + 4;
     const size_t sm_prep = (size_t)2 * DP_T * LN * 2 + (size_t)(2 * DP_T * LA + DP_T * (DP_E + 4)) * 4;
     const size_t sm_out = (size_t)(2 * DP_T * LN + 2 * max(DP_T * LN, (D + DP_T) * 72)) * 2;
@@ -610,27 +610,29 @@ static int dp_go(const DpArgs& p, int n_chunks, cudaStream_t st) {
         const size_t sm = (size_t)(8 * DP_T * LN + 2 * (D + DP_T) * (DV + 8)) * 2;                                      \
         e = cudaFuncSetAttribute(dp_walk_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);          \
         if (e != cudaSuccess) return (int)e;                                                                            \
-        dp_walk_kernel<D, DV><<<dim3(p.e / DV, p.H, p.R), DP_THREADS, sm, st>>>(p);                                     \
+        dp_walk_kernel<D, DV><<<dim3(p.e / DV, p.H, n_portions), DP_THREADS, sm, st>>>(p);                                \
     }
-    if (p.e % 32 || (long long)p.R * p.H * (p.e / 16) <= aie_sm_count()) WALK(16) else WALK(32)
+    if (p.e % 32 || (long long)n_portions * p.H * (p.e / 16) <= aie_sm_count()) WALK(16) else WALK(32)
 #undef WALK
     dp_out_kernel<D><<<dim3(n_chunks, p.H), DP_THREADS, sm_out, st>>>(p);
     AIE_LAUNCH_CHECK();
 }
 
 // The arguments are those of aie_delta_rule_chunked; scratch: W and Kw [n_chunks, H, 2, 64, d] bf16, U [n_chunks, H, 64, e], S0
-// [n_chunks, H, d, e] and decay [n_chunks, H] float32; n_chunks: the chunks of 64 tokens of all requests that bring min_len
-// tokens or more.  Takes d of 64 or 128 and e a multiple of 16, with rows that start on 16 bytes (else AIE_UNSUPPORTED).
+// [n_chunks, H, d, e] and decay [n_chunks, H] float32; n_portions, n_chunks: the requests that bring
+// min_len tokens or more, and their chunks of 64.  Takes d of 64 or 128 and e a multiple of 16, with rows that start on 16 bytes
+// (else AIE_UNSUPPORTED).
 extern "C" int aie_delta_rule_parallel(const float* q, const float* k, const float* v, int ld, const float* b_raw, int ldb,
                                        const float* a_raw, int lda, const float* a_log, const float* dt_bias, float q_scale,
                                        float unit_eps, float* state, float* out, void* W, void* Kw, float* U, float* S0, float* decay,
                                        const int* q_start, const int* q_len, const int* slots, const int* live, int R, int H, int G,
-                                       int d, int e, int max_slots, int min_len, int n_chunks, unsigned* err, cudaStream_t st) {
-    if (R <= 0 || n_chunks <= 0) return 0;
+                                       int d, int e, int max_slots, int min_len, int n_portions, int n_chunks,
+                                       unsigned* err, cudaStream_t st) {
+    if (R <= 0 || n_portions <= 0 || n_chunks <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || d <= 0 || e <= 0 || min_len < 1) return AIE_BAD_ARG;
     const size_t at = (size_t)q | (size_t)k | (size_t)v | (size_t)state | (size_t)out | (size_t)W | (size_t)Kw | (size_t)U | (size_t)S0;
-    if ((d != 64 && d != 128) || e % 16 || ld % 4 || (at & 15) || H > 65535 || R > 65535) return AIE_UNSUPPORTED;
+    if ((d != 64 && d != 128) || e % 16 || ld % 4 || (at & 15) || H > 65535 || n_portions > 65535) return AIE_UNSUPPORTED;
     const DpArgs p = {q, k, v, b_raw, a_raw, a_log, dt_bias, state, out, (bf16*)W, (bf16*)Kw, U, S0, decay, q_start, q_len, slots, live,
                       err, ld, ldb, lda, R, H, G, e, max_slots, min_len, q_scale, unit_eps};
-    return d == 64 ? dp_go<64>(p, n_chunks, st) : dp_go<128>(p, n_chunks, st);
+    return d == 64 ? dp_go<64>(p, n_portions, n_chunks, st) : dp_go<128>(p, n_portions, n_chunks, st);
 }

@@ -165,18 +165,18 @@ __global__ void __launch_bounds__(LC_THREADS, 2) lc_chunk_kernel(LcArgs p) {
 // S_c for every chunk of a request and the state behind the last; bound by the traffic of L (in L2).  A thread owns
 // four elements; eight chunks' loads are in flight while the chain of multiply-adds runs.
 __global__ void __launch_bounds__(LC_THREADS) lc_scan_kernel(LcArgs p) {
-    const int r = blockIdx.y / p.H, h = blockIdx.y % p.H;
-    const int n = chunk_count<LC_T>(p.q_len, p.R, p.min_len, r);
-    if (n == 0) return;
-    const int slot = p.slots[r];
+    __shared__ int found[2];
+    const int h = blockIdx.y % p.H;
+    int r, first;
+    portion_find<LC_T>(p.q_len, p.R, p.min_len, blockIdx.y / p.H, found, r, first);
+    if (r < 0) return;
+    const int n = chunk_count<LC_T>(p.q_len, p.R, p.min_len, r), slot = p.slots[r];
     if (slot < 0 || slot >= p.max_slots) {
         if (threadIdx.x == 0) atomicOr(p.err, AIE_DEV_SLOT_OOB);
         return;
     }
     const int e = (blockIdx.x * LC_THREADS + threadIdx.x) * 4, size = p.d * p.dv;
     if (e >= size) return;
-    int first = 0;
-    for (int i = 0; i < r; ++i) first += chunk_count<LC_T>(p.q_len, p.R, p.min_len, i);
     const int row = e / p.dv;
     float* sp = p.state + ((size_t)slot * p.H + h) * size + e;
     float* L = p.L + ((size_t)first * p.H + h) * size + e;
@@ -430,37 +430,37 @@ __global__ void __launch_bounds__(LC_THREADS, 2) lc_out_kernel(LcArgs p) {
 }
 
 template <int D, int DV>
-static int lc_go(const LcArgs& p, int n_chunks, cudaStream_t st) {
+static int lc_go(const LcArgs& p, int n_portions, int n_chunks, cudaStream_t st) {
     constexpr int KD = D > DV ? D : DV;
     const size_t sm_chunk = (size_t)LC_T * (2 * D + DV) * 4, sm_out = (size_t)LC_T * (2 * D + KD + LC_T) * 4;
     cudaError_t e = cudaFuncSetAttribute(lc_chunk_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_chunk);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(lc_out_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_out);
     if (e != cudaSuccess) return (int)e;
     lc_chunk_kernel<D, DV><<<dim3(n_chunks, p.H), LC_THREADS, sm_chunk, st>>>(p);
-    lc_scan_kernel<<<dim3((p.d * p.dv / 4 + LC_THREADS - 1) / LC_THREADS, p.R * p.H), LC_THREADS, 0, st>>>(p);
+    lc_scan_kernel<<<dim3((p.d * p.dv / 4 + LC_THREADS - 1) / LC_THREADS, n_portions * p.H), LC_THREADS, 0, st>>>(p);
     lc_out_kernel<D, DV><<<dim3(n_chunks, p.H), LC_THREADS, sm_out, st>>>(p);
     AIE_LAUNCH_CHECK();
 }
 
 // The arguments are those of aie_linear_recurrence.  L [n_chunks, H, d, dv] and G [n_chunks, H, d] float32 are scratch;
-// n_chunks: the chunks of 64 tokens of all requests that bring min_len tokens or more (the others are left alone).
+// n_portions, n_chunks: the requests that bring min_len tokens or more (the others are left alone), and their chunks of 64.
 // Takes d and dv up to 128 in steps of 4 whose rows start on 16 bytes (else AIE_UNSUPPORTED: the caller takes the
 // token-by-token kernel).
 extern "C" int aie_linear_recurrence_chunked(const float* q, const float* k, const float* v, int ld, const float* decay_tok,
                                              int ld_decay, const float* decay_head, float q_scale, float k_scale, float* state,
                                              float* out, float* L, float* G, const int* q_start, const int* q_len, const int* slots,
-                                             int R, int H, int d, int dv, int max_slots, int min_len, int n_chunks,
-                                             const float* fg_lower, const float* fg_bias, unsigned* err, cudaStream_t st) {
-    if (R <= 0 || n_chunks <= 0) return 0;
+                                             int R, int H, int d, int dv, int max_slots, int min_len, int n_portions,
+                                             int n_chunks, const float* fg_lower, const float* fg_bias, unsigned* err, cudaStream_t st) {
+    if (R <= 0 || n_portions <= 0 || n_chunks <= 0) return 0;
     if (H <= 0 || d <= 0 || dv <= 0 || min_len < 1 || (!decay_tok && !decay_head)) return AIE_BAD_ARG;
     if (fg_lower ? (!decay_tok || k) : !k) return AIE_BAD_ARG;
     const size_t at = (size_t)q | (size_t)k | (size_t)v | (size_t)decay_tok | (size_t)state | (size_t)out | (size_t)L |
                       (size_t)fg_lower | (size_t)fg_bias;
     if (d > 128 || dv > 128 || d % 4 || dv % 4 || ld % 4 || (decay_tok && ld_decay % 4) || (at & 15) ||
-        H > 65535 || (long long)R * H > 65535)
+        H > 65535 || (long long)n_portions * H > 65535)
         return AIE_UNSUPPORTED;
     const LcArgs p = {q, k, v, decay_tok, decay_head, fg_lower, fg_bias, state, out, L, G, q_start, q_len, slots, err,
                       ld, ld_decay, H, R, d, dv, max_slots, min_len, q_scale, k_scale};
-    if (d <= 64) return dv <= 64 ? lc_go<64, 64>(p, n_chunks, st) : lc_go<64, 128>(p, n_chunks, st);
-    return dv <= 64 ? lc_go<128, 64>(p, n_chunks, st) : lc_go<128, 128>(p, n_chunks, st);
+    if (d <= 64) return dv <= 64 ? lc_go<64, 64>(p, n_portions, n_chunks, st) : lc_go<64, 128>(p, n_portions, n_chunks, st);
+    return dv <= 64 ? lc_go<128, 64>(p, n_portions, n_chunks, st) : lc_go<128, 128>(p, n_portions, n_chunks, st);
 }

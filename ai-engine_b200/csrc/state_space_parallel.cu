@@ -157,17 +157,18 @@ __global__ void __launch_bounds__(SP_THREADS) sp_chunk_kernel(SpArgs p) {
 // A thread owns V neighbouring elements of a state; eight chunks' loads are in flight while the chain runs.
 template <int V>
 __global__ void __launch_bounds__(SP_THREADS) sp_scan_kernel(SpArgs p) {
-    const int r = blockIdx.y / p.H, h = blockIdx.y % p.H, n = chunk_count<SP_T>(p.q_len, p.R, p.min_len, r);
-    if (n == 0) return;
-    const int slot = p.slots[r];
+    __shared__ int found[2];
+    const int h = blockIdx.y % p.H;
+    int r, first;
+    portion_find<SP_T>(p.q_len, p.R, p.min_len, blockIdx.y / p.H, found, r, first);
+    if (r < 0) return;
+    const int n = chunk_count<SP_T>(p.q_len, p.R, p.min_len, r), slot = p.slots[r];
     if (slot < 0 || slot >= p.max_slots) {
         if (threadIdx.x == 0) atomicOr(p.err, AIE_DEV_SLOT_OOB);
         return;
     }
     const int size = p.N * p.dv, e = (blockIdx.x * SP_THREADS + threadIdx.x) * V;
     if (e >= size) return;
-    int first = 0;
-    for (int i = 0; i < r; ++i) first += chunk_count<SP_T>(p.q_len, p.R, p.min_len, i);
     float* sp = p.state + ((size_t)slot * p.H + h) * size + e;
     float* L = p.L + ((size_t)first * p.H + h) * size + e;
     const float* G = p.G + (size_t)first * p.H + h;
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
 }
 
 template <int NP>
-static int sp_go(const SpArgs& p, int n_chunks, cudaStream_t st) {
+static int sp_go(const SpArgs& p, int n_portions, int n_chunks, cudaStream_t st) {
     const int LN = NP + 8, LD = 64 + 8;
     const size_t sm_chunk = (size_t)(SP_T * LN + 2 * SP_T * LD) * 2, sm_out = (size_t)(2 * SP_T * LN + SP_T * LD + 2 * NP * LD) * 2;
     cudaError_t e = cudaFuncSetAttribute(sp_chunk_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_chunk);
@@ -354,30 +355,31 @@ static int sp_go(const SpArgs& p, int n_chunks, cudaStream_t st) {
     const int size = p.N * p.dv;
     sp_chunk_kernel<NP><<<grid, SP_THREADS, sm_chunk, st>>>(p);
     if (size % 4 == 0 && !(((size_t)p.state | (size_t)p.L) & 15))
-        sp_scan_kernel<4><<<dim3((size / 4 + SP_THREADS - 1) / SP_THREADS, p.R * p.H), SP_THREADS, 0, st>>>(p);
+        sp_scan_kernel<4><<<dim3((size / 4 + SP_THREADS - 1) / SP_THREADS, n_portions * p.H), SP_THREADS, 0, st>>>(p);
     else
-        sp_scan_kernel<1><<<dim3((size + SP_THREADS - 1) / SP_THREADS, p.R * p.H), SP_THREADS, 0, st>>>(p);
+        sp_scan_kernel<1><<<dim3((size + SP_THREADS - 1) / SP_THREADS, n_portions * p.H), SP_THREADS, 0, st>>>(p);
     sp_out_kernel<NP><<<grid, SP_THREADS, sm_out, st>>>(p);
     AIE_LAUNCH_CHECK();
 }
 
-// The arguments are those of aie_state_space_chunked; L [n_chunks, H, N, dv] and G [n_chunks, H] float32 are scratch, n_chunks
-// the chunks of 64 tokens of all requests that bring min_len tokens or more (the others are left alone).  N <= 128.
+// The arguments are those of aie_state_space_chunked; L [n_chunks, H, N, dv] and G [n_chunks, H] float32 are scratch;
+// n_portions, n_chunks: the requests that bring min_len tokens or more (the others are left alone), and their chunks of 64.
+// N <= 128.
 extern "C" int aie_state_space_parallel(const float* C, const float* B, const float* X, int ld, const float* dt_raw, int ld_dt,
                                         const float* dt_bias, const float* a_log, const float* skip, float* state, float* out,
                                         float* L, float* G, const int* q_start, const int* q_len, const int* slots, int R, int H,
-                                        int N, int dv, int hpg, int max_slots, int min_len, int n_chunks, unsigned* err,
+                                        int N, int dv, int hpg, int max_slots, int min_len, int n_portions, int n_chunks, unsigned* err,
                                         cudaStream_t st) {
-    if (R <= 0 || n_chunks <= 0) return 0;
+    if (R <= 0 || n_portions <= 0 || n_chunks <= 0) return 0;
     if (H <= 0 || N <= 0 || dv <= 0 || hpg < 1 || H % hpg || !dt_raw || !dt_bias || !a_log || min_len < 1) return AIE_BAD_ARG;
-    if (N > 128 || H > 65535 || (long long)R * H > 65535 || (dv + 63) / 64 > 65535) return AIE_UNSUPPORTED;
+    if (N > 128 || H > 65535 || (long long)n_portions * H > 65535 || (dv + 63) / 64 > 65535) return AIE_UNSUPPORTED;
     const int vec = N % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && !(((size_t)C | (size_t)B | (size_t)X | (size_t)L) & 15);
     // four or two heads a block where that still gives every SM's two places a block
     int hpb = 1;
     while (hpb < 4 && hpg % (2 * hpb) == 0 && (long long)n_chunks * (H / (2 * hpb)) * ((dv + 63) / 64) >= 2 * aie_sm_count()) hpb *= 2;
     const SpArgs p = {C, B, X, dt_raw, dt_bias, a_log, skip, state, out, L, G, q_start, q_len, slots, err,
                       ld, ld_dt, R, H, N, dv, hpg, max_slots, min_len, vec, hpb};
-    if (N <= 32) return sp_go<32>(p, n_chunks, st);
-    if (N <= 64) return sp_go<64>(p, n_chunks, st);
-    return sp_go<128>(p, n_chunks, st);
+    if (N <= 32) return sp_go<32>(p, n_portions, n_chunks, st);
+    if (N <= 64) return sp_go<64>(p, n_portions, n_chunks, st);
+    return sp_go<128>(p, n_portions, n_chunks, st);
 }

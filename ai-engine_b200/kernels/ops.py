@@ -1073,13 +1073,13 @@ def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, 
     """The portions of lc_min_len(H) tokens or more by the chunk-parallel kernels: that length; 0 (nothing is done) when there
     is none or the sizes, strides or addresses are not theirs: heads of up to 128 in steps of 4, rows that start on 16 bytes."""
     min_len = lc_min_len(H)
-    if (ctx.max_q_len < min_len or d > 128 or dv > 128 or d % 4 or dv % 4 or ld % 4 or ctx.R * H > 65535
+    if (ctx.max_q_len < min_len or d > 128 or dv > 128 or d % 4 or dv % 4 or ld % 4
             or (decay_tok is not None and decay_tok.stride(0) % 4)
             or any(t is not None and t.data_ptr() % 16 for t in (q, k, v, decay_tok, state, lower, bias))):
         return 0
     lens = ctx.h_q_len[ctx.h_q_len >= min_len]
     chunks = int(((lens + LC_CHUNK - 1) // LC_CHUNK).sum())
-    if 4 * chunks * H * d * dv > CHUNK_STATES_BYTES:
+    if 4 * chunks * H * d * dv > CHUNK_STATES_BYTES or len(lens) * H > 65535:
         return 0
     L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
     G = torch.empty((chunks, H, d), dtype=torch.float32, device=q.device)
@@ -1090,8 +1090,8 @@ def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, 
                                                 c_int(decay_tok.stride(0) if decay_tok is not None else 0), _p(decay_head),
                                                 c_float(q_scale), c_float(k_scale), _p(state), _p(out), _p(L), _p(G),
                                                 _p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d),
-                                                c_int(dv), c_int(state.shape[0]), c_int(min_len), c_int(chunks), _p(lower),
-                                                _p(bias), _p(ctx.err), _stream()), "linear_recurrence_chunked")
+                                                c_int(dv), c_int(state.shape[0]), c_int(min_len), c_int(len(lens)), c_int(chunks),
+                                                _p(lower), _p(bias), _p(ctx.err), _stream()), "linear_recurrence_chunked")
     return min_len
 
 
@@ -1142,13 +1142,14 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
             from_len = max(SSD_MIN_TOKENS, SSD_PARALLEL_TOKENS)
             lens = ctx.h_q_len[ctx.h_q_len >= from_len]
             chunks = int(((lens + SSD_CHUNK - 1) // SSD_CHUNK).sum())
-            if not chunks or ctx.R * H > 65535 or 4 * chunks * H * d * dv > CHUNK_STATES_BYTES:
+            if not chunks or len(lens) * H > 65535 or 4 * chunks * H * d * dv > CHUNK_STATES_BYTES:
                 from_len = 0
             else:
                 L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
                 G = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
                 check(library("state_space_parallel.cu").aie_state_space_parallel(
-                    *args, _p(L), _p(G), *lists, c_int(from_len), c_int(chunks), _p(ctx.err), _stream()), "state_space_parallel")
+                    *args, _p(L), _p(G), *lists, c_int(from_len), c_int(len(lens)), c_int(chunks), _p(ctx.err), _stream()),
+                    "state_space_parallel")
             if not from_len or bool(((ctx.h_q_len >= SSD_MIN_TOKENS) & (ctx.h_q_len < from_len)).any()):
                 check(library("state_space_chunked.cu").aie_state_space_chunked(
                     *args, *lists, c_int(SSD_MIN_TOKENS), c_int(max(from_len - 1, 0)), _p(ctx.err), _stream()), "state_space_chunked")
@@ -1550,7 +1551,7 @@ def _delta_in_parallel(args, lists, ctx, q, k, v, state, out, from_len: int, H: 
     lens = ctx.h_q_len[ctx.h_q_len >= from_len]
     chunks = int(((lens + DELTA_CHUNK - 1) // DELTA_CHUNK).sum())
     scratch = chunks * H * (DELTA_CHUNK * (8 * d + 4 * e) + 4 * d * e + 4)
-    if (not chunks or d not in (64, 128) or e % 16 or q.stride(0) % 4 or scratch > DELTA_PARALLEL_BYTES or max(H, ctx.R) > 65535
+    if (not chunks or d not in (64, 128) or e % 16 or q.stride(0) % 4 or scratch > DELTA_PARALLEL_BYTES or max(H, len(lens)) > 65535
             or any(t.data_ptr() % 16 for t in (q, k, v, state, out))):
         return False
     pairs = torch.empty((2, chunks, H, 2, DELTA_CHUNK, d), dtype=torch.bfloat16, device=q.device)
@@ -1558,7 +1559,8 @@ def _delta_in_parallel(args, lists, ctx, q, k, v, state, out, from_len: int, H: 
     S0 = torch.empty((chunks, H, d, e), dtype=torch.float32, device=q.device)
     decay = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
     check(library("delta_rule_parallel.cu").aie_delta_rule_parallel(
-        *args, _p(pairs[0]), _p(pairs[1]), _p(U), _p(S0), _p(decay), *lists, c_int(from_len), c_int(chunks), _p(ctx.err), _stream()),
+        *args, _p(pairs[0]), _p(pairs[1]), _p(U), _p(S0), _p(decay), *lists, c_int(from_len), c_int(len(lens)), c_int(chunks),
+        _p(ctx.err), _stream()),
         "delta_rule_parallel")
     return True
 

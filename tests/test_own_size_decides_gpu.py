@@ -24,7 +24,8 @@ def alone_and_beside(run, lens, exact):
 
 
 @pytest.mark.parametrize("keyless", [False, True])
-@pytest.mark.parametrize("H,lens", [(16, [40, 300, 1, 53, 54, 9]), (40, [41, 12, 43, 42])])
+@pytest.mark.parametrize("H,lens", [(16, [40, 300, 1, 53, 54, 9]), (40, [41, 12, 43, 42]),
+                                    (16, [1] * 33 + [70] + [3] * 34 + [130, 64])])
 def test_linear_recurrence(H, lens, keyless):
     from ai_engine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(H)
@@ -68,7 +69,8 @@ def test_float32_linear_attention_whole_and_in_portions(kind, extra):
     assert float((outs[0] - outs[1]).abs().max()) <= 1e-5 * float(outs[0].abs().max())
 
 
-@pytest.mark.parametrize("H,hpg,lens", [(4, 2, [159, 40, 160, 5, 300, 1, 64]), (32, 4, [31, 32, 130, 100])])
+@pytest.mark.parametrize("H,hpg,lens", [(4, 2, [159, 40, 160, 5, 300, 1, 64]), (32, 4, [31, 32, 130, 100]),
+                                        (4, 1, [1] * 33 + [170] + [3] * 34 + [230, 40])])
 def test_state_space(H, hpg, lens):
     from ai_engine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(H)
@@ -88,7 +90,8 @@ def test_state_space(H, hpg, lens):
     alone_and_beside(run, lens, lambda n: n >= ops.SSD_MIN_TOKENS)
 
 
-@pytest.mark.parametrize("H,G,lens", [(4, 2, [192, 40, 193, 5, 300, 1, 64]), (24, 24, [31, 32, 130, 100, 280])])
+@pytest.mark.parametrize("H,G,lens", [(4, 2, [192, 40, 193, 5, 300, 1, 64]), (24, 24, [31, 32, 130, 100, 280]),
+                                      (2, 1, [1] * 33 + [200] + [3] * 34 + [257, 40])])
 def test_delta_rule(H, G, lens):
     from ai_engine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(H)
@@ -107,3 +110,23 @@ def test_delta_rule(H, G, lens):
         return [(o, state[i]) for o, (i, _) in zip(out.split([n for _, n in reqs]), reqs)]
 
     alone_and_beside(run, lens, lambda n: n > 1)
+
+
+def test_a_prompt_beside_so_many_lone_tokens_that_a_grid_over_all_of_them_would_be_too_large(monkeypatch):
+    from ai_engine_b200.kernels import ops
+    taken, real = [], ops._recurrence_in_chunks
+    monkeypatch.setattr(ops, "_recurrence_in_chunks", lambda *a: taken.append(real(*a)) or taken[-1])
+    H, d, lens = 64, 4, [1] * 1100 + [40]
+    x = torch.randn(sum(lens), 3 * H * d, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV)
+    decay = torch.full((H,), 0.9, device=DEV)
+
+    def run(rows, lens):
+        state, ctx = torch.zeros(len(lens), H, d, d, device=DEV), Ctx(lens, list(range(len(lens))))
+        q, k, v = (rows[:, i * H * d:(i + 1) * H * d] for i in range(3))
+        out = ops.linear_recurrence(q, k, v, None, decay, 1.0, 1.0, state, ctx, H, d, d)
+        assert int(ctx.err.item()) == 0
+        return out[-40:], state[-1]
+
+    for a, b in zip(run(x, lens), run(x[-40:], [40])):
+        assert torch.equal(a, b)
+    assert taken == [ops.lc_min_len(H)] * 2
