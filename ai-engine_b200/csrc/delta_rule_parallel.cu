@@ -32,7 +32,7 @@ struct DpArgs {
     float *U, *S0, *decay;    // [n_chunks, H][64][e], [n_chunks, H][d][e], [n_chunks, H]
     const int *q_start, *q_len, *slots, *live;
     unsigned* err;
-    int ld, ldb, lda, R, H, G, e, max_slots, min_len;
+    int ld, ldb, lda, R, H, all_heads, head0, per, e, max_slots, min_len;      // H: the heads of this launch, from head0 on; per a q/k head
     float q_scale, unit_eps;
 };
 
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_prepare_kernel(DpArgs p) {
     values(0);
     dp_decays(p, a0, nt, h, la, be);
     for (int i = tid; i < DP_T * LA; i += DP_THREADS) Ts[i] = 0.f;
-    dp_units<D>(p.k + a0 * p.ld + (size_t)(h / (p.H / p.G)) * D, p.ld, nt, p.unit_eps, 1.f, KH, KL, la, p.Kw + at * 2 * DP_T * D);
+    dp_units<D>(p.k + a0 * p.ld + (size_t)((p.head0 + h) / p.per) * D, p.ld, nt, p.unit_eps, 1.f, KH, KL, la, p.Kw + at * 2 * DP_T * D);
     __syncthreads();
     if (tid == 0) p.decay[at] = expf(la[DP_T - 1]);
     // A on and below the diagonal, tiles of 16 x 16 (1/0, ... as the warps come by them)
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
         cp_async_commit();
     };
     fetch(0);
-    float* sp = p.state + ((size_t)slot * p.H + h) * D * p.e + col0;
+    float* sp = p.state + ((size_t)slot * p.all_heads + h) * D * p.e + col0;
     const bool holds = warp < D / 16;                  // rows 16 warp .. + 15 of the state
     const int sr = warp * 16 + (lane >> 2), sc = (lane & 3) * 2;
     float S[NS][4];
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_out_kernel(DpArgs p) {
     bf16* SL = SH + D * LD;
     bf16* UH = SL + D * LD;                            // [64][LD]
     bf16* UL = UH + DP_T * LD;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, hq = h / (p.H / p.G);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, hq = (p.head0 + h) / p.per;
     int r, c;
     chunk_find<DP_T>(p.q_len, p.R, p.min_len, blockIdx.x, found, r, c);
     if (r < 0) return;
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_out_kernel(DpArgs p) {
             for (int e = 0; e < 2; ++e) {
                 const int t = e ? tb : ta, j = col0 + n0 + x * 8 + (lane & 3) * 2;
                 if (t < nt && j < p.e)
-                    *reinterpret_cast<float2*>(p.out + ((a0 + t) * p.H + h) * p.e + j) = make_float2(y[x][2 * e], y[x][2 * e + 1]);
+                    *reinterpret_cast<float2*>(p.out + ((a0 + t) * p.all_heads + h) * p.e + j) = make_float2(y[x][2 * e], y[x][2 * e + 1]);
             }
     }
 }
@@ -618,21 +618,22 @@ static int dp_go(const DpArgs& p, int n_portions, int n_chunks, cudaStream_t st)
     AIE_LAUNCH_CHECK();
 }
 
-// The arguments are those of aie_delta_rule_chunked; scratch: W and Kw [n_chunks, H, 2, 64, d] bf16, U [n_chunks, H, 64, e], S0
-// [n_chunks, H, d, e] and decay [n_chunks, H] float32; n_portions, n_chunks: the requests that bring
+// The arguments are those of aie_delta_rule_chunked.  Heads head0 .. head0 + heads - 1 of the H are done; scratch: W and Kw
+// [n_chunks, heads, 2, 64, d] bf16, U [n_chunks, heads, 64, e], S0 [n_chunks, heads, d, e] and decay [n_chunks, heads] float32; n_portions, n_chunks: the requests that bring
 // min_len tokens or more, and their chunks of 64.  Takes d of 64 or 128 and e a multiple of 16, with rows that start on 16 bytes
 // (else AIE_UNSUPPORTED).
 extern "C" int aie_delta_rule_parallel(const float* q, const float* k, const float* v, int ld, const float* b_raw, int ldb,
                                        const float* a_raw, int lda, const float* a_log, const float* dt_bias, float q_scale,
                                        float unit_eps, float* state, float* out, void* W, void* Kw, float* U, float* S0, float* decay,
-                                       const int* q_start, const int* q_len, const int* slots, const int* live, int R, int H, int G,
-                                       int d, int e, int max_slots, int min_len, int n_portions, int n_chunks,
+                                       const int* q_start, const int* q_len, const int* slots, const int* live, int R, int H, int head0,
+                                       int heads, int G, int d, int e, int max_slots, int min_len, int n_portions, int n_chunks,
                                        unsigned* err, cudaStream_t st) {
     if (R <= 0 || n_portions <= 0 || n_chunks <= 0) return 0;
-    if (H <= 0 || G <= 0 || H % G || d <= 0 || e <= 0 || min_len < 1) return AIE_BAD_ARG;
+    if (heads <= 0 || head0 < 0 || head0 + heads > H || G <= 0 || H % G || d <= 0 || e <= 0 || min_len < 1) return AIE_BAD_ARG;
     const size_t at = (size_t)q | (size_t)k | (size_t)v | (size_t)state | (size_t)out | (size_t)W | (size_t)Kw | (size_t)U | (size_t)S0;
-    if ((d != 64 && d != 128) || e % 16 || ld % 4 || (at & 15) || H > 65535 || n_portions > 65535) return AIE_UNSUPPORTED;
-    const DpArgs p = {q, k, v, b_raw, a_raw, a_log, dt_bias, state, out, (bf16*)W, (bf16*)Kw, U, S0, decay, q_start, q_len, slots, live,
-                      err, ld, ldb, lda, R, H, G, e, max_slots, min_len, q_scale, unit_eps};
+    if ((d != 64 && d != 128) || e % 16 || ld % 4 || (at & 15) || heads > 65535 || n_portions > 65535) return AIE_UNSUPPORTED;
+    const size_t c = (size_t)head0 * e;
+    const DpArgs p = {q, k, v + c, b_raw + head0, a_raw + head0, a_log + head0, dt_bias + head0, state + c * d, out + c, (bf16*)W,
+                      (bf16*)Kw, U, S0, decay, q_start, q_len, slots, live, err, ld, ldb, lda, R, heads, H, head0, H / G, e, max_slots, min_len, q_scale, unit_eps};
     return d == 64 ? dp_go<64>(p, n_portions, n_chunks, st) : dp_go<128>(p, n_portions, n_chunks, st);
 }

@@ -21,7 +21,7 @@ struct LcArgs {
     float *state, *out, *L, *G;
     const int *q_start, *q_len, *slots;
     unsigned* err;
-    int ld, ld_decay, H, R, d, dv, max_slots, min_len;
+    int ld, ld_decay, H, all_heads, R, d, dv, max_slots, min_len;      // H: the heads of this launch, neighbours of all_heads
     float q_scale, k_scale;
 };
 
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(LC_THREADS) lc_scan_kernel(LcArgs p) {
     const int e = (blockIdx.x * LC_THREADS + threadIdx.x) * 4, size = p.d * p.dv;
     if (e >= size) return;
     const int row = e / p.dv;
-    float* sp = p.state + ((size_t)slot * p.H + h) * size + e;
+    float* sp = p.state + ((size_t)slot * p.all_heads + h) * size + e;
     float* L = p.L + ((size_t)first * p.H + h) * size + e;
     const float* G = p.G + ((size_t)first * p.H + h) * p.d + row;
     const size_t ls = (size_t)p.H * size, gs = (size_t)p.H * p.d;
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(LC_THREADS, 2) lc_out_kernel(LcArgs p) {
         for (int x = 0; x < NC; ++x) {
             const float4 o = hand[(m * NC + x) * LC_THREADS + (tid ^ 128)], a = half ? acc[4 + m][x] : acc[m][x];
             if (t < nt && x * 64 + col < p.dv)
-                *reinterpret_cast<float4*>(p.out + ((a0 + t) * p.H + h) * p.dv + x * 64 + col) =
+                *reinterpret_cast<float4*>(p.out + ((a0 + t) * p.all_heads + h) * p.dv + x * 64 + col) =
                     make_float4(p.q_scale * (a.x + o.x), p.q_scale * (a.y + o.y), p.q_scale * (a.z + o.z), p.q_scale * (a.w + o.w));
         }
     }
@@ -442,25 +442,28 @@ static int lc_go(const LcArgs& p, int n_portions, int n_chunks, cudaStream_t st)
     AIE_LAUNCH_CHECK();
 }
 
-// The arguments are those of aie_linear_recurrence.  L [n_chunks, H, d, dv] and G [n_chunks, H, d] float32 are scratch;
+// The arguments are those of aie_linear_recurrence.  Heads head0 .. head0 + heads - 1 of the H are done; L [n_chunks, heads, d, dv]
+// and G [n_chunks, heads, d] float32 are scratch;
 // n_portions, n_chunks: the requests that bring min_len tokens or more (the others are left alone), and their chunks of 64.
 // Takes d and dv up to 128 in steps of 4 whose rows start on 16 bytes (else AIE_UNSUPPORTED: the caller takes the
 // token-by-token kernel).
 extern "C" int aie_linear_recurrence_chunked(const float* q, const float* k, const float* v, int ld, const float* decay_tok,
                                              int ld_decay, const float* decay_head, float q_scale, float k_scale, float* state,
                                              float* out, float* L, float* G, const int* q_start, const int* q_len, const int* slots,
-                                             int R, int H, int d, int dv, int max_slots, int min_len, int n_portions,
+                                             int R, int H, int head0, int heads, int d, int dv, int max_slots, int min_len, int n_portions,
                                              int n_chunks, const float* fg_lower, const float* fg_bias, unsigned* err, cudaStream_t st) {
     if (R <= 0 || n_portions <= 0 || n_chunks <= 0) return 0;
-    if (H <= 0 || d <= 0 || dv <= 0 || min_len < 1 || (!decay_tok && !decay_head)) return AIE_BAD_ARG;
+    if (heads <= 0 || head0 < 0 || head0 + heads > H || d <= 0 || dv <= 0 || min_len < 1 || (!decay_tok && !decay_head)) return AIE_BAD_ARG;
     if (fg_lower ? (!decay_tok || k) : !k) return AIE_BAD_ARG;
     const size_t at = (size_t)q | (size_t)k | (size_t)v | (size_t)decay_tok | (size_t)state | (size_t)out | (size_t)L |
                       (size_t)fg_lower | (size_t)fg_bias;
     if (d > 128 || dv > 128 || d % 4 || dv % 4 || ld % 4 || (decay_tok && ld_decay % 4) || (at & 15) ||
-        H > 65535 || (long long)n_portions * H > 65535)
+        heads > 65535 || (long long)n_portions * heads > 65535)
         return AIE_UNSUPPORTED;
-    const LcArgs p = {q, k, v, decay_tok, decay_head, fg_lower, fg_bias, state, out, L, G, q_start, q_len, slots, err,
-                      ld, ld_decay, H, R, d, dv, max_slots, min_len, q_scale, k_scale};
+    const size_t c = (size_t)head0 * d, cv = (size_t)head0 * dv;
+    const auto from = [](const float* x, size_t n) { return x ? x + n : x; };
+    const LcArgs p = {q + c, from(k, c), v + cv, from(decay_tok, c), from(decay_head, head0), from(fg_lower, c), from(fg_bias, c),
+                      state + c * dv, out + cv, L, G, q_start, q_len, slots, err, ld, ld_decay, heads, H, R, d, dv, max_slots, min_len, q_scale, k_scale};
     if (d <= 64) return dv <= 64 ? lc_go<64, 64>(p, n_portions, n_chunks, st) : lc_go<64, 128>(p, n_portions, n_chunks, st);
     return dv <= 64 ? lc_go<128, 64>(p, n_portions, n_chunks, st) : lc_go<128, 128>(p, n_portions, n_chunks, st);
 }

@@ -20,7 +20,7 @@ struct SpArgs {
     float *state, *out, *L, *G;
     const int *q_start, *q_len, *slots;
     unsigned* err;
-    int ld, ld_dt, R, H, N, dv, hpg, max_slots, min_len, vec;
+    int ld, ld_dt, R, H, all_heads, head0, N, dv, hpg, max_slots, min_len, vec;      // H: the heads of this launch, from head0 on
     int hpb;             // neighbouring heads of one group that a block takes one after the other: B and C are read once for them
 };
 
@@ -83,8 +83,8 @@ __device__ __forceinline__ void sp_split(float a, float b, unsigned& hi, unsigne
     lo = pack_bf16(a - f.x, b - f.y);
 }
 
-template <int NP>      // rows of the state, padded (zero rows change nothing)
-__global__ void __launch_bounds__(SP_THREADS) sp_chunk_kernel(SpArgs p) {
+template <int NP>      // rows of the state, padded (zero rows change nothing); four blocks an SM: with three 53 instead of 45 us
+__global__ void __launch_bounds__(SP_THREADS, 4) sp_chunk_kernel(SpArgs p) {
     extern __shared__ __align__(16) unsigned char sp_sm[];
     __shared__ int found[2];
     __shared__ float dt[SP_T], la[SP_T];
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(SP_THREADS) sp_chunk_kernel(SpArgs p) {
     if (r < 0) return;
     const int nt = min(SP_T, p.q_len[r] - c * SP_T);
     const size_t a0 = (size_t)p.q_start[r] + c * SP_T;
-    sp_load<NP>(Bs, p.B + a0 * p.ld + (size_t)(h_first / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
+    sp_load<NP>(Bs, p.B + a0 * p.ld + (size_t)((p.head0 + h_first) / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
 #pragma unroll 1
     for (int h = h_first; h < h_first + p.hpb; ++h) {
         if (h > h_first) __syncthreads();                  // the last head's values are done with
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(SP_THREADS) sp_scan_kernel(SpArgs p) {
     }
     const int size = p.N * p.dv, e = (blockIdx.x * SP_THREADS + threadIdx.x) * V;
     if (e >= size) return;
-    float* sp = p.state + ((size_t)slot * p.H + h) * size + e;
+    float* sp = p.state + ((size_t)slot * p.all_heads + h) * size + e;
     float* L = p.L + ((size_t)first * p.H + h) * size + e;
     const float* G = p.G + (size_t)first * p.H + h;
     const size_t ls = (size_t)p.H * size;
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
     if (r < 0) return;
     const int nt = min(SP_T, p.q_len[r] - c * SP_T);
     const size_t a0 = (size_t)p.q_start[r] + c * SP_T;
-    sp_load<NP>(Cs, p.C + a0 * p.ld + (size_t)(h_first / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
-    sp_load<NP>(Bs, p.B + a0 * p.ld + (size_t)(h_first / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
+    sp_load<NP>(Cs, p.C + a0 * p.ld + (size_t)((p.head0 + h_first) / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
+    sp_load<NP>(Bs, p.B + a0 * p.ld + (size_t)((p.head0 + h_first) / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
     __syncthreads();
     const int ti = warp & 3, n0 = (warp >> 2) * 32, ta = ti * 16 + (lane >> 2), tb = ta + 8;
     unsigned cf[NP / 16][4];                           // the warp's 16 rows of C
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
                     u = fmaf(sk, xs.x, u);
                     v = fmaf(sk, xs.y, v);
                 }
-                float* o = p.out + ((a0 + t) * p.H + h) * p.dv + col0 + j;
+                float* o = p.out + ((a0 + t) * p.all_heads + h) * p.dv + col0 + j;
                 if (col0 + j < p.dv) o[0] = u;
                 if (col0 + j + 1 < p.dv) o[1] = v;
             }
@@ -362,23 +362,26 @@ static int sp_go(const SpArgs& p, int n_portions, int n_chunks, cudaStream_t st)
     AIE_LAUNCH_CHECK();
 }
 
-// The arguments are those of aie_state_space_chunked; L [n_chunks, H, N, dv] and G [n_chunks, H] float32 are scratch;
+// The arguments are those of aie_state_space_chunked.  Heads head0 .. head0 + heads - 1 of the H are done; L [n_chunks, heads, N,
+// dv] and G [n_chunks, heads] float32 are scratch;
 // n_portions, n_chunks: the requests that bring min_len tokens or more (the others are left alone), and their chunks of 64.
 // N <= 128.
 extern "C" int aie_state_space_parallel(const float* C, const float* B, const float* X, int ld, const float* dt_raw, int ld_dt,
                                         const float* dt_bias, const float* a_log, const float* skip, float* state, float* out,
-                                        float* L, float* G, const int* q_start, const int* q_len, const int* slots, int R, int H,
+                                        float* L, float* G, const int* q_start, const int* q_len, const int* slots, int R, int H, int head0, int heads,
                                         int N, int dv, int hpg, int max_slots, int min_len, int n_portions, int n_chunks, unsigned* err,
                                         cudaStream_t st) {
     if (R <= 0 || n_portions <= 0 || n_chunks <= 0) return 0;
-    if (H <= 0 || N <= 0 || dv <= 0 || hpg < 1 || H % hpg || !dt_raw || !dt_bias || !a_log || min_len < 1) return AIE_BAD_ARG;
-    if (N > 128 || H > 65535 || (long long)n_portions * H > 65535 || (dv + 63) / 64 > 65535) return AIE_UNSUPPORTED;
+    if (heads <= 0 || head0 < 0 || head0 + heads > H || N <= 0 || dv <= 0 || hpg < 1 || H % hpg || !dt_raw || !dt_bias || !a_log || min_len < 1) return AIE_BAD_ARG;
+    if (N > 128 || heads > 65535 || (long long)n_portions * heads > 65535 || (dv + 63) / 64 > 65535) return AIE_UNSUPPORTED;
     const int vec = N % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && !(((size_t)C | (size_t)B | (size_t)X | (size_t)L) & 15);
     // four or two heads a block where that still gives every SM's two places a block
     int hpb = 1;
-    while (hpb < 4 && hpg % (2 * hpb) == 0 && (long long)n_chunks * (H / (2 * hpb)) * ((dv + 63) / 64) >= 2 * aie_sm_count()) hpb *= 2;
-    const SpArgs p = {C, B, X, dt_raw, dt_bias, a_log, skip, state, out, L, G, q_start, q_len, slots, err,
-                      ld, ld_dt, R, H, N, dv, hpg, max_slots, min_len, vec, hpb};
+    while (hpb < 4 && hpg % (2 * hpb) == 0 && head0 % (2 * hpb) == 0 && heads % (2 * hpb) == 0 &&
+           (long long)n_chunks * (heads / (2 * hpb)) * ((dv + 63) / 64) >= 2 * aie_sm_count()) hpb *= 2;
+    const size_t c = (size_t)head0 * dv;
+    const SpArgs p = {C, B, X + c, dt_raw + head0, dt_bias + head0, a_log + head0, skip ? skip + head0 : skip, state + c * N, out + c, L, G,
+                      q_start, q_len, slots, err, ld, ld_dt, R, heads, H, head0, N, dv, hpg, max_slots, min_len, vec, hpb};
     if (N <= 32) return sp_go<32>(p, n_portions, n_chunks, st);
     if (N <= 64) return sp_go<64>(p, n_portions, n_chunks, st);
     return sp_go<128>(p, n_portions, n_chunks, st);

@@ -1048,8 +1048,48 @@ SSD_CHUNK = 64           # its chunk
 # n tokens each) 12 us walking the chunks against 18 in parallel (64, 1 x 64), 19 against 18 (32, 1 x 128), 33 against 24 (64, 1 x
 # 256), 36 against 27 (64, 4 x 64), 242 against 137 (64, 1 x 2048)
 SSD_PARALLEL_TOKENS = 160
-CHUNK_STATES_BYTES = 1 << 30       # the most that the states of a step's chunks may take (65,536 tokens x 16 heads of 128 x 128);
-                                   # beyond, portions go chunk after chunk or token by token and need no scratch
+# What the kernels that are parallel over chunks keep between their launches takes at most this much (16,384 tokens x 16 heads of
+# 128 x 128 of states).  More portions than that go behind one another, the heads of a longer one too: no bit depends on it.
+CHUNK_STATES_BYTES = 1 << 28
+
+
+def _portion_ranges(h_q_len, from_len: int, H: int, head_bytes: int, budget: int) -> list:
+    """The portions of from_len tokens or more as [(first request, one behind the last, portions, chunks of 64, first head, heads)],
+    each with at most `budget` bytes at head_bytes a chunk and head (one chunk-long head at the least) and 65,535 heads."""
+    out, group = [], None
+    for r in np.flatnonzero(h_q_len >= from_len).tolist():
+        c = (int(h_q_len[r]) + 63) // 64
+        if group and (group[3] + c) * H * head_bytes <= budget and (group[2] + 1) * H <= 65535:
+            group[1:4] = [r + 1, group[2] + 1, group[3] + c]
+            continue
+        heads = min(H, max(1, budget // (c * head_bytes)), 65535)
+        if heads == H:
+            group = [r, r + 1, 1, c, 0, H]
+            out.append(group)
+        else:
+            group = None
+            out += [[r, r + 1, 1, c, h, min(heads, H - h)] for h in range(0, H, heads)]
+    return out
+
+
+def _scratch(device, *sizes):
+    """A buffer and the addresses of its pieces of so many bytes (16 bytes aligned), or None where memory has no room for them
+    (callers then take a kernel that needs none)."""
+    starts = [0]
+    for n in sizes:
+        starts.append(starts[-1] + (n + 15) // 16 * 16)
+    try:
+        room = torch.empty(starts[-1], dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
+    at = room.data_ptr()
+    return room, [c_void_p(at + o) for o in starts[:-1]]
+
+
+def _range_lists(ctx, r0: int, r1: int):
+    """q_start, q_len and slots for a kernel over the requests r0 .. r1 - 1 (int32 lists: four bytes a request)."""
+    return tuple(c_void_p(t.data_ptr() + 4 * r0) for t in (ctx.q_start, ctx.q_len, ctx.slots))
+
 
 
 LC_CHUNK = 64            # chunk of the chunk-parallel kernels of the linear recurrence
@@ -1071,27 +1111,28 @@ def lc_min_len(H: int) -> int:
 
 def _recurrence_in_chunks(q, k, v, ld, decay_tok, decay_head, q_scale, k_scale, state, out, ctx, H, d, dv, lower, bias) -> int:
     """The portions of lc_min_len(H) tokens or more by the chunk-parallel kernels: that length; 0 (nothing is done) when there
-    is none or the sizes, strides or addresses are not theirs: heads of up to 128 in steps of 4, rows that start on 16 bytes."""
+    is none, memory has no room for the scratch, or the sizes, strides or addresses are not theirs: heads of up to 128 in steps of 4, rows that start on 16 bytes."""
     min_len = lc_min_len(H)
     if (ctx.max_q_len < min_len or d > 128 or dv > 128 or d % 4 or dv % 4 or ld % 4
             or (decay_tok is not None and decay_tok.stride(0) % 4)
             or any(t is not None and t.data_ptr() % 16 for t in (q, k, v, decay_tok, state, lower, bias))):
         return 0
-    lens = ctx.h_q_len[ctx.h_q_len >= min_len]
-    chunks = int(((lens + LC_CHUNK - 1) // LC_CHUNK).sum())
-    if 4 * chunks * H * d * dv > CHUNK_STATES_BYTES or len(lens) * H > 65535:
+    ranges = _portion_ranges(ctx.h_q_len, min_len, H, 4 * d * dv, CHUNK_STATES_BYTES)
+    most = max(chunks * heads for *_, chunks, _, heads in ranges)
+    room = _scratch(q.device, 4 * most * d * dv, 4 * most * d) if CHUNK_STATES_BYTES > 0 else None
+    if room is None:
         return 0
-    L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
-    G = torch.empty((chunks, H, d), dtype=torch.float32, device=q.device)
     lib = library("linear_recurrence_chunked.cu")
     T = q.shape[0]
     with region("linear_recurrence_chunked", _nb(out) + T * H * (2 * d + dv) * 4 + 2 * ctx.R * H * d * dv * 4, 4.0 * T * H * d * dv):
-        check(lib.aie_linear_recurrence_chunked(_p(q), _p(k), _p(v), c_int(ld), _p(decay_tok),
-                                                c_int(decay_tok.stride(0) if decay_tok is not None else 0), _p(decay_head),
-                                                c_float(q_scale), c_float(k_scale), _p(state), _p(out), _p(L), _p(G),
-                                                _p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d),
-                                                c_int(dv), c_int(state.shape[0]), c_int(min_len), c_int(len(lens)), c_int(chunks),
-                                                _p(lower), _p(bias), _p(ctx.err), _stream()), "linear_recurrence_chunked")
+        for r0, r1, portions, chunks, head0, heads in ranges:
+            check(lib.aie_linear_recurrence_chunked(_p(q), _p(k), _p(v), c_int(ld), _p(decay_tok),
+                                                    c_int(decay_tok.stride(0) if decay_tok is not None else 0), _p(decay_head),
+                                                    c_float(q_scale), c_float(k_scale), _p(state), _p(out), *room[1],
+                                                    *_range_lists(ctx, r0, r1), c_int(r1 - r0), c_int(H), c_int(head0), c_int(heads),
+                                                    c_int(d), c_int(dv), c_int(state.shape[0]), c_int(min_len), c_int(portions),
+                                                    c_int(chunks), _p(lower), _p(bias), _p(ctx.err), _stream()),
+                  "linear_recurrence_chunked")
     return min_len
 
 
@@ -1135,24 +1176,24 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
     if (chunked and dt_raw is not None and decay_tok is None and d <= 128 and ctx.max_q_len >= SSD_MIN_TOKENS
             and not os.environ.get("AI_ENGINE_B200_NO_CHUNKED_SCAN")):      # the switch is for measurement
         args = (_p(q), _p(k), _p(v), c_int(ld), _p(dt_raw), c_int(dt_raw.stride(0)), _p(dt_bias), _p(a_log), _p(skip), _p(state), _p(out))
-        lists = (_p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), c_int(ctx.R), c_int(H), c_int(d), c_int(dv), c_int(heads_per_group),
-                 c_int(state.shape[0]))
+        sizes = (c_int(d), c_int(dv), c_int(heads_per_group), c_int(state.shape[0]))
         with region("state_space_chunked", _nb(out) + T * H * (2 * d // heads_per_group + dv) * 4,
                     2.0 * T * H * (SSD_CHUNK * (d + dv) / 2 + 2 * d * dv)):
             from_len = max(SSD_MIN_TOKENS, SSD_PARALLEL_TOKENS)
-            lens = ctx.h_q_len[ctx.h_q_len >= from_len]
-            chunks = int(((lens + SSD_CHUNK - 1) // SSD_CHUNK).sum())
-            if not chunks or len(lens) * H > 65535 or 4 * chunks * H * d * dv > CHUNK_STATES_BYTES:
+            ranges = _portion_ranges(ctx.h_q_len, from_len, H, 4 * d * dv, CHUNK_STATES_BYTES)
+            most = max((chunks * heads for *_, chunks, _, heads in ranges), default=0)
+            room = _scratch(q.device, 4 * most * d * dv, 4 * most) if most and CHUNK_STATES_BYTES > 0 else None
+            if room is None:
                 from_len = 0
             else:
-                L = torch.empty((chunks, H, d, dv), dtype=torch.float32, device=q.device)
-                G = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
-                check(library("state_space_parallel.cu").aie_state_space_parallel(
-                    *args, _p(L), _p(G), *lists, c_int(from_len), c_int(len(lens)), c_int(chunks), _p(ctx.err), _stream()),
-                    "state_space_parallel")
+                for r0, r1, portions, chunks, head0, heads in ranges:
+                    check(library("state_space_parallel.cu").aie_state_space_parallel(
+                        *args, *room[1], *_range_lists(ctx, r0, r1), c_int(r1 - r0), c_int(H), c_int(head0), c_int(heads),
+                        *sizes, c_int(from_len), c_int(portions), c_int(chunks), _p(ctx.err), _stream()), "state_space_parallel")
             if not from_len or bool(((ctx.h_q_len >= SSD_MIN_TOKENS) & (ctx.h_q_len < from_len)).any()):
                 check(library("state_space_chunked.cu").aie_state_space_chunked(
-                    *args, *lists, c_int(SSD_MIN_TOKENS), c_int(max(from_len - 1, 0)), _p(ctx.err), _stream()), "state_space_chunked")
+                    *args, *_range_lists(ctx, 0, ctx.R), c_int(ctx.R), c_int(H), *sizes, c_int(SSD_MIN_TOKENS), c_int(max(from_len - 1, 0)),
+                    _p(ctx.err), _stream()), "state_space_chunked")
         if int(ctx.h_q_len.min()) >= SSD_MIN_TOKENS:
             return out
         max_len = SSD_MIN_TOKENS - 1                # the shorter portions and single tokens of the same step
@@ -1530,13 +1571,13 @@ def sink_attention(q: torch.Tensor, pages: torch.Tensor, gate: Optional[torch.Te
 
 DELTA_MIN_TOKENS = 32    # portions from this length on take the chunked delta-rule kernel (bfloat16 mode)
 DELTA_CHUNK = 64         # its chunk
-# A portion does in parallel what does not need the state, within this much scratch, from so many chunks of its own on (us, 16
+# A portion does in parallel what does not need the state from so many chunks of its own on (us, 16
 # heads of 128 x 128, a portion of 128 / 256 / 1024 tokens: 26 / 48 / 181 chunk after chunk, 40 / 45 / 87 in parallel; 8 heads of
 # 64 x 64: 19 / 35 / 130 and 28 / 30 / 47), or from so many (chunk, head, d e) of its own on (16 portions of 64 tokens, 16 heads
 # of 128 x 128, fill the machine alike: 129 and 86; 4 of them: 37 and 44; 16 portions of 64, 8 heads of 64 x 64: 26 and 31).
 DELTA_PARALLEL_CHUNKS = 4
 DELTA_PARALLEL_WORK = 96 * 128 * 128
-DELTA_PARALLEL_BYTES = 1 << 30
+DELTA_PARALLEL_BYTES = 1 << 28      # see CHUNK_STATES_BYTES (6,500 tokens x 16 heads of 128 x 128)
 
 
 def delta_parallel_len(H: int, d: int, e: int) -> int:
@@ -1545,23 +1586,25 @@ def delta_parallel_len(H: int, d: int, e: int) -> int:
     return max(DELTA_MIN_TOKENS, DELTA_CHUNK * (chunks - 1) + 1)
 
 
-def _delta_in_parallel(args, lists, ctx, q, k, v, state, out, from_len: int, H: int, d: int, e: int) -> bool:
-    """The chunks of portions of from_len tokens or more side by side; False: there are none, or the shapes, the rows'
-    alignment or the scratch do not fit."""
-    lens = ctx.h_q_len[ctx.h_q_len >= from_len]
-    chunks = int(((lens + DELTA_CHUNK - 1) // DELTA_CHUNK).sum())
-    scratch = chunks * H * (DELTA_CHUNK * (8 * d + 4 * e) + 4 * d * e + 4)
-    if (not chunks or d not in (64, 128) or e % 16 or q.stride(0) % 4 or scratch > DELTA_PARALLEL_BYTES or max(H, len(lens)) > 65535
+def _delta_in_parallel(args, ctx, q, k, v, state, out, from_len: int, H: int, G: int, d: int, e: int) -> bool:
+    """The chunks of portions of from_len tokens or more side by side; False: there are none, memory has no room for the
+    scratch, or the shapes or the rows' alignment do not fit."""
+    head_bytes = DELTA_CHUNK * (8 * d + 4 * e) + 4 * d * e + 4
+    ranges = _portion_ranges(ctx.h_q_len, from_len, H, head_bytes, DELTA_PARALLEL_BYTES)
+    if (not ranges or DELTA_PARALLEL_BYTES <= 0 or d not in (64, 128) or e % 16 or q.stride(0) % 4
             or any(t.data_ptr() % 16 for t in (q, k, v, state, out))):
         return False
-    pairs = torch.empty((2, chunks, H, 2, DELTA_CHUNK, d), dtype=torch.bfloat16, device=q.device)
-    U = torch.empty((chunks, H, DELTA_CHUNK, e), dtype=torch.float32, device=q.device)
-    S0 = torch.empty((chunks, H, d, e), dtype=torch.float32, device=q.device)
-    decay = torch.empty((chunks, H), dtype=torch.float32, device=q.device)
-    check(library("delta_rule_parallel.cu").aie_delta_rule_parallel(
-        *args, _p(pairs[0]), _p(pairs[1]), _p(U), _p(S0), _p(decay), *lists, c_int(from_len), c_int(len(lens)), c_int(chunks),
-        _p(ctx.err), _stream()),
-        "delta_rule_parallel")
+    most = max(chunks * heads for *_, chunks, _, heads in ranges)
+    pairs = most * 2 * DELTA_CHUNK * d * 2
+    room = _scratch(q.device, pairs, pairs, 4 * most * DELTA_CHUNK * e, 4 * most * d * e, 4 * most)
+    if room is None:
+        return False
+    for r0, r1, portions, chunks, head0, heads in ranges:
+        live = None if ctx.live is None else ctx.live.data_ptr() + 4 * r0
+        check(library("delta_rule_parallel.cu").aie_delta_rule_parallel(
+            *args, *room[1], *_range_lists(ctx, r0, r1), c_void_p(live), c_int(r1 - r0), c_int(H), c_int(head0), c_int(heads),
+            c_int(G), c_int(d), c_int(e), c_int(state.shape[0]), c_int(from_len), c_int(portions), c_int(chunks), _p(ctx.err), _stream()),
+            "delta_rule_parallel")
     return True
 
 
@@ -1595,7 +1638,7 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
                  c_int(state.shape[0]))
         with region("delta_rule_chunked", _nb(out) + T * (2 * G * d + H * e) * 4 + 2 * ctx.R * H * d * e * 4,
                     2.0 * T * H * (Q * d + Q * e + 3 * d * e)):
-            if not _delta_in_parallel(args, lists, ctx, q, k, v, state, out, from_len, H, d, e):
+            if not _delta_in_parallel(args, ctx, q, k, v, state, out, from_len, H, G, d, e):
                 from_len = 0
             if not from_len or bool(((ctx.h_q_len >= DELTA_MIN_TOKENS) & (ctx.h_q_len < from_len)).any()):
                 check(library("delta_rule_chunked.cu").aie_delta_rule_chunked(

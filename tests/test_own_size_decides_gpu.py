@@ -23,10 +23,7 @@ def alone_and_beside(run, lens, exact):
         assert torch.equal(out, out2) if exact(n) else near(out, out2), (i, n)
 
 
-@pytest.mark.parametrize("keyless", [False, True])
-@pytest.mark.parametrize("H,lens", [(16, [40, 300, 1, 53, 54, 9]), (40, [41, 12, 43, 42]),
-                                    (16, [1] * 33 + [70] + [3] * 34 + [130, 64])])
-def test_linear_recurrence(H, lens, keyless):
+def linear(H, lens, keyless):
     from ai_engine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(H)
     rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV)
@@ -43,7 +40,15 @@ def test_linear_recurrence(H, lens, keyless):
         assert int(ctx.err.item()) == 0
         return [(o, state[i]) for o, (i, _) in zip(out.split([n for _, n in reqs]), reqs)]
 
-    alone_and_beside(run, lens, lambda n: n >= ops.lc_min_len(H))
+    return run
+
+
+@pytest.mark.parametrize("keyless", [False, True])
+@pytest.mark.parametrize("H,lens", [(16, [40, 300, 1, 53, 54, 9]), (40, [41, 12, 43, 42]),
+                                    (16, [1] * 33 + [70] + [3] * 34 + [130, 64])])
+def test_linear_recurrence(H, lens, keyless):
+    from ai_engine_b200.kernels import ops
+    alone_and_beside(linear(H, lens, keyless), lens, lambda n: n >= ops.lc_min_len(H))
 
 
 @pytest.mark.parametrize("kind,extra", [("retention", [0.5, 0.9, 0.99]), ("gla", 8.0)])
@@ -69,9 +74,7 @@ def test_float32_linear_attention_whole_and_in_portions(kind, extra):
     assert float((outs[0] - outs[1]).abs().max()) <= 1e-5 * float(outs[0].abs().max())
 
 
-@pytest.mark.parametrize("H,hpg,lens", [(4, 2, [159, 40, 160, 5, 300, 1, 64]), (32, 4, [31, 32, 130, 100]),
-                                        (4, 1, [1] * 33 + [170] + [3] * 34 + [230, 40])])
-def test_state_space(H, hpg, lens):
+def state_space(H, hpg, lens):
     from ai_engine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(H)
     rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV)
@@ -87,12 +90,17 @@ def test_state_space(H, hpg, lens):
         assert int(ctx.err.item()) == 0
         return [(o, state[i]) for o, (i, _) in zip(out.split([n for _, n in reqs]), reqs)]
 
-    alone_and_beside(run, lens, lambda n: n >= ops.SSD_MIN_TOKENS)
+    return run
 
 
-@pytest.mark.parametrize("H,G,lens", [(4, 2, [192, 40, 193, 5, 300, 1, 64]), (24, 24, [31, 32, 130, 100, 280]),
-                                      (2, 1, [1] * 33 + [200] + [3] * 34 + [257, 40])])
-def test_delta_rule(H, G, lens):
+@pytest.mark.parametrize("H,hpg,lens", [(4, 2, [159, 40, 160, 5, 300, 1, 64]), (32, 4, [31, 32, 130, 100]),
+                                        (4, 1, [1] * 33 + [170] + [3] * 34 + [230, 40])])
+def test_state_space(H, hpg, lens):
+    from ai_engine_b200.kernels import ops
+    alone_and_beside(state_space(H, hpg, lens), lens, lambda n: n >= ops.SSD_MIN_TOKENS)
+
+
+def delta(H, G, lens):
     from ai_engine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(H)
     rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV)
@@ -109,7 +117,13 @@ def test_delta_rule(H, G, lens):
         assert int(ctx.err.item()) == 0
         return [(o, state[i]) for o, (i, _) in zip(out.split([n for _, n in reqs]), reqs)]
 
-    alone_and_beside(run, lens, lambda n: n > 1)
+    return run
+
+
+@pytest.mark.parametrize("H,G,lens", [(4, 2, [192, 40, 193, 5, 300, 1, 64]), (24, 24, [31, 32, 130, 100, 280]),
+                                      (2, 1, [1] * 33 + [200] + [3] * 34 + [257, 40])])
+def test_delta_rule(H, G, lens):
+    alone_and_beside(delta(H, G, lens), lens, lambda n: n > 1)
 
 
 def test_a_prompt_beside_so_many_lone_tokens_that_a_grid_over_all_of_them_would_be_too_large(monkeypatch):
@@ -130,3 +144,34 @@ def test_a_prompt_beside_so_many_lone_tokens_that_a_grid_over_all_of_them_would_
     for a, b in zip(run(x, lens), run(x[-40:], [40])):
         assert torch.equal(a, b)
     assert taken == [ops.lc_min_len(H)] * 2
+
+
+@pytest.mark.parametrize("make,sizes,lens,head_bytes", [
+    (linear, (6, False), [300, 1, 130, 200, 64, 190], 4 * 32 * 32), (state_space, (6, 3), [300, 1, 165, 40, 513, 200], 4 * 32 * 32),
+    (delta, (6, 2), [300, 1, 200, 40, 513, 200], 64 * (8 * 64 + 4 * 32) + 4 * 64 * 32 + 4)])
+def test_scratch_has_a_bound_and_no_bit_depends_on_it(make, sizes, lens, head_bytes, monkeypatch):
+    from ai_engine_b200.kernels import ops
+    reqs = list(enumerate(lens))
+    run = make(*sizes[:1], lens, sizes[1]) if make is linear else make(*sizes, lens)
+    want, sizes_asked, real = run(reqs), [], torch.empty
+    for budget in (40 * head_bytes, 10 * head_bytes, 1):          # some portions together, heads apart, one head at a time
+        for name in ("CHUNK_STATES_BYTES", "DELTA_PARALLEL_BYTES"):
+            monkeypatch.setattr(ops, name, budget)
+        with monkeypatch.context() as m:
+            m.setattr(ops, "_scratch", lambda device, *sizes, f=ops._scratch: sizes_asked.append(sum(sizes)) or f(device, *sizes))
+            got = run(reqs)
+        longest = max(-(-n // 64) for n in lens)
+        assert sizes_asked.pop() <= 1.04 * max(budget, longest * head_bytes) and not sizes_asked      # 4 %: what the decays take
+        for (a, b), (c, d) in zip(want, got):
+            assert torch.equal(a, c) and torch.equal(b, d)
+    monkeypatch.undo()
+
+    def full(shape, *a, **k):
+        raise torch.OutOfMemoryError("no room")
+
+    with monkeypatch.context() as m:                              # no room at all: a kernel that needs none
+        m.setattr(ops, "_scratch", lambda device, *sizes, f=ops._scratch: [m.setattr(torch, "empty", full), f(device, *sizes),
+                                                                          m.setattr(torch, "empty", real)][1])
+        got = run(reqs)
+    for (a, b), (c, d) in zip(want, got):
+        assert float((a - c).abs().max()) <= 2e-3 * float(a.abs().max()) and float((b - d).abs().max()) <= 2e-3 * float(b.abs().max())
