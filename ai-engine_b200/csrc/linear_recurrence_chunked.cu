@@ -400,11 +400,13 @@ __global__ void __launch_bounds__(LC_THREADS, 2) lc_out_kernel(LcArgs p) {
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
             if (m < jb) continue;
-            const float2 w = *reinterpret_cast<const float2*>(A + (rg + 8 * m) * LC_T + j);     // 0 behind the query
+            const float2 w = *reinterpret_cast<const float2*>(A + (rg + 8 * m) * LC_T + j);
+            // a value behind the query is left out, not multiplied by 0: it may be an infinity
+            const bool sees = m > jb || j <= rg + 8 * m, next = m > jb || j + 1 <= rg + 8 * m;
 #pragma unroll
             for (int x = 0; x < NC; ++x) {
-                fma4(acc[m][x], w.x, vv[0][x]);
-                fma4(acc[m][x], w.y, vv[1][x]);
+                if (sees) fma4(acc[m][x], w.x, vv[0][x]);
+                if (next) fma4(acc[m][x], w.y, vv[1][x]);
             }
         }
     }

@@ -93,3 +93,23 @@ def test_a_slot_outside_its_table_is_flagged_and_writes_no_state():
     ctx = Ctx([128], [1])
     ops.linear_recurrence(x[:, :8], x[:, 8:16], x[:, 16:], None, torch.ones(1, device=DEV), 1.0, 1.0, state, ctx, 1, 8, 8)
     assert int(ctx.err.item()) == 8 and bool((state == 1).all())
+
+
+@pytest.mark.parametrize("what", ["k", "v", "q", "decay"])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_value_that_is_not_finite_reaches_no_earlier_token(what, value):
+    from ai_engine_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    T, H, d = 200, 2, 64
+    rows, clean = torch.randn(T, 4 * H * d, generator=gen, device=DEV), None
+    rows[:, 3 * H * d:] = torch.sigmoid(rows[:, 3 * H * d:])
+    for at in (None, 5, 64, 77, 126, 199):
+        x = rows.clone()
+        if at is not None:
+            x[at, "qkv".find(what) * H * d if what != "decay" else 3 * H * d:][:H * d] = value
+        q, k, v, a = (x[:, i * H * d:(i + 1) * H * d] for i in range(4))
+        out = ops.linear_recurrence(q, k, v, a, None, 1.0, 1.0, torch.zeros(1, H, d, d, device=DEV), Ctx([T], [0]), H, d, d)
+        if at is None:
+            clean = out
+        else:
+            assert torch.equal(out[:at], clean[:at]) and not bool(torch.isfinite(out[at]).all())
