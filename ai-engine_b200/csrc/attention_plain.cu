@@ -114,8 +114,9 @@ extern "C" int aie_paged_attention_plain(const void* q, const void* k_pages, con
 // ---------------------------------------------------------------------------
 // The same for portions of prompts in float32, 64 query tokens of one request and one head a block: keys and values of a
 // chunk are read once for all of them, scores and outputs are tiles of FMAs.  A block's additions are those of the kernel
-// above, in its order (the dot product over e, the butterfly sum of a chunk's 128 weights, the values over j), so a
-// token's bits do not depend on which of the two computes it.  Bound by the FMA units and, for few heads and tokens, by
+// above, in its order (the dot product over e, the butterfly sum of a chunk's 128 weights, the values over j), and keys that a
+// query does not see take no part in them (their values may be infinities), so a token's bits do not depend on which of
+// the two computes it.  Bound by the FMA units and, for few heads and tokens, by
 // the longest block's chain of chunks.
 // A warp owns 16 query rows; lanes lie 4 x 8: rows lm + 4 i, keys ln + 8 j, output columns 4 (ln + 8 x) .. + 3.
 #define PT_Q 64
@@ -213,10 +214,13 @@ paged_attention_f32_tiles_kernel(const float* __restrict__ q, const float* __res
                 const int pos = pos0 + warp * 16 + lm + 4 * i;
                 const int lo = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
                 float mx = -INFINITY;
+                unsigned sees = 0;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     const int key = c0 + ln + 8 * j;
-                    s[i][j] = ((seen >> j) & 1) && key >= lo && key <= pos ? s[i][j] * scale : -INFINITY;
+                    const bool see = ((seen >> j) & 1) && key >= lo && key <= pos;
+                    sees |= (see ? 1u : 0u) << j;
+                    s[i][j] = see ? s[i][j] * scale : -INFINITY;
                     mx = fmaxf(mx, s[i][j]);
                 }
 #pragma unroll
@@ -227,13 +231,15 @@ paged_attention_f32_tiles_kernel(const float* __restrict__ q, const float* __res
                 for (int g = 0; g < 4; ++g) {                    // 32 keys: the butterfly 16, 8, then 4, 2, 1 over the lanes
 #pragma unroll
                     for (int x = 0; x < 4; ++x)
-                        s[i][4 * g + x] = s[i][4 * g + x] == -INFINITY ? 0.f : expf(s[i][4 * g + x] - m_new);
+                        s[i][4 * g + x] = (sees >> (4 * g + x)) & 1 ? expf(s[i][4 * g + x] - m_new) : 0.f;
                     w[g] = (s[i][4 * g] + s[i][4 * g + 2]) + (s[i][4 * g + 1] + s[i][4 * g + 3]);
 #pragma unroll
                     for (int o = 4; o > 0; o >>= 1) w[g] += __shfl_xor_sync(0xffffffffu, w[g], o);
                 }
-                const float corr = (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_new);
-                l[i] = l[i] * corr + ((w[0] + w[2]) + (w[1] + w[3]));
+                // a chunk that the query has no key in leaves its sums alone
+                const bool here = c0 <= pos && c0 + PLAIN_CHUNK > lo;
+                const float corr = !here ? 1.f : (m[i] == -INFINITY) ? 0.f : expf(m[i] - m_new);
+                if (here) l[i] = l[i] * corr + ((w[0] + w[2]) + (w[1] + w[3]));
                 m[i] = m_new;
 #pragma unroll
                 for (int x = 0; x < ND; ++x) {
@@ -256,11 +262,42 @@ paged_attention_f32_tiles_kernel(const float* __restrict__ q, const float* __res
         if (works) {
             const float* pr = p_s + (warp * 16 + lm) * ldp;
             const int nk = min(PLAIN_CHUNK, last - c0 + 1);
+            // the warp's rows from .. to (keys of the chunk) that all its queries see: outside of it each query is asked
+            const int first = pos0 + warp * 16, lo_last = window > 0 ? max(min(first + 15, last) - window + 1, 0) : 0;
+            const int from = lo_last - c0, to = first - c0;
 #pragma unroll 1
             for (int j = 0; j < nk; j += 2) {                    // a key behind the last has weight and value 0
                 float2 a[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float2*>(pr + 4 * i * ldp + j);
+                if (j < from || j + 1 > to) {
+#pragma unroll 1
+                    for (int y = 0; y < 2; ++y) {
+                        const int key = c0 + j + y;
+                        bool sees[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int pos = first + lm + 4 * i;
+                            sees[i] = key <= pos && (window <= 0 || key > pos - window);
+                        }
+#pragma unroll
+                        for (int x = 0; x < ND; ++x) {
+                            const int c = 4 * (ln + 8 * x);
+                            if (c >= d) continue;
+                            const float4 b = *reinterpret_cast<const float4*>(v_s + (j + y) * d + c);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (sees[i]) {
+                                    const float w = y ? a[i].y : a[i].x;
+                                    acc[i][x].x = fmaf(w, b.x, acc[i][x].x);
+                                    acc[i][x].y = fmaf(w, b.y, acc[i][x].y);
+                                    acc[i][x].z = fmaf(w, b.z, acc[i][x].z);
+                                    acc[i][x].w = fmaf(w, b.w, acc[i][x].w);
+                                }
+                        }
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int x = 0; x < ND; ++x) {
                     const int c = 4 * (ln + 8 * x);

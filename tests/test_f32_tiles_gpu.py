@@ -78,3 +78,40 @@ def test_attention_of_portions_has_the_plain_kernel_s_bits(H, K, d, P, reqs, win
     assert int(err.item()) == 2
     want = ops.paged_attention_plain(q, lc.k_pages, lc.v_pages, ctx.positions, ctx.token_req, bad, 0.3, 0, err)
     assert torch.equal(got, want)
+
+
+def step(H, K, d, P, reqs, seed=1):
+    """A step over filled pages: (ctx, cache, queries)."""
+    from ai_engine_b200.cache import PagedCache
+    from ai_engine_b200.engine.step import StepContext, StepEntry
+    from ai_engine_b200.parts import ATTENTION_WORK, CacheNeed, KVRequest
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    cache = PagedCache([CacheNeed(0, "m", KVRequest(K, d))], P, sum(-(-(c + n) // P) for c, n in reqs), len(reqs), 4096, torch.float32, DEV)
+    entries = []
+    for c, n in reqs:
+        s = cache.admit()
+        cache.ensure(s, c + n)
+        entries.append(StepEntry(s, c, [0] * n, []))
+    cache.groups[0].pool.normal_(generator=gen)
+    ctx = StepContext(entries, cache, torch.device(DEV), torch.zeros(1, dtype=torch.int32, device=DEV), planners=(ATTENTION_WORK,))
+    return ctx, cache.layer_cache(0, ctx)["m"], torch.randn(sum(n for _, n in reqs), H, d, generator=gen, device=DEV)
+
+
+def both(ctx, lc, q, window):
+    from ai_engine_b200.kernels import ops
+    from ai_engine_b200.parts import ATTENTION_WORK
+    return (ops.paged_attention(q, lc.k_pages, lc.v_pages, ctx, ctx.plan(ATTENTION_WORK), lc.block_table, 0.3, window),
+            ops.paged_attention_plain(q, lc.k_pages, lc.v_pages, ctx.positions, ctx.token_req, lc.block_table, 0.3, window, ctx.err))
+
+
+@pytest.mark.parametrize("window", [0, 40, 129])
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan")])
+@pytest.mark.parametrize("plane", [0, 1])
+def test_keys_and_values_that_are_not_finite_reach_the_queries_that_see_them(plane, value, window):
+    ctx, lc, q = step(4, 2, 64, 16, [(0, 150), (200, 70)])
+    planes = (lc.k_pages, lc.v_pages)[plane]
+    for r, at in ((0, 3), (0, 63), (0, 131), (1, 20), (1, 150), (1, 233)):
+        planes[int(lc.block_table[r, at // 16]), :, at % 16, ::5] = value
+    got, want = both(ctx, lc, q, window)
+    assert bool(torch.isfinite(want).any()) and not bool(torch.isfinite(want).all())
+    assert torch.equal(got.nan_to_num(nan=1e30, posinf=2e30, neginf=3e30), want.nan_to_num(nan=1e30, posinf=2e30, neginf=3e30))
