@@ -664,7 +664,8 @@ def paged_attention(q, k_pages, v_pages, ctx, work, block_table, scale: float, w
         pre_cost = (float((cl[~lone] + ql[~lone]).sum()) * K * d * 2 * es + float(ql[~lone].sum()) * H * d * 2 * es,
                     4.0 * pairs * H * d)
     if not fast and q.dtype == torch.float32 and k_pages.dtype == torch.float32 and d <= 128 and d % 4 == 0 \
-            and getattr(ctx, "max_q_len", 0) >= F32_TILE_MIN_TOKENS and getattr(work, "prefill_tiles", None) is not None:
+            and getattr(ctx, "max_q_len", 0) >= F32_TILE_MIN_TOKENS and getattr(work, "prefill_tiles", None) is not None \
+            and k_pages.shape[0] * k_pages.shape[2] <= 0x7fffffff and not any(t.data_ptr() % 16 for t in (q, k_pages, v_pages)):
         return _paged_attention_f32(q, k_pages, v_pages, ctx, work, block_table, scale, window, dec_cost, pre_cost)
     if not fast:
         return paged_attention_plain(q, k_pages, v_pages, ctx.positions, ctx.token_req, block_table,

@@ -115,3 +115,13 @@ def test_keys_and_values_that_are_not_finite_reach_the_queries_that_see_them(pla
     got, want = both(ctx, lc, q, window)
     assert bool(torch.isfinite(want).any()) and not bool(torch.isfinite(want).all())
     assert torch.equal(got.nan_to_num(nan=1e30, posinf=2e30, neginf=3e30), want.nan_to_num(nan=1e30, posinf=2e30, neginf=3e30))
+
+
+def test_operands_off_the_16_byte_grid_take_the_plain_kernel():
+    ctx, lc, q = step(2, 1, 20, 4, [(3, 70), (0, 9)])
+    off = lambda t: torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape)
+    got, want = both(ctx, lc, off(q), 0)
+    assert torch.equal(got, want)
+    planes = type("Planes", (), dict(k_pages=lc.k_pages, v_pages=off(lc.v_pages), block_table=lc.block_table))
+    got, want = both(ctx, planes, q, 33)
+    assert torch.equal(got, want) and int(ctx.err.item()) == 0
