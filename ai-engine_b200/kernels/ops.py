@@ -617,7 +617,28 @@ def prefill_takes_pairs(n_tiles: int, n_units: int, heads: int) -> bool:
     return 0.86 * math.ceil(w2) / w2 < math.ceil(w1) / w1
 
 
-F32_TILE_MIN_TOKENS = 8      # steps whose longest portion is shorter leave all tokens to the plain kernel
+# Steps whose longest portion is shorter leave all tokens to the plain kernel.  A layer of 32 heads of 64, us, plain against
+# tiles: 8 tokens behind 0 / 1,000 / 3,000 cached ones 572 / 1,056 / 2,015 against 581 / 759 / 1,135, eight times 8 behind 500 1,013
+# against 726.
+F32_TILE_MIN_TOKENS = 8
+# A chunk of 128 keys in a block's chain takes about 60 us in the plain kernel (16 blocks an SM) and 23 us in the tiled one (two
+# of 64 columns or less an SM) at heads of 64, for both in proportion to the heads' size.
+F32_CHUNK_PLAIN, F32_CHUNK_TILES = 60.0, 23.0
+
+
+def f32_tiles_pay(lens, cached, H: int, d: int, window: int, sms: int = 148) -> bool:
+    """Whether a step's portions in tiles behind its lone tokens in the plain kernel take less than all of them in the plain one
+    (the bits are the same): 16 lone tokens and 8 of a portion behind 500 cached ones each, 929 us in two kernels and 847 in one;
+    with 64 tokens of a new prompt instead, 1,010 and 1,002."""
+    lone = lens == 1
+    if not lone.any():
+        return True
+    keys = cached + lens
+    chunks = np.minimum(keys, window + 127 if window > 0 else keys) // 128 + 1
+    plain = lambda m: F32_CHUNK_PLAIN * max(int(chunks[m].max()), int((lens * chunks)[m].sum()) * H / (16 * sms))
+    tiles = (lens + 63) // 64 * chunks
+    tiled = F32_CHUNK_TILES * max(int(chunks[~lone].max()), int(tiles[~lone].sum()) * H / ((2 if d <= 64 else 1) * sms))
+    return tiled + plain(lone) < plain(lens > 0)
 
 
 def _paged_attention_f32(q, k_pages, v_pages, ctx, work, block_table, scale, window, dec_cost, pre_cost):
@@ -665,7 +686,8 @@ def paged_attention(q, k_pages, v_pages, ctx, work, block_table, scale: float, w
                     4.0 * pairs * H * d)
     if not fast and q.dtype == torch.float32 and k_pages.dtype == torch.float32 and d <= 128 and d % 4 == 0 \
             and getattr(ctx, "max_q_len", 0) >= F32_TILE_MIN_TOKENS and getattr(work, "prefill_tiles", None) is not None \
-            and k_pages.shape[0] * k_pages.shape[2] <= 0x7fffffff and not any(t.data_ptr() % 16 for t in (q, k_pages, v_pages)):
+            and k_pages.shape[0] * k_pages.shape[2] <= 0x7fffffff and not any(t.data_ptr() % 16 for t in (q, k_pages, v_pages)) \
+            and f32_tiles_pay(ctx.h_q_len, ctx.h_ctx_len, H, d, window, sm_count()):
         return _paged_attention_f32(q, k_pages, v_pages, ctx, work, block_table, scale, window, dec_cost, pre_cost)
     if not fast:
         return paged_attention_plain(q, k_pages, v_pages, ctx.positions, ctx.token_req, block_table,
