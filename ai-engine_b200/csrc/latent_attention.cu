@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(LAT_CHUNK)
 latent_attention_kernel(const float* __restrict__ q_full, const C* __restrict__ pages, O* __restrict__ out,
                         const int* __restrict__ positions, const int* __restrict__ token_req,
                         const int* __restrict__ block_table, int bt_width, int num_pages, int P, int H, int rank,
-                        int dk, int window, float scale, const float* __restrict__ sink, unsigned* err) {
+                        int dk, int window, float scale, const float* __restrict__ sink, const int* __restrict__ q_len, unsigned* err) {
     extern __shared__ __align__(16) float sm[];
     float* q_s = sm;                                   // dk (rounded up to even)
     float* p_s = q_s + ((dk + 1) & ~1);                // CHUNK
@@ -139,6 +139,7 @@ latent_attention_kernel(const float* __restrict__ q_full, const C* __restrict__ 
 
     const int t = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
     const int pos = positions[t], row = token_req[t];
+    if (q_len && q_len[row] == 1) return;              // lone tokens are another kernel's
     for (int e = tid; e < dk; e += blockDim.x) q_s[e] = q_full[((size_t)t * H + h) * dk + e];
     __syncthreads();
 
@@ -199,13 +200,13 @@ latent_attention_kernel(const float* __restrict__ q_full, const C* __restrict__ 
 template <typename C, typename O>
 static int latent_go(const float* q_full, const void* pages, void* out, const int* positions, const int* token_req,
                      const int* block_table, int bt_width, int num_pages, int P, int T, int H, int rank, int dk,
-                     int window, float scale, const float* sink, unsigned* err, cudaStream_t st) {
+                     int window, float scale, const float* sink, const int* q_len, unsigned* err, cudaStream_t st) {
     const size_t smem = (size_t)(((dk + 1) & ~1) + LAT_CHUNK + 32) * sizeof(float) + LAT_CHUNK * sizeof(long long);
     dim3 grid(T, H);
 #define GO(N)                                                                                                        \
     latent_attention_kernel<C, O, N><<<grid, LAT_CHUNK, smem, st>>>(q_full, (const C*)pages, (O*)out, positions,     \
                                                                     token_req, block_table, bt_width, num_pages, P, \
-                                                                    H, rank, dk, window, scale, sink, err)
+                                                                    H, rank, dk, window, scale, sink, q_len, err)
     if (rank <= LAT_CHUNK) GO(1);
     else if (rank <= 2 * LAT_CHUNK) GO(2);
     else if (rank <= 4 * LAT_CHUNK) GO(4);
@@ -214,18 +215,19 @@ static int latent_go(const float* q_full, const void* pages, void* out, const in
     AIE_LAUNCH_CHECK();
 }
 
+// q_len [requests] (or null): tokens of requests that bring one are left alone.
 extern "C" int aie_latent_attention(const float* q_full, const void* pages, int cache_dtype, void* out, int out_dtype,
                                     const int* positions, const int* token_req, const int* block_table, int bt_width,
                                     int num_pages, int P, int T, int H, int rank, int dk, int window, float scale,
-                                    const float* sink, unsigned* err, cudaStream_t st) {
+                                    const float* sink, const int* q_len, unsigned* err, cudaStream_t st) {
     if (T <= 0) return 0;
     if (rank <= 0 || dk < rank || H <= 0 || H > 65535) return AIE_BAD_ARG;
     if (rank > 8 * LAT_CHUNK || dk > 8192) return AIE_UNSUPPORTED;
     if (cache_dtype == AIE_F32 && out_dtype == AIE_F32)
-        return latent_go<float, float>(q_full, pages, out, positions, token_req, block_table, bt_width, num_pages, P, T, H, rank, dk, window, scale, sink, err, st);
+        return latent_go<float, float>(q_full, pages, out, positions, token_req, block_table, bt_width, num_pages, P, T, H, rank, dk, window, scale, sink, q_len, err, st);
     if (cache_dtype == AIE_BF16 && out_dtype == AIE_BF16)
-        return latent_go<bf16, bf16>(q_full, pages, out, positions, token_req, block_table, bt_width, num_pages, P, T, H, rank, dk, window, scale, sink, err, st);
+        return latent_go<bf16, bf16>(q_full, pages, out, positions, token_req, block_table, bt_width, num_pages, P, T, H, rank, dk, window, scale, sink, q_len, err, st);
     if (cache_dtype == AIE_BF16 && out_dtype == AIE_F32)
-        return latent_go<bf16, float>(q_full, pages, out, positions, token_req, block_table, bt_width, num_pages, P, T, H, rank, dk, window, scale, sink, err, st);
+        return latent_go<bf16, float>(q_full, pages, out, positions, token_req, block_table, bt_width, num_pages, P, T, H, rank, dk, window, scale, sink, q_len, err, st);
     return AIE_BAD_ARG;
 }

@@ -1,18 +1,17 @@
 // Tensor-core attention over the compressed cache (bfloat16 rows [latent (rank) | rotated key part (rot)], one per
 // token, shared by all heads): see latent_attention.cu for the formula.  All heads of a token multiply the same
-// cache rows, so the heads are the rows of the products: one CTA owns one query token and a group of 16 heads
-// (one m16 tile of mma.sync m16n8k16, bf16 in, float32 accumulate) and walks the token's visible keys in chunks
-// of 64 that start at multiples of 64 of the absolute key position (a row's additions depend on its position
-// only, not on how the prompt was cut or on the batch).  A CTA of a prompt's portion takes TQ = 4 consecutive tokens
-// of one request (four warps each): they share the gathered cache rows, whose traffic from L2 bounds the kernel,
-// and differ only in their masks.  (Lone tokens take latent_decode_kernel below.)
+// cache rows, so the heads are the rows of the products: four warps take one query token and a group of 16 heads
+// (one m16 tile of mma.sync m16n8k16, bf16 in, float32 accumulate) and walk the token's visible keys in chunks
+// of 64 that start at multiples of 64 of the absolute key position.  A CTA takes TQ = 4 consecutive tokens of a portion: they
+// share the gathered cache rows, whose traffic from L2 bounds the kernel, and differ only in their masks.  (Lone tokens
+// take latent_decode_kernel below.)
 //
 // Per chunk: the 64 cache rows are gathered page by page into shared memory by 16-byte cp.async copies (rows
 // outside the mask or the block table are zero-filled, so a probability of 0 never meets an unwritten row);
 // S = Q K^T with the chunk's keys split over the four warps; scores, mask, running maximum and sum in float32
 // in shared memory (eight threads a row); O += P V with the latent's columns split over the four warps, V being
-// the first `rank` columns of the same rows (ldmatrix.trans).  Few tokens in a step (decoding) cut each token's
-// chunks into `splits` parts that run as CTAs of their own and leave (maximum, sum, unnormalised output) for a
+// the first `rank` columns of the same rows (ldmatrix.trans).  Where the portions are few, each token's
+// chunks are cut into `splits` parts that run as CTAs of their own and leave (maximum, sum, unnormalised output) for a
 // joining kernel.  Weights enter the product with the rows rounded to bfloat16 and are summed so, or (PAIR) as two
 // bfloat16 terms each, 16 bits of mantissa, beside a float32 sum.  A sink (exp(sink[h]) in the denominator, nothing in the output) opens the running softmax of the first part.
 #include "attention_prefill.cuh"
@@ -22,15 +21,15 @@
 #define LT_THREADS 128
 #define LT_TOKENS 4
 
-template <int CW, int TQ, bool PAIR>      // latent columns per warp (rank = 4 CW); tokens per CTA; weights as two terms
-__global__ void __launch_bounds__(LT_THREADS * TQ)
+template <int CW, bool PAIR>      // latent columns per warp (rank = 4 CW); weights as two terms
+__global__ void __launch_bounds__(LT_THREADS * LT_TOKENS)
 latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restrict__ pages, bf16* __restrict__ out,
                            float* __restrict__ part_o, float* __restrict__ part_ml, const int* __restrict__ tiles,
                            const int* __restrict__ q_start, const int* __restrict__ q_len,
                            const int* __restrict__ ctx_len, const int* __restrict__ block_table, int bt_width,
                            int num_pages, int P, int H, int dk, int window, float scale, int splits,
-                           const float* __restrict__ sink, int min_len, int max_len, unsigned* err) {
-    constexpr int RANK = 4 * CW, NT = CW / 8, THREADS = LT_THREADS * TQ;
+                           const float* __restrict__ sink, unsigned* err) {
+    constexpr int RANK = 4 * CW, NT = CW / 8, TQ = LT_TOKENS, THREADS = LT_THREADS * TQ;
     extern __shared__ __align__(16) unsigned char lt_raw[];
     const int SK = dk + 8;                                        // padded row: ldmatrix rows fall on different banks
     bf16* q_all = reinterpret_cast<bf16*>(lt_raw);                // [TQ][16][SK]
@@ -45,8 +44,6 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
     pdl_launch_dependents();
     pdl_wait();
     const int row = tiles[2 * blockIdx.x], off = tiles[2 * blockIdx.x + 1];
-    const int brings = q_len[row];                                // lone tokens and longer portions are other kernels'
-    if (brings < min_len || (max_len > 0 && brings > max_len)) return;
     const int h0 = blockIdx.y * LT_ROWS, part = blockIdx.z;
     const int tid = threadIdx.x, tq = tid / LT_THREADS, ltid = tid % LT_THREADS, warp = (tid >> 5) & 3, lane = tid & 31;
     const int n_act = min(TQ, q_len[row] - off);                  // tokens of this CTA that exist
@@ -629,37 +626,34 @@ __global__ void latent_join_kernel(const float* __restrict__ part_o, const float
 }
 
 // q_full [T, H, dk] float32; pages [num_pages, P, dk] bfloat16; out [T, H, rank] bfloat16.  tiles [n_tiles, 2] =
-// (request row, offset among the tokens it brings) of units of `tq` = 4 tokens.  Requests that bring fewer than min_len or
-// (max_len > 0) more than max_len tokens are left alone.  Takes rank = 64 .. 512 in
-// steps of 64 and dk a multiple of 16 (else AIE_UNSUPPORTED: the caller takes the plain kernel).  splits > 1 needs
-// part_o [T, H, splits, rank] and part_ml [T, H, splits, 2] float32.
+// (request row, offset among the tokens it brings) of units of LT_TOKENS tokens; requests that it does not name are left
+// alone.  Takes rank = 64 .. 512 in steps of 64, dk a multiple of 16 and rows that shared memory has room for (else
+// AIE_UNSUPPORTED: the caller takes the plain kernel).  splits > 1 needs part_o [T, H, splits, rank] and part_ml [T, H,
+// splits, 2] float32.
 extern "C" int aie_latent_attention_tc(const float* q_full, const void* pages, void* out, float* part_o, float* part_ml,
-                                       const int* tiles, int n_tiles, int tq, const int* q_start, const int* q_len,
+                                       const int* tiles, int n_tiles, const int* q_start, const int* q_len,
                                        const int* ctx_len, const int* block_table, int bt_width,
                                        int num_pages, int P, int T, int H, int rank, int dk, int window, float scale,
-                                       int splits, const float* sink, int pair, int min_len, int max_len, unsigned* err, cudaStream_t st) {
+                                       int splits, const float* sink, int pair, unsigned* err, cudaStream_t st) {
     if (T <= 0 || n_tiles <= 0) return 0;
     if (rank < 64 || rank > 512 || rank % 64 || dk % 16 || dk < rank || dk > 1024 || H <= 0) return AIE_UNSUPPORTED;
-    if (splits < 1 || splits > 64 || (splits > 1 && (!part_o || !part_ml)) || tq != LT_TOKENS) return AIE_BAD_ARG;
+    if (splits < 1 || splits > 64 || (splits > 1 && (!part_o || !part_ml))) return AIE_BAD_ARG;
     const int SK = dk + 8;
-    const size_t smem = (size_t)(tq * LT_ROWS + LT_KEYS) * SK * 2 + (size_t)tq * LT_ROWS * (LT_KEYS + 8) * 2 * (pair ? 2 : 1) +
-                        (size_t)tq * (LT_ROWS * (LT_KEYS + 1) + 3 * LT_ROWS) * 4;
+    const size_t smem = (size_t)(LT_TOKENS * LT_ROWS + LT_KEYS) * SK * 2 + (size_t)LT_TOKENS * LT_ROWS * (LT_KEYS + 8) * 2 * (pair ? 2 : 1) +
+                        (size_t)LT_TOKENS * (LT_ROWS * (LT_KEYS + 1) + 3 * LT_ROWS) * 4;
     if (smem > 220 * 1024) return AIE_UNSUPPORTED;
     dim3 grid(n_tiles, (H + LT_ROWS - 1) / LT_ROWS, splits);
     if (grid.y > 65535) return AIE_UNSUPPORTED;
-#define GO2(CWV, TQV, PV)                                                                                             \
+#define GO1(CWV, PV)                                                                                                  \
     {                                                                                                                 \
-        auto kern = latent_attention_tc_kernel<CWV, TQV, PV>;                                                         \
+        auto kern = latent_attention_tc_kernel<CWV, PV>;                                                              \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                           \
-        launch_pdl(kern, grid, dim3(LT_THREADS * TQV), smem, st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, tiles,    \
-                                                   q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, H,   \
-                                                   dk, window, scale, splits, sink, min_len, max_len, err);                                   \
+        launch_pdl(kern, grid, dim3(LT_THREADS * LT_TOKENS), smem, st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, tiles, \
+                   q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, H, dk, window, scale, splits, sink, err);             \
     }
-#define GO1(CWV, TQV)                                                                                                 \
-    if (pair) GO2(CWV, TQV, true) else GO2(CWV, TQV, false)
 #define GO(CWV)                                                                                                       \
     case CWV:                                                                                                         \
-        GO1(CWV, LT_TOKENS)                                                                                           \
+        if (pair) GO1(CWV, true) else GO1(CWV, false)                                                                 \
         break;
     switch (rank / 4) {
         GO(16) GO(32) GO(48) GO(64) GO(80) GO(96) GO(112) GO(128)

@@ -994,74 +994,78 @@ def latent_prompt(q: torch.Tensor, pages: torch.Tensor, w_expand: torch.Tensor, 
             _stream()), "prefill_tc_expanded")
 
 
+def _latent_cost(q_full, pages, ctx, rank: int, window: int, mine):
+    """(bytes, operations) of the tokens of the requests `mine` (a mask)."""
+    if not (_profiling() and hasattr(ctx, "h_q_len")):
+        return 0.0, 0.0
+    H, dk = q_full.shape[1:]
+    ql, cl = ctx.h_q_len[mine].astype(float), ctx.h_ctx_len[mine].astype(float)
+    if window > 0:
+        cl = cl.clip(max=float(window))
+    return (float((cl + ql).sum()) * dk * pages.element_size() + float(ql.sum()) * H * (dk * 4 + rank * 2),
+            2.0 * float((ql * cl + ql * (ql + 1) / 2).sum()) * H * (dk + rank))
+
+
 def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table: torch.Tensor, rank: int,
                      scale: float, window: int, out_dtype: torch.dtype, work=None,
-                     sink: Optional[torch.Tensor] = None, exact_weights: bool = False, max_len: int = 0) -> torch.Tensor:
+                     sink: Optional[torch.Tensor] = None, exact_weights: bool = False) -> torch.Tensor:
     """softmax over the visible cache rows of (q_full . row) * scale, times the rows' first `rank` elements:
     [T, H, rank].  q_full [T, H, dk] float32; pages [num_pages, 1, P, dk].  `work`: the step's units of tokens
-    (`tiles` [n, 2], `tq`) for the tensor-core kernel, which bfloat16 takes when the sizes fit (a latent of
-    64 .. 512 in steps of 64, rows a multiple of 16); everything else takes the plain kernel.  sink [H] float32: the
-    denominator also holds exp(sink[h]).  exact_weights: the tensor-core kernel multiplies weights of 16 bits of mantissa
-    (two terms) instead of 8.  Lone tokens take a kernel of their own there.  max_len > 0: the tensor-core kernel leaves requests that bring more tokens alone (their rows
-    of the result stay unwritten)."""
+    (`tiles` [n, 2] of the requests `mine`: see LatentWork), with which bfloat16 with a latent of 64 .. 512 in steps of 64 and rows a multiple of 16 takes
+    the tensor cores: portions in those units where shared memory has room for four tokens' queries, lone tokens in a kernel of
+    their own; everything else takes the plain kernel.  sink [H] float32: the denominator also holds exp(sink[h]).
+    exact_weights: the tensor cores multiply weights of 16 bits of mantissa (two terms) instead of 8.  Rows of portions that the
+    units leave out stay unwritten."""
     _dev(q_full, pages, block_table, sink)
     T, H, dk = q_full.shape
     if (q_full.dtype != torch.float32 or pages.shape[3] != dk or pages.shape[1] != 1
             or (sink is not None and (sink.dtype != torch.float32 or sink.shape != (H,)))):
         raise KernelError("latent_attention: shapes or dtypes do not fit")
     out = torch.empty((T, H, rank), dtype=out_dtype, device=q_full.device)
-    cost = (float(_nb(q_full, out)), 0.0)
-    if _profiling() and hasattr(ctx, "h_q_len"):      # cache rows read once per request, products per (query, key) pair
-        pairs = rows = 0.0
-        for n, c in zip(ctx.h_q_len.tolist(), ctx.h_ctx_len.tolist()):
-            seen = [min(c + i + 1, window) if window > 0 else c + i + 1 for i in range(n)]
-            pairs += float(sum(seen))
-            rows += float(min(c + n, (window + n) if window > 0 else c + n))
-        cost = (cost[0] + rows * dk * pages.element_size(), 2.0 * pairs * H * (dk + rank))
-    if (work is not None and pages.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and rank % 64 == 0
-            and 64 <= rank <= 512 and dk % 16 == 0 and dk <= 1024
-            and (work.tq * 16 + 64) * (dk + 8) * 2 + work.tq * (9400 if exact_weights else 7000) <= 220 * 1024):
-        lib = library("latent_attention_tc.cu")
-        lone = ctx.max_q_len <= 1 or bool((ctx.h_q_len == 1).any())
-        if ctx.max_q_len > 1 and (not max_len or bool(((ctx.h_q_len > 1) & (ctx.h_q_len <= max_len)).any())):
-            # short portions; a step of few tokens cuts each token's keys into parts so that the grid fills the machine
-            keys = ctx.bt_width * ctx.page_size if ctx.bucketed else ctx.max_total_len
-            if window > 0:
-                keys = min(keys, window + 63)
-            ctas = work.tiles.shape[0] * ((H + 15) // 16)
-            splits = max(1, min(64, (keys + 63) // 64, (2 * sm_count()) // ctas))
-            part_o = part_ml = None
-            if splits > 1:
-                part_o = torch.empty((T, H, splits, rank), dtype=torch.float32, device=q_full.device)
-                part_ml = torch.empty((T, H, splits, 2), dtype=torch.float32, device=q_full.device)
-            with region("latent_attention_tc", *cost):
-                check(lib.aie_latent_attention_tc(_p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(work.tiles),
-                                                  c_int(work.tiles.shape[0]), c_int(work.tq), _p(ctx.q_start),
-                                                  _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
-                                                  c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(T), c_int(H),
-                                                  c_int(rank), c_int(dk), c_int(window), c_float(scale), c_int(splits),
-                                                  _p(sink), c_int(1 if exact_weights else 0), c_int(2 if lone else 1), c_int(max_len),
-                                                  _p(ctx.err), _stream()), "latent_attention_tc")
-        if lone:
-            # one token a request: the visible rows of all of them in equal stretches, one a CTA.  (Behind the other kernel, whose
-            # join of parts runs over every token's row.)
-            G = max(1, 2 * sm_count() // ((H + 15) // 16))
-            part_o = torch.empty((G + ctx.R, H, rank), dtype=torch.float32, device=q_full.device)
-            part_ml = torch.empty((G + ctx.R, H, 2), dtype=torch.float32, device=q_full.device)
-            with region("latent_attention_tc", *cost):
-                check(lib.aie_latent_decode(_p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(ctx.q_start), _p(ctx.q_len),
-                                            _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]),
-                                            c_int(pages.shape[2]), c_int(ctx.R), c_int(H), c_int(rank), c_int(dk), c_int(window),
-                                            c_float(scale), c_int(G), _p(sink), c_int(1 if exact_weights else 0), _p(ctx.err),
-                                            _stream()), "latent_decode")
-        return out
-    lib = library("latent_attention.cu")
-    with region("latent_attention", *cost):
-        check(lib.aie_latent_attention(_p(q_full), _p(pages), c_int(dtype_code(pages)), _p(out),
-                                       c_int(dtype_code(out)), _p(ctx.positions), _p(ctx.token_req), _p(block_table),
-                                       c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]),
-                                       c_int(T), c_int(H), c_int(rank), c_int(dk), c_int(window), c_float(scale),
-                                       _p(sink), _p(ctx.err), _stream()), "latent_attention")
+    fast = (work is not None and pages.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and rank % 64 == 0
+            and 64 <= rank <= 512 and dk % 16 == 0 and dk <= 1024)
+    lone = fast and (ctx.max_q_len <= 1 or bool((ctx.h_q_len == 1).any()))
+    if not fast or ctx.max_q_len > 1:
+        cost = _latent_cost(q_full, pages, ctx, rank, window, work.mine if fast else slice(None))
+        # four tokens' queries, 64 rows of the cache, and each token's weights and sums
+        if fast and (4 * 16 + 64) * (dk + 8) * 2 + 4 * (9400 if exact_weights else 7000) <= 220 * 1024:
+            if work.tiles.shape[0]:
+                # a step of few tokens cuts each token's keys into parts so that the grid fills the machine
+                keys = ctx.bt_width * ctx.page_size if ctx.bucketed else ctx.max_total_len
+                if window > 0:
+                    keys = min(keys, window + 63)
+                ctas = work.tiles.shape[0] * ((H + 15) // 16)
+                splits = max(1, min(64, (keys + 63) // 64, (2 * sm_count()) // ctas))
+                part_o = part_ml = None
+                if splits > 1:
+                    part_o = torch.empty((T, H, splits, rank), dtype=torch.float32, device=q_full.device)
+                    part_ml = torch.empty((T, H, splits, 2), dtype=torch.float32, device=q_full.device)
+                with region("latent_attention_tc", *cost):
+                    check(library("latent_attention_tc.cu").aie_latent_attention_tc(
+                        _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(work.tiles), c_int(work.tiles.shape[0]),
+                        _p(ctx.q_start), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
+                        c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(T), c_int(H), c_int(rank), c_int(dk), c_int(window),
+                        c_float(scale), c_int(splits), _p(sink), c_int(1 if exact_weights else 0), _p(ctx.err), _stream()),
+                        "latent_attention_tc")
+        else:
+            with region("latent_attention", *cost):
+                check(library("latent_attention.cu").aie_latent_attention(
+                    _p(q_full), _p(pages), c_int(dtype_code(pages)), _p(out), c_int(dtype_code(out)), _p(ctx.positions),
+                    _p(ctx.token_req), _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]),
+                    c_int(T), c_int(H), c_int(rank), c_int(dk), c_int(window), c_float(scale), _p(sink), _p(ctx.q_len if lone else None),
+                    _p(ctx.err), _stream()), "latent_attention")
+    if lone:
+        # one token a request: the visible rows of all of them in equal stretches, one a CTA.  (Behind the other kernel, whose
+        # join of parts runs over every token's row.)
+        G = max(1, 2 * sm_count() // ((H + 15) // 16))
+        part_o = torch.empty((G + ctx.R, H, rank), dtype=torch.float32, device=q_full.device)
+        part_ml = torch.empty((G + ctx.R, H, 2), dtype=torch.float32, device=q_full.device)
+        with region("latent_decode", *_latent_cost(q_full, pages, ctx, rank, window, ctx.h_q_len == 1)):
+            check(library("latent_attention_tc.cu").aie_latent_decode(
+                _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(ctx.q_start), _p(ctx.q_len), _p(ctx.ctx_len),
+                _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(ctx.R), c_int(H),
+                c_int(rank), c_int(dk), c_int(window), c_float(scale), c_int(G), _p(sink), c_int(1 if exact_weights else 0),
+                _p(ctx.err), _stream()), "latent_decode")
     return out
 
 

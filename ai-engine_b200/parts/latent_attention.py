@@ -23,6 +23,8 @@ nothing; the run order names the layer whose rows it reads.
 """
 from __future__ import annotations
 
+from types import SimpleNamespace
+
 import numpy as np
 import torch
 
@@ -32,20 +34,21 @@ from .base import KVRequest, Mixer, StepPlanner
 
 
 class LatentWork(StepPlanner):
-    """The work list of the tensor-core kernel: `tiles` [n, 2] = (request row, offset among the tokens it brings)
-    of units of `tq` consecutive tokens of one request, which share the cache rows they gather.  A step in which
-    every request brings one token has units of one token, all others units of four.  `prompt_tiles` [n, 2]: tiles of
-    `ops.PREFILL_TILE` tokens of the requests that bring `ops.LATENT_EXPAND_TOKENS` or more."""
+    """The work lists of the kernels for portions.  `tiles` [n, 2] = (request row, offset among the tokens it brings) of units of
+    four consecutive tokens of one request, which share the cache rows they gather, of requests that bring more than one (the
+    mask `mine`; lone tokens need no list); `short_tiles` and `short`: the same without those that bring
+    `ops.LATENT_EXPAND_TOKENS` or more, and `prompt_tiles`: these in tiles of `ops.PREFILL_TILE` tokens."""
 
     key = "latent"
 
     def plan(self, ctx):
-        tq = 1 if ctx.max_q_len <= 1 else 4
-        lens = ctx.h_q_len.tolist()
-        tiles = [(r, off) for r, n in enumerate(lens) for off in range(0, n, tq)]
-        prompts = [(r, off) for r, n in enumerate(lens) if n >= ops.LATENT_EXPAND_TOKENS for off in range(0, n, ops.PREFILL_TILE)]
-        return (dict(tiles=np.asarray(tiles, dtype=np.int32).reshape(-1, 2),
-                     prompt_tiles=np.asarray(prompts, dtype=np.int32).reshape(-1, 2)), dict(tq=tq))
+        def units(mine, size):
+            out = [(r, off) for r in np.flatnonzero(mine).tolist() for off in range(0, int(ctx.h_q_len[r]), size)]
+            return np.asarray(out, dtype=np.int32).reshape(-1, 2)
+
+        several, prompts = ctx.h_q_len > 1, ctx.h_q_len >= ops.LATENT_EXPAND_TOKENS
+        return (dict(tiles=units(several, 4), short_tiles=units(several & ~prompts, 4), prompt_tiles=units(prompts, ops.PREFILL_TILE)),
+                dict(mine=several, short=several & ~prompts))
 
 
 LATENT_WORK = LatentWork()
@@ -185,8 +188,9 @@ class LatentAttention(Mixer):
             q_plain, q_full = made[:2]
             ops.head_linear(q_plain, self.w_ukT, q_full)
             mixed = ops.latent_attention(q_full, cache.k_pages, ctx, cache.block_table, self.rank, self.scale,
-                                         self.window, self.env.dtype, work, sink=self.sink, exact_weights=self.exact_weights,
-                                         max_len=ops.LATENT_EXPAND_TOKENS - 1 if rows else 0)
+                                         self.window, self.env.dtype,
+                                         SimpleNamespace(tiles=work.short_tiles, mine=work.short) if rows else work,
+                                         sink=self.sink, exact_weights=self.exact_weights)
             ops.head_linear(mixed, self.w_uv, a)
         if rows:
             ops.latent_prompt(made[2], cache.k_pages, self.w_expand, ctx, cache.block_table, work.prompt_tiles, rows, self.scale,

@@ -13,8 +13,9 @@ DEV = "cuda:0"
     (3, 64, 16, 8, [(7 * i % 40, 1) for i in range(70)], 0, False, True),           # many requests in a stretch
     (18, 192, 32, 16, [(3000, 1)], 0, True, True),                                  # one request over many stretches
     (5, 128, 0, 32, [(900, 1), (10, 1), (300, 1)], 100, False, False), (1, 320, 48, 16, [(500, 1), (0, 1)], 1, True, False),
-    (8, 64, 80, 16, [(40, 1), (3, 7), (200, 1), (0, 2), (77, 1)], 64, False, True), (16, 448, 576, 16, [(65, 1), (1000, 1)], 0, False, False)])
-def test_lone_tokens(H, rank, rot, P, reqs, window, sink, exact):
+    (8, 64, 80, 16, [(40, 1), (3, 7), (200, 1), (0, 2), (77, 1)], 64, False, True), (16, 448, 576, 16, [(65, 1), (1000, 1)], 0, False, False),
+    (4, 192, 576, 16, [(65, 1), (30, 3), (1000, 1), (0, 9)], 0, True, False)])             # rows too long for the portions' kernel
+def test_lone_tokens(H, rank, rot, P, reqs, window, sink, exact, monkeypatch):
     from ai_engine_b200.cache import PagedCache
     from ai_engine_b200.engine.step import StepContext, StepEntry
     from ai_engine_b200.kernels import ops
@@ -40,9 +41,13 @@ def test_lone_tokens(H, rank, rot, P, reqs, window, sink, exact):
     q = torch.randn(T, H, dk, generator=gen, device=DEV).to(torch.bfloat16).float()
     sinks = torch.randn(H, generator=gen, device=DEV) if sink else None
     scale = 1.5 * dk ** -0.5
+    lib, ran = ops.library("latent_attention_tc.cu"), []
+    entry = lambda *a: ran.append(1) or lib.aie_latent_decode(*a)
+    fake = type("Lib", (), dict(aie_latent_decode=staticmethod(entry), aie_latent_attention_tc=lib.aie_latent_attention_tc))
+    monkeypatch.setattr(ops, "library", lambda name, f=ops.library: fake if name == "latent_attention_tc.cu" else f(name))
     got = ops.latent_attention(q, lc.k_pages, ctx, lc.block_table, rank, scale, window, torch.bfloat16, ctx.plan(LATENT_WORK),
                                sink=sinks, exact_weights=exact)
-    assert int(err.item()) == 0
+    assert int(err.item()) == 0 and ran == [1]                            # lone tokens have their kernel in every step
     at = 0
     for (c, n), rr in zip(reqs, rows):
         k = rr.double()
