@@ -76,10 +76,9 @@ struct AtExt {
     const float* temp;            // [H] factor of the scores, or null
     const float* slope;           // [H] slope * (i - j) is taken off the scores, or null
     const float* sink;            // [H] exp(sink) joins the denominator, or null
-    // > 0: keys and values are not in pages but in rows of their own, [key (HQ) | value (HD)] of every head side by side, a
-    // request's rows from the tile of 128 keys on that its window begins in, requests that bring this many tokens or more
-    // one behind the other
-    int min_len;
+    // not null: keys and values are not in pages but in rows of their own, [key (HQ) | value (HD)] of every head side by side;
+    // [requests] the tile of 128 rows that a request's first 128 keys would be in (those before its window are left out)
+    const int* row_tile;
 };
 
 // tanh(z) for |z| <= 1 as an odd polynomial of degree 15, two at a time (z2 = z^2 and z as packed pairs); the
@@ -245,18 +244,9 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         // pages that lie wholly before the window and hold no kept key may be gone: they are not loaded
         const int first_page = lo_min >> lp;
         auto gone = [&](int pidx) { return EXT && pidx < first_page && (pidx << lp) >= ext.keep_first; };
-        const bool in_rows = EXT && ext.min_len > 0;
+        const bool in_rows = EXT && ext.row_tile;
         const int blk_k = in_rows ? h * (HK + HV) : 0, blk_v = in_rows ? blk_k + HK : 0;
-        int row_page = 0;                                  // rows instead of pages: the request's first tile of 128
-        if (in_rows) {
-            for (int i = lane; i < r; i += 32)
-                if (q_len[i] >= ext.min_len) {
-                    const int lo = ext.window > 0 ? max(ctx_len[i] - ext.window + 1, 0) : 0;
-                    row_page += (ctx_len[i] + q_len[i] - 1) / AT_N - lo / AT_N + 1;
-                }
-            row_page = __reduce_add_sync(0xffffffffu, row_page);
-            row_page -= (ext.window > 0 ? max(ctx_len[r] - ext.window + 1, 0) : 0) / AT_N;
-        }
+        const int row_page = in_rows ? ext.row_tile[r] : 0;
         auto page_of = [&](int jj) {
             const int pidx = tile_of(jj) * ppt + lane;
             if (in_rows) return lane == 0 ? row_page + pidx : -1;
@@ -1111,20 +1101,20 @@ extern "C" int aie_paged_attention_prefill_tc_rows(const void* q, const void* pa
     if ((d != 64 && d != 128) || P < 8 || P > 128 || 128 % P || n_tiles > 65535) return AIE_UNSUPPORTED;
     if (((size_t)q & 15) || ((size_t)pages & 15) || ((size_t)out & 15)) return AIE_UNSUPPORTED;
     if (gate_logits && (((size_t)gate_logits & 15) || ld_gate % 4)) return AIE_UNSUPPORTED;
-    const AtExt ext{window, cap, gate_logits, ld_gate, keep_first, gate, temp, slope, sink, 0};
+    const AtExt ext{window, cap, gate_logits, ld_gate, keep_first, gate, temp, slope, sink, nullptr};
 #define ARGS q, pages, out, tiles, n_tiles, q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, T, H, K, tied, \
              scale, ext, err, stream
     return d == 128 ? launch_prefill_tc_rows<128>(ARGS) : launch_prefill_tc_rows<64>(ARGS);
 #undef ARGS
 }
 
-// Keys of 192 and values of 128 elements out of rows [rows][H][192 | 128] bf16 (see AtExt::min_len; rows a multiple of 128)
-// instead of pages; q [T, H, 192], out [T, H, 128].  tiles name requests that bring min_len tokens or more.
+// Keys of 192 and values of 128 elements out of rows [rows][H][192 | 128] bf16 (see AtExt::row_tile; rows a multiple of 128)
+// instead of pages; q [T, H, 192], out [T, H, 128].
 extern "C" int aie_prefill_tc_expanded(const void* q, const void* rows_kv, long long rows, void* out, const int* tiles, int n_tiles,
                                        const int* q_start, const int* q_len, const int* ctx_len, int T, int H, int window,
-                                       int min_len, const float* sink, float scale, unsigned* err, cudaStream_t stream) {
+                                       const int* row_tile, const float* sink, float scale, unsigned* err, cudaStream_t stream) {
     if (n_tiles <= 0) return 0;
-    if (H <= 0 || window < 0 || min_len < 1 || rows % AT_N || rows / AT_N > 0x7fffffffLL / AT_N) return AIE_BAD_ARG;
+    if (H <= 0 || window < 0 || !row_tile || rows % AT_N || rows / AT_N > 0x7fffffffLL / AT_N) return AIE_BAD_ARG;
     if (n_tiles > 65535 || (((size_t)q | (size_t)rows_kv | (size_t)out) & 15)) return AIE_UNSUPPORTED;
     constexpr int HD = 128, HQ = 192, BLOCKS = (HD + HQ) / 64;
     TcEncodeTiledFn fn = tc_encode_fn();
@@ -1143,7 +1133,7 @@ extern "C" int aie_prefill_tc_expanded(const void* q, const void* rows_kv, long 
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return AIE_UNSUPPORTED;
     }
-    const AtExt ext{window, 0.f, nullptr, 0, 0, nullptr, nullptr, nullptr, sink, min_len};
+    const AtExt ext{window, 0.f, nullptr, 0, 0, nullptr, nullptr, nullptr, sink, row_tile};
     auto kern = paged_prefill_tc_kernel<HD, true, HQ>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AtSmem<HD, HQ>::bytes);
     if (e != cudaSuccess) return (int)e;

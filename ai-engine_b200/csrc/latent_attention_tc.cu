@@ -744,46 +744,19 @@ extern "C" int aie_head_linear_small(const void* x, long long xt, long long xh, 
 }
 
 // ---------------------------------------------------------------------------
-// The cached rows that prompts read, one behind the other: for every request that brings min_len tokens or more, its rows
-// from the tile of 128 keys on that its first token's window begins in, to the last tile; rows outside the window or behind
-// the last token are zeros.  A block copies 32 rows of a tile, 16 bytes a thread.
+// The cached rows that portions read expanded, one behind the other: tiles [n, 2] = (request row, which 128 keys of it counted
+// from its first); rows before the window of the portion's first token or behind its last are zeros.  A block copies 32 rows
+// of a tile, 16 bytes a thread.
 #define LG_ROWS 32
 __global__ void __launch_bounds__(256)
-latent_gather_kernel(const bf16* __restrict__ pages, bf16* __restrict__ rows, const int* __restrict__ q_len,
-                     const int* __restrict__ ctx_len, const int* __restrict__ block_table, int bt_width, int num_pages, int P,
-                     int dk, int window, int min_len, int R, unsigned* err) {
-    __shared__ int found[2];
+latent_gather_kernel(const bf16* __restrict__ pages, bf16* __restrict__ rows, const int* __restrict__ tiles,
+                     const int* __restrict__ q_len, const int* __restrict__ ctx_len, const int* __restrict__ block_table,
+                     int bt_width, int num_pages, int P, int dk, int window, unsigned* err) {
     pdl_launch_dependents();
     pdl_wait();
     const int tile_i = blockIdx.x / (128 / LG_ROWS), sub = blockIdx.x % (128 / LG_ROWS), tid = threadIdx.x;
-    const auto low = [&](int r) { return window > 0 ? max(ctx_len[r] - window + 1, 0) : 0; };
-    if (tid < 32) {                                     // whose tile this is: requests in order, 32 at a time
-        int rr = -1, tile = 0, before = 0;
-        for (int base = 0; base < R && rr < 0; base += 32) {
-            const int r = base + tid;
-            const int m = r < R && q_len[r] >= min_len ? (ctx_len[r] + q_len[r] - 1) / 128 - low(r) / 128 + 1 : 0;
-            int run = m;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int up = __shfl_up_sync(0xffffffffu, run, o);
-                if (tid >= o) run += up;
-            }
-            const unsigned hit = __ballot_sync(0xffffffffu, tile_i < before + run);
-            if (hit) {
-                const int l = __ffs(hit) - 1;
-                rr = base + l;
-                tile = low(rr) / 128 + tile_i - before - __shfl_sync(0xffffffffu, run - m, l);
-            }
-            before += __shfl_sync(0xffffffffu, run, 31);
-        }
-        if (tid == 0) {
-            found[0] = rr;
-            found[1] = tile;
-        }
-    }
-    __syncthreads();
-    const int r = found[0];
-    if (r < 0) return;
-    const int key0 = found[1] * 128 + sub * LG_ROWS, lo = low(r), last = ctx_len[r] + q_len[r] - 1, pieces = dk / 8;
+    const int r = tiles[2 * tile_i], key0 = tiles[2 * tile_i + 1] * 128 + sub * LG_ROWS, pieces = dk / 8;
+    const int lo = window > 0 ? max(ctx_len[r] - window + 1, 0) : 0, last = ctx_len[r] + q_len[r] - 1;
     uint4* dst = reinterpret_cast<uint4*>(rows + ((size_t)tile_i * 128 + sub * LG_ROWS) * dk);
     for (int i = tid; i < LG_ROWS * pieces; i += 256) {
         const int key = key0 + i / pieces, c = i % pieces;
@@ -801,12 +774,12 @@ latent_gather_kernel(const bf16* __restrict__ pages, bf16* __restrict__ rows, co
 }
 
 // pages [num_pages, P, dk] bf16, dk a multiple of 8; rows [n_tiles * 128, dk].
-extern "C" int aie_latent_gather(const void* pages, void* rows, int n_tiles, const int* q_len, const int* ctx_len,
-                                 const int* block_table, int bt_width, int num_pages, int P, int dk, int window, int min_len,
-                                 int R, unsigned* err, cudaStream_t st) {
+extern "C" int aie_latent_gather(const void* pages, void* rows, const int* tiles, int n_tiles, const int* q_len, const int* ctx_len,
+                                 const int* block_table, int bt_width, int num_pages, int P, int dk, int window, unsigned* err,
+                                 cudaStream_t st) {
     if (n_tiles <= 0) return 0;
-    if (dk % 8 || P <= 0 || min_len < 1 || n_tiles > 0x1fffffff || (((size_t)pages | (size_t)rows) & 15)) return AIE_BAD_ARG;
-    launch_pdl(latent_gather_kernel, dim3((unsigned)n_tiles * (128 / LG_ROWS)), dim3(256), 0, st, (const bf16*)pages, (bf16*)rows, q_len,
-               ctx_len, block_table, bt_width, num_pages, P, dk, window, min_len, R, err);
+    if (dk % 8 || P <= 0 || n_tiles > 0x1fffffff || (((size_t)pages | (size_t)rows) & 15)) return AIE_BAD_ARG;
+    launch_pdl(latent_gather_kernel, dim3((unsigned)n_tiles * (128 / LG_ROWS)), dim3(256), 0, st, (const bf16*)pages, (bf16*)rows, tiles,
+               q_len, ctx_len, block_table, bt_width, num_pages, P, dk, window, err);
     AIE_LAUNCH_CHECK();
 }

@@ -948,49 +948,74 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
     return (q_plain, q_full, q_all) if whole else (q_plain, q_full)
 
 
-# Portions from this length on meet their keys and values expanded: 10 tokens' worth of products a key make heads of 192 and
-# 128 out of a row of 576, and a (query, key) pair then costs 640 operations instead of 2,176.
+# Portions of this many tokens or more may meet their keys and values expanded; the expanded rows of a step take no more than this.
 LATENT_EXPAND_TOKENS = 64
-LATENT_EXPAND_BYTES = 1 << 30      # the most that a step's expanded rows may take; beyond, rows are read as they are
+LATENT_EXPAND_BYTES = 1 << 30
+# Expanding takes 20 tokens' worth of multiply-adds a key and head (576 x 320 of them), and a (query, key) pair and head then
+# costs 320 instead of 1,088.  What decides is the time of either form, us, as measured on a latent of 512:
+LATENT_TILE_US = 2.4        # expanded: a tile of 128 keys in a block's chain, one block an SM for every 128 queries of a head
+LATENT_ROW_US = 0.44e-3     # ... and a cached row and head, gathered and expanded
+LATENT_PAIR_US = (0.09e-3, 0.009e-3)      # as they are: a (query, key) pair for every 16 heads begun, and for every head
+LATENT_FOLD_US = 20.0       # ... and the products that fold the queries and apply W_uv
 
 
-def latent_expanded_tiles(ctx, window: int) -> int:
-    """Tiles of 128 cache rows that the step's portions of LATENT_EXPAND_TOKENS tokens or more read under a window."""
-    n = ctx.h_q_len >= LATENT_EXPAND_TOKENS
-    c, q = ctx.h_ctx_len[n].astype(np.int64), ctx.h_q_len[n].astype(np.int64)
+def latent_expanded(lens, cached, H: int, window: int, sms: int = 148):
+    """Which portions of a step (a mask over its requests) meet their keys and values expanded: those with the longest chains of
+    key tiles stay with the rows as they are while that takes less in sum.  Whole layer, rows as they are against expanded, us:
+    16 heads, 64 tokens behind 1,000 / 3,000 / 8,000 / 30,000 cached ones 83 / 116 / 181 / 517 against 71 / 117 / 260 / 810, 128 tokens
+    90 / 157 / 301 / 946 against 66 / 127 / 260 / 807, four requests of 64 behind 3,000 265 against 192; 8 heads, 64 tokens behind
+    3,000 / 8,000 92 / 138 against 102 / 205; 64 heads, 64 behind 8,000 661 against 440.  Over 341 such points (8 to 64 heads, 64 to 512
+    tokens, 0 to 30,000 cached, 1 and 4 requests, a window of 1,024 or none) the rule took the slower form at two, by 4 us."""
+    out, some = np.zeros(len(lens), dtype=bool), np.flatnonzero(lens >= LATENT_EXPAND_TOKENS)
+    if not len(some):
+        return out
+    n, c = lens[some].astype(float), cached[some].astype(float)
     low = np.maximum(c - window + 1, 0) if window > 0 else np.zeros_like(c)
-    return int(((c + q - 1) // 128 - low // 128 + 1).sum())
+    tiles = (c + n - 1) // 128 - low // 128 + 1
+    chain = np.minimum(tiles, (window + 126) // 128 + 1) if window > 0 else tiles
+    waves = H * np.ceil(n / 128) * np.minimum(chain, c // 128 + (n + 127) // 256 + 1) / sms
+    early = np.clip(window - c, 0, n) if window > 0 else n              # tokens that see all that came before them
+    pairs = early * c + early * (early + 1) / 2 + (n - early) * window
+    fold = (LATENT_PAIR_US[0] * -(-H // 16) + LATENT_PAIR_US[1] * H) * pairs
+    order, costs = np.argsort(-chain, kind="stable"), []
+    for k in range(len(some) + 1):                                      # the k longest chains as they are
+        rest = order[k:]
+        costs.append((LATENT_FOLD_US + fold[order[:k]].sum() if k else 0.0)
+                     + (LATENT_TILE_US * max(chain[rest].max(), waves[rest].sum()) + LATENT_ROW_US * H * 128 * tiles[rest].sum()
+                        if len(rest) else 0.0))
+    out[some[order[int(np.argmin(costs)):]]] = True
+    return out
 
 
-def latent_prompt(q: torch.Tensor, pages: torch.Tensor, w_expand: torch.Tensor, ctx, block_table: torch.Tensor, tiles: torch.Tensor,
-                  n_rows: int, scale: float, window: int, sink: Optional[torch.Tensor], out: torch.Tensor) -> None:
-    """Attention of the step's portions of LATENT_EXPAND_TOKENS tokens or more over cache rows that are first expanded:
-    rows gathered one behind the other, one product with w_expand [H * (192 + 128), dk] (a head's key, its shared rotated part
-    copied by ones, and its value), then the tcgen05 prompt kernel on heads of 192 and 128.  q [T, H, 192] bfloat16, tiles
-    [n, 2] of those portions, n_rows = 128 * latent_expanded_tiles; their rows of out [T, H, 128] are written."""
-    _dev(q, pages, w_expand, block_table, tiles, sink, out)
+def latent_prompt(q: torch.Tensor, pages: torch.Tensor, w_expand: torch.Tensor, ctx, block_table: torch.Tensor, work,
+                  scale: float, window: int, sink: Optional[torch.Tensor], out: torch.Tensor) -> None:
+    """Attention of the step's portions `work.expanded` (see LatentWork) over cache rows that are first expanded: rows gathered
+    one behind the other, one product with w_expand [H * (192 + 128), dk] (a head's key, its shared rotated part copied by ones,
+    and its value), then the tcgen05 prompt kernel on heads of 192 and 128.  q [T, H, 192] bfloat16; their rows of out
+    [T, H, 128] are written."""
+    _dev(q, pages, w_expand, block_table, sink, out)
     T, H, _ = q.shape
     dk = pages.shape[3]
     if (q.shape[2] != 192 or out.shape != (T, H, 128) or w_expand.shape != (H * 320, dk) or pages.shape[1] != 1
             or any(t.dtype != torch.bfloat16 for t in (q, pages, w_expand, out))
             or (sink is not None and (sink.dtype != torch.float32 or sink.shape != (H,)))):
         raise KernelError("latent_prompt: shapes or dtypes do not fit")
-    rows = torch.empty((n_rows, dk), dtype=torch.bfloat16, device=q.device)
+    n_tiles = work.gather.shape[0]
+    rows = torch.empty((128 * n_tiles, dk), dtype=torch.bfloat16, device=q.device)
     with region("latent_gather", 2 * _nb(rows)):
         check(library("latent_attention_tc.cu").aie_latent_gather(
-            _p(pages), _p(rows), c_int(n_rows // 128), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
-            c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(dk), c_int(window), c_int(LATENT_EXPAND_TOKENS), c_int(ctx.R),
-            _p(ctx.err), _stream()), "latent_gather")
+            _p(pages), _p(rows), _p(work.gather), c_int(n_tiles), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table),
+            c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(dk), c_int(window), _p(ctx.err), _stream()),
+            "latent_gather")
     kv = linear(rows, w_expand, torch.bfloat16)
     pairs = 0.0
     if _profiling() and hasattr(ctx, "h_q_len"):
-        for n, c in zip(ctx.h_q_len.tolist(), ctx.h_ctx_len.tolist()):
-            if n >= LATENT_EXPAND_TOKENS:
-                pairs += float(sum(min(c + i + 1, window) if window > 0 else c + i + 1 for i in range(n)))
+        for n, c in zip(ctx.h_q_len[work.expanded].tolist(), ctx.h_ctx_len[work.expanded].tolist()):
+            pairs += float(sum(min(c + i + 1, window) if window > 0 else c + i + 1 for i in range(n)))
     with region("latent_prompt_tcgen05", _nb(q, kv, out), 2.0 * pairs * H * 320):
         check(library("attention_prefill_tc.cu").aie_prefill_tc_expanded(
-            _p(q), _p(kv), c_longlong(n_rows), _p(out), _p(tiles), c_int(tiles.shape[0]), _p(ctx.q_start), _p(ctx.q_len),
-            _p(ctx.ctx_len), c_int(T), c_int(H), c_int(window), c_int(LATENT_EXPAND_TOKENS), _p(sink), c_float(scale), _p(ctx.err),
+            _p(q), _p(kv), c_longlong(128 * n_tiles), _p(out), _p(work.prompt_tiles), c_int(work.prompt_tiles.shape[0]), _p(ctx.q_start),
+            _p(ctx.q_len), _p(ctx.ctx_len), c_int(T), c_int(H), c_int(window), _p(work.row_tile), _p(sink), c_float(scale), _p(ctx.err),
             _stream()), "prefill_tc_expanded")
 
 

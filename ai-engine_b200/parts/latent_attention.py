@@ -23,8 +23,6 @@ nothing; the run order names the layer whose rows it reads.
 """
 from __future__ import annotations
 
-from types import SimpleNamespace
-
 import numpy as np
 import torch
 
@@ -34,24 +32,50 @@ from .base import KVRequest, Mixer, StepPlanner
 
 
 class LatentWork(StepPlanner):
-    """The work lists of the kernels for portions.  `tiles` [n, 2] = (request row, offset among the tokens it brings) of units of
-    four consecutive tokens of one request, which share the cache rows they gather, of requests that bring more than one (the
-    mask `mine`; lone tokens need no list); `short_tiles` and `short`: the same without those that bring
-    `ops.LATENT_EXPAND_TOKENS` or more, and `prompt_tiles`: these in tiles of `ops.PREFILL_TILE` tokens."""
+    """The work lists of latent attention.  `expanded`: the mask of the requests whose keys and values are expanded (never with
+    `expands` False), `mine`: of the others that bring more than one token.  `tiles` [n, 2] = (request row, offset among the
+    tokens it brings) of units of four consecutive tokens of one request of `mine`, which share the cache rows they gather;
+    `prompt_tiles` [n, 2]: the expanded ones in tiles of `ops.PREFILL_TILE` tokens.  `gather` [n, 2] = (request row, which 128 of
+    its keys) of the rows to expand, and `row_tile` [R]: where among them a request's first 128 keys would be.  Lone tokens
+    need no list.  `prompts`: some are expanded; `folds`: some are not."""
 
-    key = "latent"
+    def __init__(self, H: int = 0, window: int = 0, expands: bool = False):
+        self.H, self.window, self.expands = H, window, expands
+        self.key = f"latent {H} {window} {expands}"
 
     def plan(self, ctx):
-        def units(mine, size):
-            out = [(r, off) for r in np.flatnonzero(mine).tolist() for off in range(0, int(ctx.h_q_len[r]), size)]
+        lens, cached = ctx.h_q_len.astype(np.int64), ctx.h_ctx_len.astype(np.int64)
+        expanded = np.zeros(len(lens), dtype=bool)
+        if self.expands and ctx.max_q_len >= ops.LATENT_EXPAND_TOKENS:
+            expanded = ops.latent_expanded(lens, cached, self.H, self.window)
+        first = (np.maximum(cached - self.window + 1, 0) if self.window > 0 else np.zeros_like(cached)) // ops.PREFILL_TILE
+        key_tiles = np.where(expanded, (cached + lens - 1) // ops.PREFILL_TILE - first + 1, 0)
+        if int(key_tiles.sum()) * ops.PREFILL_TILE * self.H * 640 > ops.LATENT_EXPAND_BYTES:
+            expanded[:], key_tiles[:] = False, 0
+        mine = (lens > 1) & ~expanded
+
+        def units(mask, size):
+            out = [(r, off) for r in np.flatnonzero(mask).tolist() for off in range(0, int(lens[r]), size)]
             return np.asarray(out, dtype=np.int32).reshape(-1, 2)
 
-        several, prompts = ctx.h_q_len > 1, ctx.h_q_len >= ops.LATENT_EXPAND_TOKENS
-        return (dict(tiles=units(several, 4), short_tiles=units(several & ~prompts, 4), prompt_tiles=units(prompts, ops.PREFILL_TILE)),
-                dict(mine=several, short=several & ~prompts))
+        rows = np.repeat(np.arange(len(lens)), key_tiles)
+        row_tile = np.cumsum(key_tiles) - key_tiles - first
+        gather = np.stack([rows, np.arange(len(rows)) - row_tile[rows]], axis=1)
+        return (dict(tiles=units(mine, 4), prompt_tiles=units(expanded, ops.PREFILL_TILE), gather=gather,
+                     row_tile=row_tile if len(rows) else row_tile[:0]),
+                dict(mine=mine, expanded=expanded, prompts=bool(len(rows)), folds=not expanded.all()))
 
 
 LATENT_WORK = LatentWork()
+_PLANNERS = {}
+
+
+def latent_work(H: int, window: int, expands: bool) -> LatentWork:
+    """The planner that all layers of these sizes share."""
+    key = (H, window, expands)
+    if key not in _PLANNERS:
+        _PLANNERS[key] = LatentWork(*key)
+    return _PLANNERS[key]
 
 
 class LatentAttention(Mixer):
@@ -156,7 +180,7 @@ class LatentAttention(Mixer):
         return KVRequest(1, self.rank + self.rot, self.cache_window, planes=1)
 
     def step_planner(self):
-        return LATENT_WORK
+        return latent_work(self.H, self.window, self.w_expand is not None)
 
     def forward(self, h, ctx, cache, add_to=None):
         T = h.shape[0]
@@ -172,29 +196,20 @@ class LatentAttention(Mixer):
             q_src = ops.linear(cq, self.w_uq, torch.float32, ctx.err)
         else:
             q_src = proj
-        work = ctx.plan(LATENT_WORK)
+        work = ctx.plan(self.step_planner())
         # portions of prompts meet their keys and values expanded; the others read the rows as they are
-        rows = 0
-        if self.w_expand is not None and work.prompt_tiles.shape[0]:
-            rows = 128 * ops.latent_expanded_tiles(ctx, self.window)
-            if rows * self.w_expand.shape[0] * 2 > ops.LATENT_EXPAND_BYTES:
-                rows = 0
-        folded = not rows or int(ctx.h_q_len.min()) < ops.LATENT_EXPAND_TOKENS
         made = ops.latent_prepare(q_src, self.H, self.d, self.rot, self.rank, self.c_weight, self.eps, inv_freq, cache.k_pages,
                                   ctx, cache.block_table, self.env.dtype, write=cache.writes and not self.shares_cache, kv=kv,
-                                  halves=self.halves, magnitude=self.magnitude, folded=folded, whole=rows > 0)
+                                  halves=self.halves, magnitude=self.magnitude, folded=work.folds, whole=work.prompts)
         a = torch.empty((T, self.H, self.dv), dtype=self.env.dtype, device=h.device)
-        if folded:
+        if work.folds:
             q_plain, q_full = made[:2]
             ops.head_linear(q_plain, self.w_ukT, q_full)
             mixed = ops.latent_attention(q_full, cache.k_pages, ctx, cache.block_table, self.rank, self.scale,
-                                         self.window, self.env.dtype,
-                                         SimpleNamespace(tiles=work.short_tiles, mine=work.short) if rows else work,
-                                         sink=self.sink, exact_weights=self.exact_weights)
+                                         self.window, self.env.dtype, work, sink=self.sink, exact_weights=self.exact_weights)
             ops.head_linear(mixed, self.w_uv, a)
-        if rows:
-            ops.latent_prompt(made[2], cache.k_pages, self.w_expand, ctx, cache.block_table, work.prompt_tiles, rows, self.scale,
-                              self.window, self.sink, a)
+        if work.prompts:
+            ops.latent_prompt(made[2], cache.k_pages, self.w_expand, ctx, cache.block_table, work, self.scale, self.window, self.sink, a)
         a = a.view(T, self.H * self.dv)
         if self.head_gate:
             g0 = first + self.rank + self.rot
