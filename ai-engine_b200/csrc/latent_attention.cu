@@ -7,7 +7,8 @@
 //
 // latent_prepare (q_plain with q_full, and q_all, may be left out: null): from the fused projection [q heads | c | kr] of the step's tokens it writes the plain
 //   query parts (compute dtype, for the folding product), the rotated query parts (float32), in q_all both parts side by
-//   side (compute dtype, for queries that meet expanded keys), and the
+//   side (compute dtype, for queries that meet expanded keys; with short_row [T] a token whose entry is >= 0 has the first two,
+//   in that row, and the others have the last), and the
 //   normalised c and rotated kr into the token's cache row.  The rotation pairs element 2i with 2i+1 over the
 //   first `rot_dims` elements of the rot-wide part (or, with `halves`, element i with i + rot_dims / 2); the
 //   angle is float(position) * inv_freq[i] in float32, and cosine and sine are multiplied by `mag`.  The latent and the key part may come from a projection
@@ -46,7 +47,7 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int ld, in
                                       const int* __restrict__ positions, const int* __restrict__ token_req,
                                       const int* __restrict__ block_table, int bt_width, int num_pages, int P,
                                       unsigned* err, const float* __restrict__ kv, int ld_kv, int halves, float mag,
-                                      A* __restrict__ q_all) {
+                                      A* __restrict__ q_all, const int* __restrict__ short_row) {
     __shared__ float red[32];
     __shared__ float2 angles[LAT_ANGLES];              // made once a token, for all heads
     pdl_launch_dependents();
@@ -61,19 +62,26 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int ld, in
         __syncthreads();
     }
     // queries: the plain part as it is, the rotated part turned by the position
+    const int tf = short_row ? short_row[t] : t;                  // the token's row of q_plain and q_full
+    if (tf < 0) {
+        q_plain = nullptr;
+        q_full = nullptr;
+    } else if (short_row) {
+        q_all = nullptr;
+    }
     const bool vec = ((d | rot | ld) & 3) == 0 && (((size_t)proj | (size_t)q_plain | (size_t)q_all) & 15) == 0;      // (rows of A: 4 elements)
     if (vec) {
         for (int e = tid * 4; e < H * d; e += blockDim.x * 4) {
             const int hh = e / d, i = e % d;
             const float4 v = *reinterpret_cast<const float4*>(row + hh * dq + i);
-            if (q_plain) store4<A>(q_plain + ((size_t)t * H + hh) * d + i, v);
+            if (q_plain) store4<A>(q_plain + ((size_t)tf * H + hh) * d + i, v);
             if (q_all) store4<A>(q_all + ((size_t)t * H + hh) * dq + i, v);
         }
     } else {
         for (int e = tid; e < H * d; e += blockDim.x) {
             const int hh = e / d, i = e % d;
             const A v = from_f32<A>(row[hh * dq + i]);
-            if (q_plain) q_plain[((size_t)t * H + hh) * d + i] = v;
+            if (q_plain) q_plain[((size_t)tf * H + hh) * d + i] = v;
             if (q_all) q_all[((size_t)t * H + hh) * dq + i] = v;
         }
     }
@@ -81,7 +89,7 @@ __global__ void latent_prepare_kernel(const float* __restrict__ proj, int ld, in
         const int hh = e / rot, i = e % rot;
         const float* qr = row + hh * dq + d;
         const float v = latent_rotated(qr, i, half, halves, pos, inv_freq, mag, tab);
-        if (q_full) q_full[((size_t)t * H + hh) * dk + rank + i] = v;
+        if (q_full) q_full[((size_t)tf * H + hh) * dk + rank + i] = v;
         if (q_all) q_all[((size_t)t * H + hh) * dq + d + i] = from_f32<A>(v);
     }
     if (!has_kv) return;
@@ -107,14 +115,15 @@ extern "C" int aie_latent_prepare(const float* proj, int ld, int T, int H, int d
                                   int has_kv, const float* c_weight, float eps, const float* inv_freq, void* q_plain,
                                   int q_dtype, float* q_full, void* pages, int cache_dtype, const int* positions,
                                   const int* token_req, const int* block_table, int bt_width, int num_pages, int P,
-                                  unsigned* err, const float* kv, int ld_kv, int halves, float mag, void* q_all, cudaStream_t st) {
+                                  unsigned* err, const float* kv, int ld_kv, int halves, float mag, void* q_all,
+                                  const int* short_row, cudaStream_t st) {
     if (T <= 0) return 0;
     if (rot_dims % 2 || rot_dims > rot || H <= 0 || d < 0 || rank <= 0) return AIE_BAD_ARG;
     const int threads = T <= 2 * aie_sm_count() ? 1024 : LAT_PREP;      // few tokens: a block has an SM to itself
 #define GO(A, C)                                                                                                      \
     launch_pdl(latent_prepare_kernel<A, C>, dim3(T), dim3(threads), 0, st, proj, ld, H, d, rot, rank, rot_dims, has_kv, c_weight, eps, inv_freq, \
                                                    (A*)q_plain, q_full, (C*)pages, positions, token_req, block_table,  \
-                                                   bt_width, num_pages, P, err, kv, ld_kv, halves, mag, (A*)q_all)
+                                                   bt_width, num_pages, P, err, kv, ld_kv, halves, mag, (A*)q_all, short_row)
     if (q_dtype == AIE_F32 && cache_dtype == AIE_F32) GO(float, float);
     else if (q_dtype == AIE_BF16 && cache_dtype == AIE_BF16) GO(bf16, bf16);
     else if (q_dtype == AIE_BF16 && cache_dtype == AIE_F32) GO(bf16, float);

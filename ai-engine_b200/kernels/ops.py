@@ -917,7 +917,8 @@ def expert_combine(y: torch.Tensor, pair_row: torch.Tensor, top: int, weight: fl
 def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_weight: Optional[torch.Tensor],
                    eps: float, inv_freq: torch.Tensor, pages: torch.Tensor, ctx, block_table: torch.Tensor,
                    q_dtype: torch.dtype, write: bool, kv: Optional[torch.Tensor] = None, halves: bool = False,
-                   magnitude: float = 1.0, folded: bool = True, whole: bool = False):
+                   magnitude: float = 1.0, folded: bool = True, whole: bool = False, short_row: Optional[torch.Tensor] = None,
+                   n_short: int = 0):
     """From the fused projection [q heads (d plain | rot rotated) | latent (rank) | shared key part (rot)] of a
     step: (q_plain [T, H, d] in q_dtype, q_full [T, H, rank + rot] float32 whose last rot columns hold the
     rotated query parts); with `write`, the normalised latent and the rotated key part go into the tokens'
@@ -925,7 +926,8 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
     [T, >= rank + rot] (rows any stride) instead of the columns behind the queries.  halves: the rotation pairs
     element i with i + rot_dims / 2 instead of 2i with 2i + 1.  magnitude: factor of all cosines and sines.
     folded False: (None, None) for the two; whole: a third result [T, H, d + rot] in q_dtype, a head's plain and rotated
-    parts side by side."""
+    parts side by side.  short_row (int32 [T], with n_short entries that are not negative): these tokens have rows of the first
+    two results [n_short, H, .], in that order, the others rows of the third."""
     _dev(proj, c_weight, inv_freq, pages, block_table)
     T, ld = proj.shape
     need = H * (d + rot) + ((rank + rot) if write and kv is None else 0)
@@ -933,18 +935,20 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
         raise KernelError("latent_prepare: the latent projection is a float32 view [T, >= rank + rot]")
     if proj.dtype != torch.float32 or ld < need or pages.shape[1] != 1 or pages.shape[3] != rank + rot:
         raise KernelError("latent_prepare: shapes or dtypes do not fit")
-    q_plain = torch.empty((T, H, d), dtype=q_dtype, device=proj.device) if folded else None
-    q_full = torch.empty((T, H, rank + rot), dtype=torch.float32, device=proj.device) if folded else None
+    n = T if short_row is None else n_short
+    q_plain = torch.empty((n, H, d), dtype=q_dtype, device=proj.device) if folded else None
+    q_full = torch.empty((n, H, rank + rot), dtype=torch.float32, device=proj.device) if folded else None
     q_all = torch.empty((T, H, d + rot), dtype=q_dtype, device=proj.device) if whole else None
     lib = library("latent_attention.cu")
-    with region("latent_prepare", _nb(proj, q_plain, q_all) + (T * H * rot * 4 if folded else 0)):
+    with region("latent_prepare", _nb(proj, q_plain, q_all) + (n * H * rot * 4 if folded else 0)):
         check(lib.aie_latent_prepare(_p(proj), c_int(ld), c_int(T), c_int(H), c_int(d), c_int(rot), c_int(rank),
                                      c_int(2 * inv_freq.shape[0]), c_int(1 if write else 0), _p(c_weight),
                                      c_float(eps), _p(inv_freq), _p(q_plain), c_int(dtype_code(q_dtype)), _p(q_full),
                                      _p(pages), c_int(dtype_code(pages)), _p(ctx.positions), _p(ctx.token_req),
                                      _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]),
                                      c_int(pages.shape[2]), _p(ctx.err), _p(kv), c_int(kv.stride(0) if kv is not None else 0),
-                                     c_int(1 if halves else 0), c_float(magnitude), _p(q_all), _stream()), "latent_prepare")
+                                     c_int(1 if halves else 0), c_float(magnitude), _p(q_all), _p(short_row), _stream()),
+              "latent_prepare")
     return (q_plain, q_full, q_all) if whole else (q_plain, q_full)
 
 
@@ -1033,14 +1037,14 @@ def _latent_cost(q_full, pages, ctx, rank: int, window: int, mine):
 
 def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table: torch.Tensor, rank: int,
                      scale: float, window: int, out_dtype: torch.dtype, work=None,
-                     sink: Optional[torch.Tensor] = None, exact_weights: bool = False) -> torch.Tensor:
+                     sink: Optional[torch.Tensor] = None, exact_weights: bool = False, compact: bool = False) -> torch.Tensor:
     """softmax over the visible cache rows of (q_full . row) * scale, times the rows' first `rank` elements:
     [T, H, rank].  q_full [T, H, dk] float32; pages [num_pages, 1, P, dk].  `work`: the step's units of tokens
     (`tiles` [n, 2] of the requests `mine`: see LatentWork), with which bfloat16 with a latent of 64 .. 512 in steps of 64 and rows a multiple of 16 takes
     the tensor cores: portions in those units where shared memory has room for four tokens' queries, lone tokens in a kernel of
     their own; everything else takes the plain kernel.  sink [H] float32: the denominator also holds exp(sink[h]).
     exact_weights: the tensor cores multiply weights of 16 bits of mantissa (two terms) instead of 8.  Rows of portions that the
-    units leave out stay unwritten."""
+    units leave out stay unwritten.  compact: q_full and the result hold the rows of `work.short_tokens` only."""
     _dev(q_full, pages, block_table, sink)
     T, H, dk = q_full.shape
     if (q_full.dtype != torch.float32 or pages.shape[3] != dk or pages.shape[1] != 1
@@ -1049,6 +1053,7 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
     out = torch.empty((T, H, rank), dtype=out_dtype, device=q_full.device)
     fast = (work is not None and pages.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and rank % 64 == 0
             and 64 <= rank <= 512 and dk % 16 == 0 and dk <= 1024)
+    starts = work.short_start if compact else ctx.q_start
     lone = fast and (ctx.max_q_len <= 1 or bool((ctx.h_q_len == 1).any()))
     if not fast or ctx.max_q_len > 1:
         cost = _latent_cost(q_full, pages, ctx, rank, window, work.mine if fast else slice(None))
@@ -1068,15 +1073,15 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
                 with region("latent_attention_tc", *cost):
                     check(library("latent_attention_tc.cu").aie_latent_attention_tc(
                         _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(work.tiles), c_int(work.tiles.shape[0]),
-                        _p(ctx.q_start), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
+                        _p(starts), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table), c_int(block_table.shape[1]),
                         c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(T), c_int(H), c_int(rank), c_int(dk), c_int(window),
                         c_float(scale), c_int(splits), _p(sink), c_int(1 if exact_weights else 0), _p(ctx.err), _stream()),
                         "latent_attention_tc")
         else:
+            positions, token_req = ((t.index_select(0, work.short_tokens) if compact else t) for t in (ctx.positions, ctx.token_req))
             with region("latent_attention", *cost):
                 check(library("latent_attention.cu").aie_latent_attention(
-                    _p(q_full), _p(pages), c_int(dtype_code(pages)), _p(out), c_int(dtype_code(out)), _p(ctx.positions),
-                    _p(ctx.token_req), _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]),
+                    _p(q_full), _p(pages), c_int(dtype_code(pages)), _p(out), c_int(dtype_code(out)), _p(positions), _p(token_req), _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]),
                     c_int(T), c_int(H), c_int(rank), c_int(dk), c_int(window), c_float(scale), _p(sink), _p(ctx.q_len if lone else None),
                     _p(ctx.err), _stream()), "latent_attention")
     if lone:
@@ -1087,7 +1092,7 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
         part_ml = torch.empty((G + ctx.R, H, 2), dtype=torch.float32, device=q_full.device)
         with region("latent_decode", *_latent_cost(q_full, pages, ctx, rank, window, ctx.h_q_len == 1)):
             check(library("latent_attention_tc.cu").aie_latent_decode(
-                _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(ctx.q_start), _p(ctx.q_len), _p(ctx.ctx_len),
+                _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(starts), _p(ctx.q_len), _p(ctx.ctx_len),
                 _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(ctx.R), c_int(H),
                 c_int(rank), c_int(dk), c_int(window), c_float(scale), c_int(G), _p(sink), c_int(1 if exact_weights else 0),
                 _p(ctx.err), _stream()), "latent_decode")
@@ -1270,11 +1275,15 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
     return out
 
 
-def gather_rows(src: torch.Tensor, rows: torch.Tensor, zero_fill: bool = True, live: Optional[int] = None) -> torch.Tensor:
+def gather_rows(src: torch.Tensor, rows: torch.Tensor, zero_fill: bool = True, live: Optional[int] = None,
+                out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """out[r] = src[rows[r]]; where rows[r] < 0, zeros, or nothing is written (zero_fill False).  live: how many rows
-    are not padding (for the byte count of a profile)."""
-    _dev(src, rows)
-    out = torch.empty((rows.shape[0], src.shape[1]), dtype=src.dtype, device=src.device)
+    are not padding (for the byte count of a profile).  out: a tensor of that shape to write to."""
+    _dev(src, rows, out)
+    if out is None:
+        out = torch.empty((rows.shape[0], src.shape[1]), dtype=src.dtype, device=src.device)
+    elif out.shape != (rows.shape[0], src.shape[1]) or out.dtype != src.dtype or not out.is_contiguous():
+        raise KernelError("gather_rows: out does not fit")
     lib = library("sequence_ops.cu")
     with region("gather_rows", 2 * (live if live is not None and not zero_fill else out.shape[0]) * out.shape[1] * out.element_size()):
         check(lib.aie_gather_rows(_p(src), _p(rows), _p(out), c_int(dtype_code(src)), c_int(rows.shape[0]),

@@ -37,7 +37,9 @@ class LatentWork(StepPlanner):
     tokens it brings) of units of four consecutive tokens of one request of `mine`, which share the cache rows they gather;
     `prompt_tiles` [n, 2]: the expanded ones in tiles of `ops.PREFILL_TILE` tokens.  `gather` [n, 2] = (request row, which 128 of
     its keys) of the rows to expand, and `row_tile` [R]: where among them a request's first 128 keys would be.  Lone tokens
-    need no list.  `prompts`: some are expanded; `folds`: some are not."""
+    need no list.  `prompts`: some are expanded; `folds`: some are not.  `mixed`: some are expanded and some not; the tokens of these others, `short_tokens` [n_short], are then handled
+    one behind the other: `short_row` [T] has a token's place among them (-1: expanded), `short_start` [R] that of a request's
+    first."""
 
     def __init__(self, H: int = 0, window: int = 0, expands: bool = False):
         self.H, self.window, self.expands = H, window, expands
@@ -61,9 +63,15 @@ class LatentWork(StepPlanner):
         rows = np.repeat(np.arange(len(lens)), key_tiles)
         row_tile = np.cumsum(key_tiles) - key_tiles - first
         gather = np.stack([rows, np.arange(len(rows)) - row_tile[rows]], axis=1)
-        return (dict(tiles=units(mine, 4), prompt_tiles=units(expanded, ops.PREFILL_TILE), gather=gather,
-                     row_tile=row_tile if len(rows) else row_tile[:0]),
-                dict(mine=mine, expanded=expanded, prompts=bool(len(rows)), folds=not expanded.all()))
+        arrays = dict(tiles=units(mine, 4), prompt_tiles=units(expanded, ops.PREFILL_TILE), gather=gather,
+                      row_tile=row_tile if len(rows) else row_tile[:0])
+        mixed, n_short = bool(len(rows)) and not expanded.all(), int(lens[~expanded].sum())
+        if mixed:
+            short = np.repeat(~expanded, lens)
+            brings = np.where(expanded, 0, lens)
+            arrays.update(short_row=np.where(short, np.cumsum(short) - 1, -1), short_start=np.cumsum(brings) - brings,
+                          short_tokens=np.flatnonzero(short))
+        return arrays, dict(mine=mine, expanded=expanded, prompts=bool(len(rows)), folds=not expanded.all(), mixed=mixed, n_short=n_short)
 
 
 LATENT_WORK = LatentWork()
@@ -200,14 +208,19 @@ class LatentAttention(Mixer):
         # portions of prompts meet their keys and values expanded; the others read the rows as they are
         made = ops.latent_prepare(q_src, self.H, self.d, self.rot, self.rank, self.c_weight, self.eps, inv_freq, cache.k_pages,
                                   ctx, cache.block_table, self.env.dtype, write=cache.writes and not self.shares_cache, kv=kv,
-                                  halves=self.halves, magnitude=self.magnitude, folded=work.folds, whole=work.prompts)
+                                  halves=self.halves, magnitude=self.magnitude, folded=work.folds, whole=work.prompts,
+                                  short_row=work.short_row if work.mixed else None, n_short=work.n_short)
         a = torch.empty((T, self.H, self.dv), dtype=self.env.dtype, device=h.device)
         if work.folds:
             q_plain, q_full = made[:2]
             ops.head_linear(q_plain, self.w_ukT, q_full)
             mixed = ops.latent_attention(q_full, cache.k_pages, ctx, cache.block_table, self.rank, self.scale,
-                                         self.window, self.env.dtype, work, sink=self.sink, exact_weights=self.exact_weights)
-            ops.head_linear(mixed, self.w_uv, a)
+                                         self.window, self.env.dtype, work, sink=self.sink, exact_weights=self.exact_weights,
+                                         compact=work.mixed)
+            own = torch.empty_like(a[:work.n_short]) if work.mixed else a
+            ops.head_linear(mixed, self.w_uv, own)
+            if work.mixed:
+                ops.gather_rows(own.view(work.n_short, -1), work.short_row, zero_fill=False, live=work.n_short, out=a.view(T, -1))
         if work.prompts:
             ops.latent_prompt(made[2], cache.k_pages, self.w_expand, ctx, cache.block_table, work, self.scale, self.window, self.sink, a)
         a = a.view(T, self.H * self.dv)

@@ -54,3 +54,43 @@ def test_a_page_outside_the_pool_is_flagged():
     lc.block_table[0, 2] = 99
     part.forward(rnd(gen, 70, 128).to(torch.bfloat16).cuda(), ctx, lc)
     assert int(rig.err.item()) == 2
+
+
+def test_tokens_beside_a_prompt_are_the_only_ones_that_are_folded(monkeypatch):
+    """Four decoded tokens and a short portion beside two prompts: the products that fold and unfold see their rows alone, and
+    every request has the bits that it has in a step of its own kind."""
+    from ai_engine_b200.kernels import ops
+    gen = torch.Generator().manual_seed(4)
+    m = lm(2, 128, 64, 128, 64, 0.1, None)
+    part, t = latent_part(m, 128, 1e-5, "bfloat16", gen)
+    load(part, {k: v.to(torch.bfloat16) for k, v in t.items()}, torch.bfloat16)
+    rows_seen, real = [], ops.head_linear
+    monkeypatch.setattr(ops, "head_linear", lambda x, w, out: rows_seen.append(x.shape[0]) or real(x, w, out))
+    before, brings = (40, 0, 7, 300, 20, 0, 99), (1, 100, 1, 1, 7, 70, 1)
+    seqs = [rnd(gen, c + n, 128).to(torch.bfloat16).cuda() for c, n in zip(before, brings)]
+
+    def run(groups):
+        rig = Rig(part, DT["bfloat16"], page=16, pages=64, max_seqs=8)
+        slots, out = [rig.admit() for _ in seqs], {}
+
+        def step(who, rows):
+            portions = [(slots[i], len(x)) for i, x in zip(who, rows)]
+            ctx, lc = rig.step(portions)
+            got = part.forward(torch.cat(rows), ctx, lc)
+            rig.done(portions)
+            return (got.sum(0) if got.dim() == 3 else got).split([len(x) for x in rows])
+
+        for i, c in enumerate(before):
+            if c:
+                step([i], [seqs[i][:c]])
+        rows_seen.clear()
+        for who in groups:
+            out.update(zip(who, step(who, [seqs[i][before[i]:] for i in who])))
+        return [out[i] for i in range(len(seqs))], list(rows_seen)
+
+    together, seen = run([list(range(7))])
+    assert seen == [11, 11]                                       # 1 + 1 + 1 + 7 + 1
+    apart, _ = run([[0, 2, 3, 6], [4], [1, 5]])
+    for a, b in zip(together, apart):
+        # the joins of parts and the output's product follow the step's shape: bfloat16 roundings of equal sums
+        assert float((a.float() - b.float()).abs().max()) <= 2.0 ** -6 * float(b.float().abs().max())

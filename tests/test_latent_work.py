@@ -46,3 +46,13 @@ def test_lists_name_every_token_and_every_row_once():
                 assert w.gather[at].tolist() == [r, k] and w.row_tile[r] + k == at
                 at += 1
         assert at == len(w.gather) and len(w.row_tile) == (len(reqs) if at else 0)
+        assert w.mixed == (bool(at) and not w.expanded.all())
+        if w.mixed:                                               # what is not expanded, token behind token
+            tokens, t = [], 0
+            for r, (_, n) in enumerate(reqs):
+                if not w.expanded[r]:
+                    assert w.short_start[r] == len(tokens)
+                    tokens += range(t, t + n)
+                t += n
+            assert w.short_tokens.tolist() == tokens and w.n_short == len(tokens)
+            assert [w.short_row[i] for i in tokens] == list(range(len(tokens))) and (w.short_row >= 0).sum() == len(tokens)
