@@ -1108,23 +1108,24 @@ extern "C" int aie_paged_attention_prefill_tc_rows(const void* q, const void* pa
 #undef ARGS
 }
 
-// Keys of 192 and values of 128 elements out of rows [rows][H][192 | 128] bf16 (see AtExt::row_tile; rows a multiple of 128)
-// instead of pages; q [T, H, 192], out [T, H, 128].
+// Heads head0 .. head0 + heads - 1 of H over keys of 192 and values of 128 elements out of rows [rows][heads][192 | 128] bf16 (see
+// AtExt::row_tile; rows a multiple of 128) instead of pages; q [T, H, 192], out [T, H, 128].
 extern "C" int aie_prefill_tc_expanded(const void* q, const void* rows_kv, long long rows, void* out, const int* tiles, int n_tiles,
-                                       const int* q_start, const int* q_len, const int* ctx_len, int T, int H, int window,
-                                       const int* row_tile, const float* sink, float scale, unsigned* err, cudaStream_t stream) {
+                                       const int* q_start, const int* q_len, const int* ctx_len, int T, int H, int head0,
+                                       int heads, int window, const int* row_tile, const float* sink, float scale, unsigned* err, cudaStream_t stream) {
     if (n_tiles <= 0) return 0;
-    if (H <= 0 || window < 0 || !row_tile || rows % AT_N || rows / AT_N > 0x7fffffffLL / AT_N) return AIE_BAD_ARG;
+    if (heads <= 0 || head0 < 0 || head0 + heads > H || window < 0 || !row_tile || rows % AT_N || rows / AT_N > 0x7fffffffLL / AT_N) return AIE_BAD_ARG;
     if (n_tiles > 65535 || (((size_t)q | (size_t)rows_kv | (size_t)out) & 15)) return AIE_UNSUPPORTED;
     constexpr int HD = 128, HQ = 192, BLOCKS = (HD + HQ) / 64;
     TcEncodeTiledFn fn = tc_encode_fn();
     if (!fn) return AIE_UNSUPPORTED;
     CUtensorMap mq, mk, mv;
-    int rc = tc_make_map_2d(&mq, q, (unsigned long long)T, (unsigned long long)H * HQ, (unsigned long long)H * HQ * 2, AT_M, 64);
+    int rc = tc_make_map_2d(&mq, (const bf16*)q + (size_t)head0 * HQ, (unsigned long long)T, (unsigned long long)heads * HQ,
+                            (unsigned long long)H * HQ * 2, AT_M, 64);
     if (rc) return rc;
     // [groups of 8 rows][blocks of 64 columns of all heads][8 rows][64]: a box takes a head's key blocks, or its value blocks
-    const cuuint64_t row_bytes = (cuuint64_t)H * BLOCKS * 128;
-    const cuuint64_t dims[4] = {64, 8, (cuuint64_t)H * BLOCKS, (cuuint64_t)(rows / 8)}, strides[3] = {row_bytes, 128, row_bytes * 8};
+    const cuuint64_t row_bytes = (cuuint64_t)heads * BLOCKS * 128;
+    const cuuint64_t dims[4] = {64, 8, (cuuint64_t)heads * BLOCKS, (cuuint64_t)(rows / 8)}, strides[3] = {row_bytes, 128, row_bytes * 8};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     for (int v = 0; v < 2; ++v) {
         const cuuint32_t box[4] = {64, 8, (cuuint32_t)((v ? HD : HQ) / 64), AT_N / 8};
@@ -1133,11 +1134,11 @@ extern "C" int aie_prefill_tc_expanded(const void* q, const void* rows_kv, long 
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return AIE_UNSUPPORTED;
     }
-    const AtExt ext{window, 0.f, nullptr, 0, 0, nullptr, nullptr, nullptr, sink, row_tile};
+    const AtExt ext{window, 0.f, nullptr, 0, 0, nullptr, nullptr, nullptr, sink ? sink + head0 : sink, row_tile};
     auto kern = paged_prefill_tc_kernel<HD, true, HQ>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AtSmem<HD, HQ>::bytes);
     if (e != cudaSuccess) return (int)e;
-    launch_pdl(kern, dim3(H, n_tiles), dim3(AT_THREADS), AtSmem<HD, HQ>::bytes, stream, mq, mk, mv, (bf16*)out, tiles, n_tiles,
+    launch_pdl(kern, dim3(heads, n_tiles), dim3(AT_THREADS), AtSmem<HD, HQ>::bytes, stream, mq, mk, mv, (bf16*)out + (size_t)head0 * HD, tiles, n_tiles,
                q_start, q_len, ctx_len, (const int*)nullptr, 0, (int)(rows / AT_N), AT_N, H, 1, scale, err, ext);
     AIE_LAUNCH_CHECK();
 }

@@ -952,9 +952,12 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
     return (q_plain, q_full, q_all) if whole else (q_plain, q_full)
 
 
-# Portions of this many tokens or more may meet their keys and values expanded; the expanded rows of a step take no more than this.
+# Portions of this many tokens or more may meet their keys and values expanded.  Expanded rows take at most this much at a time
+# (26,214 rows x 16 heads; one head's rows of one portion at the least): more portions than that go behind one another, the
+# heads of a longer one too, and no bit depends on it.
 LATENT_EXPAND_TOKENS = 64
-LATENT_EXPAND_BYTES = 1 << 30
+LATENT_EXPAND_BYTES = 1 << 28
+LATENT_EXPAND_ROW = 2 * (192 + 128)      # bytes of a row and head
 # Expanding takes 20 tokens' worth of multiply-adds a key and head (576 x 320 of them), and a (query, key) pair and head then
 # costs 320 instead of 1,088.  What decides is the time of either form, us, as measured on a latent of 512:
 LATENT_TILE_US = 2.4        # expanded: a tile of 128 keys in a block's chain, one block an SM for every 128 queries of a head
@@ -1004,23 +1007,34 @@ def latent_prompt(q: torch.Tensor, pages: torch.Tensor, w_expand: torch.Tensor, 
             or any(t.dtype != torch.bfloat16 for t in (q, pages, w_expand, out))
             or (sink is not None and (sink.dtype != torch.float32 or sink.shape != (H,)))):
         raise KernelError("latent_prompt: shapes or dtypes do not fit")
-    n_tiles = work.gather.shape[0]
-    rows = torch.empty((128 * n_tiles, dk), dtype=torch.bfloat16, device=q.device)
-    with region("latent_gather", 2 * _nb(rows)):
-        check(library("latent_attention_tc.cu").aie_latent_gather(
-            _p(pages), _p(rows), _p(work.gather), c_int(n_tiles), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table),
-            c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(dk), c_int(window), _p(ctx.err), _stream()),
-            "latent_gather")
-    kv = linear(rows, w_expand, torch.bfloat16)
     pairs = 0.0
     if _profiling() and hasattr(ctx, "h_q_len"):
         for n, c in zip(ctx.h_q_len[work.expanded].tolist(), ctx.h_ctx_len[work.expanded].tolist()):
             pairs += float(sum(min(c + i + 1, window) if window > 0 else c + i + 1 for i in range(n)))
-    with region("latent_prompt_tcgen05", _nb(q, kv, out), 2.0 * pairs * H * 320):
-        check(library("attention_prefill_tc.cu").aie_prefill_tc_expanded(
-            _p(q), _p(kv), c_longlong(128 * n_tiles), _p(out), _p(work.prompt_tiles), c_int(work.prompt_tiles.shape[0]), _p(ctx.q_start),
-            _p(ctx.q_len), _p(ctx.ctx_len), c_int(T), c_int(H), c_int(window), _p(work.row_tile), _p(sink), c_float(scale), _p(ctx.err),
-            _stream()), "prefill_tc_expanded")
+    for g0, g1, p0, p1, step in work.groups:
+        rows = torch.empty((128 * (g1 - g0), dk), dtype=torch.bfloat16, device=q.device)
+        with region("latent_gather", 2 * _nb(rows)):
+            check(library("latent_attention_tc.cu").aie_latent_gather(
+                _p(pages), _p(rows), _p(work.gather[g0:g1]), c_int(g1 - g0), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table),
+                c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(dk), c_int(window), _p(ctx.err),
+                _stream()), "latent_gather")
+        head = 0
+        while head < H:
+            heads = min(step, H - head)
+            try:
+                kv = linear(rows, w_expand[320 * head:320 * (head + heads)], torch.bfloat16)
+            except torch.OutOfMemoryError:
+                if step == 1:
+                    raise
+                step = max(1, step // 4)                    # fewer heads at a time
+                continue
+            share = (p1 - p0) / work.prompt_tiles.shape[0] * heads / H
+            with region("latent_prompt_tcgen05", share * _nb(q, out) + _nb(kv), share * 2.0 * pairs * H * 320):
+                check(library("attention_prefill_tc.cu").aie_prefill_tc_expanded(
+                    _p(q), _p(kv), c_longlong(128 * (g1 - g0)), _p(out), _p(work.prompt_tiles[p0:p1]), c_int(p1 - p0), _p(ctx.q_start),
+                    _p(ctx.q_len), _p(ctx.ctx_len), c_int(T), c_int(H), c_int(head), c_int(heads), c_int(window), _p(work.row_tile),
+                    _p(sink), c_float(scale), _p(ctx.err), _stream()), "prefill_tc_expanded")
+            head += heads
 
 
 def _latent_cost(q_full, pages, ctx, rank: int, window: int, mine):

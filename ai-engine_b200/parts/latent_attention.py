@@ -36,7 +36,8 @@ class LatentWork(StepPlanner):
     `expands` False), `mine`: of the others that bring more than one token.  `tiles` [n, 2] = (request row, offset among the
     tokens it brings) of units of four consecutive tokens of one request of `mine`, which share the cache rows they gather;
     `prompt_tiles` [n, 2]: the expanded ones in tiles of `ops.PREFILL_TILE` tokens.  `gather` [n, 2] = (request row, which 128 of
-    its keys) of the rows to expand, and `row_tile` [R]: where among them a request's first 128 keys would be.  Lone tokens
+    its keys) of the rows to expand.  They are expanded in `groups`, each (first, one behind the last of `gather`, the same of
+    `prompt_tiles`, heads at a time), and `row_tile` [R] says where in its group a request's first 128 keys would be.  Lone tokens
     need no list.  `prompts`: some are expanded; `folds`: some are not.  `mixed`: some are expanded and some not; the tokens of these others, `short_tokens` [n_short], are then handled
     one behind the other: `short_row` [T] has a token's place among them (-1: expanded), `short_start` [R] that of a request's
     first."""
@@ -49,11 +50,10 @@ class LatentWork(StepPlanner):
         lens, cached = ctx.h_q_len.astype(np.int64), ctx.h_ctx_len.astype(np.int64)
         expanded = np.zeros(len(lens), dtype=bool)
         if self.expands and ctx.max_q_len >= ops.LATENT_EXPAND_TOKENS:
-            expanded = ops.latent_expanded(lens, cached, self.H, self.window)
+            if ops.LATENT_EXPAND_BYTES > 0:
+                expanded = ops.latent_expanded(lens, cached, self.H, self.window)
         first = (np.maximum(cached - self.window + 1, 0) if self.window > 0 else np.zeros_like(cached)) // ops.PREFILL_TILE
         key_tiles = np.where(expanded, (cached + lens - 1) // ops.PREFILL_TILE - first + 1, 0)
-        if int(key_tiles.sum()) * ops.PREFILL_TILE * self.H * 640 > ops.LATENT_EXPAND_BYTES:
-            expanded[:], key_tiles[:] = False, 0
         mine = (lens > 1) & ~expanded
 
         def units(mask, size):
@@ -61,8 +61,18 @@ class LatentWork(StepPlanner):
             return np.asarray(out, dtype=np.int32).reshape(-1, 2)
 
         rows = np.repeat(np.arange(len(lens)), key_tiles)
-        row_tile = np.cumsum(key_tiles) - key_tiles - first
-        gather = np.stack([rows, np.arange(len(rows)) - row_tile[rows]], axis=1)
+        before = np.cumsum(key_tiles) - key_tiles
+        gather = np.stack([rows, np.arange(len(rows)) - (before - first)[rows]], axis=1)
+        row_tile, groups = before - first, []
+        most = max(1, ops.LATENT_EXPAND_BYTES // (ops.PREFILL_TILE * ops.LATENT_EXPAND_ROW))      # tiles x heads at a time
+        for r in np.flatnonzero(expanded).tolist():
+            n, q = int(key_tiles[r]), -(-int(lens[r]) // ops.PREFILL_TILE)
+            if groups and (before[r] + n - groups[-1][0]) * self.H <= most:
+                groups[-1][1::2] = [int(before[r]) + n, groups[-1][3] + q]
+            else:
+                at = groups[-1][3] if groups else 0
+                groups.append([int(before[r]), int(before[r]) + n, at, at + q, min(self.H, max(1, most // n))])
+            row_tile[r] -= groups[-1][0]
         arrays = dict(tiles=units(mine, 4), prompt_tiles=units(expanded, ops.PREFILL_TILE), gather=gather,
                       row_tile=row_tile if len(rows) else row_tile[:0])
         mixed, n_short = bool(len(rows)) and not expanded.all(), int(lens[~expanded].sum())
@@ -71,7 +81,7 @@ class LatentWork(StepPlanner):
             brings = np.where(expanded, 0, lens)
             arrays.update(short_row=np.where(short, np.cumsum(short) - 1, -1), short_start=np.cumsum(brings) - brings,
                           short_tokens=np.flatnonzero(short))
-        return arrays, dict(mine=mine, expanded=expanded, prompts=bool(len(rows)), folds=not expanded.all(), mixed=mixed, n_short=n_short)
+        return arrays, dict(mine=mine, expanded=expanded, groups=[tuple(g) for g in groups], prompts=bool(len(rows)), folds=not expanded.all(), mixed=mixed, n_short=n_short)
 
 
 LATENT_WORK = LatentWork()

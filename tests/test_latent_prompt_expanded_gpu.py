@@ -94,3 +94,36 @@ def test_tokens_beside_a_prompt_are_the_only_ones_that_are_folded(monkeypatch):
     for a, b in zip(together, apart):
         # the joins of parts and the output's product follow the step's shape: bfloat16 roundings of equal sums
         assert float((a.float() - b.float()).abs().max()) <= 2.0 ** -6 * float(b.float().abs().max())
+
+
+@pytest.mark.parametrize("window", [None, 100])
+def test_expanded_rows_have_a_bound_and_no_bit_depends_on_it(window, monkeypatch):
+    from ai_engine_b200.kernels import ops
+    gen = torch.Generator().manual_seed(6)
+    m = dict(lm(5, 128, 64, 128, 64, 0.1, window))
+    part, t = latent_part(m, 128, 1e-5, "bfloat16", gen)
+    load(part, {k: v.to(torch.bfloat16) for k, v in t.items()}, torch.bfloat16)
+    seqs, cuts = [rnd(gen, n, 128).to(torch.bfloat16) for n in (200, 70, 300, 90)], [[200], [70], [130, 170], [5, 85]]
+    products, real = [], ops.linear
+    monkeypatch.setattr(ops, "linear", lambda x, w, *a: products.append((w.shape[0] % 320 == 0 and x.shape[0] % 128 == 0
+                                                                       and x.shape[1] == 128, x.shape[0] * w.shape[0] * 2)) or real(x, w, *a))
+    run = lambda: Rig(part, DT["bfloat16"], page=16, pages=64).run(seqs, cuts)
+    want, most = run(), max(size for mine, size in products if mine)
+    for bound in (most // 2, 128 * 640 * 3, 1):
+        monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", bound)
+        products.clear()
+        got = run()
+        sizes = [size for mine, size in products if mine]
+        assert len(sizes) > 2 and max(sizes) <= max(bound, 3 * 128 * 640)            # three tiles: the longest portion, one head
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+    monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", 1 << 28)
+    full = [3]                                                    # no room for three products: fewer heads at a time
+
+    def tight(x, w, *a):
+        if w.shape[0] > 320 and w.shape[0] % 320 == 0 and x.shape[0] % 128 == 0 and full[0]:
+            full[0] -= 1
+            raise torch.OutOfMemoryError("no room")
+        return real(x, w, *a)
+
+    monkeypatch.setattr(ops, "linear", tight)
+    assert all(torch.equal(a, b) for a, b in zip(want, run())) and full[0] < 3

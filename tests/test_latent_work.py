@@ -28,7 +28,9 @@ def test_which_portions_are_expanded(H, window, reqs, expanded):
     assert not plan(reqs, H, window, expands=False).expanded.any()
 
 
-def test_lists_name_every_token_and_every_row_once():
+@pytest.mark.parametrize("bound", [1 << 28, 40 << 20, 5 << 20, 1])
+def test_lists_name_every_token_and_every_row_once(bound, monkeypatch):
+    monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", bound)
     rng = random.Random(1)
     for _ in range(200):
         window, H = rng.choice([0, 1, 100, 128, 129, 1024]), rng.choice([1, 16, 40])
@@ -42,9 +44,17 @@ def test_lists_name_every_token_and_every_row_once():
         for r in np.flatnonzero(w.expanded).tolist():
             c, n = reqs[r]
             low = max(c - window + 1, 0) // 128 if window else 0
+            start = next(g0 for g0, g1, *_ in w.groups if g0 <= at < g1)
             for k in range(low, (c + n - 1) // 128 + 1):
-                assert w.gather[at].tolist() == [r, k] and w.row_tile[r] + k == at
+                assert w.gather[at].tolist() == [r, k] and w.row_tile[r] + k == at - start
                 at += 1
+        ends = [0, 0]
+        for g0, g1, p0, p1, heads in w.groups:                    # one behind the other, whole requests, within the bound
+            assert [g0, p0] == ends and 1 <= heads <= H and (heads == 1 or (g1 - g0) * heads * 128 * 640 <= bound)
+            assert set(w.gather[g0:g1, 0].tolist()) == set(w.prompt_tiles[p0:p1, 0].tolist())
+            assert heads == H or len(set(w.gather[g0:g1, 0].tolist())) == 1
+            ends = [g1, p1]
+        assert ends == [len(w.gather), len(w.prompt_tiles)]
         assert at == len(w.gather) and len(w.row_tile) == (len(reqs) if at else 0)
         assert w.mixed == (bool(at) and not w.expanded.all())
         if w.mixed:                                               # what is not expanded, token behind token
