@@ -954,7 +954,7 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
 
 # Portions of this many tokens or more may meet their keys and values expanded.  Expanded rows take at most this much at a time
 # (26,214 rows x 16 heads; one head's rows of one portion at the least): more portions than that go behind one another, the
-# heads of a longer one too, and no bit depends on it.
+# heads of a longer one too.
 LATENT_EXPAND_TOKENS = 64
 LATENT_EXPAND_BYTES = 1 << 28
 LATENT_EXPAND_ROW = 2 * (192 + 128)      # bytes of a row and head
@@ -1038,9 +1038,10 @@ def latent_prompt(q: torch.Tensor, pages: torch.Tensor, w_expand: torch.Tensor, 
 
 
 def _latent_cost(q_full, pages, ctx, rank: int, window: int, mine):
-    """(bytes, operations) of the tokens of the requests `mine` (a mask)."""
+    """(bytes, operations) of the tokens of the requests that `mine` (a mask, or a function of the lengths) picks."""
     if not (_profiling() and hasattr(ctx, "h_q_len")):
         return 0.0, 0.0
+    mine = mine(ctx.h_q_len) if callable(mine) else mine
     H, dk = q_full.shape[1:]
     ql, cl = ctx.h_q_len[mine].astype(float), ctx.h_ctx_len[mine].astype(float)
     if window > 0:
@@ -1104,7 +1105,7 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
         G = max(1, 2 * sm_count() // ((H + 15) // 16))
         part_o = torch.empty((G + ctx.R, H, rank), dtype=torch.float32, device=q_full.device)
         part_ml = torch.empty((G + ctx.R, H, 2), dtype=torch.float32, device=q_full.device)
-        with region("latent_decode", *_latent_cost(q_full, pages, ctx, rank, window, ctx.h_q_len == 1)):
+        with region("latent_decode", *_latent_cost(q_full, pages, ctx, rank, window, lambda lens: lens == 1)):
             check(library("latent_attention_tc.cu").aie_latent_decode(
                 _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(starts), _p(ctx.q_len), _p(ctx.ctx_len),
                 _p(block_table), c_int(block_table.shape[1]), c_int(pages.shape[0]), c_int(pages.shape[2]), c_int(ctx.R), c_int(H),

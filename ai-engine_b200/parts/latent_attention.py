@@ -130,6 +130,7 @@ class LatentAttention(Mixer):
             raise ValueError("latent attention: a layer that reads another's cache has neither a query latent nor a gate")
         self.w_uq = self.cq_weight = self.sink = None
         self.w_in = self.w_ukT = self.w_uv = self.w_o = self.c_weight = self._no_rope = self.w_expand = None
+        self.planner = latent_work(self.H, self.window, False)
 
     def tensor_specs(self):
         t, dq = self.spec.tensors, self.d + self.rot
@@ -178,6 +179,7 @@ class LatentAttention(Mixer):
             w[:, self.d:self.d + self.rot, self.rank:] = torch.eye(self.rot, dtype=torch.bfloat16, device=uk.device)
             w[:, self.d + self.rot:, :self.rank] = self.w_uv
             self.w_expand = w.view(-1, self.rank + self.rot)
+            self.planner = latent_work(self.H, self.window, True)
         self.w_o = source.get(t["o"])
         if self.has_sink:
             self.sink = source.get(t["sink"]).float().contiguous()
@@ -198,7 +200,7 @@ class LatentAttention(Mixer):
         return KVRequest(1, self.rank + self.rot, self.cache_window, planes=1)
 
     def step_planner(self):
-        return latent_work(self.H, self.window, self.w_expand is not None)
+        return self.planner
 
     def forward(self, h, ctx, cache, add_to=None):
         T = h.shape[0]
@@ -214,7 +216,7 @@ class LatentAttention(Mixer):
             q_src = ops.linear(cq, self.w_uq, torch.float32, ctx.err)
         else:
             q_src = proj
-        work = ctx.plan(self.step_planner())
+        work = ctx.plan(self.planner)
         # portions of prompts meet their keys and values expanded; the others read the rows as they are
         made = ops.latent_prepare(q_src, self.H, self.d, self.rot, self.rank, self.c_weight, self.eps, inv_freq, cache.k_pages,
                                   ctx, cache.block_table, self.env.dtype, write=cache.writes and not self.shares_cache, kv=kv,
