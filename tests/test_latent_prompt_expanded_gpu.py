@@ -18,8 +18,7 @@ def test_portions_over_expanded_rows(heads, rank, page, window, scaling, monkeyp
     hidden, lens = 128, (420, 64, 200, 90)
     cuts = [[129, 64, 1, 128, 63, 35], [64], [1, 130, 2, 67], [63, 27]]
     # queries of deviation 0.3 sqrt(128) on keys of 0.3 sqrt(rank): scores of about 1.5.  A score's relative error (a rounded
-    # query on a rounded key, or its latent form: 2^-9 each) is then an error of 1.5 x 2^-8.5 in the exponent; scores ten
-    # times as large, with which this was first written, bring either path to 2.6 % at a latent of 512
+    # query on a rounded key, or its latent form: 2^-9 each) is then an error of 1.5 x 2^-8.5 in the exponent
     m = lm(heads, 128, 64, 128, rank, 1.5 / (0.3 * 128 ** 0.5 * 0.3 * rank ** 0.5 * 128 ** 0.5), window, 20000.0, scaling)
     gen = torch.Generator().manual_seed(rank + (window or 0))
     part, t = latent_part(m, hidden, 1e-5, "bfloat16", gen)
@@ -127,3 +126,49 @@ def test_expanded_rows_have_a_bound_and_no_bit_depends_on_it(window, monkeypatch
 
     monkeypatch.setattr(ops, "linear", tight)
     assert all(torch.equal(a, b) for a, b in zip(want, run())) and full[0] < 3
+
+
+def test_a_query_latent_a_gate_a_head_and_a_rotation_of_halves(monkeypatch):
+    """The other design's layer: queries through a latent of their own, a gate a head, pairs half a rotation apart, no sink and
+    softmax weights of 8 bits where rows are read as they are."""
+    import plain_fokisun as pf
+    from ai_engine_b200.kernels import ops
+    from test_fokisun_parts_gpu import latent_part as gated_part
+    gen = torch.Generator().manual_seed(8)
+    m = dict(heads=3, dim=128, rot_dim=64, vdim=128, kv_rank=128, q_rank=72, scale=0.004, rot=dict(base=20000.0, dims=64))
+    part, t = gated_part(m, 96, 1e-5, "bfloat16", gen)
+    load(part, {k: v.to(torch.bfloat16) for k, v in t.items()}, torch.bfloat16)
+    assert part.w_expand is not None and part.halves and part.head_gate and part.q_rank and not part.exact_weights
+    seqs, cuts, calls, real = [rnd(gen, n, 96) for n in (300, 150)], [[200, 1, 99], [3, 64, 83]], [], ops.latent_prompt
+    refs = [pf.latent_attention(s.double(), f64(t), "", m, 1e-5) for s in seqs]
+    monkeypatch.setattr(ops, "latent_prompt", lambda *a, **k: calls.append(1) or real(*a, **k))
+    run = lambda: Rig(part, DT["bfloat16"], page=16, pages=64).run([s.to(torch.bfloat16) for s in seqs], cuts)
+    got = run()
+    assert len(calls) == 3
+    monkeypatch.setattr(ops, "LATENT_EXPAND_BYTES", 0)
+    folded = run()
+    errors = [[float((o - r).norm() / r.norm()) for o, r in zip(os, refs)] for os in (got, folded)]
+    # scores of about 1: 2^-8.5 of them in the exponent; queries' latent, latents, values, gate, outputs and their projection 2^-9 each
+    assert len(calls) == 3 and max(errors[0]) <= 6 * 2.0 ** -9 and sum(errors[0]) <= 1.05 * sum(errors[1]), errors
+
+
+def test_a_layer_that_reads_another_s_cache(monkeypatch):
+    from ai_engine_b200.kernels import ops
+    from test_pifutar_parts_gpu import latent_part as sharing_part, latent_tensors
+    gen = torch.Generator().manual_seed(3)
+    m = dict(heads=2, dim=128, rot_dim=64, vdim=128, kv_rank=64, scale=0.05, rot=dict(base=10000.0, dims=64))
+    ts = latent_tensors(torch.bfloat16, 64, m, gen)
+    owner = load(sharing_part(torch.bfloat16, 64, m, False), ts, torch.bfloat16)
+    reader = load(sharing_part(torch.bfloat16, 64, m, True), {k: v for k, v in ts.items() if not k.startswith("dkv")}, torch.bfloat16)
+    rig, h = Rig(owner, torch.bfloat16, page=16, pages=32), torch.randn(230, 64, generator=gen).to(torch.bfloat16).cuda()
+    slot, at = rig.admit(), 0
+    for n in (130, 100):
+        ctx, lc = rig.step([(slot, n)])
+        want = owner.forward(h[at:at + n], ctx, lc)
+        pages = lc.k_pages.clone()
+        got = reader.forward(h[at:at + n], ctx, lc)                # the same weights: the same rows, which it must not write
+        a, b = (o.sum(0) if o.dim() == 3 else o for o in (got, want))
+        assert float((a.float() - b.float()).abs().max()) <= 2.0 ** -6 * float(b.float().abs().max())      # queries by another product
+        assert torch.equal(pages.nan_to_num(7.0), lc.k_pages.nan_to_num(7.0))
+        rig.done([(slot, n)])
+        at += n

@@ -35,6 +35,8 @@ def reference(q, k, v, a, S, lens, slots):
 def test_chunks_against_the_recurrence(form, H, d, e, lens, monkeypatch):
     from ai_engine_b200.kernels import ops
     monkeypatch.setattr(ops, "LC_MIN_WORK", 0)              # small steps too
+    taken, real = [], ops._recurrence_in_chunks
+    monkeypatch.setattr(ops, "_recurrence_in_chunks", lambda *a: taken.append(real(*a)) or taken[-1])
     gen = torch.Generator(device=DEV).manual_seed(d * 7 + e + len(lens))
     T, slots = sum(lens), list(range(len(lens)))[::-1]
     rnd = lambda *s: torch.randn(*s, generator=gen, device=DEV)
@@ -60,6 +62,7 @@ def test_chunks_against_the_recurrence(form, H, d, e, lens, monkeypatch):
     ctx, state = Ctx(lens, slots), state0.clone()
     out = ops.linear_recurrence(q, None if form == "keyless" else k, v, decay_tok, decay_head, scale, 1.0, state, ctx, H, d, e,
                                 forget_lower=lower, forget_bias=bias)
+    assert taken == [ops.LC_MIN_TOKENS]
     ref, ref_state = reference(q64, k64, v64, a64, state0.double(), lens, slots)
     mag, mag_state = reference(q64.abs(), k64.abs(), v64.abs(), a64, state0.double().abs(), lens, slots)
     # every term is rounded once per factor and addition that it passes: at most two a token of its chunk, a chunk of its

@@ -31,8 +31,12 @@ def test_chunks_in_parallel(H, hpg, N, dv, lens, pad, monkeypatch):
         assert int(ctx.err.item()) == 0
         return out, state
 
+    entered, real = [], ops.library
+    monkeypatch.setattr(ops, "library", lambda name: entered.append(name) or real(name))
     out, state = run(True)
+    assert "state_space_parallel.cu" in entered and "state_space_chunked.cu" not in entered
     other, other_state = run(False)
+    assert entered.count("state_space_parallel.cu") == 1 and "state_space_chunked.cu" in entered
     rounded = lambda t, n: t.to(torch.bfloat16).double().reshape(T, n, -1).repeat_interleave(H // n, dim=1)
     dt = torch.nn.functional.softplus(dt_raw.double() + dt_bias.double())
     a = torch.exp(-torch.exp(a_log.double()) * dt)
