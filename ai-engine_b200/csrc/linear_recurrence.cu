@@ -13,8 +13,9 @@
 // The columns of S never mix: column j needs only v_t[j].  A warp owns 32 / lanes columns of one (request,
 // head); `lanes` threads share a column, each with RPT consecutive rows of S in registers, and a token costs
 // each thread 2 RPT multiply-adds and a shuffle reduction over its column's lanes.  Tokens of a portion run
-// in order, so a portion of any length continues where the previous step left the state, and a request's
-// result does not depend on what else is in the batch.  The eight warps of a block belong to one (request, head):
+// in order, so a portion of any length continues where the previous step left the state, whose bits depend neither on how a
+// prompt was cut nor on what else is in the batch (an output's do up to the order of the sum over a column's rows: RPT and
+// `lanes` follow the step's shape).  The eight warps of a block belong to one (request, head):
 // they stage the queries, keys and decays of up to sixteen tokens at a time in shared memory with coalesced
 // loads and then walk those tokens from there, so a token does not cost a round trip to memory.
 #include "common.cuh"
