@@ -958,8 +958,9 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
 LATENT_EXPAND_TOKENS = 64
 LATENT_EXPAND_BYTES = 1 << 28
 LATENT_EXPAND_ROW = 2 * (192 + 128)      # bytes of a row and head
-# Expanding takes 20 tokens' worth of multiply-adds a key and head (576 x 320 of them), and a (query, key) pair and head then
-# costs 320 instead of 1,088.  What decides is the time of either form, us, as measured on a latent of 512:
+# On a latent of 512, expanding a key takes 576 x 320 multiply-adds a head, and a (query, key) pair and head then costs 320
+# instead of 1,088: in arithmetic 240 queries a key pay for it, but the two forms reach very different rates.  What decides is
+# the time of either, us, as measured there:
 LATENT_TILE_US = 2.4        # expanded: a tile of 128 keys in a block's chain, one block an SM for every 128 queries of a head
 LATENT_ROW_US = 0.44e-3     # ... and a cached row and head, gathered and expanded
 LATENT_PAIR_US = (0.09e-3, 0.009e-3)      # as they are: a (query, key) pair for every 16 heads begun, and for every head
