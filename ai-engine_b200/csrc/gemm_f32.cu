@@ -7,6 +7,7 @@
 // The reference multiplies x[B,S,in] by a weight kept as [in,out]
 // (crates/ai-engine-runtime/src/arch/linear.rs:106-123); the product is the same.
 #include "common.cuh"
+#include <type_traits>
 
 #define BM 64
 #define BN 64
@@ -100,33 +101,45 @@ static int gemm_f32_go(const void* A, const void* W, void* C, int c_dtype, const
 }
 
 // ---------------------------------------------------------------------------
-// The same product for float32 operands whose rows start on 16 bytes: blocks of 64 x 64 outputs, a thread 8 x 4 of them (a
-// warp's lanes lie 4 x 8 over its quarter), tiles of 64 k brought by cp.async into two stages, k innermost as in memory
-// (rows 68 floats apart: the eight rows that lanes read at a time fall on different banks).  Each output is still one
-// thread's sum over k in order: bits do not depend on the tile.  Warps whose rows all lie behind M only help loading.
-// Bound by what shared memory hands to registers (12 floats a thread for 32 multiply-adds: two thirds of the FMA rate)
-// and, on small grids, by latency.  513 tokens, us, before -> now: 2,048 x 2,048 213 -> 123; 3,072 x 2,048 305 -> 174;
-// 2,048 x 8,192 878 -> 461; 16,384 x 2,048 1,518 -> 881 (39 TFLOP/s).  Tiles of 64 x 128 and 128 x 128 with 8 x 8 or
-// 16 x 8 a thread were within 4 % on the largest grids and 15 to 100 % slower on the others, tiles of 16 and 32 k
-// 33 and 3 % slower in sum.
-#define GT_M 64
-#define GT_N 64
-#define GT_K 64
-#define GT_LD (GT_K + 4)
-#define GT_STAGES 2
-#define GT_THREADS 128
-#define GT_TM 8
-#define GT_TN 4
+// The same product for float32 operands whose rows start on 16 bytes: blocks of 64 x 16 TN outputs, a thread TM x 4 of them in
+// pairs of rows, so that one packed instruction (fma.rn.f32x2, each half rounded as fmaf) does two multiply-adds: registers
+// alone it reaches 62 TFLOP/s here, fmaf 51.  Each output is still one thread's sum over k in order: bits do not depend on
+// the tile.  The pairs want the rows next to one another, so tiles of 16 k go through registers into shared memory with k
+// outermost, four buffers, two tiles between barriers; a row of k group g lies at row ^ 8 g, which keeps the transposing
+// stores off one another's banks.
+// Bound by what shared memory hands to registers (512 bytes of a warp in four cycles): 8 x 4 outputs a thread want 12 floats
+// for 16 packed instructions, 16 x 4 want 20 for 32 (58 TFLOP/s on large grids; 8 x 8 is 2 % behind, 16 x 8 spills).  The wide
+// form has half as many blocks, so which is faster is a matter of rounds (gemm_f32_aligned).
+// us, before (64 x 64 tiles of fmaf, k innermost) -> now, weights from memory: 513 tokens 16,384 x 2,048 913 -> 656,
+// 2,048 x 8,192 491 -> 433, 3,072 x 2,048 179 -> 159, 2,048 x 2,048 128 -> 110; 2,048 tokens 16,384 x 2,048 3,170 -> 2,453;
+// one token 16,384 x 2,048 120 -> 72, 2,048 x 2,048 72 -> 64.
+// AHEAD: with one block an SM a tile's latency shows, so its lines are asked into L2 eight tiles early: one token
+// 84 -> 64, 200 tokens 2,048 x 8,192 320 -> 280; with more blocks it costs 3 %.
+#define GP_M 64
+#define GP_K 16
+#define GP_THREADS 128
 
-template <typename OT>
-__global__ void __launch_bounds__(GT_THREADS, 3)
-gemm_f32_tiled_kernel(const float* __restrict__ A, const float* __restrict__ W, OT* __restrict__ C,
+__device__ __forceinline__ unsigned long long gp_pair(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void gp_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+template <int TM, bool AHEAD, typename OT>
+__global__ void __launch_bounds__(GP_THREADS, TM == 16 ? 3 : 4)
+gemm_f32_pairs_kernel(const float* __restrict__ A, const float* __restrict__ W, OT* __restrict__ C,
                       const int* __restrict__ a_rows, const int* __restrict__ tile_w, int M, int N, int K, int lda, int ldc,
                       long long a_bs, long long w_bs, long long c_bs) {
-    constexpr int ROW = GT_K / 4, PIECES = (GT_M + GT_N) * ROW / GT_THREADS, STEP = GT_THREADS / ROW, STAGE = (GT_M + GT_N) * GT_LD;
-    extern __shared__ __align__(16) float gt_sm[];
-    const int tid = threadIdx.x, lane = tid & 31, wm = tid >> 6, wn = (tid >> 5) & 1;
-    const int m0 = blockIdx.y * GT_M, n0 = blockIdx.x * GT_N;
+    // warps lie GP_M / (4 TM) x the rest over the block, a warp's lanes 4 x 8
+    constexpr int TN = 4, WM = GP_M / (4 * TM), BN_ = 4 / WM * 8 * TN, PA = GP_M / 32, PW = BN_ / 32, LINES = (GP_M + BN_ + GP_THREADS - 1) / GP_THREADS;
+    extern __shared__ __align__(16) float gp_sm[];
+    float(*as)[GP_K][GP_M] = reinterpret_cast<float(*)[GP_K][GP_M]>(gp_sm);                       // four buffers each
+    float(*ws)[GP_K][BN_] = reinterpret_cast<float(*)[GP_K][BN_]>(gp_sm + 4 * GP_K * GP_M);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wm = warp % WM, wn = warp / WM;
+    const int m0 = blockIdx.y * GP_M, n0 = blockIdx.x * BN_;
     A += (long long)blockIdx.z * a_bs;
     C += (long long)blockIdx.z * c_bs;
     if (tile_w) {
@@ -136,93 +149,165 @@ gemm_f32_tiled_kernel(const float* __restrict__ A, const float* __restrict__ W, 
     } else {
         W += (long long)blockIdx.z * w_bs;
     }
-    // a thread's pieces of a tile: 16 bytes at column k4 of every STEP-th row, GT_M rows of A, then those of W
-    const int row0 = tid / ROW, k4 = (tid % ROW) * 4;
-    int arow[GT_M / STEP];                          // -1: a row of zeros
+    // a thread's pieces of a tile: 16 bytes at column k4 of every 32nd row, the rows of A, then those of W
+    const int row0 = tid >> 2, k4 = tid & 3;
+    const float* asrc[PA];                          // null: a row of zeros
 #pragma unroll
-    for (int i = 0; i < GT_M / STEP; ++i) {
-        const int m = m0 + row0 + i * STEP;
-        arow[i] = m < M ? (a_rows ? a_rows[m] : m) : -1;
+    for (int i = 0; i < PA; ++i) {
+        const int m = m0 + row0 + i * 32, r = m < M ? (a_rows ? a_rows[m] : m) : -1;
+        asrc[i] = r >= 0 ? A + (size_t)r * lda + k4 * 4 : nullptr;
     }
-    const int blocks = (K + GT_K - 1) / GT_K;
-    auto fetch = [&](int kb) {
-        if (kb < blocks) {
-            const unsigned dst = (unsigned)__cvta_generic_to_shared(gt_sm + (kb % GT_STAGES) * STAGE + row0 * GT_LD + k4);
-            const int k = kb * GT_K + k4;
+    const float* wsrc = W + (size_t)(n0 + row0) * K + k4 * 4;
+    const int wrows = N - n0 - row0;                // rows 32 i below this are there
+    const int blocks = (K + GP_K - 1) / GP_K;
+    const float* line[AHEAD ? LINES : 1];           // rows whose lines this thread asks for
+    if (AHEAD) {
 #pragma unroll
-            for (int i = 0; i < PIECES; ++i) {
-                const float* src = W;
-                bool ok = k < K;
-                if (i < GT_M / STEP) {
-                    ok = ok && arow[i < GT_M / STEP ? i : 0] >= 0;
-                    if (ok) src = A + (size_t)arow[i < GT_M / STEP ? i : 0] * lda + k;
-                } else {
-                    const int n = n0 + row0 + (i - GT_M / STEP) * STEP;
-                    ok = ok && n < N;
-                    if (ok) src = W + (size_t)n * K + k;
-                }
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + i * STEP * GT_LD * 4), "l"(src),
-                             "r"(ok ? 16 : 0) : "memory");
+        for (int i = 0; i < LINES; ++i) {
+            const int row = tid + i * GP_THREADS, m = m0 + row, n = n0 + row - GP_M;
+            line[i] = nullptr;
+            if (row < GP_M) {
+                const int r = m < M ? (a_rows ? a_rows[m] : m) : -1;
+                if (r >= 0) line[i] = A + (size_t)r * lda;
+            } else if (row < GP_M + BN_ && n < N) {
+                line[i] = W + (size_t)n * K;
             }
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    float acc[GT_TM][GT_TN];
-#pragma unroll
-    for (int i = 0; i < GT_TM; ++i)
-#pragma unroll
-        for (int j = 0; j < GT_TN; ++j) acc[i][j] = 0.f;
-    const int lm = wm * 4 * GT_TM + (lane >> 3), ln = wn * 8 * GT_TN + (lane & 7);        // rows lm + 4 i, columns ln + 8 j
-    const bool works = m0 + wm * 4 * GT_TM < M;
-#pragma unroll
-    for (int s = 0; s < GT_STAGES - 1; ++s) fetch(s);
-#pragma unroll 1
-    for (int kb = 0; kb < blocks; ++kb) {
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(GT_STAGES - 2) : "memory");
-        __syncthreads();
-        fetch(kb + GT_STAGES - 1);
-        if (!works) continue;
-        const float* as = gt_sm + (kb % GT_STAGES) * STAGE + lm * GT_LD;
-        const float* ws = gt_sm + (kb % GT_STAGES) * STAGE + (GT_M + ln) * GT_LD;
-#pragma unroll 2
-        for (int k = 0; k < GT_K; k += 4) {
-            float4 a[GT_TM], w[GT_TN];
-#pragma unroll
-            for (int i = 0; i < GT_TM; ++i) a[i] = *reinterpret_cast<const float4*>(as + 4 * i * GT_LD + k);
-#pragma unroll
-            for (int j = 0; j < GT_TN; ++j) w[j] = *reinterpret_cast<const float4*>(ws + 8 * j * GT_LD + k);
-#pragma unroll
-            for (int x = 0; x < 4; ++x)
-#pragma unroll
-                for (int i = 0; i < GT_TM; ++i)
-#pragma unroll
-                    for (int j = 0; j < GT_TN; ++j)
-                        acc[i][j] = x == 0 ? fmaf(a[i].x, w[j].x, acc[i][j]) : x == 1 ? fmaf(a[i].y, w[j].y, acc[i][j])
-                                  : x == 2 ? fmaf(a[i].z, w[j].z, acc[i][j]) : fmaf(a[i].w, w[j].w, acc[i][j]);
-        }
     }
+    float4 next[PA + PW];
+    auto fetch = [&](int kb) {
+        const bool in = kb * GP_K + k4 * 4 < K;
 #pragma unroll
-    for (int i = 0; i < GT_TM; ++i) {
-        const int m = m0 + lm + 4 * i;
+        for (int i = 0; i < PA; ++i)
+            next[i] = in && asrc[i] ? __ldg(reinterpret_cast<const float4*>(asrc[i] + (size_t)kb * GP_K)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < PW; ++i)
+            next[PA + i] = in && i * 32 < wrows ? __ldg(reinterpret_cast<const float4*>(wsrc + (size_t)i * 32 * K + (size_t)kb * GP_K))
+                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto put = [&](int kb) {
+        const int s = kb & 3;
+#pragma unroll
+        for (int i = 0; i < PA + PW; ++i) {
+            const int row = (row0 + (i < PA ? i : i - PA) * 32) ^ (8 * k4);
+            float* at = i < PA ? &as[s][4 * k4][row] : &ws[s][4 * k4][row];
+            const int ld = i < PA ? GP_M : BN_;
+            at[0] = next[i].x;
+            at[ld] = next[i].y;
+            at[2 * ld] = next[i].z;
+            at[3 * ld] = next[i].w;
+        }
+    };
+    // a warp's 4 TM rows x 8 TN columns: a lane's rows lm + 16 i + (0 .. 3), its columns ln + (0 .. 3)
+    const int lm = wm * 4 * TM + (lane >> 3) * 4, ln = wn * 8 * TN + (lane & 7) * 4;
+    unsigned long long acc[TM / 2][TN];             // rows 2 i and 2 i + 1 of the lane's
+#pragma unroll
+    for (int i = 0; i < TM / 2; ++i)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+    const bool works = m0 + wm * 4 * TM < M;        // a warp whose rows all lie behind M only helps loading
+    auto multiply = [&](int kb, auto gc) {
+        constexpr int G = decltype(gc)::value;
+        const int s = kb & 3;
+#pragma unroll
+        for (int k = 0; k < GP_K; ++k) {
+            const int x = 8 * (k >> 2);
+            ulonglong2 a[G];
+#pragma unroll
+            for (int i = 0; i < G; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(&as[s][k][(lm + 16 * i) ^ x]);
+            const float4 w = *reinterpret_cast<const float4*>(&ws[s][k][ln ^ x]);
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const float wj = j == 0 ? w.x : j == 1 ? w.y : j == 2 ? w.z : w.w;
+                const unsigned long long ww = gp_pair(wj, wj);
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    gp_fma2(acc[2 * i][j], a[i].x, ww);
+                    gp_fma2(acc[2 * i + 1][j], a[i].y, ww);
+                }
+            }
+        }
+    };
+    auto walk = [&](auto gc) {
+        fetch(0);
+        put(0);
+        fetch(1);
+        put(1);
+        __syncthreads();
+#pragma unroll 1
+        for (int kb = 0; kb < blocks; kb += 2) {    // behind the last block all are zeros
+            const bool more = kb + 2 < blocks;
+            if (AHEAD && (kb + 8) * GP_K < K) {
+#pragma unroll
+                for (int i = 0; i < LINES; ++i)
+                    if (line[i]) asm volatile("prefetch.global.L2 [%0];" ::"l"(line[i] + (kb + 8) * GP_K));
+            }
+            if (more) fetch(kb + 2);
+            if (works) multiply(kb, gc);
+            if (more) {
+                put(kb + 2);
+                fetch(kb + 3);
+            }
+            if (works && kb + 1 < blocks) multiply(kb + 1, gc);
+            if (more) put(kb + 3);
+            __syncthreads();
+        }
+    };
+    // the wide form's warps have all the block's rows, and the same ones: 16 or 32 of them where there are no more
+    if (TM == 16 && m0 + 16 >= M) walk(std::integral_constant<int, 1>());
+    else if (TM == 16 && m0 + 32 >= M) walk(std::integral_constant<int, 2>());
+    else walk(std::integral_constant<int, TM / 4>());
+    const bool wide = sizeof(OT) == 4 && ldc % 4 == 0 && (((size_t)C) & 15) == 0;
+    const int n = n0 + ln;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + lm + (i >> 2) * 16 + (i & 3);
         if (m >= M) continue;
+        float o[TN];
 #pragma unroll
-        for (int j = 0; j < GT_TN; ++j) {
-            const int n = n0 + ln + 8 * j;
-            if (n < N) C[(size_t)m * ldc + n] = from_f32<OT>(acc[i][j]);
+        for (int j = 0; j < TN; ++j) o[j] = __uint_as_float((i & 1) ? (unsigned)(acc[i >> 1][j] >> 32) : (unsigned)acc[i >> 1][j]);
+        OT* to = C + (size_t)m * ldc + n;
+        if (wide && n + TN <= N) {
+            *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < TN; ++j)
+                if (n + j < N) to[j] = from_f32<OT>(o[j]);
         }
     }
 }
 
-template <typename OT>
-static int gemm_f32_tiled(const float* A, const float* W, OT* C, const int* a_rows, const int* tile_w, int M, int N, int K,
+template <int TM, bool AHEAD, typename OT>
+static int gemm_f32_pairs(const float* A, const float* W, OT* C, const int* a_rows, const int* tile_w, int M, int N, int K,
                           int lda, int ldc, int batch, long long a_bs, long long w_bs, long long c_bs, cudaStream_t stream) {
-    constexpr int smem = GT_STAGES * (GT_M + GT_N) * GT_LD * 4;
-    dim3 grid((N + GT_N - 1) / GT_N, (M + GT_M - 1) / GT_M, batch);
+    constexpr int BN_ = 8 * TM, smem = 4 * GP_K * (GP_M + BN_) * 4;
+    dim3 grid((N + BN_ - 1) / BN_, (M + GP_M - 1) / GP_M, batch);
     if (grid.y > 65535 || batch > 65535) return AIE_UNSUPPORTED;
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_tiled_kernel<OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_f32_pairs_kernel<TM, AHEAD, OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    gemm_f32_tiled_kernel<OT><<<grid, GT_THREADS, smem, stream>>>(A, W, C, a_rows, tile_w, M, N, K, lda, ldc, a_bs, w_bs, c_bs);
+    gemm_f32_pairs_kernel<TM, AHEAD, OT><<<grid, GP_THREADS, smem, stream>>>(A, W, C, a_rows, tile_w, M, N, K, lda, ldc, a_bs, w_bs, c_bs);
     AIE_LAUNCH_CHECK();
+}
+
+// Which form: rounds of blocks over the SMs, a last tile of rows counted by what it takes (in tenths, measured at 1, 33 and 64
+// rows) and a tenth of a round let off.  At 2,048 of K a block an SM takes 50 us beside others in the narrow form and 86 in
+// the wide one, and 10 and 24 more the first time.  Measured at 66 sizes (1 .. 2,048 rows, six weights) the rule's choice is
+// the fastest of the three or within 4 % of it, 7 % at 257 rows of 2,048 columns.
+template <typename OT>
+static int gemm_f32_aligned(const float* A, const float* W, OT* C, const int* a_rows, const int* tile_w, int M, int N, int K,
+                            int lda, int ldc, int batch, long long a_bs, long long w_bs, long long c_bs, cudaStream_t st) {
+    const int rest = M % GP_M;
+    const auto rounds = [&](int columns, int last) {
+        const long long tenths = (long long)batch * ((N + columns - 1) / columns) * (10 * (M / GP_M) + last);
+        return (tenths + 9 * 148 - 1) / (10 * 148) + ((tenths + 9 * 148 - 1) < 10 * 148);
+    };
+    const long long narrow = rounds(64, rest == 0 ? 0 : rest <= 32 ? 6 : 10);
+    const long long wide = rounds(128, rest == 0 ? 0 : rest <= 16 ? 4 : rest <= 32 ? 6 : 10);
+#define GO(TM, AHEAD) return gemm_f32_pairs<TM, AHEAD, OT>(A, W, C, a_rows, tile_w, M, N, K, lda, ldc, batch, a_bs, w_bs, c_bs, st)
+    if (7 * wide + 2 < 4 * narrow + 1) GO(16, false);
+    if (narrow == 1) GO(8, true);
+    GO(8, false);
+#undef GO
 }
 
 // The general form.  A [M, lda] (float32 or bfloat16, widened on load), W [N, K], C [M, ldc] (float32 or
@@ -238,11 +323,11 @@ extern "C" int aie_gemm_f32_ex(const void* A, int a_dtype, const void* W, int w_
     if (a_dtype == AIE_F32 && w_dtype == AIE_F32 && K % 4 == 0 && lda % 4 == 0 && a_bs % 4 == 0 && w_bs % 4 == 0 &&
         !(((size_t)A | (size_t)W) & 15)) {
         if (c_dtype == AIE_F32)
-            return gemm_f32_tiled<float>((const float*)A, (const float*)W, (float*)C, a_rows, tile_w, M, N, K, lda, ldc, batch,
-                                         a_bs, w_bs, c_bs, stream);
+            return gemm_f32_aligned<float>((const float*)A, (const float*)W, (float*)C, a_rows, tile_w, M, N, K, lda, ldc, batch,
+                                           a_bs, w_bs, c_bs, stream);
         if (c_dtype == AIE_BF16)
-            return gemm_f32_tiled<bf16>((const float*)A, (const float*)W, (bf16*)C, a_rows, tile_w, M, N, K, lda, ldc, batch,
-                                        a_bs, w_bs, c_bs, stream);
+            return gemm_f32_aligned<bf16>((const float*)A, (const float*)W, (bf16*)C, a_rows, tile_w, M, N, K, lda, ldc, batch,
+                                          a_bs, w_bs, c_bs, stream);
     }
 #define GO(AT, WT) return gemm_f32_go<AT, WT>(A, W, C, c_dtype, a_rows, tile_w, M, N, K, lda, ldc, batch, a_bs, w_bs, c_bs, stream)
     if (a_dtype == AIE_F32 && w_dtype == AIE_F32) GO(float, float);
