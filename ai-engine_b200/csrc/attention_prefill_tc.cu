@@ -30,10 +30,18 @@
 // The extended form (EXT) of this kernel adds, for layers that want them: a window (key tiles before it are never
 // loaded, nor are pages that the window has passed) that may keep the first keys, a factor a head and a distance bias on
 // the scores, a sink in the denominator, a gate a token and head, scores kept within +-cap by a tanh, probabilities that enter the
-// product with the values as two bfloat16 terms (the rounded one over the first half of the scores' columns, what
-// rounding left over the second: 16 bits of mantissa), a sigmoid gate on every output element, and cache rows
+// product with the values as two bfloat16 terms (of every 32 keys the rounded ones over the first 16 of the scores' columns,
+// what rounding left over the others: 16 bits of mantissa), a sigmoid gate on every output element, and cache rows
 // [k | v] or, with the values being the keys, [k] of one plane.  A portion of 1,900 tokens after 1,000 and a prompt of 148,
-// 16 heads of 128, window 1,024 with four kept keys, bias, sink and gates: 83 us (mma.sync kernel: 183 us).
+// 16 heads of 128, window 1,024 with four kept keys, bias, sink and gates: 62 us (82 with a thread a row; mma.sync kernel: 183 us).
+// Its softmax has eight warps, two threads a query row (64 keys each, their maxima exchanged in shared memory behind a barrier of the
+// two warps): what it does to a score is three to ten instructions more than in the plain form, and one warp a scheduler then
+// waited for its own results and for instructions (a row unrolled in 255 registers).  Cycles a key tile at heads of 128, by clock:
+// a thread a row in registers 4,200, the same in loops over 32 columns that read tensor memory twice 3,250, in one pass against
+// an older maximum 3,650, two threads a row 2,530 (670 up to the maximum, which the products' use of tensor memory stretches from
+// 260; 1,500 of exponentials, 1,024 the least; 330 to hand over).  Two query tiles a CTA as below: 2,630 a tile.  2,048
+// tokens after 6,000 on 32 heads 346 -> 318 us, with bounded scores 698 -> 509; 2,048 after 1,024 on 16 heads with keys of 192 and a
+// window of 1,024: 69 -> 45.
 // The value rows of keys past the sequence's last token are zeroed in shared memory before the
 // last tile's P . V, so a probability of 0 never meets what an unwritten cache slot holds.
 // The softmax warps hand a tile's probabilities to the issuing warp at a named hardware barrier (bar.arrive /
@@ -51,17 +59,21 @@
 #define AT_BAR_P 1            // named barriers 1, 2: the probabilities of an even / odd key tile are in tensor memory
                               // (two, because a softmax warp may be a tile ahead of another: its arrival for
                               // tile j + 1 must not count for tile j)
+// columns of the probabilities of keys 16 ks .. 16 ks + 15 (the extended form's second terms lie 16 further)
+#define AT_P_COL(ext, ks) (unsigned)((ext) ? 32 * ((ks) >> 1) + 8 * ((ks) & 1) : 8 * (ks))
+#define AT_EXT_THREADS 320      // the extended form: 8 softmax warps, two threads a query row
+#define AT_BAR_ROW 3          // ... whose two warps of the same 32 rows meet at named barriers 3 .. 6
 #define AT_RESCALE_STEP 8.0f     // a row's reference maximum moves in steps of more than this (log2 units)
 
 // HD: head size, HD / 64 halves of 64 columns.  A tile of 128 keys (or queries) holds 16 KB per half.
 // HQ: elements of queries and keys (HD those of values) when they differ.
-template <int HD, int HQ = HD> struct AtSmem {
+template <int HD, int HQ = HD, bool EXT = false> struct AtSmem {
     static constexpr int tile = HQ / 64 * AT_HALF_BYTES, v_tile = HD / 64 * AT_HALF_BYTES;
-    // [alignment slack | 1 KB: barriers | Q | K x NST | V x NST]
+    // [alignment slack | 1 KB: barriers (the extended form: 2 KB, what a row's threads tell one another behind them) | Q | K x NST | V x NST]
     // rings of NST key tiles and NST value tiles: as deep as 227 KB allow (3 at head size 128), because a
     // tile is requested when its buffer is freed and a ring of two leaves the products waiting for loads
     static constexpr int NST = HQ > 128 ? 2 : (HD >= 128 ? 3 : 4);
-    static constexpr int q_off = 1024, k_off = q_off + tile, v_off = k_off + NST * tile, end = v_off + NST * v_tile;
+    static constexpr int q_off = EXT ? 2048 : 1024, k_off = q_off + tile, v_off = k_off + NST * tile, end = v_off + NST * v_tile;
     static constexpr int bytes = 1024 + end;
 };
 
@@ -151,8 +163,112 @@ __device__ __forceinline__ float at_hi(unsigned long long v) {
                    "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),   \
                    "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory")
 
+// What the softmax of the extended form does to 32 scores of one row, in registers (columns 32 c .. 32 c + 31 of a key tile whose
+// first key is `kbase`; sv holds them as they come from tensor memory).
+struct AtShape {
+    float z_of, m2, slope2;      // factor below the tanh (capped), factor and bias of the scores (shaped)
+    bool capped, shaped;
+    int qpos, low, low_last, keep_first, p_first;      // masks; low_last, p_first: the last row's `low`, the first row's position
+};
+__device__ __forceinline__ void at_tanh32(unsigned (&sv)[32], float z_of) {      // s <- tanh(s z_of)
+    float big = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) big = at_max3(big, fabsf(__uint_as_float(sv[i])), fabsf(__uint_as_float(sv[i + 1])));
+    if (__all_sync(0xffffffffu, big * fabsf(z_of) <= 1.f)) {
+        constexpr float tc[8] = AT_TANH_COEFS;
+        const unsigned long long zz = at_pack2(z_of, z_of);
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+            const unsigned long long z = at_mul2(at_pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), zz);
+            const unsigned long long y = at_mul2(z, z);
+            unsigned long long p = at_pack2(tc[7], tc[7]);
+#pragma unroll
+            for (int c = 6; c >= 0; --c) p = at_fma2(p, y, at_pack2(tc[c], tc[c]));
+            p = at_mul2(p, z);
+            sv[i] = __float_as_uint(at_lo(p));
+            sv[i + 1] = __float_as_uint(at_hi(p));
+        }
+    } else {
+        const float k2 = 2.f * 1.4426950408889634f * z_of;      // tanh(z) = 1 - 2 / (1 + 2^(2 z log2 e))
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            float e, q;
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__uint_as_float(sv[i]) * k2));
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(1.f + e));
+            sv[i] = __float_as_uint(fmaf(-2.f, q, 1.f));
+        }
+    }
+}
+__device__ __forceinline__ void at_shape32(unsigned (&sv)[32], const AtShape& a, int key0) {
+    if (a.shaped) {
+        const unsigned long long off2 = at_pack2((float)(key0 - a.qpos), (float)(key0 - a.qpos));
+        const unsigned long long m2 = at_pack2(a.m2, a.m2), b2 = at_pack2(a.slope2, a.slope2);
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+            unsigned long long dist;            // j - i, exact
+            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(dist) : "l"(off2), "l"(at_pack2((float)i, (float)(i + 1))));
+            const unsigned long long x = at_fma2(at_pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), m2, at_mul2(dist, b2));
+            sv[i] = __float_as_uint(at_lo(x));
+            sv[i + 1] = __float_as_uint(at_hi(x));
+        }
+    }
+    if (__builtin_expect(key0 + 31 > a.p_first, 0)) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (key0 + i > a.qpos) sv[i] = 0xff800000u;      // -inf: not visible
+    }
+    if (__builtin_expect(key0 < a.low_last, 0)) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (key0 + i < a.low && key0 + i >= a.keep_first) sv[i] = 0xff800000u;
+    }
+}
+// 32 columns on their way out of tensor memory have landed (the registers are named so that nothing reads them before)
+#define AT_LANDED32(v)                                                                                                \
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n"                                                                   \
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),    \
+                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), \
+                   "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), \
+                   "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])  \
+                 :: "memory")
+__device__ __forceinline__ float at_scores32(unsigned (&sv)[32], const AtShape& a, int key0) {      // ... their largest
+    if (__builtin_expect(a.capped, 0)) at_tanh32(sv, a.z_of);
+    at_shape32(sv, a, key0);
+    float m0 = -INFINITY, m1 = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+        m0 = at_max3(m0, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+        m1 = at_max3(m1, __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]));
+    }
+    return fmaxf(m0, m1);
+}
+// Probabilities 2^(s sl2 - m) of 32 keys as two bfloat16 terms over the scores they come from: the rounded ones in the first 16
+// columns, what rounding left in the others, two keys to a column.  They are added to sum_a and sum_b (packed halves).
+__device__ __forceinline__ void at_exp32(const unsigned (&sv)[32], unsigned taddr, float sl2, float m, unsigned long long& sum_a,
+                                         unsigned long long& sum_b) {
+    const unsigned long long sl2_2 = at_pack2(sl2, sl2), negm_2 = at_pack2(-m, -m), minus = at_pack2(-1.f, -1.f);
+    unsigned p[32];
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+        const unsigned long long x2 = at_fma2(at_pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), sl2_2, negm_2);
+        float e0, e1;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(at_lo(x2)));
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(at_hi(x2)));
+        const unsigned long long e2 = at_pack2(e0, e1);
+        if (i & 2) asm("add.rn.f32x2 %0, %1, %2;" : "=l"(sum_b) : "l"(sum_b), "l"(e2));
+        else asm("add.rn.f32x2 %0, %1, %2;" : "=l"(sum_a) : "l"(sum_a), "l"(e2));
+        const __nv_bfloat162 bb = __floats2bfloat162_rn(e0, e1);
+        const float2 f = __bfloat1622float2(bb);
+        const unsigned long long left = at_fma2(at_pack2(f.x, f.y), minus, e2);
+        const __nv_bfloat162 rr = __floats2bfloat162_rn(at_lo(left), at_hi(left));
+        p[i >> 1] = *reinterpret_cast<const unsigned*>(&bb);
+        p[16 + (i >> 1)] = *reinterpret_cast<const unsigned*>(&rr);
+    }
+    AT_ST32(p, taddr);
+}
+
 template <int HD, bool EXT, int HQ = HD>
-__global__ void __launch_bounds__(AT_THREADS, 1)
+__global__ void __launch_bounds__(EXT ? AT_EXT_THREADS : AT_THREADS, 1)
 paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, bf16* __restrict__ out,
                         const int* __restrict__ tiles, int n_tiles, const int* __restrict__ q_start,
@@ -162,9 +278,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     extern __shared__ unsigned char at_raw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>(((size_t)at_raw + 1023) & ~(size_t)1023);
     unsigned long long* q_full = reinterpret_cast<unsigned long long*>(sm);
-    constexpr int NST = AtSmem<HD, HQ>::NST;           // stages of the key ring and of the value ring
-    unsigned long long* kv_full = q_full + 1;      // [NST] keys and values of a tile have landed
-    unsigned long long* k_empty = kv_full + NST;   // [NST] the scores have read the keys
+    constexpr int NST = AtSmem<HD, HQ, EXT>::NST;           // stages of the key ring and of the value ring
+    unsigned long long* kv_full = q_full + 1;      // [NST] keys and values of a tile have landed (extended form: the keys)
+    unsigned long long* v_full = kv_full + NST;    // [NST] extended form: the values of a tile have landed
+    unsigned long long* k_empty = v_full + NST;    // [NST] the scores have read the keys
     unsigned long long* v_empty = k_empty + NST;   // [NST] P . V has read the values
     unsigned long long* s_full = v_empty + NST;    // [2] score buffers
     unsigned long long* p_ready = s_full + 2;
@@ -175,14 +292,20 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                                                    // may come here while that one is still to be issued
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_last + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    float(*row_x)[AT_M] = reinterpret_cast<float(*)[AT_M]>(sm + 1024);      // (extended form) what a row's two threads tell one another
     constexpr int HV = HD / 64, HK = HQ / 64;      // halves of 64 columns of values, of queries and keys
-    constexpr int KTILE = AtSmem<HD, HQ>::tile, TILE = AtSmem<HD, HQ>::v_tile;      // bytes of a 128-row tile of keys, of values
+    constexpr int KTILE = AtSmem<HD, HQ, EXT>::tile, TILE = AtSmem<HD, HQ, EXT>::v_tile;      // bytes of a 128-row tile of keys, of values
     constexpr int KGROUP = HK * 1024, GROUP = HV * 1024;      // bytes of 8 rows (all halves) of a key tile, of a value tile
-    unsigned char* q_s = sm + AtSmem<HD, HQ>::q_off;
-    unsigned char* k_s = sm + AtSmem<HD, HQ>::k_off;   // stage st at + st * KTILE
-    unsigned char* v_s = sm + AtSmem<HD, HQ>::v_off;   // ... + st * TILE
+    unsigned char* q_s = sm + AtSmem<HD, HQ, EXT>::q_off;
+    unsigned char* k_s = sm + AtSmem<HD, HQ, EXT>::k_off;   // stage st at + st * KTILE
+    unsigned char* v_s = sm + AtSmem<HD, HQ, EXT>::v_off;   // ... + st * TILE
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (EXT && tid == 0) {
+        tma_prefetch_map(&map_q);
+        tma_prefetch_map(&map_k);
+        tma_prefetch_map(&map_v);
+    }
     // later tiles hold more keys: start them first, for all heads (heads run fastest in the grid, so the heads
     // of a group, which read the same keys, start side by side)
     const int tile_i = n_tiles - 1 - (int)blockIdx.y;
@@ -205,6 +328,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         mbar_init(q_full, 1);
         for (int s = 0; s < NST; ++s) {
             mbar_init(&kv_full[s], 1);
+            mbar_init(&v_full[s], 1);
             mbar_init(&k_empty[s], 1);
             mbar_init(&v_empty[s], 1);
         }
@@ -266,33 +390,52 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             if (have && !valid) atomicOr(err, AIE_DEV_PAGE_OOB);
             // a missing page is flagged; page 0 stands in for it so that the byte count of the barrier holds
             const int group0 = (((valid ? page : 0) * K + kvh) << lp) >> 3;     // first group of 8 rows of the page
-            // one barrier counts the bytes of the tile's keys and values: the products wait once per tile
-            if (lane == 0) {
-                const unsigned ph = ((j / NST) & 1) ^ 1;
-                ok = mbar_wait(&k_empty[st], ph, abort_flag, err) && mbar_wait(&v_empty[st], ph, abort_flag, err);
-                if (ok && !missing) mbar_expect_tx(&kv_full[st], (unsigned)n_pages * (unsigned)P * (unsigned)((HQ + HD) * 2));
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (!ok) break;
-            if (EXT && missing) {
-                // the value rows of pages that are not loaded are zeroed before the tile's barrier is armed (their
-                // scores are masked, whatever the keys' places hold)
-                for (; missing; missing &= missing - 1) {
-                    const int r0 = (__ffs(missing) - 1) * P;
-                    for (int i = lane; i < P * HV * 8; i += 32) {
-                        const int row = r0 + i / (HV * 8), c = i % (HV * 8);
-                        *reinterpret_cast<uint4*>(v_s + st * TILE + (row >> 3) * GROUP + (c >> 3) * 1024 + (row & 7) * 128 + (c & 7) * 16) =
-                            make_uint4(0, 0, 0, 0);
-                    }
+            if constexpr (EXT) {
+                // keys and values each when their place is free: the keys of a tile are wanted a softmax before its values, and
+                // their place is free a softmax before (one barrier for both: 3,440 cycles a tile at keys of 192, 1,350 of
+                // them between the place of the values and the keys' arrival)
+                const unsigned ph = ((j / NST) & 1) ^ 1, bytes = (unsigned)(n_pages - n_lost) * (unsigned)P * 2u;
+                if (lane == 0) {
+                    ok = mbar_wait(&k_empty[st], ph, abort_flag, err);
+                    if (ok) mbar_expect_tx(&kv_full[st], bytes * HQ);
                 }
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (!ok) break;
+                if (have) tma_load_4d(k_s + st * KTILE + lane * P * (HQ * 2), &map_k, &kv_full[st], 0, 0, blk_k, group0);
                 __syncwarp();
-                if (lane == 0) mbar_expect_tx(&kv_full[st], (unsigned)(n_pages - n_lost) * (unsigned)P * (unsigned)((HQ + HD) * 2));
+                if (lane == 0) ok = mbar_wait(&v_empty[st], ph, abort_flag, err);
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (!ok) break;
+                if (missing) {
+                    // the value rows of pages that are not loaded are zeroed before the tile's barrier is armed (their
+                    // scores are masked, whatever the keys' places hold)
+                    for (; missing; missing &= missing - 1) {
+                        const int r0 = (__ffs(missing) - 1) * P;
+                        for (int i = lane; i < P * HV * 8; i += 32) {
+                            const int row = r0 + i / (HV * 8), c = i % (HV * 8);
+                            *reinterpret_cast<uint4*>(v_s + st * TILE + (row >> 3) * GROUP + (c >> 3) * 1024 + (row & 7) * 128 + (c & 7) * 16) =
+                                make_uint4(0, 0, 0, 0);
+                        }
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    __syncwarp();
+                }
+                if (lane == 0) mbar_expect_tx(&v_full[st], bytes * HD);
                 __syncwarp();
-            }
-            if (have) {
-                tma_load_4d(k_s + st * KTILE + lane * P * (HQ * 2), &map_k, &kv_full[st], 0, 0, blk_k, group0);
-                tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &kv_full[st], 0, 0, blk_v, group0);
+                if (have) tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &v_full[st], 0, 0, blk_v, group0);
+            } else {
+                // one barrier counts the bytes of the tile's keys and values: the products wait once per tile
+                if (lane == 0) {
+                    const unsigned ph = ((j / NST) & 1) ^ 1;
+                    ok = mbar_wait(&k_empty[st], ph, abort_flag, err) && mbar_wait(&v_empty[st], ph, abort_flag, err);
+                    if (ok) mbar_expect_tx(&kv_full[st], (unsigned)n_pages * (unsigned)P * (unsigned)((HQ + HD) * 2));
+                }
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                if (!ok) break;
+                if (have) {
+                    tma_load_4d(k_s + st * KTILE + lane * P * (HQ * 2), &map_k, &kv_full[st], 0, 0, blk_k, group0);
+                    tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &kv_full[st], 0, 0, blk_v, group0);
+                }
             }
             __syncwarp();
             page = page_next;
@@ -304,7 +447,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             const int first_bad = p_last + 1 - tile_of(j) * AT_N;       // rows [first_bad, 128) are not keys
             bool ok2 = true;
             if (first_bad < AT_N) {
-                if (lane == 0) ok2 = mbar_wait(&kv_full[st], (j / NST) & 1, abort_flag, err);
+                if (lane == 0) ok2 = ok && mbar_wait(EXT ? &v_full[st] : &kv_full[st], (j / NST) & 1, abort_flag, err);
                 ok2 = __shfl_sync(0xffffffffu, ok2 ? 1 : 0, 0) != 0;
                 if (ok2) {
                     unsigned char* vd = v_s + st * TILE;
@@ -321,7 +464,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             if (lane == 0) mbar_arrive_plain(v_fixed);
         }
     } else if (warp == 1) {
-        // the whole warp walks the tiles (it meets the softmax warps at a named barrier); lane 0 issues
+        // the whole warp walks the tiles (it meets the softmax warps at a named barrier); one lane issues
         {
             const unsigned idesc_s = umma_idesc(AT_N), idesc_o = umma_idesc(HD, true);
             // descriptors of the first step of each operand, built once; a step or a stage further along is an
@@ -338,8 +481,9 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 umma_commit(&k_empty[st]);
                 umma_commit(&s_full[j & 1]);
             };
-            bool ok = true;                 // lane 0's; once false, the warp only keeps its appointments at the barrier
-            if (lane == 0) {
+            const bool lead = tc_elect();
+            bool ok = true;                 // that lane's; once false, the warp only keeps its appointments at the barrier
+            if (lead) {
                 ok = mbar_wait(q_full, 0, abort_flag, err);
                 if (ok) ok = mbar_wait(&kv_full[0], 0, abort_flag, err);
                 if (ok) {
@@ -350,7 +494,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             int st = 0, ph = 0;             // stage and phase of tile j in the rings
             for (int j = 0; j < n_kt; ++j) {
                 const int st1 = st + 1 == NST ? 0 : st + 1, ph1 = st + 1 == NST ? ph ^ 1 : ph;      // of tile j + 1
-                if (lane == 0 && ok && j + 1 < n_kt) {
+                if (lead && ok && j + 1 < n_kt) {
                     // the next tile's scores, while this tile's softmax runs.  They go over the P of tile
                     // j - 1, which the P . V issued before them has read: the tensor pipe runs what one thread
                     // issues in order.
@@ -360,15 +504,16 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                         issue_scores(j + 1, st1);
                     }
                 }
-                if (lane == 0 && ok && j == n_kt - 1) ok = mbar_wait(v_fixed, 0, abort_flag, err);
+                if (EXT && lead && ok) ok = mbar_wait(&v_full[st], ph, abort_flag, err);
+                if (lead && ok && j == n_kt - 1) ok = mbar_wait(v_fixed, 0, abort_flag, err);
                 // the tile's probabilities are written: the 128 softmax threads arrive, this warp waits.  A hardware
                 // barrier: an mbarrier test costs the issuing thread some hundred cycles while the tensor pipe reads
                 // shared memory, and this hand-over is on the tile's critical path (P . V, then the scores of the tile
                 // after the next, which the softmax warps wait for).  (The tile's values landed with its keys.)
-                asm volatile("bar.sync %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"(AT_M + 32) : "memory");
+                asm volatile("bar.sync %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"((EXT ? 2 : 1) * AT_M + 32) : "memory");
                 st = st1;
                 ph = ph1;
-                if (lane != 0 || !ok) continue;
+                if (!lead || !ok) continue;
                 const int st0 = st == 0 ? NST - 1 : st - 1;      // the stage of tile j again
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 // O += P . V over 128 keys: 8 steps of 16 keys; P is in tensor memory (two keys to a column),
@@ -377,12 +522,12 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 const unsigned tp = tmem_base + (unsigned)((j & 1) * AT_N);
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks)
-                    umma_a_tmem(tmem_base + 256u, tp + (unsigned)(ks * 8), dv + (unsigned long long)((ks * 2 * GROUP) >> 4),
+                    umma_a_tmem(tmem_base + 256u, tp + AT_P_COL(EXT, ks), dv + (unsigned long long)((ks * 2 * GROUP) >> 4),
                                 idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
                 if (EXT) {
 #pragma unroll
                     for (int ks = 0; ks < 8; ++ks)           // what rounding left of the probabilities
-                        umma_a_tmem(tmem_base + 256u, tp + 64u + (unsigned)(ks * 8),
+                        umma_a_tmem(tmem_base + 256u, tp + 16u + AT_P_COL(EXT, ks),
                                     dv + (unsigned long long)((ks * 2 * GROUP) >> 4), idesc_o, 1u);
                 }
                 umma_commit(&v_empty[st0]);
@@ -400,194 +545,235 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
         const bool capped = EXT && ext.cap > 0.f;
         const float scale_h = EXT && ext.temp ? scale * ext.temp[h] : scale;
         const float sl2 = capped ? ext.cap * log2e : scale_h * log2e;      // scores in units of log2(e): exp2 below
-        const float z_of = capped ? scale_h / ext.cap : 0.f, z_abs = fabsf(z_of);
+        const float z_of = capped ? scale_h / ext.cap : 0.f;
         // with a bias or a factor of its own, a head's scores are brought to those units before their maximum is taken
         const bool shaped = EXT && (ext.slope || ext.temp);
         const float slope2 = EXT && ext.slope ? ext.slope[h] * log2e : 0.f, sl2_e = shaped ? 1.f : sl2;
         const int low = EXT && ext.window > 0 ? qpos - ext.window + 1 : 0;      // first key this row reads
         const int low_last = EXT && ext.window > 0 ? p_last - ext.window + 1 : 0;
-        float m_run = -INFINITY, l_run = 0.f;
-        bool ok = true;
-        for (int j = 0; j < n_kt; ++j) {
-            // (a warp that gave up still arrives at the barrier for every tile: the issuing warp waits there
-            // without a limit)
-            const unsigned tmem_s = tmem_base + (unsigned)((j & 1) * AT_N);
+        const AtShape shape{z_of, sl2, slope2, capped, shaped, qpos, low, low_last, ext.keep_first, p0};
+        if constexpr (EXT) {
+            // two threads a query row: half 0 takes the first 64 keys of a tile and the first half of the output's columns.  One warp a
+            // scheduler (a thread a row) spent two thirds of its time waiting for its own instructions: 3,250 cycles a tile.
+            const int half = (warp - 2) >> 2;
+            float m_run = -INFINITY, l_run = 0.f;
+            bool ok = true;
+            for (int j = 0; j < n_kt; ++j) {
+                // (a warp that gave up still meets the others at both barriers for every tile: they wait there without a limit)
+                const unsigned ts = tmem_base + (unsigned)((j & 1) * AT_N + half * 64) + lane_addr;
+                if (ok) {
+                    if (lane == 0) ok = mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag, err);
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                }
+                unsigned sa[32], sb[32];
+                const int key0 = tile_of(j) * AT_N + half * 64;
+                if (ok) {
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    AT_LD32(sa, ts);
+                    AT_LD32(sb, ts + 32u);
+                    AT_LANDED32(sa);
+                    AT_LANDED32(sb);
+                    row_x[half][row] = fmaxf(at_scores32(sa, shape, key0), at_scores32(sb, shape, key0 + 32)) * sl2_e;
+                }
+                asm volatile("bar.sync %0, 64;\n" ::"r"(AT_BAR_ROW + quarter) : "memory");
+                const float tmax = fmaxf(row_x[0][row], row_x[1][row]);
+                asm volatile("bar.sync %0, 64;\n" ::"r"(AT_BAR_ROW + quarter) : "memory");      // both have read
+                if (ok) {
+                    // the row's reference maximum moves only by more than AT_RESCALE_STEP
+                    float m_new = m_run, corr = 1.0f;
+                    if (tmax > m_run + AT_RESCALE_STEP) {
+                        m_new = tmax;
+                        corr = (m_run == -INFINITY) ? 0.f : exp2f(m_run - tmax);
+                    }
+                    const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+                    m_run = m_new;
+                    // rows whose reference maximum moved rescale their row of O once the previous P . V has landed
+                    if (j > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
+                        if (lane == 0) ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, err);
+                        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll 1
+                        for (int c0 = half * (HD / 2); ok && c0 < (half + 1) * (HD / 2); c0 += 32) {
+                            unsigned ov[32];
+                            AT_LD32(ov, tmem_o + lane_addr + (unsigned)c0);
+                            AT_LANDED32(ov);
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+                            AT_ST32(ov, tmem_o + lane_addr + (unsigned)c0);
+                        }
+                    }
+                    unsigned long long sum_a = 0ull, sum_b = 0ull;
+                    at_exp32(sa, ts, sl2_e, m_use, sum_a, sum_b);
+                    at_exp32(sb, ts + 32u, sl2_e, m_use, sum_a, sum_b);
+                    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(sum_a) : "l"(sum_a), "l"(sum_b));
+                    l_run = l_run * corr + (at_lo(sum_a) + at_hi(sum_a));
+                    asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                }
+                asm volatile("bar.arrive %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"(2 * AT_M + 32) : "memory");
+            }
+            row_x[half][row] = l_run;
+            asm volatile("bar.sync %0, 64;\n" ::"r"(AT_BAR_ROW + quarter) : "memory");
+            l_run = row_x[0][row] + row_x[1][row];
+            // the last P . V, then this row of O divided by the row's sum
             if (ok) {
-                if (lane == 0) ok = mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag, err);
+                if (lane == 0) ok = mbar_wait(o_last, 0, abort_flag, err);
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             }
-            if (!ok) {
-                asm volatile("bar.arrive %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"(AT_M + 32) : "memory");
-                continue;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const int kbase = tile_of(j) * AT_N;
-            const bool edge = kbase + AT_N - 1 > p0;     // the tile touches the diagonal or the sequence's end
-            // the row of scores in registers (all four loads in flight at once), masked; its maximum
-            unsigned sv[128];
-            AT_LD32((sv + 0), tmem_s + lane_addr + 0);
-            AT_LD32((sv + 32), tmem_s + lane_addr + 32);
-            AT_LD32((sv + 64), tmem_s + lane_addr + 64);
-            AT_LD32((sv + 96), tmem_s + lane_addr + 96);
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            if (capped) {
-                // s <- tanh(s scale / cap), times cap where the exponent is made
-                float big = 0.f;
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                if (ext.sink) l_run += exp2f(ext.sink[h] * log2e - m_run);
+                float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+                if (ext.gate && row < rows_valid) inv *= ext.gate[(size_t)(t0 + row) * H + h];
+                bf16* dst = out + ((size_t)(t0 + row) * H + h) * HD;
+#pragma unroll 1
+                for (int c0 = half * (HD / 2); c0 < (half + 1) * (HD / 2); c0 += 32) {
+                    unsigned ov[32];
+                    AT_LD32(ov, tmem_o + lane_addr + (unsigned)c0);
+                    AT_LANDED32(ov);
+                    if (ext.gate_logits && row < rows_valid) {
+                        const float4* gl = reinterpret_cast<const float4*>(ext.gate_logits + (size_t)(t0 + row) * ext.ld_gate + (size_t)h * HD + c0);
 #pragma unroll
-                for (int i = 0; i < 128; i += 2)
-                    big = at_max3(big, fabsf(__uint_as_float(sv[i])), fabsf(__uint_as_float(sv[i + 1])));
-                if (__all_sync(0xffffffffu, big * z_abs <= 1.f)) {
-                    constexpr float tc[8] = AT_TANH_COEFS;
-                    const unsigned long long zz = at_pack2(z_of, z_of);
-#pragma unroll
-                    for (int i = 0; i < 128; i += 2) {
-                        const unsigned long long z = at_mul2(at_pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), zz);
-                        const unsigned long long y = at_mul2(z, z);
-                        unsigned long long p = at_pack2(tc[7], tc[7]);
-#pragma unroll
-                        for (int c = 6; c >= 0; --c) p = at_fma2(p, y, at_pack2(tc[c], tc[c]));
-                        p = at_mul2(p, z);
-                        sv[i] = __float_as_uint(at_lo(p));
-                        sv[i + 1] = __float_as_uint(at_hi(p));
+                        for (int i = 0; i < 8; ++i) {
+                            const float4 g = gl[i];
+                            ov[4 * i] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i]), 1.f + __expf(-g.x)));
+                            ov[4 * i + 1] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i + 1]), 1.f + __expf(-g.y)));
+                            ov[4 * i + 2] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i + 2]), 1.f + __expf(-g.z)));
+                            ov[4 * i + 3] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i + 3]), 1.f + __expf(-g.w)));
+                        }
                     }
-                } else {
-                    const float k2 = 2.f * log2e * z_of;      // tanh(z) = 1 - 2 / (1 + 2^(2 z log2 e))
+                    if (row < rows_valid) {
 #pragma unroll
-                    for (int i = 0; i < 128; ++i) {
-                        float e, q;
-                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__uint_as_float(sv[i]) * k2));
-                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(1.f + e));
-                        sv[i] = __float_as_uint(fmaf(-2.f, q, 1.f));
+                        for (int i = 0; i < 32; i += 8) {
+                            unsigned pk[4];
+#pragma unroll
+                            for (int e = 0; e < 8; e += 2) {
+                                __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(ov[i + e]) * inv,
+                                                                         __uint_as_float(ov[i + e + 1]) * inv);
+                                pk[e >> 1] = *reinterpret_cast<unsigned*>(&b);
+                            }
+                            *reinterpret_cast<uint4*>(dst + c0 + i) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                        }
                     }
                 }
             }
-            if (shaped) {
-                const unsigned long long off2 = at_pack2((float)(kbase - qpos), (float)(kbase - qpos));
-                const unsigned long long m2 = at_pack2(sl2, sl2), b2 = at_pack2(slope2, slope2);
-#pragma unroll
-                for (int i = 0; i < 128; i += 2) {
-                    unsigned long long dist;            // j - i, exact
-                    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(dist) : "l"(off2), "l"(at_pack2((float)i, (float)(i + 1))));
-                    const unsigned long long x = at_fma2(at_pack2(__uint_as_float(sv[i]), __uint_as_float(sv[i + 1])), m2, at_mul2(dist, b2));
-                    sv[i] = __float_as_uint(at_lo(x));
-                    sv[i + 1] = __float_as_uint(at_hi(x));
+        } else {
+            float m_run = -INFINITY, l_run = 0.f;
+            bool ok = true;
+            for (int j = 0; j < n_kt; ++j) {
+                // (a warp that gave up still arrives at the barrier for every tile: the issuing warp waits there
+                // without a limit)
+                const unsigned tmem_s = tmem_base + (unsigned)((j & 1) * AT_N);
+                if (ok) {
+                    if (lane == 0) ok = mbar_wait(&s_full[j & 1], (j >> 1) & 1, abort_flag, err);
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 }
-            }
-            if (edge) {
-#pragma unroll
-                for (int i = 0; i < 128; ++i)
-                    if (kbase + i > qpos) sv[i] = 0xff800000u;      // -inf: not visible
-            }
-            if (EXT && kbase < low_last) {
-#pragma unroll
-                for (int i = 0; i < 128; ++i)
-                    if (kbase + i < low && kbase + i >= ext.keep_first) sv[i] = 0xff800000u;
-            }
-            float tmax = -INFINITY, tmax2 = -INFINITY;
-#pragma unroll
-            for (int i = 0; i < 128; i += 4) {
-                tmax = at_max3(tmax, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
-                tmax2 = at_max3(tmax2, __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]));
-            }
-            tmax = fmaxf(tmax, tmax2) * sl2_e;
-            // the row's reference maximum moves only by more than AT_RESCALE_STEP
-            float m_new = m_run, corr = 1.0f;
-            if (tmax > m_run + AT_RESCALE_STEP) {
-                m_new = tmax;
-                corr = (m_run == -INFINITY) ? 0.f : exp2f(m_run - tmax);
-            }
-            const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-            m_run = m_new;
-            // rows whose reference maximum moved rescale their row of O once the previous P . V has landed
-            if (j > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
-                if (lane == 0) ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, err);
-                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (!ok) {
                     asm volatile("bar.arrive %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"(AT_M + 32) : "memory");
                     continue;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const int kbase = tile_of(j) * AT_N;
+                const bool edge = kbase + AT_N - 1 > p0;     // the tile touches the diagonal or the sequence's end
+                // the row of scores in registers (all four loads in flight at once), masked; its maximum
+                unsigned sv[128];
+                AT_LD32((sv + 0), tmem_s + lane_addr + 0);
+                AT_LD32((sv + 32), tmem_s + lane_addr + 32);
+                AT_LD32((sv + 64), tmem_s + lane_addr + 64);
+                AT_LD32((sv + 96), tmem_s + lane_addr + 96);
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                if (edge) {
+#pragma unroll
+                    for (int i = 0; i < 128; ++i)
+                        if (kbase + i > qpos) sv[i] = 0xff800000u;      // -inf: not visible
+                }
+                float tmax = -INFINITY, tmax2 = -INFINITY;
+#pragma unroll
+                for (int i = 0; i < 128; i += 4) {
+                    tmax = at_max3(tmax, __uint_as_float(sv[i]), __uint_as_float(sv[i + 1]));
+                    tmax2 = at_max3(tmax2, __uint_as_float(sv[i + 2]), __uint_as_float(sv[i + 3]));
+                }
+                tmax = fmaxf(tmax, tmax2) * sl2;
+                // the row's reference maximum moves only by more than AT_RESCALE_STEP
+                float m_new = m_run, corr = 1.0f;
+                if (tmax > m_run + AT_RESCALE_STEP) {
+                    m_new = tmax;
+                    corr = (m_run == -INFINITY) ? 0.f : exp2f(m_run - tmax);
+                }
+                const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
+                m_run = m_new;
+                // rows whose reference maximum moved rescale their row of O once the previous P . V has landed
+                if (j > 0 && __any_sync(0xffffffffu, corr != 1.0f)) {
+                    if (lane == 0) ok = mbar_wait(o_done, (j - 1) & 1, abort_flag, err);
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                    if (!ok) {
+                        asm volatile("bar.arrive %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"(AT_M + 32) : "memory");
+                        continue;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+#pragma unroll
+                    for (int c0 = 0; c0 < HD; c0 += 32) {
+                        unsigned ov[32];
+                        AT_LD32(ov, tmem_o + lane_addr + c0);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
+                        AT_ST32(ov, tmem_o + lane_addr + c0);
+                    }
+                }
+                // probabilities exp2(s * sl2 - m), their sum, packed to bf16 and written over the scores, 32 columns
+                // at a time: two keys to a column, so the P of columns [32 c, 32 c + 32) lands on [16 c, 16 c + 16)
+                const unsigned long long sl2_2 = at_pack2(sl2, sl2), negm_2 = at_pack2(-m_use, -m_use);
+                unsigned long long psum2 = 0ull, psum2b = 0ull;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    unsigned pk[16];
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        unsigned long long x2;
+                        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x2) : "l"(at_pack2(__uint_as_float(sv[32 * c + i]), __uint_as_float(sv[32 * c + i + 1]))), "l"(sl2_2), "l"(negm_2));
+                        float e0, e1;
+                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(at_lo(x2)));
+                        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(at_hi(x2)));
+                        if (i & 2) asm("add.rn.f32x2 %0, %1, %2;" : "=l"(psum2b) : "l"(psum2b), "l"(at_pack2(e0, e1)));
+                        else asm("add.rn.f32x2 %0, %1, %2;" : "=l"(psum2) : "l"(psum2), "l"(at_pack2(e0, e1)));
+                        __nv_bfloat162 bb = __floats2bfloat162_rn(e0, e1);
+                        pk[i >> 1] = *reinterpret_cast<unsigned*>(&bb);
+                    }
+                    AT_ST16(pk, tmem_s + lane_addr + (unsigned)(16 * c));
+                }
+                asm("add.rn.f32x2 %0, %1, %2;" : "=l"(psum2) : "l"(psum2), "l"(psum2b));
+                l_run = l_run * corr + (at_lo(psum2) + at_hi(psum2));
+                asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                asm volatile("bar.arrive %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"(AT_M + 32) : "memory");
+            }
+            // the last P . V, then this row of O divided by the row's sum
+            if (ok) {
+                if (lane == 0) ok = mbar_wait(o_last, 0, abort_flag, err);
+                ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            }
+            if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                const float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
+                bf16* dst = out + ((size_t)(t0 + row) * H + h) * HD;
 #pragma unroll
                 for (int c0 = 0; c0 < HD; c0 += 32) {
                     unsigned ov[32];
                     AT_LD32(ov, tmem_o + lane_addr + c0);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    if (row < rows_valid) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * corr);
-                    AT_ST32(ov, tmem_o + lane_addr + c0);
-                }
-            }
-            // probabilities exp2(s * sl2 - m), their sum, packed to bf16 and written over the scores, 32 columns
-            // at a time: two keys to a column, so the P of columns [32 c, 32 c + 32) lands on [16 c, 16 c + 16)
-            const unsigned long long sl2_2 = at_pack2(sl2_e, sl2_e), negm_2 = at_pack2(-m_use, -m_use);
-            unsigned long long psum2 = 0ull, psum2b = 0ull;
+                        for (int i = 0; i < 32; i += 8) {
+                            unsigned pk[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                unsigned pk[16], pr[EXT ? 16 : 1];
-#pragma unroll
-                for (int i = 0; i < 32; i += 2) {
-                    unsigned long long x2;
-                    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x2) : "l"(at_pack2(__uint_as_float(sv[32 * c + i]), __uint_as_float(sv[32 * c + i + 1]))), "l"(sl2_2), "l"(negm_2));
-                    float e0, e1;
-                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(at_lo(x2)));
-                    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(at_hi(x2)));
-                    if (i & 2) asm("add.rn.f32x2 %0, %1, %2;" : "=l"(psum2b) : "l"(psum2b), "l"(at_pack2(e0, e1)));
-                    else asm("add.rn.f32x2 %0, %1, %2;" : "=l"(psum2) : "l"(psum2), "l"(at_pack2(e0, e1)));
-                    __nv_bfloat162 bb = __floats2bfloat162_rn(e0, e1);
-                    pk[i >> 1] = *reinterpret_cast<unsigned*>(&bb);
-                    if (EXT) {
-                        const float2 f = __bfloat1622float2(bb);
-                        __nv_bfloat162 rr = __floats2bfloat162_rn(e0 - f.x, e1 - f.y);
-                        pr[EXT ? i >> 1 : 0] = *reinterpret_cast<unsigned*>(&rr);
-                    }
-                }
-                AT_ST16(pk, tmem_s + lane_addr + (unsigned)(16 * c));
-                if constexpr (EXT) AT_ST16(pr, tmem_s + lane_addr + (unsigned)(64 + 16 * c));
-            }
-            asm("add.rn.f32x2 %0, %1, %2;" : "=l"(psum2) : "l"(psum2), "l"(psum2b));
-            l_run = l_run * corr + (at_lo(psum2) + at_hi(psum2));
-            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            asm volatile("bar.arrive %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"(AT_M + 32) : "memory");
-        }
-        // the last P . V, then this row of O divided by the row's sum
-        if (ok) {
-            if (lane == 0) ok = mbar_wait(o_last, 0, abort_flag, err);
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        }
-        if (ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            if (EXT && ext.sink) l_run += exp2f(ext.sink[h] * log2e - m_run);
-            float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
-            if (EXT && ext.gate && row < rows_valid) inv *= ext.gate[(size_t)(t0 + row) * H + h];
-            bf16* dst = out + ((size_t)(t0 + row) * H + h) * HD;
-#pragma unroll
-            for (int c0 = 0; c0 < HD; c0 += 32) {
-                unsigned ov[32];
-                AT_LD32(ov, tmem_o + lane_addr + c0);
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                if (EXT && ext.gate_logits && row < rows_valid) {
-                    const float4* gl = reinterpret_cast<const float4*>(ext.gate_logits + (size_t)(t0 + row) * ext.ld_gate + (size_t)h * HD + c0);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float4 g = gl[i];
-                        ov[4 * i] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i]), 1.f + __expf(-g.x)));
-                        ov[4 * i + 1] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i + 1]), 1.f + __expf(-g.y)));
-                        ov[4 * i + 2] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i + 2]), 1.f + __expf(-g.z)));
-                        ov[4 * i + 3] = __float_as_uint(__fdividef(__uint_as_float(ov[4 * i + 3]), 1.f + __expf(-g.w)));
-                    }
-                }
-                if (row < rows_valid) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        unsigned pk[4];
-#pragma unroll
-                        for (int e = 0; e < 8; e += 2) {
-                            __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(ov[i + e]) * inv,
-                                                                     __uint_as_float(ov[i + e + 1]) * inv);
-                            pk[e >> 1] = *reinterpret_cast<unsigned*>(&b);
+                            for (int e = 0; e < 8; e += 2) {
+                                __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(ov[i + e]) * inv,
+                                                                         __uint_as_float(ov[i + e + 1]) * inv);
+                                pk[e >> 1] = *reinterpret_cast<unsigned*>(&b);
+                            }
+                            *reinterpret_cast<uint4*>(dst + c0 + i) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                         }
-                        *reinterpret_cast<uint4*>(dst + c0 + i) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
                     }
                 }
             }
@@ -599,6 +785,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     if (*abort_flag && tid == 0) {      // give copies in flight a bounded time to land
         for (int s = 0; s < NST; ++s) {
             for (unsigned i = 0; i < (1u << 16) && !mbar_try_wait(&kv_full[s], 0) && !mbar_try_wait(&kv_full[s], 1); ++i) {}
+            for (unsigned i = 0; EXT && i < (1u << 16) && !mbar_try_wait(&v_full[s], 0) && !mbar_try_wait(&v_full[s], 1); ++i) {}
         }
     }
     __syncthreads();
@@ -1060,8 +1247,8 @@ static int launch_prefill_tc_rows(const void* q, const void* pages, void* out, c
     rc = tc_make_map_rows8(&mv, (const bf16*)pages + (tied ? 0 : HD), rows, HD / 64, P / 8, bytes);
     if (rc) return rc;
     auto kern = paged_prefill_tc_kernel<HD, true>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AtSmem<HD>::bytes);
-    launch_pdl(kern, dim3(H, n_tiles), dim3(AT_THREADS), AtSmem<HD>::bytes, stream, mq, mk, mv, (bf16*)out, tiles, n_tiles,
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AtSmem<HD, HD, true>::bytes);
+    launch_pdl(kern, dim3(H, n_tiles), dim3(AT_EXT_THREADS), AtSmem<HD, HD, true>::bytes, stream, mq, mk, mv, (bf16*)out, tiles, n_tiles,
                q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, H, K, scale, err, ext);
     AIE_LAUNCH_CHECK();
 }
@@ -1136,9 +1323,9 @@ extern "C" int aie_prefill_tc_expanded(const void* q, const void* rows_kv, long 
     }
     const AtExt ext{window, 0.f, nullptr, 0, 0, nullptr, nullptr, nullptr, sink ? sink + head0 : sink, row_tile};
     auto kern = paged_prefill_tc_kernel<HD, true, HQ>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AtSmem<HD, HQ>::bytes);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AtSmem<HD, HQ, true>::bytes);
     if (e != cudaSuccess) return (int)e;
-    launch_pdl(kern, dim3(heads, n_tiles), dim3(AT_THREADS), AtSmem<HD, HQ>::bytes, stream, mq, mk, mv, (bf16*)out + (size_t)head0 * HD, tiles, n_tiles,
+    launch_pdl(kern, dim3(heads, n_tiles), dim3(AT_EXT_THREADS), AtSmem<HD, HQ, true>::bytes, stream, mq, mk, mv, (bf16*)out + (size_t)head0 * HD, tiles, n_tiles,
                q_start, q_len, ctx_len, (const int*)nullptr, 0, (int)(rows / AT_N), AT_N, H, 1, scale, err, ext);
     AIE_LAUNCH_CHECK();
 }

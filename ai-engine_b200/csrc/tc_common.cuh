@@ -43,6 +43,19 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     return false;
 }
 
+// True in one lane of a converged warp.  Products are issued under this and not under `lane == 0`: the compiler knows that a
+// single thread runs then and keeps descriptors in uniform registers.  Cycles between two tcgen05.mma of one issuing thread (when
+// the tensor pipe itself takes fewer): 32 to 39; under `lane == 0` 60 with constant descriptors, 106 to 178 with computed ones.
+__device__ __forceinline__ bool tc_elect() {
+    unsigned p;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+
+// asks for a tensor map ahead of the first copy that uses it
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, unsigned long long* bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                  ::"r"(tc_smem(dst)), "l"(map), "r"(tc_smem(bar)), "r"(x), "r"(y) : "memory");
