@@ -7,8 +7,9 @@
 // Operands, terms and sums are those of the other kernel: C, B and x enter rounded to bfloat16, w * X, W and the state as
 // pairs of bfloat16 values, sums are float32.  Products run on mma.sync: a chunk's tiles are 64 x 64, W is made in the
 // registers that the scores come in and meets X from there.  Bound by the traffic of the states (32 KB a chunk and head
-// of 128 x 64, written, read, written and read again).  2,048 tokens x 64 heads in eight groups: 45 + 18 + 69 us, walked 260 us;
-// with a head a block, which reads B and C anew, 46 + 18 + 80 us.
+// of 128 x 64, written, read, written and read again).  2,048 tokens x 64 heads in eight groups: 35 + 17 + 62 us, walked 260 us;
+// 45 + 18 + 69 when results went four bytes at a time, the first warp made each head's decays while the others waited and the next
+// head's state was asked for only when it was wanted; then with a head a block, which reads B and C anew, 46 + 18 + 80 us.
 #include "attention_prefill.cuh"
 #include "chunk_find.cuh"
 
@@ -48,12 +49,13 @@ __device__ __forceinline__ void sp_load(bf16* dst, const float* src, size_t ld, 
     }
 }
 
-// step sizes and running sums of the log decays of a chunk's tokens (a token behind the end: no step, no decay); dt and la
-// hold 64 floats, done by the first warp, to be followed by a barrier
-__device__ __forceinline__ float sp_decays(const SpArgs& p, size_t a0, int nt, int h, float* dt, float* la) {
-    float end = 0.f;
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
+// step sizes and running sums of the log decays of a chunk's tokens (a token behind the end: no step, no decay) for the block's
+// heads, 64 floats each, a warp a head, to be followed by a barrier.  (By the first warp from head to head the others waited for it.)
+#define SP_HEADS 4          // heads a block takes at most
+__device__ __forceinline__ void sp_decays(const SpArgs& p, size_t a0, int nt, int h_first, float (*dts)[SP_T], float (*las)[SP_T]) {
+    if ((int)threadIdx.x < 32 * p.hpb) {
+        const int lane = threadIdx.x & 31, h = h_first + (threadIdx.x >> 5);
+        float *dt = dts[threadIdx.x >> 5], *la = las[threadIdx.x >> 5];
         const float rate = expf(p.a_log[h]), bias = p.dt_bias[h];
         float d[2];
 #pragma unroll
@@ -73,9 +75,7 @@ __device__ __forceinline__ float sp_decays(const SpArgs& p, size_t a0, int nt, i
         }
         la[2 * lane] = run - v1;
         la[2 * lane + 1] = run;
-        end = __shfl_sync(0xffffffffu, run, 31);
     }
-    return end;
 }
 __device__ __forceinline__ void sp_split(float a, float b, unsigned& hi, unsigned& lo) {
     hi = pack_bf16(a, b);
@@ -83,11 +83,15 @@ __device__ __forceinline__ void sp_split(float a, float b, unsigned& hi, unsigne
     lo = pack_bf16(a - f.x, b - f.y);
 }
 
-template <int NP>      // rows of the state, padded (zero rows change nothing); four blocks an SM: with three 53 instead of 45 us
+__device__ __forceinline__ void sp_copy(float* dst, const float* src, bool ok) {      // 16 bytes; zeros when not ok
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+template <int NP>      // rows of the state, padded (zero rows change nothing); four blocks an SM: with three a fifth slower
 __global__ void __launch_bounds__(SP_THREADS, 4) sp_chunk_kernel(SpArgs p) {
     extern __shared__ __align__(16) unsigned char sp_sm[];
     __shared__ int found[2];
-    __shared__ float dt[SP_T], la[SP_T];
+    __shared__ float dts[SP_HEADS][SP_T], las[SP_HEADS][SP_T];
     constexpr int LN = NP + 8, LD = 64 + 8;
     bf16* Bs = reinterpret_cast<bf16*>(sp_sm);         // [64][NP]
     bf16* XH = Bs + SP_T * LN;                         // [64][64] x, then w * X, rounded
@@ -98,15 +102,16 @@ __global__ void __launch_bounds__(SP_THREADS, 4) sp_chunk_kernel(SpArgs p) {
     if (r < 0) return;
     const int nt = min(SP_T, p.q_len[r] - c * SP_T);
     const size_t a0 = (size_t)p.q_start[r] + c * SP_T;
+    sp_decays(p, a0, nt, h_first, dts, las);
     sp_load<NP>(Bs, p.B + a0 * p.ld + (size_t)((p.head0 + h_first) / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
 #pragma unroll 1
     for (int h = h_first; h < h_first + p.hpb; ++h) {
         if (h > h_first) __syncthreads();                  // the last head's values are done with
         sp_load<64>(XH, p.X + a0 * p.ld + (size_t)h * p.dv + col0, p.ld, nt, p.dv - col0, p.vec);
-        const float end = sp_decays(p, a0, nt, h, dt, la);
-        if (tid == 0 && blockIdx.z == 0) p.G[(size_t)blockIdx.x * p.H + h] = expf(end);
         __syncthreads();
+        const float *dt = dts[h - h_first], *la = las[h - h_first];
         const float l_end = la[SP_T - 1];
+        if (tid == 0 && blockIdx.z == 0) p.G[(size_t)blockIdx.x * p.H + h] = expf(l_end);
 #pragma unroll
         for (int it = 0; it < SP_T * 32 / SP_THREADS; ++it) {
             const int i = tid + it * SP_THREADS, t = i >> 5, j = (i & 31) * 2;
@@ -147,6 +152,10 @@ __global__ void __launch_bounds__(SP_THREADS, 4) sp_chunk_kernel(SpArgs p) {
                 for (int e = 0; e < 2; ++e) {
                     const int n = m0 + (lane >> 2) + 8 * e, j = col0 + n0 + x * 8 + (lane & 3) * 2;
                     if (n >= p.N) continue;
+                    if (p.vec) {
+                        if (j < p.dv) *reinterpret_cast<float2*>(L + (size_t)n * p.dv + j) = make_float2(acc[x][2 * e], acc[x][2 * e + 1]);
+                        continue;
+                    }
                     if (j < p.dv) L[(size_t)n * p.dv + j] = acc[x][2 * e];
                     if (j + 1 < p.dv) L[(size_t)n * p.dv + j + 1] = acc[x][2 * e + 1];
                 }
@@ -211,19 +220,24 @@ template <int NP>
 __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
     extern __shared__ __align__(16) unsigned char sp_sm[];
     __shared__ int found[2];
-    __shared__ float dt[SP_T], la[SP_T];
+    __shared__ float dts[SP_HEADS][SP_T], las[SP_HEADS][SP_T];
     constexpr int LN = NP + 8, LD = 64 + 8;
     bf16* Cs = reinterpret_cast<bf16*>(sp_sm);         // [64][NP]
     bf16* Bs = Cs + SP_T * LN;                         // [64][NP]
     bf16* Xs = Bs + SP_T * LN;                         // [64][64]
     bf16* SH = Xs + SP_T * LD;                         // [NP][64]
     bf16* SL = SH + NP * LD;
+    // with `vec` the next head's state (over C and B, which live in registers then) and values, as they are in memory
+    float* St = reinterpret_cast<float*>(sp_sm);       // [NP][64]
+    float* Xt = reinterpret_cast<float*>(SL + NP * LD);        // [64][64]
+    static_assert(NP * 64 * 4 <= 2 * SP_T * LN * 2, "the state lies over C and B");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h_first = blockIdx.y * p.hpb, col0 = blockIdx.z * 64;
     int r, c;
     chunk_find<SP_T>(p.q_len, p.R, p.min_len, blockIdx.x, found, r, c);
     if (r < 0) return;
     const int nt = min(SP_T, p.q_len[r] - c * SP_T);
     const size_t a0 = (size_t)p.q_start[r] + c * SP_T;
+    sp_decays(p, a0, nt, h_first, dts, las);
     sp_load<NP>(Cs, p.C + a0 * p.ld + (size_t)((p.head0 + h_first) / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
     sp_load<NP>(Bs, p.B + a0 * p.ld + (size_t)((p.head0 + h_first) / p.hpg) * p.N, p.ld, nt, p.N, p.vec);
     __syncthreads();
@@ -247,28 +261,51 @@ __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
             mma16816(g[sj][1], cf[k], b2, b3);
         }
     }
+    auto fetch = [&](int h) {
+        const float* S = p.L + ((size_t)blockIdx.x * p.H + h) * p.N * p.dv + col0;
+        const float* X = p.X + a0 * p.ld + (size_t)h * p.dv + col0;
+#pragma unroll
+        for (int it = 0; it < NP * 16 / SP_THREADS; ++it) {
+            const int i = tid + it * SP_THREADS, n = i >> 4, j = (i & 15) * 4;
+            const bool ok = n < p.N && col0 + j < p.dv;
+            sp_copy(St + i * 4, ok ? S + (size_t)n * p.dv + j : S, ok);
+        }
+#pragma unroll
+        for (int it = 0; it < SP_T * 16 / SP_THREADS; ++it) {
+            const int i = tid + it * SP_THREADS, t = i >> 4, j = (i & 15) * 4;
+            const bool ok = t < nt && col0 + j < p.dv;
+            sp_copy(Xt + i * 4, ok ? X + (size_t)t * p.ld + j : p.X, ok);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    if (p.vec) {
+        __syncthreads();                                   // C and B are in registers
+        fetch(h_first);
+    }
 #pragma unroll 1
     for (int h = h_first; h < h_first + p.hpb; ++h) {
-        if (h > h_first) __syncthreads();                  // the last head's state and values are done with
         const float* S = p.L + ((size_t)blockIdx.x * p.H + h) * p.N * p.dv + col0;
         if (p.vec) {
-            constexpr int PER = NP * 16 / SP_THREADS;
-            float4 v[PER];
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+            __syncthreads();                               // ... for all threads, and the last head's operands are done with
 #pragma unroll
-            for (int it = 0; it < PER; ++it) {
+            for (int it = 0; it < NP * 16 / SP_THREADS; ++it) {
                 const int i = tid + it * SP_THREADS, n = i >> 4, j = (i & 15) * 4;
-                v[it] = n < p.N && col0 + j < p.dv ? *reinterpret_cast<const float4*>(S + (size_t)n * p.dv + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int it = 0; it < PER; ++it) {
-                const int i = tid + it * SP_THREADS, n = i >> 4, j = (i & 15) * 4;
+                const float4 v = *reinterpret_cast<const float4*>(St + i * 4);
                 uint2 hi, lo;
-                sp_split(v[it].x, v[it].y, hi.x, lo.x);
-                sp_split(v[it].z, v[it].w, hi.y, lo.y);
+                sp_split(v.x, v.y, hi.x, lo.x);
+                sp_split(v.z, v.w, hi.y, lo.y);
                 *reinterpret_cast<uint2*>(SH + n * LD + j) = hi;
                 *reinterpret_cast<uint2*>(SL + n * LD + j) = lo;
             }
+#pragma unroll
+            for (int it = 0; it < SP_T * 16 / SP_THREADS; ++it) {
+                const int i = tid + it * SP_THREADS, t = i >> 4, j = (i & 15) * 4;
+                const float4 v = *reinterpret_cast<const float4*>(Xt + i * 4);
+                *reinterpret_cast<uint2*>(Xs + t * LD + j) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+            }
         } else {
+            if (h > h_first) __syncthreads();              // the last head's state and values are done with
             for (int i = tid; i < NP * 64; i += SP_THREADS) {
                 const int n = i >> 6, j = i & 63;
                 const float v = n < p.N && col0 + j < p.dv ? S[(size_t)n * p.dv + j] : 0.f;
@@ -276,10 +313,11 @@ __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
                 SH[n * LD + j] = hi;
                 SL[n * LD + j] = __float2bfloat16_rn(v - __bfloat162float(hi));
             }
+            sp_load<64>(Xs, p.X + a0 * p.ld + (size_t)h * p.dv + col0, p.ld, nt, p.dv - col0, false);
         }
-        sp_load<64>(Xs, p.X + a0 * p.ld + (size_t)h * p.dv + col0, p.ld, nt, p.dv - col0, p.vec);
-        sp_decays(p, a0, nt, h, dt, la);
         __syncthreads();
+        if (p.vec && h + 1 < h_first + p.hpb) fetch(h + 1);      // lands while this head's products run
+        const float *dt = dts[h - h_first], *la = las[h - h_first];
         const float lta = la[ta], ltb = la[tb];
         float y[4][4] = {};
 #pragma unroll
@@ -338,6 +376,10 @@ __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
                     v = fmaf(sk, xs.y, v);
                 }
                 float* o = p.out + ((a0 + t) * p.all_heads + h) * p.dv + col0 + j;
+                if (p.vec) {
+                    if (col0 + j < p.dv) *reinterpret_cast<float2*>(o) = make_float2(u, v);
+                    continue;
+                }
                 if (col0 + j < p.dv) o[0] = u;
                 if (col0 + j + 1 < p.dv) o[1] = v;
             }
@@ -347,7 +389,7 @@ __global__ void __launch_bounds__(SP_THREADS, 2) sp_out_kernel(SpArgs p) {
 template <int NP>
 static int sp_go(const SpArgs& p, int n_portions, int n_chunks, cudaStream_t st) {
     const int LN = NP + 8, LD = 64 + 8;
-    const size_t sm_chunk = (size_t)(SP_T * LN + 2 * SP_T * LD) * 2, sm_out = (size_t)(2 * SP_T * LN + SP_T * LD + 2 * NP * LD) * 2;
+    const size_t sm_chunk = (size_t)(SP_T * LN + 2 * SP_T * LD) * 2, sm_out = (size_t)(2 * SP_T * LN + SP_T * LD + 2 * NP * LD) * 2 + SP_T * 64 * 4;
     cudaError_t e = cudaFuncSetAttribute(sp_chunk_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_chunk);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(sp_out_kernel<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_out);
     if (e != cudaSuccess) return (int)e;
@@ -374,10 +416,10 @@ extern "C" int aie_state_space_parallel(const float* C, const float* B, const fl
     if (R <= 0 || n_portions <= 0 || n_chunks <= 0) return 0;
     if (heads <= 0 || head0 < 0 || head0 + heads > H || N <= 0 || dv <= 0 || hpg < 1 || H % hpg || !dt_raw || !dt_bias || !a_log || min_len < 1) return AIE_BAD_ARG;
     if (N > 128 || heads > 65535 || (long long)n_portions * heads > 65535 || (dv + 63) / 64 > 65535) return AIE_UNSUPPORTED;
-    const int vec = N % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && !(((size_t)C | (size_t)B | (size_t)X | (size_t)L) & 15);
+    const int vec = N % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && !(((size_t)C | (size_t)B | (size_t)X | (size_t)L) & 15) && !((size_t)out & 7);
     // four or two heads a block where that still gives every SM's two places a block
     int hpb = 1;
-    while (hpb < 4 && hpg % (2 * hpb) == 0 && head0 % (2 * hpb) == 0 && heads % (2 * hpb) == 0 &&
+    while (hpb < SP_HEADS && hpg % (2 * hpb) == 0 && head0 % (2 * hpb) == 0 && heads % (2 * hpb) == 0 &&
            (long long)n_chunks * (heads / (2 * hpb)) * ((dv + 63) / 64) >= 2 * aie_sm_count()) hpb *= 2;
     const size_t c = (size_t)head0 * dv;
     const SpArgs p = {C, B, X + c, dt_raw + head0, dt_bias + head0, a_log + head0, skip ? skip + head0 : skip, state + c * N, out + c, L, G,
