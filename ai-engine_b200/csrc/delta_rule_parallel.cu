@@ -3,15 +3,16 @@
 // part that does not depend on the columns once for every block of columns: 11.5 us a chunk, 184 us for 1024 tokens of 16
 // heads of 128 x 128).  With T = (I + A)^-1,
 //     U = T (beta V) - T (beta exp(l) K) S_0 = U0 - W S_0
-// so that three kernels do it, for those 1024 tokens in 26 + 43 + 23 us:
+// so that three kernels do it, for those 1024 tokens in 26 + 29 + 23 us:
 //   prepare  every (chunk, head): unit keys, A, T, U0 and W, the keys times exp(l_Q - l_s), the chunk's decay
 //   walk     every (request, head, 16 or 32 columns): U = U0 - W S,  S <- exp(l_Q) S + (w K)^T U  from chunk to chunk; U takes
 //            U0's place, the states that chunks start from are kept
 //   out      every (chunk, head): O = exp(l_t) Q S_0 + P U
-// The walk is the chain that bounds it, 2.7 us a chunk with 16 columns a block and 3.5 with 32: two products, two barriers and the
-// exchange of the state one after the other on eight warps an SM, no unit near its limit (shared memory 50 %, L2 26 %).  A third
-// stage of W and the keys in shared memory changed nothing; both straight from L2 to the registers of their products: 2.4 us at
-// d = 128, but 5 % slower at d = 64.
+// The walk is the chain that bounds it, 1.8 us a chunk with 16 columns a block: two products, two barriers and the exchange of the
+// state one after the other on eight warps an SM, no unit near its limit.  W, the keys and U0 lie in memory as the walk wants them
+// in shared memory and come in three bulk copies a chunk, and what goes back goes 16 bytes a thread from shared memory: 16 bytes a
+// thread through cp.async and four bytes at a time back it was 2.7 us (3.5 with 32 columns), a bulk copy a row 3.3.  Without any
+// traffic 1.45.  W and keys straight from L2 to the registers of their products: 2.4 us.
 // T is made in float32: diagonal blocks of 16 by forward substitution, what is below from them.  T, beta V and beta exp(l)
 // enter the products of U0 and W as three bfloat16 values, all 24 bits; on the FMA units prepare took 39 us.  Everything else
 // enters mma.sync as pairs of bfloat16 values, as before, with float32 sums; the products that the state or the output is summed
@@ -20,6 +21,7 @@
 // accumulators.
 #include "attention_prefill.cuh"
 #include "chunk_find.cuh"
+#include "tc_common.cuh"
 
 #define DP_T 64
 #define DP_THREADS 256
@@ -28,8 +30,8 @@
 struct DpArgs {
     const float *q, *k, *v, *b_raw, *a_raw, *a_log, *dt_bias;
     float *state, *out;
-    bf16 *W, *Kw;             // [n_chunks, H, 2][64][d]: rounded value, rest
-    float *U, *S0, *decay;    // [n_chunks, H][64][e], [n_chunks, H][d][e], [n_chunks, H]
+    bf16 *W, *Kw;             // [n_chunks, H, 2][64][d]: rounded value, rest; eight columns j of row t at place j ^ (t & 7) (dp_at)
+    float *U, *S0, *decay;    // [n_chunks, H][e / 16][64][16], [n_chunks, H][d][e], [n_chunks, H]
     const int *q_start, *q_len, *slots, *live;
     unsigned* err;
     int ld, ldb, lda, R, H, all_heads, head0, per, e, max_slots, min_len;      // H: the heads of this launch, from head0 on; per a q/k head
@@ -47,12 +49,13 @@ __device__ __forceinline__ void dp_split3(float a, float b, unsigned& hi, unsign
     const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hi)), g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&lo));
     tail = pack_bf16((a - f.x) - g.x, (b - f.y) - g.y);
 }
-__device__ __forceinline__ void dp_fetch(void* dst, const void* src) { cp_async16(dst, src, true); }
-// columns j and j + 1 of a row of pairs that takes the place of one of float32 values: 16 rounded values, their 16 rests, ...
-__device__ __forceinline__ void dp_put(float* row, int j, unsigned hi, unsigned lo) {
-    unsigned* at = reinterpret_cast<unsigned*>(row) + (j & ~15) + ((j & 15) >> 1);
-    at[0] = hi;
-    at[8] = lo;
+// where column c of row t of W and Kw lies: as in shared memory, so that a chunk's come in one copy and ldmatrix reads eight rows
+// without conflicts
+template <int D> __device__ __forceinline__ int dp_at(int t, int c) { return t * D + ((c & ~7) ^ ((t & 7) << 3)) + (c & 7); }
+// from global to shared memory, both on 16 bytes; the bytes count on the barrier
+__device__ __forceinline__ void dp_bulk(void* dst, const void* src, int bytes, unsigned long long* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                 ::"r"(tc_smem(dst)), "l"(src), "r"(bytes), "r"(tc_smem(bar)) : "memory");
 }
 // acc += (ah + al) (bh + bl) without al bl, which is as small as what the pairs leave out
 __device__ __forceinline__ void dp_mma3(float* acc, const unsigned* ah, const unsigned* al, unsigned bh0, unsigned bh1, unsigned bl0, unsigned bl1) {
@@ -96,8 +99,8 @@ __device__ __forceinline__ void dp_units(const float* x, size_t ld, int nt, floa
             *reinterpret_cast<unsigned*>(lo + t * (D + 8) + V * lane + i) = l;
             if (Kw) {
                 dp_split(a * w, b * w, h, l);
-                *reinterpret_cast<unsigned*>(Kw + t * D + V * lane + i) = h;
-                *reinterpret_cast<unsigned*>(Kw + (DP_T + t) * D + V * lane + i) = l;
+                *reinterpret_cast<unsigned*>(Kw + dp_at<D>(t, V * lane + i)) = h;
+                *reinterpret_cast<unsigned*>(Kw + DP_T * D + dp_at<D>(t, V * lane + i)) = l;
             }
         }
     }
@@ -284,7 +287,7 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_prepare_kernel(DpArgs p) {
             for (int y = 0; y < 2; ++y) {
                 unsigned hi, lo;
                 dp_split(g[x][2 * y], g[x][2 * y + 1], hi, lo);
-                bf16* w = p.W + (at * 2 * DP_T + ta + 8 * y) * D + n0 + x * 8 + sc;
+                bf16* w = p.W + at * 2 * DP_T * D + dp_at<D>(ta + 8 * y, n0 + x * 8 + sc);
                 *reinterpret_cast<unsigned*>(w) = hi;
                 *reinterpret_cast<unsigned*>(w + DP_T * D) = lo;
             }
@@ -314,9 +317,9 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_prepare_kernel(DpArgs p) {
                 mma16816(g, th[sj], t0, t1);
                 mma16816(g, tt[sj], b0, b1);
             }
-            float* u = p.U + (at * DP_T + ta) * p.e + c0 + n0 + sc;
+            float* u = p.U + at * DP_T * p.e + (size_t)((c0 + n0) / 16 * DP_T + ta) * 16 + (n0 & 8) + sc;
             *reinterpret_cast<float2*>(u) = make_float2(g[0], g[1]);
-            *reinterpret_cast<float2*>(u + 8 * p.e) = make_float2(g[2], g[3]);
+            *reinterpret_cast<float2*>(u + 8 * 16) = make_float2(g[2], g[3]);
         }
     }
 }
@@ -327,12 +330,15 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_prepare_kernel(DpArgs p) {
 template <int D, int DV>
 __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
     extern __shared__ __align__(16) unsigned char dp_sm[];
-    constexpr int LN = D + 8, LD = DV + 8, ST = 4 * DP_T * LN, NU = DV / 16, NS = DV / 8;
-    bf16* stage = reinterpret_cast<bf16*>(dp_sm);      // two of [WH | WL | KH | KL], each [64][LN]
+    constexpr int LD = DV + 8, ST = 4 * DP_T * D, NU = DV / 16, NS = DV / 8;
+    bf16* stage = reinterpret_cast<bf16*>(dp_sm);      // two of [WH | WL | KH | KL], each [64][D] (dp_at)
     bf16* SH = stage + 2 * ST;                         // [D][LD]
     bf16* SL = SH + D * LD;
     bf16* UH = SL + D * LD;                            // [64][LD]
     bf16* UL = UH + DP_T * LD;
+    float* Us = reinterpret_cast<float*>(UL + DP_T * LD);          // two of [DV / 16][64][16]: U0
+    __shared__ unsigned long long bars[2];             // a chunk's operands have landed
+    __shared__ int gave_up;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, col0 = blockIdx.x * DV, h = blockIdx.y;
     __shared__ int found[2];
     int r, first;
@@ -343,20 +349,36 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
         if (tid == 0) atomicOr(p.err, AIE_DEV_SLOT_OOB);
         return;
     }
+    // A chunk's operands come in three bulk copies (16 bytes at a time through the load/store units they took 12 of 43 us, in a
+    // bulk copy a row 53)
     auto fetch = [&](int c) {
-        if (c < n) {
-            const size_t at = (size_t)(first + c) * p.H + h;
-            bf16* dst = stage + (c & 1) * ST;
-#pragma unroll
-            for (int it = 0; it < 4 * DP_T * D / 8 / DP_THREADS; ++it) {
-                const int i = tid + it * DP_THREADS, row = i / (D / 8), x = (i % (D / 8)) * 8;      // rows of W's pair, then of the keys'
-                const bf16* src = row < 2 * DP_T ? p.W + (at * 2 * DP_T + row) * D + x : p.Kw + (at * 2 * DP_T + row - 2 * DP_T) * D + x;
-                dp_fetch(dst + row * LN + x, src);
-            }
-        }
-        cp_async_commit();
+        if (c >= n || tid != 0) return;
+        const size_t at = (size_t)(first + c) * p.H + h;
+        constexpr int PAIR = 2 * DP_T * D * 2, COLS = DP_T * DV * 4;
+        unsigned long long* bar = &bars[c & 1];
+        mbar_expect_tx(bar, 2 * PAIR + COLS);
+        dp_bulk(stage + (c & 1) * ST, p.W + at * 2 * DP_T * D, PAIR, bar);
+        dp_bulk(stage + (c & 1) * ST + 2 * DP_T * D, p.Kw + at * 2 * DP_T * D, PAIR, bar);
+        dp_bulk(Us + (c & 1) * DP_T * DV, p.U + at * DP_T * p.e + (size_t)col0 * DP_T, COLS, bar);
     };
-    fetch(0);
+    if (tid == 0) {
+        gave_up = 0;
+        mbar_init(&bars[0], 1);
+        mbar_init(&bars[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        fetch(0);
+    }
+    __syncthreads();
+    // a matrix of pairs in shared memory to rows (`row` floats apart, groups of 16 columns `group` apart) that take the place of
+    // float32 ones: 16 rounded values, their 16 rests, ...; 16 bytes a thread
+    auto store = [&](float* dst, size_t row_step, size_t group_step, const bf16* hi, const bf16* lo, int rows) {
+        for (int i = tid; i < rows * DV / 4; i += DP_THREADS) {
+            const int row = i / (DV / 4), x = i % (DV / 4), j = (x >> 2) * 16;      // x & 3: the rounded ones' halves, the rests'
+            *reinterpret_cast<uint4*>(dst + row * row_step + (x >> 2) * group_step + (x & 3) * 4) =
+                *reinterpret_cast<const uint4*>((x & 2 ? lo : hi) + row * LD + j + (x & 1) * 8);
+        }
+    };
     float* sp = p.state + ((size_t)slot * p.all_heads + h) * D * p.e + col0;
     const bool holds = warp < D / 16;                  // rows 16 warp .. + 15 of the state
     const int sr = warp * 16 + (lane >> 2), sc = (lane & 3) * 2;
@@ -369,26 +391,11 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
             S[x][2 * y] = v.x, S[x][2 * y + 1] = v.y;
         }
     const int ut = (warp & 3) * 16 + (lane >> 2), un = (warp >> 2) * 8 * NU;
-    float u[NU][4], decay;                             // U0 and the decay of the chunk, loaded a chunk ahead
-    auto load = [&](int c) {
-        if (c >= n) return;
-        const size_t at = (size_t)(first + c) * p.H + h;
-        const float* U = p.U + (at * DP_T + ut) * p.e + col0 + un + sc;
-#pragma unroll
-        for (int x = 0; x < NU; ++x)
-#pragma unroll
-            for (int y = 0; y < 2; ++y) {
-                const float2 v = *reinterpret_cast<const float2*>(U + (size_t)8 * y * p.e + x * 8);
-                u[x][2 * y] = v.x, u[x][2 * y + 1] = v.y;
-            }
-        decay = p.decay[at];
-    };
-    load(0);
+    float decay = p.decay[(size_t)first * p.H + h];      // of the chunk, loaded a chunk ahead
     for (int c = 0; c < n; ++c) {
         const size_t at = (size_t)(first + c) * p.H + h;
-        float* U = p.U + at * DP_T * p.e + col0;
+        float* U = p.U + at * DP_T * p.e + (size_t)col0 * DP_T;
         if (holds) {
-            float* S0 = p.S0 + at * D * p.e + col0;
 #pragma unroll
             for (int x = 0; x < NS; ++x)
 #pragma unroll
@@ -397,20 +404,20 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
                     dp_split(S[x][2 * y], S[x][2 * y + 1], hi, lo);
                     *reinterpret_cast<unsigned*>(SH + (sr + 8 * y) * LD + x * 8 + sc) = hi;
                     *reinterpret_cast<unsigned*>(SL + (sr + 8 * y) * LD + x * 8 + sc) = lo;
-                    dp_put(S0 + (size_t)(sr + 8 * y) * p.e, x * 8 + sc, hi, lo);
                 }
         }
-        cp_async_wait<0>();
+        mbar_wait(&bars[c & 1], (c >> 1) & 1, &gave_up, p.err);
         __syncthreads();                               // this chunk's operands and state are here; the last chunk is done with
         fetch(c + 1);
+        store(p.S0 + at * D * p.e + col0, p.e, 16, SH, SL, D);
         const bf16* WH = stage + (c & 1) * ST;
         float a[NU][4] = {}, ahl[NU][4] = {}, alh[NU][4] = {};     // three chains of products
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
             unsigned ah[4], al[4];
-            const int aat = ((warp & 3) * 16 + (lane & 15)) * LN + k * 16 + (lane >> 4) * 8;
+            const int aat = dp_at<D>((warp & 3) * 16 + (lane & 15), k * 16 + (lane >> 4) * 8);
             ldsm_x4(ah[0], ah[1], ah[2], ah[3], WH + aat);
-            ldsm_x4(al[0], al[1], al[2], al[3], WH + DP_T * LN + aat);
+            ldsm_x4(al[0], al[1], al[2], al[3], WH + DP_T * D + aat);
             const int bat = (k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + un + (NU > 1 ? (lane >> 4) * 8 : 0);
             unsigned b[4], l[4];
             ldsm_x4_t(b[0], b[1], b[2], b[3], SH + bat);
@@ -427,19 +434,20 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
         for (int x = 0; x < NU; ++x)
 #pragma unroll
             for (int y = 0; y < 2; ++y) {
-                const float v0 = u[x][2 * y] - (a[x][2 * y] + (ahl[x][2 * y] + alh[x][2 * y]));
-                const float v1 = u[x][2 * y + 1] - (a[x][2 * y + 1] + (ahl[x][2 * y + 1] + alh[x][2 * y + 1]));
+                const float2 u0 = *reinterpret_cast<const float2*>(Us + (c & 1) * DP_T * DV + (((un + x * 8) >> 4) * DP_T + ut + 8 * y) * 16 + ((un + x * 8) & 8) + sc);
+                const float v0 = u0.x - (a[x][2 * y] + (ahl[x][2 * y] + alh[x][2 * y]));
+                const float v1 = u0.y - (a[x][2 * y + 1] + (ahl[x][2 * y + 1] + alh[x][2 * y + 1]));
                 unsigned hi, lo;
                 dp_split(v0, v1, hi, lo);
-                dp_put(U + (size_t)(ut + 8 * y) * p.e, un + x * 8 + sc, hi, lo);
                 *reinterpret_cast<unsigned*>(UH + (ut + 8 * y) * LD + un + x * 8 + sc) = hi;
                 *reinterpret_cast<unsigned*>(UL + (ut + 8 * y) * LD + un + x * 8 + sc) = lo;
             }
         const float g = decay;
-        load(c + 1);
+        if (c + 1 < n) decay = p.decay[at + p.H];
         __syncthreads();
+        store(U, 16, DP_T * 16, UH, UL, DP_T);
         if (holds) {
-            const bf16* KH = WH + 2 * DP_T * LN;
+            const bf16* KH = WH + 2 * DP_T * D;
 #pragma unroll
             for (int x = 0; x < NS; ++x)
 #pragma unroll
@@ -447,9 +455,9 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
 #pragma unroll
             for (int k = 0; k < DP_T; k += 16) {
                 unsigned ah[4], al[4];
-                const int aat = (k + (lane & 7) + ((lane >> 4) << 3)) * LN + warp * 16 + ((lane >> 3) & 1) * 8;
+                const int aat = dp_at<D>(k + (lane & 7) + ((lane >> 4) << 3), warp * 16 + ((lane >> 3) & 1) * 8);
                 ldsm_x4_t(ah[0], ah[1], ah[2], ah[3], KH + aat);
-                ldsm_x4_t(al[0], al[1], al[2], al[3], KH + DP_T * LN + aat);
+                ldsm_x4_t(al[0], al[1], al[2], al[3], KH + DP_T * D + aat);
 #pragma unroll
                 for (int x = 0; x < NS; x += 2) {
                     const int bat = (k + (lane & 7) + ((lane >> 3) & 1) * 8) * LD + x * 8 + (lane >> 4) * 8;
@@ -534,7 +542,8 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_out_kernel(DpArgs p) {
         for (int it = 0; it < (D + DP_T) * 16 / DP_THREADS; ++it) {
             const int i = tid + it * DP_THREADS, row = i >> 4, j = ((i >> 2) & 3) * 16;
             const bool state = row < D, rest = i & 2, ok = col0 + j < p.e;
-            const float* src = (state ? p.S0 + (at * D + row) * p.e : p.U + (at * DP_T + row - D) * p.e) + (ok ? col0 + j : 0) + (i & 3) * 4;
+            const int cj = ok ? col0 + j : 0;
+            const float* src = (state ? p.S0 + (at * D + row) * p.e + cj : p.U + at * DP_T * p.e + (size_t)(cj / 16 * DP_T + row - D) * 16) + (i & 3) * 4;
             bf16* dst = (state ? (rest ? SL : SH) + row * LD : (rest ? UL : UH) + (row - D) * LD) + j + (i & 1) * 8;
             cp_async16(dst, src, ok);
         }
@@ -607,7 +616,7 @@ static int dp_go(const DpArgs& p, int n_portions, int n_chunks, cudaStream_t st)
     // 16 columns a block while all blocks run at once; 32 read W and the keys half as often
 #define WALK(DV)                                                                                                        \
     {                                                                                                                   \
-        const size_t sm = (size_t)(8 * DP_T * LN + 2 * (D + DP_T) * (DV + 8)) * 2;                                      \
+        const size_t sm = (size_t)(8 * DP_T * D + 2 * (D + DP_T) * (DV + 8)) * 2 + (size_t)2 * DP_T * DV * 4;           \
         e = cudaFuncSetAttribute(dp_walk_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);          \
         if (e != cudaSuccess) return (int)e;                                                                            \
         dp_walk_kernel<D, DV><<<dim3(p.e / DV, p.H, n_portions), DP_THREADS, sm, st>>>(p);                                \
