@@ -1,0 +1,273 @@
+// Products of rows grouped by expert, C[row] = W[expert of the row's tile] . X[row] with X in tiles of 64 rows of one expert each
+// (bfloat16, float32 sums in tensor memory): the kernel for experts that have several tiles, whose weights are then read for all of
+// them at once.  gemm_tc.cu's grouped form takes one or two tiles a block and is bound by what its operands cost between L2 and
+// shared memory (32 KB for 256 cycles of products); here an item is 128 rows of an expert's weights against up to four of its
+// tiles (48 KB for 512 cycles), one block an SM walks items, and an item's epilogue runs while the next one's products do:
+//   warp 0 (one lane)  TMA loads of W [128 x 64] and of the tiles' X [64 x 64] into a ring of four stages;
+//   warp 1 (one lane)  four tcgen05.mma (K = 16) a stage into one of two accumulators of 256 columns;
+//   warps 2-9          the epilogue of the accumulator before (lane = weight row, column = token; two warps share a quarter of the
+//                      rows and take half of the columns each: with one the unit of a short K took longer than the products).
+// Items are walked in steps of the grid, those of four tiles first, the weight tiles of the same X side by side.
+// GLU: W [2 F, K] holds F gate rows, then F up rows.  A weight tile takes 64 of either in groups of 16, so that a warp's 32 lanes hold
+// a unit's gate and up sixteen lanes apart; act = min(gate, limit) * sigmoid(slope * it) * (up kept within +-limit + shift), as
+// clamped_glu makes it out of float32 sums, is stored in bfloat16.
+// Bound by L2: 48 KB a stage and SM at 43 bytes a cycle (12 TB/s over the chip), 1,120 cycles for 512 of products; 32 experts of 2,048 x
+// 2,048 with 1,024 rows each 301 -> 273 us, 1.0 PFLOP/s; gate and up with the unit behind them 355 -> 238.
+// Every wait is bounded (see tc_common.cuh).
+#include "tc_common.cuh"
+
+#define GG_BM 128
+#define GG_BK 64
+#define GG_TILE 64          // rows of X a tile
+#define GG_MOST 4           // tiles an item
+#define GG_STAGES 4
+#define GG_THREADS 320
+#define GG_MAX_TILES 2048   // tiles of a launch
+#define GG_W_BYTES (GG_BM * GG_BK * 2)
+#define GG_X_BYTES (GG_TILE * GG_BK * 2)
+#define GG_STAGE_BYTES (GG_W_BYTES + GG_MOST * GG_X_BYTES)
+// [alignment slack | 1 KB: barriers | list of items | ring]
+#define GG_LIST_BYTES (GG_MAX_TILES * 8)
+#define GG_SMEM (2048 + GG_LIST_BYTES + GG_STAGES * GG_STAGE_BYTES)
+
+struct GgGlu {
+    float limit, slope, shift;
+};
+
+template <bool GLU, typename OT>
+__global__ void __launch_bounds__(GG_THREADS, 1)
+gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, OT* __restrict__ C,
+                    const int* __restrict__ tile_w, int n_tiles, int N, int K, int ldc, unsigned* err, const GgGlu glu) {
+    extern __shared__ unsigned char gg_raw[];
+    unsigned char* bars = reinterpret_cast<unsigned char*>(((size_t)gg_raw + 1023) & ~(size_t)1023);
+    unsigned long long* full = reinterpret_cast<unsigned long long*>(bars);
+    unsigned long long* empty = full + GG_STAGES;
+    unsigned long long* acc_full = empty + GG_STAGES;      // [2]
+    unsigned long long* acc_empty = acc_full + 2;          // [2] the epilogue has read it
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(acc_empty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* n_groups_s = reinterpret_cast<int*>(tmem_slot + 2);
+    int2* list = reinterpret_cast<int2*>(bars + 1024);     // (first tile * 4 + tiles - 1, expert)
+    unsigned char* ring = bars + 1024 + GG_LIST_BYTES;
+    int* tw = reinterpret_cast<int*>(ring);                // the tiles' experts and the items that begin there, until the list is made
+    unsigned char* code = ring + GG_MAX_TILES * 4;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        tma_prefetch_map(&map_w);
+        tma_prefetch_map(&map_x);
+        for (int s = 0; s < GG_STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(&acc_full[a], 1);
+            mbar_init(&acc_empty[a], 8);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
+    }
+    pdl_launch_dependents();
+    pdl_wait();                                            // the list of tiles and the rows are earlier kernels' output
+    for (int i = tid; i < n_tiles; i += GG_THREADS) tw[i] = tile_w[i];
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const unsigned tmem = *tmem_slot;
+    if (warp == 0) {
+        // a run of an expert's tiles is cut into items of four from its start; the same list in every block
+        int run = 0;
+        for (int base = 0; base < n_tiles; base += 32) {
+            const int y = base + lane;
+            const int e = y < n_tiles ? tw[y] : -1;
+            const unsigned starts = __ballot_sync(0xffffffffu, y == 0 || (y < n_tiles && tw[y - 1] != e));
+            const unsigned mine = starts & (0xffffffffu >> (31 - lane));
+            const int first = mine ? base + 31 - __clz(mine) : run;
+            if (starts) run = base + 31 - __clz(starts);
+            if (y < n_tiles) {
+                int n = 0;
+                if (e >= 0 && (y - first) % GG_MOST == 0) {
+                    n = 1;
+                    while (n < GG_MOST && y + n < n_tiles && tw[y + n] == e) ++n;
+                }
+                code[y] = (unsigned char)n;
+            }
+        }
+        __syncwarp();
+        int at = 0;
+        for (int n = GG_MOST; n > 0; --n)
+            for (int base = 0; base < n_tiles; base += 32) {
+                const int y = base + lane;
+                const bool takes = y < n_tiles && code[y] == n;
+                const unsigned hit = __ballot_sync(0xffffffffu, takes);
+                if (takes) list[at + __popc(hit & ((1u << lane) - 1))] = make_int2(y * 4 + n - 1, tw[y]);
+                at += __popc(hit);
+            }
+        if (lane == 0) *n_groups_s = at;
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");      // the ring was written to by threads
+    __syncthreads();
+    const int per_tile = GLU ? GG_BM / 2 : GG_BM, NT = (GLU ? N / 2 : N) / per_tile, items = *n_groups_s * NT;
+    const int kbs = (K + GG_BK - 1) / GG_BK;
+
+    if (warp == 0) {
+        if (tc_elect()) {
+            int s = 0;
+            unsigned ph = 1;
+            bool ok = true;
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+                const int2 g = list[item / NT];
+                const int y = g.x >> 2, n = (g.x & 3) + 1, w0 = g.y * N + (item % NT) * per_tile;
+                for (int kb = 0; kb < kbs; ++kb) {
+                    ok = mbar_wait(&empty[s], ph, abort_flag, err);
+                    if (!ok) break;
+                    unsigned char* st = ring + s * GG_STAGE_BYTES;
+                    mbar_expect_tx(&full[s], GG_W_BYTES + n * GG_X_BYTES);
+                    if (GLU) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            tma_load_2d(st + q * 4096, &map_w, &full[s], kb * GG_BK, w0 + q * 16);
+                            tma_load_2d(st + q * 4096 + 2048, &map_w, &full[s], kb * GG_BK, w0 + N / 2 + q * 16);
+                        }
+                    } else {
+                        tma_load_2d(st, &map_w, &full[s], kb * GG_BK, w0);
+                    }
+                    for (int i = 0; i < n; ++i)
+                        tma_load_2d(st + GG_W_BYTES + i * GG_X_BYTES, &map_x, &full[s], kb * GG_BK, (y + i) * GG_TILE);
+                    if (++s == GG_STAGES) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (tc_elect()) {
+            int s = 0, a = 0;
+            unsigned ph = 0, aph = 1;
+            bool ok = true;
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+                const int n = (list[item / NT].x & 3) + 1;
+                const unsigned idesc = umma_idesc(n * GG_TILE), d = tmem + (unsigned)(a * 256);
+                ok = mbar_wait(&acc_empty[a], aph, abort_flag, err);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                for (int kb = 0; kb < kbs; ++kb) {
+                    ok = mbar_wait(&full[s], ph, abort_flag, err);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                    unsigned char* st = ring + s * GG_STAGE_BYTES;
+                    const unsigned long long da = umma_desc(st), db = umma_desc(st + GG_W_BYTES);
+#pragma unroll
+                    for (int j = 0; j < GG_BK / 16; ++j) umma(d, da + 2 * j, db + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
+                    umma_commit(&empty[s]);
+                    if (++s == GG_STAGES) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (ok) umma_commit(&acc_full[a]);
+                if (a == 1) aph ^= 1;
+                a ^= 1;
+            }
+        }
+    } else {
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        int a = 0;
+        unsigned aph = 0;
+        for (int item = blockIdx.x; item < items; item += gridDim.x) {
+            const int2 g = list[item / NT];
+            const int n = (g.x & 3) + 1, t0 = (g.x >> 2) * GG_TILE;
+            bool ok = true;
+            if (lane == 0) ok = mbar_wait(&acc_full[a], aph, abort_flag, err);
+            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const unsigned at = tmem + (unsigned)(a * 256) + ((unsigned)(quarter * 32) << 16);
+#pragma unroll 1
+            for (int c0 = half * 32 * n; c0 < (half + 1) * 32 * n; c0 += 32) {
+                unsigned v[32];
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                             "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+                             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                               "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+                               "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+                               "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                             : "r"(at + (unsigned)c0));
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                if (GLU) {
+                    // lanes 0 .. 15 hold gates and take the even tokens, the others ups and the odd ones
+                    const bool low = lane < 16;
+                    OT* to = C + (size_t)(t0 + c0 + (low ? 0 : 1)) * ldc + (item % NT) * per_tile + quarter * 16 + (lane & 15);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        const float own0 = __uint_as_float(v[j]), own1 = __uint_as_float(v[j + 1]);
+                        const float other = __shfl_xor_sync(0xffffffffu, low ? own1 : own0, 16);
+                        const float gate = fminf(low ? own0 : other, glu.limit);
+                        const float up = fminf(fmaxf(low ? other : own1, -glu.limit), glu.limit);
+                        to[(size_t)j * ldc] = from_f32<OT>(gate / (1.0f + expf(-glu.slope * gate)) * (up + glu.shift));
+                    }
+                } else {
+                    OT* to = C + (size_t)(t0 + c0) * ldc + (item % NT) * per_tile + quarter * 32 + lane;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) to[(size_t)j * ldc] = from_f32<OT>(__uint_as_float(v[j]));
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_plain(&acc_empty[a]);
+            if (a == 1) aph ^= 1;
+            a ^= 1;
+        }
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (*abort_flag && tid == 0) {      // give copies in flight a bounded time to land
+        for (int s = 0; s < GG_STAGES; ++s)
+            for (unsigned i = 0; i < (1u << 16) && !mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1); ++i) {}
+    }
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512));
+    }
+}
+
+template <bool GLU, typename OT>
+static int gg_go(const CUtensorMap& mw, const CUtensorMap& mx, void* C, const int* tile_w, int n_tiles, int N, int K, int ldc,
+                 unsigned* err, const GgGlu& glu, cudaStream_t st) {
+    auto kern = gemm_grouped_kernel<GLU, OT>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GG_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    const long long most = (long long)n_tiles * (N / GG_BM), sms = aie_sm_count();
+    e = launch_pdl(kern, dim3((unsigned)(most < sms ? most : sms)), dim3(GG_THREADS), GG_SMEM, st, mw, mx, (OT*)C, tile_w, n_tiles, N, K, ldc, err, glu);
+    return (int)e;
+}
+
+// X [tiles * 64, K], W [E, N, K] bfloat16, tile_w [tiles] (-1: the tile is skipped and its rows of C are left as they are).  C [rows, ldc]
+// float32 or bfloat16; with `glu` (W holds N / 2 gate rows, then as many up rows) C [rows, ldc >= N / 2] is bfloat16.
+extern "C" int aie_gemm_grouped(const void* X, const void* W, void* C, int out_dtype, int tiles, int N, int K, int ldc, int E,
+                                const int* tile_w, int glu, float limit, float slope, float shift, unsigned* err, cudaStream_t stream) {
+    if (tiles <= 0 || N <= 0) return 0;
+    if (!tile_w || E <= 0) return AIE_BAD_ARG;
+    if (K <= 0 || K % 8 || N % GG_BM || tiles > GG_MAX_TILES || ((size_t)X & 15) || ((size_t)W & 15) ||
+        (long long)E * N > 0x7fffffffLL || (glu && out_dtype != AIE_BF16))
+        return AIE_UNSUPPORTED;
+    CUtensorMap mw, mx;
+    int rc = tc_make_map_2d(&mw, W, (unsigned long long)E * N, K, (unsigned long long)K * 2, glu ? 16 : GG_BM, GG_BK);
+    if (rc) return rc;
+    rc = tc_make_map_2d(&mx, X, (unsigned long long)tiles * GG_TILE, K, (unsigned long long)K * 2, GG_TILE, GG_BK);
+    if (rc) return rc;
+    const GgGlu g{limit, slope, shift};
+    if (glu) return gg_go<true, bf16>(mw, mx, C, tile_w, tiles, N, K, ldc, err, g, stream);
+    if (out_dtype == AIE_F32) return gg_go<false, float>(mw, mx, C, tile_w, tiles, N, K, ldc, err, g, stream);
+    if (out_dtype == AIE_BF16) return gg_go<false, bf16>(mw, mx, C, tile_w, tiles, N, K, ldc, err, g, stream);
+    return AIE_BAD_ARG;
+}

@@ -1307,17 +1307,45 @@ def gather_rows(src: torch.Tensor, rows: torch.Tensor, zero_fill: bool = True, l
     return out
 
 
+GROUPED_MAX_TILES = 2048      # tiles that the kernel of csrc/gemm_grouped.cu lists
+
+
+def grouped_takes_items(tiles: int, E: int, N: int) -> bool:
+    """Whether a product of rows grouped by expert takes the kernel whose blocks walk items of up to four tiles: from 2.6 tiles an
+    expert on (its share of the empty ones too) and 1,024 columns.  us, one or two tiles a block against items, at 64 / 100 /
+    128 / 192 / 214 / 320 / 1,024 rows an expert: 32 experts of 2,048 x 2,048 55 / 65 / 71 / 84 / 92 / 124 / 301 against 59 / 62 / 63 / 71
+    / 87 / 120 / 273; of 2,048 x 1,024 34 / 39 / 41 / 49 / 55 / 72 / 183 and 36 / 36 / 39 / 42 / 49 / 68 / 160; 8 of 4,096 x 2,048 30 / 39 /
+    39 / 43 / 54 / 60 / 162 and 32 / 33 / 34 / 37 / 47 / 60 / 143; 128 of 512 x 1,024 34 / 41 / 44 / 54 / 59 / 74 and 38 / 43 / 47 / 53 / 63 /
+    79."""
+    return 5 * tiles >= 13 * E and N >= 1024 and tiles <= GROUPED_MAX_TILES
+
+
+def _grouped_items(x, w, tile_w, out, err, row_src, live, glu=None) -> None:
+    """The kernel whose blocks walk items of 128 weight rows and up to four tiles (see csrc/gemm_grouped.cu)."""
+    E, N, K = w.shape
+    xs = gather_rows(x, row_src, zero_fill=False, live=live) if row_src is not None else x
+    _dev(xs, w, tile_w, out, err)
+    limit, slope, shift = glu or (float("inf"), 1.0, 0.0)
+    with region("gemm_grouped", _nb(xs, w, out), 2.0 * out.shape[0] * N * K):
+        check(library("gemm_grouped.cu").aie_gemm_grouped(
+            _p(xs), _p(w), _p(out), c_int(dtype_code(out)), c_int(tile_w.shape[0]), c_int(N), c_int(K), c_int(out.shape[1]), c_int(E),
+            _p(tile_w), c_int(1 if glu else 0), c_float(limit), c_float(slope), c_float(shift), _p(err), _stream()), "gemm_grouped")
+
+
 def grouped_linear(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, out_dtype: torch.dtype,
                    err: torch.Tensor, row_src: Optional[torch.Tensor] = None, live: Optional[int] = None) -> torch.Tensor:
     """Rows grouped in tiles of EXPERT_TILE, tile i multiplied with the weight w[tile_w[i]] of the stack w [E, N, K]
     (tile_w[i] < 0: the tile is skipped, its output rows are undefined).  x [rows, K], or, with `row_src`
     [rows], the rows x[row_src[r]] (where row_src[r] < 0 the output row is undefined: every row is a product of its
     own).  bfloat16 operands whose N is a multiple of 128 and K of 8
-    take the tcgen05 kernel, everything else the float32 kernel on the CUDA cores."""
+    take the tcgen05 kernels, everything else the float32 kernel on the CUDA cores."""
     E, N, K = w.shape
     rows = tile_w.shape[0] * EXPERT_TILE
     out = torch.empty((rows, N), dtype=out_dtype, device=x.device)
     if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and N % 128 == 0 and K % 8 == 0:
+        if grouped_takes_items(tile_w.shape[0], E, N):
+            _grouped_items(x, w, tile_w, out, err, row_src, live)
+            return out
         xs = gather_rows(x, row_src, zero_fill=False, live=live) if row_src is not None else x
         _dev(xs, w, tile_w, err)
         lib = library("gemm_tc.cu")
@@ -1327,6 +1355,22 @@ def grouped_linear(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, out_d
                                           _stream()), "gemm_tc_grouped")
         return out
     return gemm_f32_ex(x, w, out, rows, N, K, K, N, w_bs=N * K, a_rows=row_src, tile_w=tile_w)
+
+
+def grouped_glu(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, limit: float, alpha: float, shift: float,
+                out_dtype: torch.dtype, err: torch.Tensor, row_src: torch.Tensor, live: Optional[int] = None) -> torch.Tensor:
+    """clamped_glu of grouped_linear's float32 result, w [E, 2 F, K] with the gate's rows first: [rows, F] in out_dtype.  In bfloat16
+    the unit is applied to the product's sums, the same bits: us, product and unit against one kernel, at 3 / 64 / 128 / 214 / 1,024 rows
+    an expert: 32 experts of 2,048 x 2,048 59 / 65 / 82 / 107 / 355 against 55 / 57 / 61 / 81 / 238, of 1,024 x 512 11 / 16 / 23 / 33 / 106
+    and 9 / 13 / 15 / 21 / 67; 128 of 512 x 1,024 40 / 46 / 59 / 79 and 34 / 37 / 44 / 56."""
+    E, N, K = w.shape
+    if (x.dtype == w.dtype == out_dtype == torch.bfloat16 and N % 128 == 0 and K % 8 == 0
+            and tile_w.shape[0] <= GROUPED_MAX_TILES):
+        out = torch.empty((tile_w.shape[0] * EXPERT_TILE, N // 2), dtype=out_dtype, device=x.device)
+        _grouped_items(x, w, tile_w, out, err, row_src, live, (limit, alpha, shift))
+        return out
+    gu = grouped_linear(x, w, tile_w, torch.float32, err, row_src=row_src, live=live)
+    return clamped_glu(gu, N // 2, limit, alpha, shift, out_dtype, rows=row_src)
 
 
 # ---------------------------------------------------------------------------
