@@ -745,9 +745,9 @@ extern "C" int aie_head_linear_small(const void* x, long long xt, long long xh, 
 
 // ---------------------------------------------------------------------------
 // The cached rows that portions read expanded, one behind the other: tiles [n, 2] = (request row, which 128 keys of it counted
-// from its first); rows before the window of the portion's first token or behind its last are zeros.  A block copies 32 rows
-// of a tile, 16 bytes a thread.
-#define LG_ROWS 32
+// from its first); rows before the window of the portion's first token or behind its last are zeros.  A block copies 8 rows
+// of a tile, 16 bytes a thread (32 rows: 3,072 rows of 576 took 9.3 us in 96 blocks, now 5.3).
+#define LG_ROWS 8
 __global__ void __launch_bounds__(256)
 latent_gather_kernel(const bf16* __restrict__ pages, bf16* __restrict__ rows, const int* __restrict__ tiles,
                      const int* __restrict__ q_len, const int* __restrict__ ctx_len, const int* __restrict__ block_table,
