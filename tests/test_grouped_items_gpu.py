@@ -1,5 +1,5 @@
 """The grouped tcgen05 product whose blocks walk items of up to four tiles of an expert: runs of one to nine and more than 32 tiles,
-empty tiles between, more items than SMs, a remainder of K; with and without the gated unit, which gives the bits of the unit on
+empty tiles between, more items than SMs, a remainder of K, one block an item and two; with and without the gated unit, which gives the bits of the unit on
 the float32 product."""
 import pytest
 import torch
@@ -10,7 +10,8 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("runs,N,K", [
     ([(0, 1), (1, 3), (-1, 2), (2, 2), (0, 4), (1, 5), (2, 9)], 128, 64), ([(1, 33), (0, 65), (1, 1)], 256, 72), ([(-1, 3)], 128, 64),
-    ([(2, 1)], 384, 520), ([(0, 7), (-1, 1), (2, 6), (1, 40)], 1152, 1032)])
+    ([(2, 1)], 384, 520), ([(0, 7), (-1, 1), (2, 6), (1, 40)], 1152, 1032),
+    ([(0, 7), (-1, 1), (2, 6), (1, 40)], 1280, 1032), ([(-1, 3)], 256, 1024), ([(2, 1)], 256, 1024)])
 def test_items_of_up_to_four_tiles(runs, N, K):
     from ai_engine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(K + N)
