@@ -1313,10 +1313,10 @@ GROUPED_MAX_TILES = 2048      # tiles that the kernel of csrc/gemm_grouped.cu li
 def grouped_takes_items(tiles: int, E: int, N: int) -> bool:
     """Whether a product of rows grouped by expert takes the kernel whose blocks walk items of up to four tiles: from 2.6 tiles an
     expert on (its share of the empty ones too) and 1,024 columns.  us, one or two tiles a block against items, at 64 / 100 /
-    128 / 192 / 214 / 320 / 1,024 rows an expert: 32 experts of 2,048 x 2,048 55 / 65 / 71 / 84 / 92 / 124 / 301 against 59 / 62 / 63 / 71
-    / 87 / 120 / 273; of 2,048 x 1,024 34 / 39 / 41 / 49 / 55 / 72 / 183 and 36 / 36 / 39 / 42 / 49 / 68 / 160; 8 of 4,096 x 2,048 30 / 39 /
-    39 / 43 / 54 / 60 / 162 and 32 / 33 / 34 / 37 / 47 / 60 / 143; 128 of 512 x 1,024 34 / 41 / 44 / 54 / 59 / 74 and 38 / 43 / 47 / 53 / 63 /
-    79."""
+    128 / 192 / 214 / 320 / 1,024 rows an expert: 32 experts of 2,048 x 2,048 54 / 63 / 67 / 79 / 89 / 118 / 293 against 55 / 58 / 59 / 64
+    / 78 / 105 / 233; of 2,048 x 1,024 33 / 38 / 40 / 48 / 55 / 71 / 176 and 35 / 35 / 37 / 39 / 46 / 61 / 139; 8 of 4,096 x 2,048 30 / 39 /
+    38 / 41 / 54 / 58 / 157 and 30 / 31 / 32 / 34 / 41 / 53 / 126; 128 of 512 x 1,024 34 / 40 / 43 / 53 / 59 / 73 and 37 / 42 / 46 / 52 / 61 /
+    77."""
     return 5 * tiles >= 13 * E and N >= 1024 and tiles <= GROUPED_MAX_TILES
 
 
@@ -1361,8 +1361,8 @@ def grouped_glu(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, limit: f
                 out_dtype: torch.dtype, err: torch.Tensor, row_src: torch.Tensor, live: Optional[int] = None) -> torch.Tensor:
     """clamped_glu of grouped_linear's float32 result, w [E, 2 F, K] with the gate's rows first: [rows, F] in out_dtype.  In bfloat16
     the unit is applied to the product's sums, the same bits: us, product and unit against one kernel, at 3 / 64 / 128 / 214 / 1,024 rows
-    an expert: 32 experts of 2,048 x 2,048 59 / 65 / 82 / 107 / 355 against 55 / 57 / 61 / 81 / 238, of 1,024 x 512 11 / 16 / 23 / 33 / 106
-    and 9 / 13 / 15 / 21 / 67; 128 of 512 x 1,024 40 / 46 / 59 / 79 and 34 / 37 / 44 / 56."""
+    an expert: 32 experts of 2,048 x 2,048 59 / 64 / 79 / 105 / 350 against 51 / 52 / 55 / 71 / 217, of 1,024 x 512 11 / 16 / 23 / 33 / 106
+    and 9 / 12 / 15 / 21 / 66; 128 of 512 x 1,024 40 / 45 / 59 / 79 and 32 / 36 / 44 / 56."""
     E, N, K = w.shape
     if (x.dtype == w.dtype == out_dtype == torch.bfloat16 and N % 128 == 0 and K % 8 == 0
             and tile_w.shape[0] <= GROUPED_MAX_TILES):
