@@ -512,6 +512,71 @@ extern "C" int aie_gated_decay(const float* z, const float* bias, float* out, lo
     AIE_LAUNCH_CHECK();
 }
 
+// The same of the logits of a short product, z = x[t] . w[n] over up to LRD_RANK terms in their order.  The product's own kernel and the
+// one above move 8 bytes an element out and in again; this one is bound by the two exponentials and the logarithm (about 100
+// instructions an element).  A thread keeps its channel's weights and walks LRD_TOKENS tokens, whose x lie in shared memory: us at 1 / 64 /
+// 256 / 2,048 / 8,192 tokens of 2,048 channels, two kernels 3.7 / 4.6 / 5.4 / 17.8 / 62, this 1.9 / 3.4 / 3.8 / 13.6 / 46 (two channels a
+// thread 2.0 / 5.6 / 5.9 / 14.4 / 45).  vec: rows of w start on 16 bytes and are LRD_RANK long.
+#define LRD_RANK 16
+#define LRD_TOKENS 16
+template <typename WT>
+__global__ void __launch_bounds__(128)
+low_rank_decay_kernel(const float* __restrict__ x, int ldx, const WT* __restrict__ w, const float* __restrict__ bias,
+                      float* __restrict__ out, int T, int N, int rank, float inv_tau, int vec) {
+    __shared__ __align__(16) float xs[LRD_TOKENS][LRD_RANK];
+    const int n = blockIdx.x * 128 + threadIdx.x, t0 = blockIdx.y * LRD_TOKENS, nt = min(LRD_TOKENS, T - t0);
+    for (int i = threadIdx.x; i < LRD_TOKENS * LRD_RANK; i += 128) {
+        const int t = i / LRD_RANK, r = i % LRD_RANK;
+        xs[t][r] = t < nt && r < rank ? x[(size_t)(t0 + t) * ldx + r] : 0.f;
+    }
+    __syncthreads();
+    if (n >= N) return;
+    const WT* row = w + (size_t)n * rank;
+    float wr[LRD_RANK];
+#pragma unroll
+    for (int r = 0; r < LRD_RANK; r += 4) {
+        const float4 v = vec ? load4<WT>(row + r) : make_float4(0.f, 0.f, 0.f, 0.f);
+        wr[r] = v.x;
+        wr[r + 1] = v.y;
+        wr[r + 2] = v.z;
+        wr[r + 3] = v.w;
+    }
+    if (!vec) {
+#pragma unroll
+        for (int r = 0; r < LRD_RANK; ++r)
+            if (r < rank) wr[r] = to_f32<WT>(row[r]);
+    }
+    const float b = bias ? bias[n] : 0.f;
+#pragma unroll 2
+    for (int t = 0; t < nt; ++t) {
+        float z = 0.f;
+#pragma unroll
+        for (int r = 0; r < LRD_RANK; r += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(&xs[t][r]);
+            z = fmaf(a.w, wr[r + 3], fmaf(a.z, wr[r + 2], fmaf(a.y, wr[r + 1], fmaf(a.x, wr[r], z))));
+        }
+        const float v = z + b;
+        out[(size_t)(t0 + t) * N + n] = expf((fminf(v, 0.f) - log1pf(expf(-fabsf(v)))) * inv_tau);
+    }
+}
+
+// x: float32 rows of stride ldx; w [N, rank] float32 or bfloat16; AIE_UNSUPPORTED for a rank the kernel does not keep.
+extern "C" int aie_low_rank_decay(const float* x, int ldx, const void* w, int w_dtype, const float* bias, float* out, int T, int N,
+                                  int rank, float tau, cudaStream_t st) {
+    if (T <= 0) return 0;
+    if (N <= 0 || rank <= 0 || !(tau > 0.f)) return AIE_BAD_ARG;
+    if (rank > LRD_RANK || T > 65535 * LRD_TOKENS) return AIE_UNSUPPORTED;
+    const int vec = rank == LRD_RANK && !((size_t)w & 15);
+    const dim3 grid((N + 127) / 128, (T + LRD_TOKENS - 1) / LRD_TOKENS);
+    if (w_dtype == AIE_F32)
+        low_rank_decay_kernel<float><<<grid, 128, 0, st>>>(x, ldx, (const float*)w, bias, out, T, N, rank, 1.0f / tau, vec);
+    else if (w_dtype == AIE_BF16)
+        low_rank_decay_kernel<bf16><<<grid, 128, 0, st>>>(x, ldx, (const bf16*)w, bias, out, T, N, rank, 1.0f / tau, vec);
+    else
+        return AIE_BAD_ARG;
+    AIE_LAUNCH_CHECK();
+}
+
 // ---------------------------------------------------------------------------
 // Experts chosen by a table of the token's id: pair p = (token t, choice s) goes to expert table[id[t], s]
 // (ids null: the table has a row per token of the step, as a router leaves it).  Experts E .. E + ident - 1 are

@@ -95,10 +95,7 @@ class DecayLinearAttention(Mixer):
         v, g = proj[:, 2 * Hd:2 * Hd + Hv], proj[:, 2 * Hd + Hv:2 * Hd + 2 * Hv]
         decay_tok = None
         if self.decay is None:
-            T = h.shape[0]
-            z = torch.empty((T, Hd), dtype=torch.float32, device=h.device)
-            ops.gemm_f32_ex(proj[:, 2 * Hd + 2 * Hv:], self.w_a2, z, T, Hd, self.r, proj.stride(0), Hd)
-            decay_tok = ops.gated_decay(z, self.a2_bias, self.tau)
+            decay_tok = ops.low_rank_decay(proj[:, 2 * Hd + 2 * Hv:], self.w_a2, self.a2_bias, self.tau)
         o = ops.linear_recurrence(q, k, v, decay_tok, self.decay_head, self.q_scale, self.k_scale, cache.state, ctx,
                                   self.H, self.d, self.dv, in_order=self.env.dtype == torch.float32)
         y = ops.head_norm_gate(o, g, self.out_weight, self.eps, self.env.dtype)
