@@ -15,6 +15,7 @@
 // joining kernel.  Weights enter the product with the rows rounded to bfloat16 and are summed so, or (PAIR) as two
 // bfloat16 terms each, 16 bits of mantissa, beside a float32 sum.  A sink (exp(sink[h]) in the denominator, nothing in the output) opens the running softmax of the first part.
 #include "attention_prefill.cuh"
+#include "tc_common.cuh"
 
 #define LT_KEYS 64
 #define LT_ROWS 16
@@ -248,12 +249,16 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
 // Requests that bring one token.  What bounds them is the stream of their cache rows, so the rows are cut evenly over the
 // machine whatever the requests' lengths: the visible chunks of 32 keys of all such requests stand in one line, CTA i takes
 // the i-th of gridDim.x equal stretches of it, and the rows of the next chunk are on their way, across the requests' ends,
-// while a chunk is multiplied; two CTAs share an SM, so that one's chain of products and softmax fills the other's waits.  Eight warps: the scores' products are split over four groups of
-// eight keys and two halves of a row, the values' over eight ranges of the latent's columns.  A stretch that holds a whole
+// while a chunk is multiplied; two CTAs share an SM, so that one's chain of products and softmax fills the other's waits.  Eight warps
+// multiply: the scores' products are split over four groups of eight keys and two halves of a row, the values' over eight ranges of
+// the latent's columns.  A ninth looks the rows up, a lane a key, and asks for each with one bulk copy whose bytes count on the stage's
+// barrier (rows that are not to be seen it fills with zeros): with 16-byte copies by the other eight, which all looked up the
+// same places, four of five of their instructions were addresses.  A stretch that holds a whole
 // request writes its result; others leave (maximum, sum, unnormalised output) in slot CTA + request for the join.
-// 64 requests of 512 .. 4,096 keys, 16 heads, a latent of 512 (170 MB of rows, 26 us at the copy bandwidth): 63 us; 162 us with
-// a CTA a (request, quarter of its keys) that loaded and multiplied in turn, 109 us with one CTA an SM and four chunks in
-// flight, whose eight warps waited on one another.
+// 64 requests of 512 .. 4,096 keys, 16 heads, a latent of 512 (170 MB of rows, 26 us at the copy bandwidth): 47 us, 63 with the copies
+// in the warps that multiply; 162 us with a CTA a (request, quarter of its keys) that loaded and multiplied in turn, 109 us with one
+// CTA an SM and four chunks in flight, whose eight warps waited on one another.  Bound by the chain of a chunk's products, softmax and
+// products, 870 -> 250 instructions a warp.  Every wait is bounded (see tc_common.cuh).
 #define LD_KEYS 32
 #define LD_THREADS 256
 #define LD_MIN_CHUNKS 2       // a stretch is at least this long: a CTA's start costs about as much as two chunks
@@ -274,8 +279,17 @@ __device__ __forceinline__ int ld_stretch(const int* q_len, const int* ctx_len, 
     return max((total + G - 1) / G, LD_MIN_CHUNKS);
 }
 
+__device__ __forceinline__ void ld_sync() { asm volatile("barrier.sync 1, %0;\n" ::"n"(LD_THREADS) : "memory"); }
+// the same, and whether any of the threads says so
+__device__ __forceinline__ bool ld_sync_any(bool mine) {
+    int any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+                 : "=r"(any) : "r"(mine ? 1 : 0), "n"(LD_THREADS) : "memory");
+    return any != 0;
+}
+
 template <int NT, bool PAIR, int CTAS>     // NT: tiles of 8 latent columns a warp (rank = 64 NT); CTAS: blocks an SM
-__global__ void __launch_bounds__(LD_THREADS, CTAS)
+__global__ void __launch_bounds__(LD_THREADS + 32, CTAS)
 latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ pages, bf16* __restrict__ out,
                      float* __restrict__ part_o, float* __restrict__ part_ml, const int* __restrict__ q_start,
                      const int* __restrict__ q_len, const int* __restrict__ ctx_len, const int* __restrict__ block_table,
@@ -291,9 +305,21 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
     float* m_s = s_s + 2 * LT_ROWS * SS;                          // [16] running maximum, sum, correction
     float* l_s = m_s + LT_ROWS;
     float* c_s = l_s + LT_ROWS;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h0 = blockIdx.y * LT_ROWS, pieces = dk / 8;
+    __shared__ unsigned long long full[NST], empty[NST];
+    __shared__ int abort_word;
+    volatile int* abort_flag = &abort_word;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h0 = blockIdx.y * LT_ROWS;
+    if (tid == 0) {
+        for (int i = 0; i < NST; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], LD_THREADS / 32);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
     pdl_launch_dependents();
     pdl_wait();
+    __syncthreads();
     int total, first;
     const int per = ld_stretch(q_len, ctx_len, R, window, gridDim.x, total);
     const int begin = blockIdx.x * per, cnt = min(total - begin, per);
@@ -315,178 +341,191 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
         }
         before += __shfl_sync(0xffffffffu, run, 31);
     }
-    int lr = r, lc = c, lfirst, ln = ld_chunks(q_len, ctx_len, R, window, r, lfirst);      // the chunk that is asked for next
-    // lane l: place (page * P + offset) of key l of the chunk that is asked for next, -1: none or not to be seen.  Looked up a
-    // chunk ahead, so that no copy waits for a block table.
-    auto places = [&](int i) {
-        int at = -1;
-        if (i < cnt) {
-            const int pos = ctx_len[lr], kp = (lfirst + lc) * LD_KEYS + lane;
-            if (kp <= pos && (window <= 0 || kp > pos - window)) {
-                const int pidx = kp / P, page = pidx < bt_width ? block_table[(size_t)lr * bt_width + pidx] : -1;
-                if (page < 0 || page >= num_pages) atomicOr(err, AIE_DEV_PAGE_OOB);
-                else at = page * P + (kp - pidx * P);
-            }
-            if (++lc == ln && i + 1 < cnt) {
-                lc = 0;
-                do ln = ld_chunks(q_len, ctx_len, R, window, ++lr, lfirst);
-                while (ln == 0 && lr < R);
-            }
-        }
-        return at;
-    };
-    int next_at = places(0);
-    auto fetch = [&](int i) {
-        if (i < cnt) {
-            bf16* dst = k_s + ((i % NST) * LD_KEYS + warp * (LD_KEYS / 8)) * SK + lane * 8;
-#pragma unroll
-            for (int jj = 0; jj < LD_KEYS / 8; ++jj) {
-                const int at = __shfl_sync(0xffffffffu, next_at, warp * (LD_KEYS / 8) + jj);
-                const bf16* src = pages + (size_t)max(at, 0) * dk + lane * 8;
-                for (int x = lane; x < pieces; x += 32, src += 256) cp_async16(dst + jj * SK + (x - lane) * 8, src, at >= 0);
-            }
-        }
-        cp_async_commit();
-        next_at = places(i + 1);
-    };
-    fetch(0);
-    const int steps = dk / 16, kg = warp & 3, kh = warp >> 2;
-    const int step0 = kh ? (steps + 1) / 2 : 0, step1 = kh ? steps : (steps + 1) / 2;
-    float acc[NT][4];
-    int n = 0, c_begin = 0, pos = 0, lo = 0;
-    bool fresh = true;
-    for (int i = 0; i < cnt; ++i) {
-        if (fresh) {                                              // a request begins: its queries, an empty softmax
-            fresh = false;
-            n = ld_chunks(q_len, ctx_len, R, window, r, first);
-            c_begin = c;
-            pos = ctx_len[r];
-            lo = window > 0 ? max(pos - window + 1, 0) : 0;
-            if (i > 0) __syncthreads();                           // the last one's sums have been read
-            const int t = q_start[r];
-            for (int rr = warp; rr < LT_ROWS; rr += LD_THREADS / 32) {
-                const bool on = h0 + rr < H;
-                const float* src = q_full + ((size_t)t * H + h0 + rr) * dk;
-                for (int x = lane * 4; x < dk; x += 128) {
-                    const float4 v = on ? *reinterpret_cast<const float4*>(src + x) : make_float4(0.f, 0.f, 0.f, 0.f);
-                    *reinterpret_cast<uint2*>(q_s + rr * SK + x) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    if (warp == LD_THREADS / 32) {                                // the warp that asks for rows, a chunk ahead of the others
+        int lr = r, lc = c, lfirst, ln = ld_chunks(q_len, ctx_len, R, window, r, lfirst);
+        // lane l: place (page * P + offset) of key l of the chunk that is asked for next, -1: none or not to be seen
+        auto places = [&](int i) {
+            int at = -1;
+            if (i < cnt) {
+                const int pos = ctx_len[lr], kp = (lfirst + lc) * LD_KEYS + lane;
+                if (kp <= pos && (window <= 0 || kp > pos - window)) {
+                    const int pidx = kp / P, page = pidx < bt_width ? block_table[(size_t)lr * bt_width + pidx] : -1;
+                    if (page < 0 || page >= num_pages) atomicOr(err, AIE_DEV_PAGE_OOB);
+                    else at = page * P + (kp - pidx * P);
+                }
+                if (++lc == ln && i + 1 < cnt) {
+                    lc = 0;
+                    do ln = ld_chunks(q_len, ctx_len, R, window, ++lr, lfirst);
+                    while (ln == 0 && lr < R);
                 }
             }
-            if (tid < LT_ROWS) {
-                const bool leaks = sink && c == 0 && h0 + tid < H;
-                m_s[tid] = leaks ? sink[h0 + tid] : -INFINITY;
-                l_s[tid] = leaks ? 1.f : 0.f;
-            }
-#pragma unroll
-            for (int x = 0; x < NT; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
-        }
-        cp_async_wait<NST - 2>();
-        __syncthreads();                                          // chunk i is here for all; chunk i - 1 is done with
-        fetch(i + NST - 1);
-        const bf16* ks = k_s + (i % NST) * LD_KEYS * SK;
-        {
-            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
-            const bf16* qa = q_s + (lane & 15) * SK + (lane >> 4) * 8;
-            const bf16* kb = ks + (kg * 8 + (lane & 7)) * SK + (lane >> 3) * 8;
-#pragma unroll 3
-            for (int st = step0; st < step1; st += 2) {           // two steps of 16: one load of keys
-                unsigned a[4], b0, b1, b2, b3;
-                ldsm_x4(b0, b1, b2, b3, kb + st * 16);
-                ldsm_x4(a[0], a[1], a[2], a[3], qa + st * 16);
-                mma16816(s0, a, b0, b1);
-                if (st + 1 < step1) {
-                    ldsm_x4(a[0], a[1], a[2], a[3], qa + st * 16 + 16);
-                    mma16816(s1, a, b2, b3);
-                }
-            }
-            float* d = s_s + kh * LT_ROWS * SS + (lane >> 2) * SS + kg * 8 + (lane & 3) * 2;
-            *reinterpret_cast<float2*>(d) = make_float2(s0[0] + s1[0], s0[1] + s1[1]);
-            *reinterpret_cast<float2*>(d + 8 * SS) = make_float2(s0[2] + s1[2], s0[3] + s1[3]);
-        }
-        __syncthreads();
-        {                                                         // running softmax: sixteen threads a row, two keys a thread
-            const int row = tid >> 4, g = tid & 15, key = (first + c) * LD_KEYS + 2 * g;
-            const float2 x = *reinterpret_cast<const float2*>(s_s + row * SS + 2 * g);
-            const float2 y = *reinterpret_cast<const float2*>(s_s + (LT_ROWS + row) * SS + 2 * g);
-            const float v0 = key >= lo && key <= pos ? (x.x + y.x) * scale : -INFINITY;
-            const float v1 = key + 1 >= lo && key + 1 <= pos ? (x.y + y.y) * scale : -INFINITY;
-            float mx = fmaxf(v0, v1);
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            const float m_old = m_s[row], m_new = fmaxf(m_old, mx);
-            const float p0 = v0 == -INFINITY ? 0.f : expf(v0 - m_new), p1 = v1 == -INFINITY ? 0.f : expf(v1 - m_new);
-            const unsigned pb = pack_bf16(p0, p1);
-            const float2 pf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pb));
-            *reinterpret_cast<unsigned*>(p_s + row * SP + 2 * g) = pb;
-            if (PAIR) *reinterpret_cast<unsigned*>(p_s + (LT_ROWS + row) * SP + 2 * g) = pack_bf16(p0 - pf.x, p1 - pf.y);
-            float sum = PAIR ? p0 + p1 : pf.x + pf.y;             // the sum of what the product will multiply
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            return at;
+        };
+        int at = places(0);
+        for (int i = 0; i < cnt; ++i) {
+            unsigned long long* bar = &full[i % NST];
+            bool ok = true;
+            if (i >= NST) ok = mbar_wait(&empty[i % NST], (i / NST - 1) & 1, abort_flag, err);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            bf16* dst = k_s + ((i % NST) * LD_KEYS + lane) * SK;
+            if (at < 0)
+                for (int x = 0; x < dk; x += 8) *reinterpret_cast<uint4*>(dst + x) = make_uint4(0, 0, 0, 0);
+            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");      // (a later copy may land on such a row)
+            const int rows = __popc(__ballot_sync(0xffffffffu, at >= 0));
+            if (lane == 0) mbar_expect_tx(bar, rows * dk * 2);
             __syncwarp();
-            if (g == 0) {
-                const float corr = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
-                c_s[row] = corr;
-                l_s[row] = l_s[row] * corr + sum;
-                m_s[row] = m_new;
-            }
+            if (at >= 0)
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
+                             ::"r"(tc_smem(dst)), "l"(pages + (size_t)at * dk), "r"(dk * 2), "r"(tc_smem(bar)) : "memory");
+            at = places(i + 1);
         }
-        __syncthreads();
-        {                                                         // O = O * corr + P V over this warp's columns
-            const float ca = c_s[lane >> 2], cb = c_s[(lane >> 2) + 8];
+    } else {
+        const int steps = dk / 16, kg = warp & 3, kh = warp >> 2;
+        const int step0 = kh ? (steps + 1) / 2 : 0, step1 = kh ? steps : (steps + 1) / 2;
+        float acc[NT][4];
+        int n = 0, c_begin = 0, pos = 0, lo = 0;
+        bool fresh = true;
+        for (int i = 0; i < cnt; ++i) {
+            if (fresh) {                                              // a request begins: its queries, an empty softmax
+                fresh = false;
+                n = ld_chunks(q_len, ctx_len, R, window, r, first);
+                c_begin = c;
+                pos = ctx_len[r];
+                lo = window > 0 ? max(pos - window + 1, 0) : 0;
+                if (i > 0) ld_sync();                                 // the last one's sums have been read
+                const int t = q_start[r];
+                for (int rr = warp; rr < LT_ROWS; rr += LD_THREADS / 32) {
+                    const bool on = h0 + rr < H;
+                    const float* src = q_full + ((size_t)t * H + h0 + rr) * dk;
+                    for (int x = lane * 4; x < dk; x += 128) {
+                        const float4 v = on ? *reinterpret_cast<const float4*>(src + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+                        *reinterpret_cast<uint2*>(q_s + rr * SK + x) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+                    }
+                }
+                if (tid < LT_ROWS) {
+                    const bool leaks = sink && c == 0 && h0 + tid < H;
+                    m_s[tid] = leaks ? sink[h0 + tid] : -INFINITY;
+                    l_s[tid] = leaks ? 1.f : 0.f;
+                }
 #pragma unroll
-            for (int x = 0; x < NT; ++x) {
-                acc[x][0] *= ca;
-                acc[x][1] *= ca;
-                acc[x][2] *= cb;
-                acc[x][3] *= cb;
+                for (int x = 0; x < NT; ++x) acc[x][0] = acc[x][1] = acc[x][2] = acc[x][3] = 0.f;
+                ld_sync();
             }
+            const bool ok = mbar_wait(&full[i % NST], (i / NST) & 1, abort_flag, err);
+            __syncwarp();
+            const bf16* ks = k_s + (i % NST) * LD_KEYS * SK;
+            {
+                float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+                const bf16* qa = q_s + (lane & 15) * SK + (lane >> 4) * 8;
+                const bf16* kb = ks + (kg * 8 + (lane & 7)) * SK + (lane >> 3) * 8;
+#pragma unroll 3
+                for (int st = step0; st < step1; st += 2) {           // two steps of 16: one load of keys
+                    unsigned a[4], b0, b1, b2, b3;
+                    ldsm_x4(b0, b1, b2, b3, kb + st * 16);
+                    ldsm_x4(a[0], a[1], a[2], a[3], qa + st * 16);
+                    mma16816(s0, a, b0, b1);
+                    if (st + 1 < step1) {
+                        ldsm_x4(a[0], a[1], a[2], a[3], qa + st * 16 + 16);
+                        mma16816(s1, a, b2, b3);
+                    }
+                }
+                float* d = s_s + kh * LT_ROWS * SS + (lane >> 2) * SS + kg * 8 + (lane & 3) * 2;
+                *reinterpret_cast<float2*>(d) = make_float2(s0[0] + s1[0], s0[1] + s1[1]);
+                *reinterpret_cast<float2*>(d + 8 * SS) = make_float2(s0[2] + s1[2], s0[3] + s1[3]);
+            }
+            // all scores are there; nobody multiplies the weights and values of the chunk before any more
+            if (ld_sync_any(!ok)) break;
+            {                                                         // running softmax: sixteen threads a row, two keys a thread
+                const int row = tid >> 4, g = tid & 15, key = (first + c) * LD_KEYS + 2 * g;
+                const float2 x = *reinterpret_cast<const float2*>(s_s + row * SS + 2 * g);
+                const float2 y = *reinterpret_cast<const float2*>(s_s + (LT_ROWS + row) * SS + 2 * g);
+                const float v0 = key >= lo && key <= pos ? (x.x + y.x) * scale : -INFINITY;
+                const float v1 = key + 1 >= lo && key + 1 <= pos ? (x.y + y.y) * scale : -INFINITY;
+                float mx = fmaxf(v0, v1);
 #pragma unroll
-            for (int kk = 0; kk < LD_KEYS; kk += 16) {
-                unsigned a[4], a2[4];
-                ldsm_x4(a[0], a[1], a[2], a[3], p_s + (lane & 15) * SP + kk + (lane >> 4) * 8);
-                if (PAIR) ldsm_x4(a2[0], a2[1], a2[2], a2[3], p_s + LT_ROWS * SP + (lane & 15) * SP + kk + (lane >> 4) * 8);
-                const bf16* vb = ks + (kk + (lane & 7) + ((lane >> 3) & 1) * 8) * SK + warp * 8 * NT + (lane >> 4) * 8;
+                for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                const float m_old = m_s[row], m_new = fmaxf(m_old, mx);
+                const float p0 = v0 == -INFINITY ? 0.f : expf(v0 - m_new), p1 = v1 == -INFINITY ? 0.f : expf(v1 - m_new);
+                const unsigned pb = pack_bf16(p0, p1);
+                const float2 pf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pb));
+                *reinterpret_cast<unsigned*>(p_s + row * SP + 2 * g) = pb;
+                if (PAIR) *reinterpret_cast<unsigned*>(p_s + (LT_ROWS + row) * SP + 2 * g) = pack_bf16(p0 - pf.x, p1 - pf.y);
+                float sum = PAIR ? p0 + p1 : pf.x + pf.y;             // the sum of what the product will multiply
 #pragma unroll
-                for (int np = 0; np < (NT + 1) / 2; ++np) {
-                    unsigned b0, b1, b2, b3;
-                    ldsm_x4_t(b0, b1, b2, b3, vb + np * 16);
-                    mma16816(acc[2 * np], a, b0, b1);
-                    if (2 * np + 1 < NT) mma16816(acc[2 * np + 1 < NT ? 2 * np + 1 : 0], a, b2, b3);
-                    if (PAIR) {
-                        mma16816(acc[2 * np], a2, b0, b1);
-                        if (2 * np + 1 < NT) mma16816(acc[2 * np + 1 < NT ? 2 * np + 1 : 0], a2, b2, b3);
+                for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                __syncwarp();
+                if (g == 0) {
+                    const float corr = m_old == -INFINITY ? 0.f : expf(m_old - m_new);
+                    c_s[row] = corr;
+                    l_s[row] = l_s[row] * corr + sum;
+                    m_s[row] = m_new;
+                }
+            }
+            ld_sync();
+            {                                                         // O = O * corr + P V over this warp's columns
+                const float ca = c_s[lane >> 2], cb = c_s[(lane >> 2) + 8];
+#pragma unroll
+                for (int x = 0; x < NT; ++x) {
+                    acc[x][0] *= ca;
+                    acc[x][1] *= ca;
+                    acc[x][2] *= cb;
+                    acc[x][3] *= cb;
+                }
+#pragma unroll
+                for (int kk = 0; kk < LD_KEYS; kk += 16) {
+                    unsigned a[4], a2[4];
+                    ldsm_x4(a[0], a[1], a[2], a[3], p_s + (lane & 15) * SP + kk + (lane >> 4) * 8);
+                    if (PAIR) ldsm_x4(a2[0], a2[1], a2[2], a2[3], p_s + LT_ROWS * SP + (lane & 15) * SP + kk + (lane >> 4) * 8);
+                    const bf16* vb = ks + (kk + (lane & 7) + ((lane >> 3) & 1) * 8) * SK + warp * 8 * NT + (lane >> 4) * 8;
+#pragma unroll
+                    for (int np = 0; np < (NT + 1) / 2; ++np) {
+                        unsigned b0, b1, b2, b3;
+                        ldsm_x4_t(b0, b1, b2, b3, vb + np * 16);
+                        mma16816(acc[2 * np], a, b0, b1);
+                        if (2 * np + 1 < NT) mma16816(acc[2 * np + 1 < NT ? 2 * np + 1 : 0], a, b2, b3);
+                        if (PAIR) {
+                            mma16816(acc[2 * np], a2, b0, b1);
+                            if (2 * np + 1 < NT) mma16816(acc[2 * np + 1 < NT ? 2 * np + 1 : 0], a2, b2, b3);
+                        }
                     }
                 }
             }
-        }
-        ++c;
-        if (c < n && i + 1 < cnt) continue;
-        // the request, or the stretch, ends here
-        const int ra = lane >> 2, rb = ra + 8, t = q_start[r];
-        const bool whole = c_begin == 0 && c == n;
-        const size_t slot = (size_t)(blockIdx.x + r) * H;
-        const float ia = whole ? (l_s[ra] > 0.f ? 1.0f / l_s[ra] : 0.f) : 1.f, ib = whole ? (l_s[rb] > 0.f ? 1.0f / l_s[rb] : 0.f) : 1.f;
+            __syncwarp();
+            if (lane == 0) mbar_arrive_plain(&empty[i % NST]);
+            ++c;
+            if (c < n && i + 1 < cnt) continue;
+            // the request, or the stretch, ends here
+            const int ra = lane >> 2, rb = ra + 8, t = q_start[r];
+            const bool whole = c_begin == 0 && c == n;
+            const size_t slot = (size_t)(blockIdx.x + r) * H;
+            const float ia = whole ? (l_s[ra] > 0.f ? 1.0f / l_s[ra] : 0.f) : 1.f, ib = whole ? (l_s[rb] > 0.f ? 1.0f / l_s[rb] : 0.f) : 1.f;
 #pragma unroll
-        for (int x = 0; x < NT; ++x) {
-            const int col = warp * 8 * NT + x * 8 + (lane & 3) * 2;
+            for (int x = 0; x < NT; ++x) {
+                const int col = warp * 8 * NT + x * 8 + (lane & 3) * 2;
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int hh = h0 + (e ? rb : ra);
-                if (hh >= H) continue;
-                const float u = acc[x][2 * e] * (e ? ib : ia), v = acc[x][2 * e + 1] * (e ? ib : ia);
-                if (whole) *reinterpret_cast<unsigned*>(out + ((size_t)t * H + hh) * RANK + col) = pack_bf16(u, v);
-                else *reinterpret_cast<float2*>(part_o + (slot + hh) * RANK + col) = make_float2(u, v);
+                for (int e = 0; e < 2; ++e) {
+                    const int hh = h0 + (e ? rb : ra);
+                    if (hh >= H) continue;
+                    const float u = acc[x][2 * e] * (e ? ib : ia), v = acc[x][2 * e + 1] * (e ? ib : ia);
+                    if (whole) *reinterpret_cast<unsigned*>(out + ((size_t)t * H + hh) * RANK + col) = pack_bf16(u, v);
+                    else *reinterpret_cast<float2*>(part_o + (slot + hh) * RANK + col) = make_float2(u, v);
+                }
             }
+            if (!whole && tid < LT_ROWS && h0 + tid < H) {
+                part_ml[(slot + h0 + tid) * 2] = m_s[tid];
+                part_ml[(slot + h0 + tid) * 2 + 1] = l_s[tid];
+            }
+            c = 0;
+            fresh = true;
+            if (i + 1 < cnt)
+                do n = ld_chunks(q_len, ctx_len, R, window, ++r, first);
+                while (n == 0 && r < R);
         }
-        if (!whole && tid < LT_ROWS && h0 + tid < H) {
-            part_ml[(slot + h0 + tid) * 2] = m_s[tid];
-            part_ml[(slot + h0 + tid) * 2 + 1] = l_s[tid];
-        }
-        c = 0;
-        fresh = true;
-        if (i + 1 < cnt)
-            do n = ld_chunks(q_len, ctx_len, R, window, ++r, first);
-            while (n == 0 && r < R);
+    }
+    __syncthreads();
+    if (*abort_flag && tid == 0) {      // give copies in flight a bounded time to land
+        for (int i = 0; i < NST; ++i)
+            for (unsigned k = 0; k < (1u << 16) && !mbar_try_wait(&full[i], 0) && !mbar_try_wait(&full[i], 1); ++k) {}
     }
 }
 
@@ -567,7 +606,7 @@ extern "C" int aie_latent_decode(const float* q_full, const void* pages, void* o
         auto kern = latent_decode_kernel<NT, PV, CTAS>;                                                                 \
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                         \
         if (e == cudaSuccess)                                                                                           \
-            e = launch_pdl(kern, grid, dim3(LD_THREADS), smem, st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, \
+            e = launch_pdl(kern, grid, dim3(LD_THREADS + 32), smem, st, q_full, (const bf16*)pages, (bf16*)out, part_o, part_ml, \
                            q_start, q_len, ctx_len, block_table, bt_width, num_pages, P, R, H, dk, window, scale, sink, err); \
     }
 #define GO(NT)                                                                                                          \
