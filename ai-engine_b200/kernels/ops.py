@@ -28,7 +28,7 @@ def dtype_code(t) -> int:
 
 
 def _p(t: Optional[torch.Tensor]):
-    return c_void_p(0 if t is None else t.data_ptr())
+    return None if t is None else c_void_p(t.data_ptr())
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -43,7 +43,9 @@ def _stream():
 
 
 def _nb(*ts) -> int:
-    """Bytes of the given tensors (what a kernel that touches each once has to move)."""
+    """Bytes of the given tensors (what a kernel that touches each once has to move); 0 while nobody records them."""
+    if not _profiling():
+        return 0
     return sum(t.numel() * t.element_size() for t in ts if t is not None)
 
 
@@ -73,7 +75,7 @@ def embed_gather(ids: torch.Tensor, table: torch.Tensor, err: torch.Tensor,
     _dev(ids, table, err)
     T, (V, D) = ids.shape[0], table.shape
     if out is None:
-        out = torch.empty((T, D), dtype=torch.float32, device=table.device)
+        out = table.new_empty(T, D, dtype=torch.float32)
     lib = library("elementwise.cu")
     with region("embed_gather", T * D * table.element_size() + _nb(out)):
         check(lib.aie_embed_gather(_p(ids), _p(table), c_int(dtype_code(table)), _p(out), c_int(T),
@@ -111,7 +113,7 @@ def add_rmsnorm(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Te
         raise KernelError("add_rmsnorm: delta shape differs from x")
     n = x.shape[0] if rows is None else rows.shape[0]
     if out is None:
-        out = torch.empty((n, D), dtype=out_dtype, device=x.device)
+        out = x.new_empty(n, D, dtype=out_dtype)
     lib = library("elementwise.cu")
     stored = write_back and rows is None and delta is not None      # without a branch to add, the stream is as it was
     with region("add_rmsnorm", n * D * 4 * (2 if stored else 1) + (_nb(delta) if rows is None else 0) + _nb(out)):
@@ -141,8 +143,8 @@ def add_rmsnorm_pair(x: torch.Tensor, delta: Optional[torch.Tensor], w1: torch.T
         parts, stride = (delta.shape[0], delta.stride(0)) if delta.dim() == 3 else (1, 0)
         if delta.shape[-2:] != x.shape:
             raise KernelError("add_rmsnorm_pair: delta differs in shape from x")
-    out1 = torch.empty((T, D), dtype=out_dtype, device=x.device)
-    out2 = torch.empty((T, D), dtype=out_dtype, device=x.device) if w2 is not None else None
+    out1 = x.new_empty(T, D, dtype=out_dtype)
+    out2 = x.new_empty(T, D, dtype=out_dtype) if w2 is not None else None
     stored = any(t is not None for t in (delta, extra, step))
     lib = library("elementwise.cu")
     with region("add_rmsnorm_pair", (2 if stored else 1) * _nb(x) + _nb(delta, extra, out1, out2)):
@@ -166,7 +168,7 @@ def silu_mul(gu: torch.Tensor, out: Optional[torch.Tensor] = None, block: int = 
     T, F2 = gu.shape
     F = F2 // 2
     if out is None:
-        out = torch.empty((T, F), dtype=gu.dtype, device=gu.device)
+        out = gu.new_empty(T, F, dtype=gu.dtype)
     lib = library("elementwise.cu")
     with region("silu_mul", _nb(gu, out)):
         check(lib.aie_silu_mul(_p(gu), _p(out), c_int(dtype_code(gu)), c_int(T), c_int(F), c_int(block),
@@ -199,7 +201,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, rows: Optional[torch.Tensor] = No
         raise KernelError(f"gemm_f32: inner sizes differ ({K} vs {w.shape[1]})")
     M = a.shape[0] if rows is None else rows.shape[0]
     if out is None:
-        out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+        out = a.new_empty(M, N, dtype=torch.float32)
     lib = library("gemm_f32.cu")
     with region("gemm_f32", _nb(w, out) + M * K * 4, 2.0 * M * N * K):
         check(lib.aie_gemm_f32(_p(a), _p(w), c_int(dtype_code(w)), _p(out), _p(rows), c_int(M), c_int(N),
@@ -273,11 +275,11 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, err: torch
             raise KernelError("gemm_tc: the buffer for the parts does not fit")
         raw_parts = splits > 1
     elif raw_parts and splits > 1:
-        out = torch.empty((splits, T, N), dtype=torch.float32, device=x.device)
+        out = x.new_empty(splits, T, N, dtype=torch.float32)
     else:
         raw_parts = False
         splits = min(splits, 8)              # joined inside a cluster of at most 8 CTAs
-        out = torch.empty((T, N // 2 if swiglu else N), dtype=out_dtype, device=x.device)
+        out = x.new_empty(T, N // 2 if swiglu else N, dtype=out_dtype)
     lib = library("gemm_tc.cu")
     with region("gemm_tc_swiglu" if swiglu else "gemm_tc", _nb(x, w, out), 2.0 * T * N * K):
         check(lib.aie_gemm_tc(_p(x), _p(w), _p(out), c_int(dtype_code(out)), c_int(T), c_int(N), c_int(K),
@@ -408,7 +410,7 @@ def linear_rope_kv(x: torch.Tensor, w_qkv: torch.Tensor, k_pages: torch.Tensor, 
     kb = (Kin + 63) // 64
     splits = max(1, min(8, kb // 8, (3 * sm_count()) // max(1, N // 128)))
     splits = -(-kb // -(-kb // splits))
-    q_out = torch.empty((T, H, d), dtype=torch.bfloat16, device=x.device)
+    q_out = x.new_empty(T, H, d, dtype=torch.bfloat16)
     lib = library("gemm_tc.cu")
     with region("gemm_tc_rope", _nb(x, w_qkv) + T * N * 2, 2.0 * T * N * Kin):
         check(lib.aie_gemm_tc_rope(_p(x), _p(w_qkv), c_int(T), c_int(N), c_int(Kin), c_int(bn), c_int(splits),
@@ -440,7 +442,7 @@ def rope_kv_write(qkv: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tenso
         raise KernelError("rope_kv_write: qkv must be in the cache's dtype or float32")
     rot = inv_freq.shape[0] * 2
     if q_out is None:
-        q_out = torch.empty((T, H, d), dtype=k_pages.dtype, device=qkv.device)
+        q_out = qkv.new_empty(T, H, d, dtype=k_pages.dtype)
     lib = library("rope_kv.cu")
     with region("rope_kv_write", _nb(qkv) + T * (H + 2 * K) * d * k_pages.element_size()):
         check(lib.aie_rope_kv_write(_p(qkv), c_int(dtype_code(qkv)), c_int(parts), c_longlong(part_stride),
@@ -516,8 +518,8 @@ def paged_attention_decode(q, k_pages, v_pages, dec_tokens, positions, token_req
     n = dec_tokens.shape[0]
     part_o = part_lse = counters = None
     if splits > 1:
-        part_o = torch.empty((n, H, splits, d), dtype=torch.float32, device=q.device)
-        part_lse = torch.empty((n, H, splits), dtype=torch.float32, device=q.device)
+        part_o = q.new_empty(n, H, splits, d, dtype=torch.float32)
+        part_lse = q.new_empty(n, H, splits, dtype=torch.float32)
         if join_in_kernel:
             counters = _decode_counters(q.device, n * K * ((H // K + 7) // 8))
     lib = library("attention_fast.cu")
@@ -782,7 +784,7 @@ def short_conv(h: torch.Tensor, w: torch.Tensor, state: torch.Tensor, ctx, out_d
         raise KernelError("short_conv: inputs, taps and state are float32")
     if w.shape[0] != D or state.shape[1:] != (max(taps - 1, 0), D):
         raise KernelError("short_conv: shapes do not fit")
-    out = torch.empty((T, D), dtype=out_dtype, device=h.device)
+    out = h.new_empty(T, D, dtype=out_dtype)
     lib = library("sequence_ops.cu")
     with region("short_conv", _nb(h, out)):
         check(lib.aie_short_conv(_p(h), _p(w), _p(state), _p(out), c_int(dtype_code(out)), _p(ctx.q_start),
@@ -818,7 +820,7 @@ def polynorm(z: torch.Tensor, coef: torch.Tensor, eps: float, out_dtype: torch.d
     if z.dtype != torch.float32 or coef.dtype != torch.float32 or coef.numel() != 4:
         raise KernelError("polynorm: float32 input and four float32 coefficients")
     T, F = z.shape
-    out = torch.empty((T, F), dtype=out_dtype, device=z.device)
+    out = z.new_empty(T, F, dtype=out_dtype)
     lib = library("sequence_ops.cu")
     with region("polynorm", _nb(z, out)):
         check(lib.aie_polynorm(_p(z), _p(coef), _p(out), c_int(dtype_code(out)), c_int(T), c_int(F), c_float(eps),
@@ -835,7 +837,7 @@ def head_norm_gate(o: torch.Tensor, gate: Optional[torch.Tensor], weight: Option
     if o.dtype != torch.float32 or (gate is not None and (gate.dtype != torch.float32 or gate.stride(1) != 1
                                                           or gate.shape != (T, H * dv))):
         raise KernelError("head_norm_gate: shapes or dtypes do not fit")
-    out = torch.empty((T, H * dv), dtype=out_dtype, device=o.device)
+    out = o.new_empty(T, H * dv, dtype=out_dtype)
     lib = library("sequence_ops.cu")
     with region("head_norm_gate", 2 * _nb(o) + _nb(out)):
         check(lib.aie_head_norm_gate(_p(o), _p(gate), c_int(gate.stride(0) if gate is not None else 0), _p(weight), _p(out),
@@ -852,7 +854,7 @@ def clamped_glu(gu: torch.Tensor, F: int, limit: float, alpha: float, shift: flo
     if gu.dtype != torch.float32 or gu.stride(1) != 1 or gu.shape[1] < 2 * F:
         raise KernelError("clamped_glu: float32 [T, >= 2F] input")
     T = gu.shape[0]
-    out = torch.empty((T, F), dtype=out_dtype, device=gu.device)
+    out = gu.new_empty(T, F, dtype=out_dtype)
     lib = library("sequence_ops.cu")
     with region("clamped_glu", 2 * T * F * 4 + _nb(out)):
         check(lib.aie_clamped_glu(_p(gu), c_int(gu.stride(0)), _p(out), c_int(dtype_code(out)), c_longlong(T),
@@ -883,10 +885,10 @@ def low_rank_decay(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor
     if x.dtype != torch.float32 or x.shape[1] != rank or x.stride(1) != 1:
         raise KernelError("low_rank_decay: x is a float32 view [T, rank]")
     if rank > LOW_RANK_DECAY or T > 1 << 19:
-        z = torch.empty((T, N), dtype=torch.float32, device=x.device)
+        z = x.new_empty(T, N, dtype=torch.float32)
         return gated_decay(gemm_f32_ex(x, w, z, T, N, rank, x.stride(0), N), bias, tau)
     _dev(w, bias)
-    out = torch.empty((T, N), dtype=torch.float32, device=x.device)
+    out = x.new_empty(T, N, dtype=torch.float32)
     with region("low_rank_decay", _nb(w, out) + T * rank * 4, 2.0 * T * N * rank):
         check(library("sequence_ops.cu").aie_low_rank_decay(
             _p(x), c_int(x.stride(0)), _p(w), c_int(dtype_code(w)), _p(bias), _p(out), c_int(T), c_int(N), c_int(rank), c_float(tau),
@@ -926,7 +928,7 @@ def expert_combine(y: torch.Tensor, pair_row: torch.Tensor, top: int, weight: fl
     if y.dtype != torch.float32 or (shared is not None and (shared.dtype != torch.float32 or gate is None or
                                                             gate.dtype != torch.float32)):
         raise KernelError("expert_combine: float32 operands")
-    out = torch.empty((T, D), dtype=torch.float32, device=y.device)
+    out = y.new_empty(T, D, dtype=torch.float32)
     lib = library("sequence_ops.cu")
     with region("expert_combine", (top + 2) * T * D * 4):
         check(lib.aie_expert_combine(_p(y), _p(pair_row), c_int(top), c_float(weight), _p(shared), _p(gate),
@@ -957,9 +959,9 @@ def latent_prepare(proj: torch.Tensor, H: int, d: int, rot: int, rank: int, c_we
     if proj.dtype != torch.float32 or ld < need or pages.shape[1] != 1 or pages.shape[3] != rank + rot:
         raise KernelError("latent_prepare: shapes or dtypes do not fit")
     n = T if short_row is None else n_short
-    q_plain = torch.empty((n, H, d), dtype=q_dtype, device=proj.device) if folded else None
-    q_full = torch.empty((n, H, rank + rot), dtype=torch.float32, device=proj.device) if folded else None
-    q_all = torch.empty((T, H, d + rot), dtype=q_dtype, device=proj.device) if whole else None
+    q_plain = proj.new_empty(n, H, d, dtype=q_dtype) if folded else None
+    q_full = proj.new_empty(n, H, rank + rot, dtype=torch.float32) if folded else None
+    q_all = proj.new_empty(T, H, d + rot, dtype=q_dtype) if whole else None
     lib = library("latent_attention.cu")
     with region("latent_prepare", _nb(proj, q_plain, q_all) + (n * H * rot * 4 if folded else 0)):
         check(lib.aie_latent_prepare(_p(proj), c_int(ld), c_int(T), c_int(H), c_int(d), c_int(rot), c_int(rank),
@@ -1034,7 +1036,7 @@ def latent_prompt(q: torch.Tensor, pages: torch.Tensor, w_expand: torch.Tensor, 
         for n, c in zip(ctx.h_q_len[work.expanded].tolist(), ctx.h_ctx_len[work.expanded].tolist()):
             pairs += float(sum(min(c + i + 1, window) if window > 0 else c + i + 1 for i in range(n)))
     for g0, g1, p0, p1, step in work.groups:
-        rows = torch.empty((128 * (g1 - g0), dk), dtype=torch.bfloat16, device=q.device)
+        rows = q.new_empty(128 * (g1 - g0), dk, dtype=torch.bfloat16)
         with region("latent_gather", 2 * _nb(rows)):
             check(library("latent_attention_tc.cu").aie_latent_gather(
                 _p(pages), _p(rows), _p(work.gather[g0:g1]), c_int(g1 - g0), _p(ctx.q_len), _p(ctx.ctx_len), _p(block_table),
@@ -1087,7 +1089,7 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
     if (q_full.dtype != torch.float32 or pages.shape[3] != dk or pages.shape[1] != 1
             or (sink is not None and (sink.dtype != torch.float32 or sink.shape != (H,)))):
         raise KernelError("latent_attention: shapes or dtypes do not fit")
-    out = torch.empty((T, H, rank), dtype=out_dtype, device=q_full.device)
+    out = q_full.new_empty(T, H, rank, dtype=out_dtype)
     fast = (work is not None and pages.dtype == torch.bfloat16 and out_dtype == torch.bfloat16 and rank % 64 == 0
             and 64 <= rank <= 512 and dk % 16 == 0 and dk <= 1024)
     starts = work.short_start if compact else ctx.q_start
@@ -1105,8 +1107,8 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
                 splits = max(1, min(64, (keys + 63) // 64, (2 * sm_count()) // ctas))
                 part_o = part_ml = None
                 if splits > 1:
-                    part_o = torch.empty((T, H, splits, rank), dtype=torch.float32, device=q_full.device)
-                    part_ml = torch.empty((T, H, splits, 2), dtype=torch.float32, device=q_full.device)
+                    part_o = q_full.new_empty(T, H, splits, rank, dtype=torch.float32)
+                    part_ml = q_full.new_empty(T, H, splits, 2, dtype=torch.float32)
                 with region("latent_attention_tc", *cost):
                     check(library("latent_attention_tc.cu").aie_latent_attention_tc(
                         _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(work.tiles), c_int(work.tiles.shape[0]),
@@ -1125,8 +1127,8 @@ def latent_attention(q_full: torch.Tensor, pages: torch.Tensor, ctx, block_table
         # one token a request: the visible rows of all of them in equal stretches, one a CTA.  (Behind the other kernel, whose
         # join of parts runs over every token's row.)
         G = max(1, 2 * sm_count() // ((H + 15) // 16))
-        part_o = torch.empty((G + ctx.R, H, rank), dtype=torch.float32, device=q_full.device)
-        part_ml = torch.empty((G + ctx.R, H, 2), dtype=torch.float32, device=q_full.device)
+        part_o = q_full.new_empty(G + ctx.R, H, rank, dtype=torch.float32)
+        part_ml = q_full.new_empty(G + ctx.R, H, 2, dtype=torch.float32)
         with region("latent_decode", *_latent_cost(q_full, pages, ctx, rank, window, lambda lens: lens == 1)):
             check(library("latent_attention_tc.cu").aie_latent_decode(
                 _p(q_full), _p(pages), _p(out), _p(part_o), _p(part_ml), _p(starts), _p(ctx.q_len), _p(ctx.ctx_len),
@@ -1265,7 +1267,7 @@ def linear_recurrence(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_t
             or (not keyless and (k.dtype != torch.float32 or k.stride(0) != ld))
             or state.shape[1:] != (H, d, dv) or state.dtype != torch.float32):
         raise KernelError("linear_recurrence: shapes or dtypes do not fit")
-    out = torch.empty((T, H, dv), dtype=torch.float32, device=q.device)
+    out = q.new_empty(T, H, dv, dtype=torch.float32)
     max_len = 0
     if (chunked and dt_raw is not None and decay_tok is None and d <= 128 and ctx.max_q_len >= SSD_MIN_TOKENS
             and not os.environ.get("AI_ENGINE_B200_NO_CHUNKED_SCAN")):      # the switch is for measurement
@@ -1318,7 +1320,7 @@ def gather_rows(src: torch.Tensor, rows: torch.Tensor, zero_fill: bool = True, l
     are not padding (for the byte count of a profile).  out: a tensor of that shape to write to."""
     _dev(src, rows, out)
     if out is None:
-        out = torch.empty((rows.shape[0], src.shape[1]), dtype=src.dtype, device=src.device)
+        out = src.new_empty(rows.shape[0], src.shape[1], dtype=src.dtype)
     elif out.shape != (rows.shape[0], src.shape[1]) or out.dtype != src.dtype or not out.is_contiguous():
         raise KernelError("gather_rows: out does not fit")
     lib = library("sequence_ops.cu")
@@ -1362,7 +1364,7 @@ def grouped_linear(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, out_d
     take the tcgen05 kernels, everything else the float32 kernel on the CUDA cores."""
     E, N, K = w.shape
     rows = tile_w.shape[0] * EXPERT_TILE
-    out = torch.empty((rows, N), dtype=out_dtype, device=x.device)
+    out = x.new_empty(rows, N, dtype=out_dtype)
     if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and N % 128 == 0 and K % 8 == 0:
         if grouped_takes_items(tile_w.shape[0], E, N):
             _grouped_items(x, w, tile_w, out, err, row_src, live)
@@ -1387,7 +1389,7 @@ def grouped_glu(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, limit: f
     E, N, K = w.shape
     if (x.dtype == w.dtype == out_dtype == torch.bfloat16 and N % 128 == 0 and K % 8 == 0
             and tile_w.shape[0] <= GROUPED_MAX_TILES):
-        out = torch.empty((tile_w.shape[0] * EXPERT_TILE, N // 2), dtype=out_dtype, device=x.device)
+        out = x.new_empty(tile_w.shape[0] * EXPERT_TILE, N // 2, dtype=out_dtype)
         _grouped_items(x, w, tile_w, out, err, row_src, live, (limit, alpha, shift))
         return out
     gu = grouped_linear(x, w, tile_w, torch.float32, err, row_src=row_src, live=live)
@@ -1414,7 +1416,7 @@ def causal_conv(u: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
         raise KernelError("causal_conv: shapes do not fit")
     if activation not in (None, "silu"):
         raise KernelError(f"causal_conv: activation `{activation}` is not known (silu)")
-    out = torch.empty((T, C + dup_n), dtype=out_dtype, device=u.device)
+    out = u.new_empty(T, C + dup_n, dtype=out_dtype)
     lib = library("sequence_ops.cu")
     with region("causal_conv", T * C * 4 + _nb(out)):
         check(lib.aie_causal_conv(_p(u), c_int(u.stride(0)), _p(w), _p(bias), _p(state), _p(out), c_int(dtype_code(out)),
@@ -1434,7 +1436,7 @@ def gate_group_norm(y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, part
     if (y.dtype != torch.float32 or z.dtype != torch.float32 or z.shape != (T, W) or z.stride(1) != 1
             or weight.dtype != torch.float32 or weight.shape != (W,) or parts < 1 or W % parts):
         raise KernelError("gate_group_norm: shapes or dtypes do not fit")
-    out = torch.empty((T, W), dtype=out_dtype, device=y.device)
+    out = y.new_empty(T, W, dtype=out_dtype)
     lib = library("sequence_ops.cu")
     with region("gate_group_norm", 2 * _nb(y) + _nb(out)):
         check(lib.aie_gate_group_norm(_p(y), _p(z), c_int(z.stride(0)), _p(weight), _p(out), c_int(dtype_code(out)),
@@ -1455,9 +1457,9 @@ def route_topk(logits: torch.Tensor, correction: Optional[torch.Tensor], groups:
     if logits.dtype != torch.float32 or logits.stride(1) != 1 or (correction is not None and (correction.dtype != torch.float32 or
                                                                     correction.shape != (E,))):
         raise KernelError("route_topk: float32 logits and correction")
-    ids = torch.empty((T, top), dtype=torch.int32, device=logits.device)
-    weights = torch.empty((T, top), dtype=torch.float32, device=logits.device)
-    scratch = torch.empty((T, E), dtype=torch.float32, device=logits.device)
+    ids = logits.new_empty(T, top, dtype=torch.int32)
+    weights = logits.new_empty(T, top, dtype=torch.float32)
+    scratch = logits.new_empty(T, E, dtype=torch.float32)
     lib = library("sequence_ops.cu")
     with region("route_topk", 3 * _nb(scratch)):
         check(lib.aie_route_topk(_p(logits), c_int(logits.stride(0)), _p(scratch), _p(correction), c_int(T), c_int(E), c_int(groups), c_int(keep),
@@ -1479,7 +1481,7 @@ def expert_combine_weighted(y: torch.Tensor, pair_row: torch.Tensor, weights: to
     D = h.shape[1]
     if y.dtype != torch.float32 or weights.dtype != torch.float32 or y.shape[1] != D or pair_row.numel() != T * top:
         raise KernelError("expert_combine_weighted: shapes or dtypes do not fit")
-    out = torch.empty((T, D), dtype=torch.float32, device=y.device)
+    out = y.new_empty(T, D, dtype=torch.float32)
     lib = library("sequence_ops.cu")
     with region("expert_combine", (top + 2) * T * D * 4):
         check(lib.aie_expert_combine_weighted(_p(y), _p(pair_row), _p(weights), c_int(top), _p(h), c_int(dtype_code(h)),
@@ -1577,7 +1579,7 @@ def join_streams(x: torch.Tensor, delta: Optional[torch.Tensor], y: torch.Tensor
         parts, stride = (delta.shape[0], delta.stride(0)) if delta.dim() == 3 else (1, 0)
         if delta.shape[-2:] != x.shape:
             raise KernelError("join_streams: delta differs in shape from x")
-    out = torch.empty((T, 2 * D), dtype=out_dtype, device=x.device)
+    out = x.new_empty(T, 2 * D, dtype=out_dtype)
     lib = library("elementwise.cu")
     with region("join_streams", _nb(x, delta, y, out)):
         check(lib.aie_join_streams(_p(x), _p(delta), c_int(dtype_code(delta) if delta is not None else 0), c_int(parts),
@@ -1597,8 +1599,8 @@ def sink_attn_prepare(proj: torch.Tensor, bias: Optional[torch.Tensor], pages: t
     if (proj.dtype != torch.float32 or ld < H * d + G * (d + e) + H or pages.shape[1] != G or pages.shape[3] != d + e
             or (bias is not None and (bias.dtype != torch.float32 or bias.numel() != H * d + G * (d + e)))):
         raise KernelError("sink_attn_prepare: shapes or dtypes do not fit")
-    q = torch.empty((T, H, d), dtype=pages.dtype, device=proj.device)
-    gate = torch.empty((T, H), dtype=torch.float32, device=proj.device)
+    q = proj.new_empty(T, H, d, dtype=pages.dtype)
+    gate = proj.new_empty(T, H, dtype=torch.float32)
     lib = library("sink_attention.cu")
     with region("sink_attn_prepare", _nb(proj, q) + T * G * (d + e) * pages.element_size()):
         check(lib.aie_sink_attn_prepare(_p(proj), c_int(ld), _p(bias), _p(q), c_int(dtype_code(q)), _p(pages),
@@ -1651,7 +1653,7 @@ def sink_attention(q: torch.Tensor, pages: torch.Tensor, gate: Optional[torch.Te
         raise KernelError("sink_attention: the gate's logits are a float32 view [T, H * e]")
     extras = (c_float(softcap), c_int(1 if tied else 0), _p(gate_logits),
               c_int(gate_logits.stride(0) if gate_logits is not None else 0))
-    out = torch.empty((T, H, e), dtype=out_dtype, device=q.device)
+    out = q.new_empty(T, H, e, dtype=out_dtype)
     out32 = out if out_dtype == torch.float32 else None
     cost = (0.0, 0.0)
     if _profiling() and hasattr(ctx, "h_q_len"):
@@ -1678,8 +1680,8 @@ def sink_attention(q: torch.Tensor, pages: torch.Tensor, gate: Optional[torch.Te
             S = min(decode_splits(n, G, H // G, keys), 64)
             part_o = part_lse = None
             if S > 1:
-                part_o = torch.empty((n, H, S, e), dtype=torch.float32, device=q.device)
-                part_lse = torch.empty((n, H, S), dtype=torch.float32, device=q.device)
+                part_o = q.new_empty(n, H, S, e, dtype=torch.float32)
+                part_lse = q.new_empty(n, H, S, dtype=torch.float32)
             share = float(n) / T
             with region("sink_attention_decode", cost[0] * share, cost[1] * share):
                 check(fast.aie_sink_attention_decode(_p(q), _p(pages), _p(out), _p(part_o), _p(part_lse), _p(gate),
@@ -1768,7 +1770,7 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
             or b_raw.dtype != torch.float32 or a_raw.dtype != torch.float32 or b_raw.stride(1) != 1 or a_raw.stride(1) != 1
             or state.shape[1:] != (H, d, e) or state.dtype != torch.float32 or H % G or d > 256):
         raise KernelError("delta_rule: shapes or dtypes do not fit")
-    out = torch.empty((T, H, e), dtype=torch.float32, device=q.device)
+    out = q.new_empty(T, H, e, dtype=torch.float32)
     max_len = 0
     if (chunked and d <= 128 and ctx.max_q_len >= DELTA_MIN_TOKENS
             and not os.environ.get("AI_ENGINE_B200_NO_CHUNKED_SCAN")):      # the switch is for measurement
@@ -1776,16 +1778,17 @@ def delta_rule(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b_raw: torch.T
         from_len = delta_parallel_len(H, d, e)
         args = (_p(q), _p(k), _p(v), c_int(ld), _p(b_raw), c_int(b_raw.stride(0)), _p(a_raw), c_int(a_raw.stride(0)), _p(a_log),
                 _p(dt_bias), c_float(q_scale), c_float(unit_eps), _p(state), _p(out))
-        lists = (_p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), _p(ctx.live), c_int(ctx.R), c_int(H), c_int(G), c_int(d), c_int(e),
-                 c_int(state.shape[0]))
         with region("delta_rule_chunked", _nb(out) + T * (2 * G * d + H * e) * 4 + 2 * ctx.R * H * d * e * 4,
                     2.0 * T * H * (Q * d + Q * e + 3 * d * e)):
             if not _delta_in_parallel(args, ctx, q, k, v, state, out, from_len, H, G, d, e):
                 from_len = 0
-            if not from_len or bool(((ctx.h_q_len >= DELTA_MIN_TOKENS) & (ctx.h_q_len < from_len)).any()):
+            least = int(ctx.h_q_len.min())
+            if not from_len or (least < from_len and bool(((ctx.h_q_len >= DELTA_MIN_TOKENS) & (ctx.h_q_len < from_len)).any())):
+                lists = (_p(ctx.q_start), _p(ctx.q_len), _p(ctx.slots), _p(ctx.live), c_int(ctx.R), c_int(H), c_int(G), c_int(d),
+                         c_int(e), c_int(state.shape[0]))
                 check(library("delta_rule_chunked.cu").aie_delta_rule_chunked(
                     *args, *lists, c_int(DELTA_MIN_TOKENS), c_int(max(from_len - 1, 0)), _p(ctx.err), _stream()), "delta_rule_chunked")
-        if int(ctx.h_q_len.min()) >= DELTA_MIN_TOKENS:
+        if least >= DELTA_MIN_TOKENS:
             return out
         max_len = DELTA_MIN_TOKENS - 1              # the shorter portions and single tokens of the same step
     lib = library("delta_rule.cu")
@@ -1818,7 +1821,7 @@ def add_dyt(x: torch.Tensor, delta: Optional[torch.Tensor], weight: torch.Tensor
         if delta.shape[-2:] != x.shape:
             raise KernelError("add_dyt: delta differs in shape from x")
     n = x.shape[0] if rows is None else rows.shape[0]
-    out = torch.empty((n, D), dtype=out_dtype, device=x.device)
+    out = x.new_empty(n, D, dtype=out_dtype)
     stored = write_back and rows is None and delta is not None
     lib = library("elementwise.cu")
     with region("add_dyt", n * D * 4 * (2 if stored else 1) + (_nb(delta) if rows is None else 0) + _nb(out)):
@@ -1920,8 +1923,8 @@ def normed_attn_prepare(proj: torch.Tensor, bias: Optional[torch.Tensor], q_weig
             or (q_weight is not None and (k_weight is None or q_weight.numel() != nq or k_weight.numel() != nk))
             or (mix_from is not None and (mix_from.dtype != torch.float32 or mix_from.shape != (T, G * e) or mix_lambda is None))):
         raise KernelError("normed_attn_prepare: shapes or dtypes do not fit")
-    q = torch.empty((T, H, d), dtype=pages.dtype, device=proj.device)
-    kept = torch.empty((T, G * e), dtype=torch.float32, device=proj.device) if keep_values else None
+    q = proj.new_empty(T, H, d, dtype=pages.dtype)
+    kept = proj.new_empty(T, G * e, dtype=torch.float32) if keep_values else None
     lib = library("sink_attention.cu")
     with region("normed_attn_prepare", T * n * 4 + _nb(q, kept, mix_from) + T * G * w * pages.element_size()):
         check(lib.aie_normed_attn_prepare(_p(proj), c_int(ld), _p(bias), _p(q_weight), _p(k_weight), c_float(eps),
@@ -1942,7 +1945,7 @@ def slice_rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out_dtype: 
     T, n = x.shape
     if x.dtype != torch.float32 or x.stride(1) != 1 or weight.dtype != torch.float32 or weight.shape != (n,):
         raise KernelError("slice_rmsnorm: a float32 view and one float32 weight per column")
-    out = torch.empty((T, n), dtype=out_dtype, device=x.device)
+    out = x.new_empty(T, n, dtype=out_dtype)
     lib = library("sequence_ops.cu")
     with region("slice_rmsnorm", T * n * 4 + _nb(out)):
         check(lib.aie_slice_rmsnorm(_p(x), c_int(x.stride(0)), _p(weight), _p(out), c_int(dtype_code(out)), c_int(T), c_int(n),
@@ -1970,8 +1973,8 @@ def token_shift(x: torch.Tensor, shift: torch.Tensor, state: torch.Tensor, ctx, 
     T, D = x.shape
     if any(t.dtype != torch.float32 for t in (x, shift, state)) or shift.shape != (D,) or state.shape[1:] != (D,):
         raise KernelError("token_shift: a float32 stream [T, D], weights [D] and state [slots, D]")
-    out = torch.empty((T, D), dtype=out_dtype, device=x.device)
-    same = torch.empty((T, D), dtype=out_dtype, device=x.device) if plain and out_dtype != x.dtype else None
+    out = x.new_empty(T, D, dtype=out_dtype)
+    same = x.new_empty(T, D, dtype=out_dtype) if plain and out_dtype != x.dtype else None
     lib = library("gated_stream.cu")
     with region("token_shift", _nb(x, out, same)):
         check(lib.aie_token_shift(_p(x), _p(shift), _p(state), _p(out), _p(same), c_int(dtype_code(out)), _p(ctx.q_start),
@@ -2019,14 +2022,14 @@ def gated_norm_add(x: torch.Tensor, y, weight: torch.Tensor, eps: float, out_dty
         ldz = gate.stride(-2)
         nb += zparts * T * D * 4
     code = dtype_code(out_dtype or f32)
-    out = torch.empty((T, D), dtype=out_dtype, device=x.device) if out_dtype is not None and out_dtype != f32 else None
+    out = x.new_empty(T, D, dtype=out_dtype) if out_dtype is not None and out_dtype != f32 else None
     shift = state = shifted = None
     if next_shift is not None:
         shift, state = next_shift
         _dev(shift, state)
         if ctx is None or ctx.max_q_len != 1 or state.shape[1:] != (D,) or shift.shape != (D,) or out_dtype is None:
             raise KernelError("gated_norm_add: the next layer's shift is made in steps of lone tokens only")
-        shifted = torch.empty((T, D), dtype=out_dtype, device=x.device)
+        shifted = x.new_empty(T, D, dtype=out_dtype)
         nb += 2 * T * D * 4
     lib = library("gated_stream.cu")
     with region("gated_norm_add", 2 * _nb(x) + nb + _nb(out, shifted)):
@@ -2049,7 +2052,7 @@ def side_gate(z: torch.Tensor, ids: torch.Tensor, table: torch.Tensor, offset: i
         raise KernelError("side_gate: shapes or dtypes do not fit")
     T = z.shape[-2]
     parts, stride = (z.shape[0], z.stride(0)) if z.dim() == 3 else (1, 0)
-    out = torch.empty((T, n), dtype=out_dtype, device=z.device)
+    out = z.new_empty(T, n, dtype=out_dtype)
     lib = library("gated_stream.cu")
     with region("side_gate", parts * T * n * 4 + T * n * table.element_size() + _nb(out)):
         check(lib.aie_side_gate(_p(z), c_int(parts), c_longlong(stride), c_int(z.stride(-2)), _p(ids), _p(table),
@@ -2065,7 +2068,7 @@ def map_difference(a: torch.Tensor, lam: float, eps: float, factor: float, out_d
     T, H2, e = a.shape
     if a.dtype != torch.float32 or H2 % 2:
         raise KernelError("map_difference: float32 [T, 2 H, e]")
-    out = torch.empty((T, H2 // 2 * e), dtype=out_dtype, device=a.device)
+    out = a.new_empty(T, H2 // 2 * e, dtype=out_dtype)
     lib = library("gated_stream.cu")
     with region("map_difference", _nb(a, out)):
         check(lib.aie_map_difference(_p(a), c_float(lam), c_float(eps), c_float(factor), _p(out), c_int(dtype_code(out)),
@@ -2082,8 +2085,8 @@ def route_chosen(z: torch.Tensor, bias: Optional[torch.Tensor], E: int, top: int
         raise KernelError("route_chosen: float32 logits and bias")
     T = z.shape[-2]
     parts, stride = (z.shape[0], z.stride(0)) if z.dim() == 3 else (1, 0)
-    ids = torch.empty((T, top), dtype=torch.int32, device=z.device)
-    weights = torch.empty((T, top), dtype=torch.float32, device=z.device)
+    ids = z.new_empty(T, top, dtype=torch.int32)
+    weights = z.new_empty(T, top, dtype=torch.float32)
     lib = library("gated_stream.cu")
     with region("route_chosen", parts * T * E * 4 + _nb(ids, weights)):
         check(lib.aie_route_chosen(_p(z), c_int(parts), c_longlong(stride), c_int(z.stride(-2)), _p(bias), c_int(T), c_int(E),

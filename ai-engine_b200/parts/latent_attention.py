@@ -222,7 +222,7 @@ class LatentAttention(Mixer):
                                   ctx, cache.block_table, self.env.dtype, write=cache.writes and not self.shares_cache, kv=kv,
                                   halves=self.halves, magnitude=self.magnitude, folded=work.folds, whole=work.prompts,
                                   short_row=work.short_row if work.mixed else None, n_short=work.n_short)
-        a = torch.empty((T, self.H, self.dv), dtype=self.env.dtype, device=h.device)
+        a = h.new_empty(T, self.H, self.dv, dtype=self.env.dtype)
         if work.folds:
             q_plain, q_full = made[:2]
             ops.head_linear(q_plain, self.w_ukT, q_full)
