@@ -258,7 +258,7 @@ latent_attention_tc_kernel(const float* __restrict__ q_full, const bf16* __restr
 // 64 requests of 512 .. 4,096 keys, 16 heads, a latent of 512 (170 MB of rows, 26 us at the copy bandwidth): 47 us, 63 with the copies
 // in the warps that multiply; 162 us with a CTA a (request, quarter of its keys) that loaded and multiplied in turn, 109 us with one
 // CTA an SM and four chunks in flight, whose eight warps waited on one another.  Bound by the chain of a chunk's products, softmax and
-// products, 870 -> 250 instructions a warp.  Every wait is bounded (see tc_common.cuh).
+// products.  Every wait is bounded (see tc_common.cuh).
 #define LD_KEYS 32
 #define LD_THREADS 256
 #define LD_MIN_CHUNKS 2       // a stretch is at least this long: a CTA's start costs about as much as two chunks
