@@ -101,7 +101,7 @@ static int gemm_f32_go(const void* A, const void* W, void* C, int c_dtype, const
 }
 
 // ---------------------------------------------------------------------------
-// The same product for float32 operands whose rows start on 16 bytes: blocks of 64 x 16 TN outputs, a thread TM x 4 of them in
+// The same product for float32 operands whose rows start on 16 bytes: blocks of 64 x 64 or 64 x 128 outputs, a thread TM x 4 of them in
 // pairs of rows, so that one packed instruction (fma.rn.f32x2, each half rounded as fmaf) does two multiply-adds: registers
 // alone it reaches 62 TFLOP/s here, fmaf 51.  Each output is still one thread's sum over k in order: bits do not depend on
 // the tile.  The pairs want the rows next to one another, so tiles of 16 k go through registers into shared memory with k

@@ -595,6 +595,7 @@ extern "C" int aie_latent_decode(const float* q_full, const void* pages, void* o
     if (R <= 0) return 0;
     if (rank < 64 || rank > 512 || rank % 64 || dk % 16 || dk < rank || dk > 1024 || H <= 0) return AIE_UNSUPPORTED;
     if (G < 1 || G > 4096 || !part_o || !part_ml || P <= 0 || (long long)num_pages * P > 0x7fffffffLL) return AIE_BAD_ARG;
+    if (((size_t)q_full | (size_t)pages) & 15) return AIE_BAD_ARG;      // (rows are copied from 16 bytes on)
     const dim3 grid(G, (H + LT_ROWS - 1) / LT_ROWS);
     if (grid.y > 65535 || H > 65535) return AIE_UNSUPPORTED;
     const size_t smem = (size_t)(LT_ROWS + 2 * LD_KEYS) * (dk + 8) * 2 + 64 + (size_t)(pair ? 2 : 1) * LT_ROWS * (LD_KEYS + 8) * 2 +
