@@ -292,6 +292,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                                                    // may come here while that one is still to be issued
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_last + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* asked = reinterpret_cast<int*>(tmem_slot + 2);      // [2] key tiles, value tiles that were asked for (see tc_drain)
     float(*row_x)[AT_M] = reinterpret_cast<float(*)[AT_M]>(sm + 1024);      // (extended form) what a row's two threads tell one another
     constexpr int HV = HD / 64, HK = HQ / 64;      // halves of 64 columns of values, of queries and keys
     constexpr int KTILE = AtSmem<HD, HQ, EXT>::tile, TILE = AtSmem<HD, HQ, EXT>::v_tile;      // bytes of a 128-row tile of keys, of values
@@ -376,7 +377,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             if (in_rows) return lane == 0 ? row_page + pidx : -1;
             return (lane < ppt && (pidx << lp) <= p_last && pidx < bt_width && !gone(pidx)) ? bt[pidx] : -1;
         };
-        int page = page_of(0);
+        int page = page_of(0), n_k = 0, n_v = 0;
         bool ok = true;
         for (int j = 0; j < n_kt && ok; ++j) {
             const int st = j % NST;
@@ -402,6 +403,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                 if (!ok) break;
                 if (have) tma_load_4d(k_s + st * KTILE + lane * P * (HQ * 2), &map_k, &kv_full[st], 0, 0, blk_k, group0);
+                n_k = j + 1;
                 __syncwarp();
                 if (lane == 0) ok = mbar_wait(&v_empty[st], ph, abort_flag, err);
                 ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -423,6 +425,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 if (lane == 0) mbar_expect_tx(&v_full[st], bytes * HD);
                 __syncwarp();
                 if (have) tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &v_full[st], 0, 0, blk_v, group0);
+                n_v = j + 1;
             } else {
                 // one barrier counts the bytes of the tile's keys and values: the products wait once per tile
                 if (lane == 0) {
@@ -436,9 +439,14 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                     tma_load_4d(k_s + st * KTILE + lane * P * (HQ * 2), &map_k, &kv_full[st], 0, 0, blk_k, group0);
                     tma_load_4d(v_s + st * TILE + lane * P * (HD * 2), &map_v, &kv_full[st], 0, 0, blk_v, group0);
                 }
+                n_k = j + 1;
             }
             __syncwarp();
             page = page_next;
+        }
+        if (lane == 0) {
+            asked[0] = n_k;
+            asked[1] = n_v;
         }
         __syncwarp();
         // the last tile: zero the value rows of keys past the sequence's end (whole warp)
@@ -782,11 +790,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (*abort_flag && tid == 0) {      // give copies in flight a bounded time to land
-        for (int s = 0; s < NST; ++s) {
-            for (unsigned i = 0; i < (1u << 16) && !mbar_try_wait(&kv_full[s], 0) && !mbar_try_wait(&kv_full[s], 1); ++i) {}
-            for (unsigned i = 0; EXT && i < (1u << 16) && !mbar_try_wait(&v_full[s], 0) && !mbar_try_wait(&v_full[s], 1); ++i) {}
-        }
+    if (*abort_flag && tid == 0) {
+        tc_drain(q_full, 1, 1);
+        tc_drain(kv_full, NST, asked[0]);
+        if (EXT) tc_drain(v_full, NST, asked[1]);
     }
     __syncthreads();
     if (warp == 1) {
@@ -852,6 +859,7 @@ paged_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __
     unsigned long long* v_fixed = o_done + 2;
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(v_fixed + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* asked = reinterpret_cast<int*>(tmem_slot + 2);      // slots of the ring that were asked for (see tc_drain)
     constexpr int HV = HD / 64;
     constexpr int TILE = At2Smem<HD>::tile;
     constexpr int GROUP = HV * 1024;
@@ -918,7 +926,7 @@ paged_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __
         };
         int page = page_of(0);
         bool ok = true;
-        int slot = 0, ph = 0;           // ring position of the next item (K0 V0 K1 V1 ...)
+        int slot = 0, ph = 0, n_items = 0;           // ring position of the next item (K0 V0 K1 V1 ...), how many there were
         for (int j = 0; j < n_kt && ok; ++j) {
             const int page_next = j + 1 < n_kt ? page_of(j + 1) : -1;
             const int n_pages = min(ppt, ((p_last - j * AT_N) >> lp) + 1);
@@ -937,6 +945,7 @@ paged_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __
                 if (have)
                     tma_load_4d(kv_s + slot * TILE + lane * P * (HD * 2), item == 0 ? &map_k : &map_v, &full[slot], 0, 0, 0,
                                 group0);
+                ++n_items;
                 __syncwarp();
                 if (++slot == NS) {
                     slot = 0;
@@ -945,6 +954,7 @@ paged_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __
             }
             page = page_next;
         }
+        if (lane == 0) *asked = n_items;
         __syncwarp();
         // the last tile: zero the value rows of keys past the sequence's end (whole warp)
         {
@@ -1178,10 +1188,9 @@ paged_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __
 
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (*abort_flag && tid == 0) {      // give copies in flight a bounded time to land
-        for (int s = 0; s < NS; ++s) {
-            for (unsigned i = 0; i < (1u << 16) && !mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1); ++i) {}
-        }
+    if (*abort_flag && tid == 0) {
+        tc_drain(q_full, 1, 1);
+        tc_drain(full, NS, *asked);
     }
     __syncthreads();
     if (warp == 9) {

@@ -104,6 +104,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(acc_empty + 2);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     int* n_groups_s = reinterpret_cast<int*>(tmem_slot + 2);
+    int* asked_s = n_groups_s + 1;                         // stages of the ring that this block asked for (see tc_drain)
     int2* list = reinterpret_cast<int2*>(bars + 1024);     // (first tile * 4 + tiles - 1, expert)
     unsigned char* ring = bars + 1024 + GG_LIST_BYTES;
     int* tw = reinterpret_cast<int*>(ring);                // the tiles' experts and the items that begin there, until the list is made
@@ -182,7 +183,7 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     if (warp == 0) {
         if (tc_elect()) {
-            int s = 0;
+            int s = 0, asked = 0;
             unsigned ph = 1;
             bool ok = true;
             for (int item = first_item; item < items && ok; item += step) {
@@ -205,12 +206,14 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                     }
                     for (int i = 0; i < n; ++i)
                         gg_load<CTAS>(st + GG_W_BYTES + i * XB, &map_x, &full[s], kb * GG_BK, x0 + i * (GG_TILE / CTAS));
+                    ++asked;
                     if (++s == STAGES) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
             }
+            *asked_s = asked;
             // a pair's products free the stages in both blocks: all have been freed before either block leaves
             for (int i = 0; CTAS == 2 && i < STAGES && ok; ++i) {
                 ok = mbar_wait(&empty[s], ph, abort_flag, err);
@@ -302,10 +305,9 @@ gemm_grouped_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (*abort_flag && tid == 0) {      // give copies in flight a bounded time to land
-        for (int s = 0; s < STAGES; ++s)
-            for (unsigned i = 0; i < (1u << 16) && !mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1); ++i) {}
-    }
+    // a pair's copies all count on the first block's barriers, and both leave together: the second waits on one that nothing arrives
+    // at until it runs out, which gives copies that the first had not armed yet their time
+    if (*abort_flag && tid == 0) tc_drain(full, rank == 0 ? STAGES : 1, rank == 0 ? *asked_s : 1);
     __syncthreads();
     if (CTAS == 2) gg_cluster_sync();                      // nobody leaves while the other still reaches for its barriers
     if (warp == 1) {

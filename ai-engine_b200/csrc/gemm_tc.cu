@@ -164,6 +164,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     unsigned long long* accum = empty + 8;
     unsigned* tmem_slot = reinterpret_cast<unsigned*>(accum + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int* asked = reinterpret_cast<int*>(tmem_slot + 2);  // stages of the ring that were asked for (for the way out, see tc_drain)
     float* tile_s = reinterpret_cast<float*>(base);      // [BN][128] partial tile, after the ring is idle
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -216,7 +217,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 load_x(base + i * TcSmem<BN>::stage_bytes, &full[i], (kb_begin + i) * TC_BK);
             int s = 0;                  // (a stage and its phase are counted along: a division here stood between two requests)
             unsigned ph = 0;
-            for (int i = pre; i < nkb; ++i) {
+            int i = pre;
+            for (; i < nkb; ++i) {
                 if (!mbar_wait(&empty[s], ph, abort_flag, err)) break;
                 unsigned char* st = base + s * TcSmem<BN>::stage_bytes;
                 mbar_expect_tx(&full[s], bytes);
@@ -228,6 +230,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     ph ^= 1;
                 }
             }
+            *asked = i;
         }
     } else if (warp == 1) {
         if (tc_elect() && nkb > 0) {
@@ -375,10 +378,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // leave together; on an abort, give copies in flight a bounded time to land first
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
-    if (*abort_flag && tid == 0) {
-        for (int s = 0; s < STAGES; ++s)
-            for (unsigned i = 0; i < (1u << 16) && !mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1); ++i) {}
-    }
+    if (*abort_flag && tid == 0) tc_drain(full, STAGES, *asked);
     __syncthreads();
     if (warp == 1) {
         __syncwarp();

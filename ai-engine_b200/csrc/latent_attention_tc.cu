@@ -306,7 +306,7 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
     float* l_s = m_s + LT_ROWS;
     float* c_s = l_s + LT_ROWS;
     __shared__ unsigned long long full[NST], empty[NST];
-    __shared__ int abort_word;
+    __shared__ int abort_word, asked;                             // asked: chunks whose rows were asked for (see tc_drain)
     volatile int* abort_flag = &abort_word;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h0 = blockIdx.y * LT_ROWS;
     if (tid == 0) {
@@ -361,8 +361,8 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
             }
             return at;
         };
-        int at = places(0);
-        for (int i = 0; i < cnt; ++i) {
+        int at = places(0), i = 0;
+        for (; i < cnt; ++i) {
             unsigned long long* bar = &full[i % NST];
             bool ok = true;
             if (i >= NST) ok = mbar_wait(&empty[i % NST], (i / NST - 1) & 1, abort_flag, err);
@@ -379,6 +379,7 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
                              ::"r"(tc_smem(dst)), "l"(pages + (size_t)at * dk), "r"(dk * 2), "r"(tc_smem(bar)) : "memory");
             at = places(i + 1);
         }
+        if (lane == 0) asked = i;
     } else {
         const int steps = dk / 16, kg = warp & 3, kh = warp >> 2;
         const int step0 = kh ? (steps + 1) / 2 : 0, step1 = kh ? steps : (steps + 1) / 2;
@@ -523,10 +524,7 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
         }
     }
     __syncthreads();
-    if (*abort_flag && tid == 0) {      // give copies in flight a bounded time to land
-        for (int i = 0; i < NST; ++i)
-            for (unsigned k = 0; k < (1u << 16) && !mbar_try_wait(&full[i], 0) && !mbar_try_wait(&full[i], 1); ++k) {}
-    }
+    if (*abort_flag && tid == 0) tc_drain(full, NST, asked);
 }
 
 // One block a (request, head): the parts that the stretches of latent_decode_kernel left of it, in their order.

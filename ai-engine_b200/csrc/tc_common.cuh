@@ -5,7 +5,12 @@
 
 #include "common.cuh"
 
+#ifndef TC_WAIT_LIMIT              // polls before a wait gives up, and before a block that leaves early stops waiting for its copies
 #define TC_WAIT_LIMIT (1u << 24)
+#endif
+#ifndef TC_DRAIN_LIMIT
+#define TC_DRAIN_LIMIT (1u << 16)
+#endif
 
 __device__ __forceinline__ unsigned tc_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -41,6 +46,16 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
     *abort_flag = 1;
     atomicOr(err, AIE_DEV_WAIT_TIMEOUT);
     return false;
+}
+
+// For a block whose roles gave up: copies that are still in flight are given a bounded time to land before it leaves, because its
+// shared memory is another block's afterwards.  `asked` stages were armed, one after the other around the ring `full`: the last time
+// stage s was, it was for phase (asked - 1 - s) / stages.  The parity must be that phase's own (the one before always reads as over).
+__device__ __forceinline__ void tc_drain(unsigned long long* full, int stages, int asked) {
+    for (int s = 0; s < stages && s < asked; ++s) {
+        const unsigned parity = (unsigned)((asked - 1 - s) / stages) & 1u;
+        for (unsigned i = 0; i < TC_DRAIN_LIMIT && !mbar_try_wait(&full[s], parity); ++i) {}
+    }
 }
 
 // True in one lane of a converged warp.  Products are issued under this and not under `lane == 0`: the compiler knows that a
