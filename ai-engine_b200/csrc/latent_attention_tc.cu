@@ -372,6 +372,7 @@ latent_decode_kernel(const float* __restrict__ q_full, const bf16* __restrict__ 
                 for (int x = 0; x < dk; x += 8) *reinterpret_cast<uint4*>(dst + x) = make_uint4(0, 0, 0, 0);
             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");      // (a later copy may land on such a row)
             const int rows = __popc(__ballot_sync(0xffffffffu, at >= 0));
+            __syncwarp();                                         // lane 0's arrival publishes all lanes' zeros: a vote orders no memory
             if (lane == 0) mbar_expect_tx(bar, rows * dk * 2);
             __syncwarp();
             if (at >= 0)
