@@ -326,7 +326,10 @@ __global__ void __launch_bounds__(DP_THREADS, 2) dp_prepare_kernel(DpArgs p) {
 
 // From chunk to chunk.  Eight warps: U in tiles of 16 tokens x DV / 2 columns; the state in D / 16 tiles of 16 rows x DV columns,
 // float32 in its warp's accumulators, as pairs in shared memory for the next chunk.  The next chunk's W and keys are on
-// their way meanwhile.
+// their way meanwhile.  The wait for them is bounded (see tc_common.cuh): a block that gives up leaves the request's state as it was.
+#ifndef DP_STRAY          // bytes that a chunk's barrier waits for beyond those that come: for the test of a wait that runs out
+#define DP_STRAY 0
+#endif
 template <int D, int DV>
 __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
     extern __shared__ __align__(16) unsigned char dp_sm[];
@@ -356,7 +359,7 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
         const size_t at = (size_t)(first + c) * p.H + h;
         constexpr int PAIR = 2 * DP_T * D * 2, COLS = DP_T * DV * 4;
         unsigned long long* bar = &bars[c & 1];
-        mbar_expect_tx(bar, 2 * PAIR + COLS);
+        mbar_expect_tx(bar, 2 * PAIR + COLS + DP_STRAY);
         dp_bulk(stage + (c & 1) * ST, p.W + at * 2 * DP_T * D, PAIR, bar);
         dp_bulk(stage + (c & 1) * ST + 2 * DP_T * D, p.Kw + at * 2 * DP_T * D, PAIR, bar);
         dp_bulk(Us + (c & 1) * DP_T * DV, p.U + at * DP_T * p.e + (size_t)col0 * DP_T, COLS, bar);
@@ -406,8 +409,12 @@ __global__ void __launch_bounds__(DP_THREADS, 1) dp_walk_kernel(DpArgs p) {
                     *reinterpret_cast<unsigned*>(SL + (sr + 8 * y) * LD + x * 8 + sc) = lo;
                 }
         }
-        mbar_wait(&bars[c & 1], (c >> 1) & 1, &gave_up, p.err);
-        __syncthreads();                               // this chunk's operands and state are here; the last chunk is done with
+        const bool ok = mbar_wait(&bars[c & 1], (c >> 1) & 1, &gave_up, p.err);
+        if (__syncthreads_or(!ok)) {                   // this chunk's operands and state are here; the last chunk is done with
+            if (tid == 0) tc_drain(bars, 2, c + 1);
+            __syncthreads();
+            return;
+        }
         fetch(c + 1);
         store(p.S0 + at * D * p.e + col0, p.e, 16, SH, SL, D);
         const bf16* WH = stage + (c & 1) * ST;
