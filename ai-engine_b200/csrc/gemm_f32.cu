@@ -293,20 +293,28 @@ static int gemm_f32_pairs(const float* A, const float* W, OT* C, const int* a_ro
 // rows) and a tenth of a round let off.  At 2,048 of K a block an SM takes 50 us beside others in the narrow form and 86 in
 // the wide one, and 10 and 24 more the first time.  Measured at 66 sizes (1 .. 2,048 rows, six weights) the rule's choice is
 // the fastest of the three or within 4 % of it, 7 % at 257 rows of 2,048 columns.
-template <typename OT>
-static int gemm_f32_aligned(const float* A, const float* W, OT* C, const int* a_rows, const int* tile_w, int M, int N, int K,
-                            int lda, int ldc, int batch, long long a_bs, long long w_bs, long long c_bs, cudaStream_t st) {
+enum { GP_NARROW = 0, GP_AHEAD = 1, GP_WIDE = 2 };      // 64 columns a block, the same with lines asked for early, 128 columns
+static int gemm_f32_form(int M, int N, int batch, long long sms) {
     const int rest = M % GP_M;
     const auto rounds = [&](int columns, int last) {
         const long long tenths = (long long)batch * ((N + columns - 1) / columns) * (10 * (M / GP_M) + last);
-        return (tenths + 9 * 148 - 1) / (10 * 148) + ((tenths + 9 * 148 - 1) < 10 * 148);
+        return (tenths + 9 * sms - 1) / (10 * sms) + ((tenths + 9 * sms - 1) < 10 * sms);
     };
     const long long narrow = rounds(64, rest == 0 ? 0 : rest <= 32 ? 6 : 10);
     const long long wide = rounds(128, rest == 0 ? 0 : rest <= 16 ? 4 : rest <= 32 ? 6 : 10);
+    return 7 * wide + 2 < 4 * narrow + 1 ? GP_WIDE : narrow == 1 ? GP_AHEAD : GP_NARROW;
+}
+extern "C" int aie_gemm_f32_form(int M, int N, int batch, int sms) { return gemm_f32_form(M, N, batch, sms); }      // for tests
+
+template <typename OT>
+static int gemm_f32_aligned(const float* A, const float* W, OT* C, const int* a_rows, const int* tile_w, int M, int N, int K,
+                            int lda, int ldc, int batch, long long a_bs, long long w_bs, long long c_bs, cudaStream_t st) {
 #define GO(TM, AHEAD) return gemm_f32_pairs<TM, AHEAD, OT>(A, W, C, a_rows, tile_w, M, N, K, lda, ldc, batch, a_bs, w_bs, c_bs, st)
-    if (7 * wide + 2 < 4 * narrow + 1) GO(16, false);
-    if (narrow == 1) GO(8, true);
-    GO(8, false);
+    switch (gemm_f32_form(M, N, batch, aie_sm_count())) {
+        case GP_WIDE: GO(16, false);
+        case GP_AHEAD: GO(8, true);
+        default: GO(8, false);
+    }
 #undef GO
 }
 
