@@ -9,7 +9,8 @@
 //                      128-byte-swizzled atoms, the two halves of a group side by side), a ring of
 //                      three buffers for keys and one of three for values (four at head size 64: a
 //                      tile is requested when its buffer is freed, and a ring of two left the
-//                      products waiting for loads), one mbarrier per stage counting the bytes of both;
+//                      products waiting for loads), one mbarrier per stage counting the bytes of both
+//                      (the extended form: one for the keys, one for the values);
 //                      the loop has no division and
 //                      reads the next tile's page id while this tile's boxes are issued;
 //   warp 1 (one lane)  issues S = Q . K^T (8 x tcgen05.mma of K = 16) into one of two score buffers in
@@ -18,7 +19,8 @@
 //                      O += P . V (8 x tcgen05.mma; P is read from tensor memory, where the softmax
 //                      wrote it over the scores; V is the MN-major operand: its rows are keys), and
 //                      commits to the mbarriers the others wait on;
-//   warps 2-5          softmax, one thread per query row: the row of S in registers (tcgen05.ld), masked
+//   warps 2-5          softmax, one thread per query row (the extended form below: warps 2-9, two threads per
+//                      row): the row of S in registers (tcgen05.ld), masked
 //                      on tiles that touch the diagonal or the sequence's end, its maximum; then
 //                      the probabilities and their running sum (float32; the scale-and-subtract and
 //                      the sum as packed f32x2 instructions), written as bf16 pairs into tensor
@@ -284,8 +286,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     unsigned long long* k_empty = v_full + NST;    // [NST] the scores have read the keys
     unsigned long long* v_empty = k_empty + NST;   // [NST] P . V has read the values
     unsigned long long* s_full = v_empty + NST;    // [2] score buffers
-    unsigned long long* p_ready = s_full + 2;
-    unsigned long long* o_done = p_ready + 1;
+    unsigned long long* o_done = s_full + 2;
     unsigned long long* v_fixed = o_done + 1;
     unsigned long long* o_last = v_fixed + 1;      // the last P . V; o_done, which every tile's P . V completes, does not
                                                    // tell it from the one before the last: a softmax warp that is a tile ahead
@@ -514,10 +515,11 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                 }
                 if (EXT && lead && ok) ok = mbar_wait(&v_full[st], ph, abort_flag, err);
                 if (lead && ok && j == n_kt - 1) ok = mbar_wait(v_fixed, 0, abort_flag, err);
-                // the tile's probabilities are written: the 128 softmax threads arrive, this warp waits.  A hardware
-                // barrier: an mbarrier test costs the issuing thread some hundred cycles while the tensor pipe reads
-                // shared memory, and this hand-over is on the tile's critical path (P . V, then the scores of the tile
-                // after the next, which the softmax warps wait for).  (The tile's values landed with its keys.)
+                // the tile's probabilities are written: the softmax threads (128, in the extended form 256) arrive, this warp
+                // waits.  A hardware barrier: an mbarrier test costs the issuing thread some hundred cycles while the tensor pipe
+                // reads shared memory, and this hand-over is on the tile's critical path (P . V, then the scores of the tile
+                // after the next, which the softmax warps wait for).  (The tile's values landed with its keys; in the extended
+                // form they have a barrier of their own, waited for above.)
                 asm volatile("bar.sync %0, %1;\n" ::"r"(AT_BAR_P + (j & 1)), "r"((EXT ? 2 : 1) * AT_M + 32) : "memory");
                 st = st1;
                 ph = ph1;
@@ -543,7 +545,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
             }
         }
     } else {
-        // softmax: one thread per query row (warp w reads lanes 32 * (w % 4) .. + 31 of tensor memory)
+        // softmax: one thread per query row, in the extended form two (warp w reads lanes 32 * (w % 4) .. + 31 of tensor memory)
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         const int qpos = p0 + row;
