@@ -11,12 +11,13 @@
 // From a K of 1,024 on (and an even number of weight tiles) two blocks of a cluster share an item of 256 weight rows, with
 // cta_group::2: each loads its own 128 rows and half of X's (32 KB a stage and SM instead of 48, so six stages), the first one issues
 // the products of both, each block keeps the sums of its weight rows and has its own epilogue.  A short K is bound by the epilogue and
-// loses what the pair costs to join: 32 experts of 1,024 x 512 with 1,024 rows each 67 us as one block, 71 as two.
+// loses what the pair costs to join (see gg_go).
 // GLU: W [2 F, K] holds F gate rows, then F up rows.  A weight tile takes 64 of either in groups of 16, so that a warp's 32 lanes hold
 // a unit's gate and up sixteen lanes apart; act = min(gate, limit) * sigmoid(slope * it) * (up kept within +-limit + shift), as
 // clamped_glu makes it out of float32 sums, is stored in bfloat16.
-// Bound by L2 (12 TB/s over the chip): 32 experts of 2,048 x 2,048 with 1,024 rows each 301 us as two tiles a block, 262 as items of one
-// block, 245 as items of two; gate and up with the unit behind them 355, 235, 216.  An L2 policy that evicts the weights first: 72 -> 81.
+// Bound by L2 (12 TB/s over the chip).  32 experts of 2,048 x 2,048, us, a launch by itself on a cold L2: 214 rows each 101 as two tiles a
+// block, 85 as items of one block, 80 as items of two, 1,024 rows each 276, 231, 199; gate and up with the unit 120 (two kernels), 92, 89
+// and 347, 237, 237.  An L2 policy that evicts the weights first: 72 -> 81.
 // Every wait is bounded (see tc_common.cuh).
 #include "tc_common.cuh"
 
@@ -345,7 +346,11 @@ static int gg_launch(const CUtensorMap& mw, const CUtensorMap& mx, void* C, cons
 template <bool GLU, typename OT>
 static int gg_go(const void* X, const void* W, void* C, const int* tile_w, int n_tiles, int N, int K, int ldc, int E, unsigned* err,
                  const GgGlu& glu, cudaStream_t st) {
-    const int ctas = N / GG_BM % 2 || K < 1024 ? 1 : 2;      // (a short product is bound by its epilogue, see above)
+    // Where two blocks take over, us as one block / as two (32 experts, N = 2,048, a launch by itself on a cold L2), at K = 512, 640, 768,
+    // 896, 1,024, 1,536, 2,048: float32 results with 214 rows each 36/38 41/42 45/44 49/47 53/51 70/65 85/80, with 1,024 rows 99/96 109/101
+    // 120/108 131/115 142/124 186/158 231/199; the unit with 214 rows 41/44 44/46 47/49 51/53 55/57 75/74 92/89, with 1,024 rows 115/122
+    // 119/127 125/132 132/138 141/148 190/192 237/237.  Plain results gain from 768 on, the unit from some 1,500: one line between them.
+    const int ctas = N / GG_BM % 2 || K < 1024 ? 1 : 2;
     CUtensorMap mw, mx;
     int rc = tc_make_map_2d(&mw, W, (unsigned long long)E * N, K, (unsigned long long)K * 2, GLU ? 16 : GG_BM, GG_BK);
     if (rc) return rc;

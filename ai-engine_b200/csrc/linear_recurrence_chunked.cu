@@ -251,8 +251,9 @@ __device__ __forceinline__ void lc_diagonal(const float* qs, const float* ks, co
 }
 
 // s[4 a + b] = q_(i0 + a) . k_(j0 + b) over every SHARES-th piece of four channels: 8 loads of 16 bytes for 64 multiply-adds (a dot
-// product a thread, 2 or 4 of them with the same key, took 3 or 5 for 8 or 16: 2,048 tokens x 16 heads
-// 86.3 -> 85.0 us, a layer that brings them in two steps 258 -> 254).  at: the share, and which of the
+// product a thread, 2 or 4 of them with the same key, took 3 or 5 for 8 or 16: all three kernels at 300 /
+// 1,024 / 2,048 / 4,000 tokens x 16 heads 49.5 / 73.9 / 139.4 / 245.9 -> 48.2 / 71.8 / 137.3 / 243.3 us, the
+// middle halves of 40 runs each within 0.2; ragged prompts in two steps 257 -> 253).  at: the share, and which of the
 // piece's neighbours comes first: threads that read other rows side by side start on other banks.
 template <int D, int SHARES>
 __device__ __forceinline__ void lc_pairs(const float* qs, const float* ks, int i0, int j0, int at, float* s) {

@@ -1335,11 +1335,11 @@ GROUPED_MAX_TILES = 2048      # tiles that the kernel of csrc/gemm_grouped.cu li
 
 def grouped_takes_items(tiles: int, E: int, N: int) -> bool:
     """Whether a product of rows grouped by expert takes the kernel whose blocks walk items of up to four tiles: from 2.6 tiles an
-    expert on (its share of the empty ones too) and 1,024 columns.  us, one or two tiles a block against items, at 64 / 100 /
-    128 / 192 / 214 / 320 / 1,024 rows an expert: 32 experts of 2,048 x 2,048 54 / 63 / 67 / 79 / 89 / 118 / 293 against 55 / 58 / 59 / 64
-    / 78 / 105 / 233; of 2,048 x 1,024 33 / 38 / 40 / 48 / 55 / 71 / 176 and 35 / 35 / 37 / 39 / 46 / 61 / 139; 8 of 4,096 x 2,048 30 / 39 /
-    38 / 41 / 54 / 58 / 157 and 30 / 31 / 32 / 34 / 41 / 53 / 126; 128 of 512 x 1,024 34 / 40 / 43 / 53 / 59 / 73 and 37 / 42 / 46 / 52 / 61 /
-    77."""
+    expert on (its share of the empty ones too) and 1,024 columns.  us, float32 results, a launch by itself on a cold L2, one or two tiles
+    a block against items, at 64 / 100 / 128 / 192 / 214 / 320 / 1,024 rows an expert: 32 experts of 2,048 x 2,048 68 / 74 / 74 / 86 / 100
+    / 121 / 272 against 68 / 70 / 72 / 74 / 80 / 121 / 201; of 2,048 x 1,024 41 / 47 / 47 / 57 / 61 / 76 / 174 and 41 / 43 / 43 / 47 / 51 /
+    74 / 123; 8 of 4,096 x 2,048 37 / 47 / 47 / 51 / 66 / 70 / 141 and 41 / 41 / 41 / 43 / 45 / 69 / 100; 128 of 512 x 1,024 43 / 51 / 51 / 59
+    / 68 / 80 / 186 and 45 / 51 / 51 / 57 / 68 / 94 / 162."""
     return 5 * tiles >= 13 * E and N >= 1024 and tiles <= GROUPED_MAX_TILES
 
 
@@ -1383,9 +1383,9 @@ def grouped_linear(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, out_d
 def grouped_glu(x: torch.Tensor, w: torch.Tensor, tile_w: torch.Tensor, limit: float, alpha: float, shift: float,
                 out_dtype: torch.dtype, err: torch.Tensor, row_src: torch.Tensor, live: Optional[int] = None) -> torch.Tensor:
     """clamped_glu of grouped_linear's float32 result, w [E, 2 F, K] with the gate's rows first: [rows, F] in out_dtype.  In bfloat16
-    the unit is applied to the product's sums, the same bits: us, product and unit against one kernel, at 3 / 64 / 128 / 214 / 1,024 rows
-    an expert: 32 experts of 2,048 x 2,048 59 / 64 / 79 / 105 / 350 against 51 / 52 / 55 / 71 / 217, of 1,024 x 512 11 / 16 / 23 / 33 / 106
-    and 9 / 12 / 15 / 21 / 66; 128 of 512 x 1,024 40 / 45 / 59 / 79 and 32 / 36 / 44 / 56."""
+    the unit is applied to the product's sums, the same bits: us, a launch by itself on a cold L2, product and unit against one kernel, at
+    3 / 64 / 128 / 214 / 1,024 rows an expert: 32 experts of 2,048 x 2,048 75 / 75 / 85 / 120 / 347 against 70 / 70 / 76 / 92 / 237, of
+    1,024 x 512 24 / 24 / 32 / 42 / 112 and 18 / 18 / 23 / 31 / 70; 128 of 512 x 1,024 52 / 52 / 62 / 89 / 259 and 45 / 45 / 53 / 72 / 176."""
     E, N, K = w.shape
     if (x.dtype == w.dtype == out_dtype == torch.bfloat16 and N % 128 == 0 and K % 8 == 0
             and tile_w.shape[0] <= GROUPED_MAX_TILES):
